@@ -372,6 +372,39 @@ GemvArgs head_args(ribn_b200_executor* ex, int rows, const ActOperand& in) {
     return a;
 }
 
+// Norm, rotary, cache append and attention of layer l over the step's raw q / k / v, into ex->attn.  When every row adds
+// one token (fused_attention) it is one pass, which can also leave the result in `operand`.
+bool fused_attention(const ribn_b200_executor* ex, const StepPlan& plan) { return plan.n_rows == plan.n_tokens && ex->cfg.head_dim >= 64; }
+
+cudaError_t run_attention(ribn_b200_executor* ex, const StepPlan& plan, int l, bool programmatic, const ActOperand& operand, int& launches) {
+    const ribn_b200_config& c = ex->cfg;
+    cudaStream_t s = ex->stream;
+    const int T = plan.n_tokens;
+    Tensor* t = &ex->lt(l, 0);
+    __half* ck = ex->cache_k + (long long)l * ex->layer_stride;
+    __half* cv = ex->cache_v + (long long)l * ex->layer_stride;
+    if (fused_attention(ex, plan)) {
+        DecodeAttention d{};
+        d.q = ex->q; d.k = ex->k; d.v = ex->v;
+        d.q_norm = (const float*)t[kAttnQNorm].raw; d.k_norm = (const float*)t[kAttnKNorm].raw;
+        d.inv_freq = ex->inv_freq; d.eps = c.rms_eps;
+        d.cache_k = ck; d.cache_v = cv;
+        d.page_tables = ex->d_page_tables; d.pages_per_sequence = ex->pages_per_sequence;
+        d.token_seq = ex->meta.token_seq; d.token_pos = ex->meta.token_pos; d.token_slot = ex->meta.token_slot;
+        d.n_tokens = T; d.q_heads = c.q_heads; d.kv_heads = c.kv_heads; d.head_dim = c.head_dim;
+        d.window = 0; d.max_keys = plan.max_keys;
+        d.partial = ex->scratch.attn_partial; d.partial_bytes = ex->scratch.attn_partial_bytes;
+        d.out = ex->attn; d.operand = operand;
+        d.programmatic = programmatic;
+        return launch_attention_decode(s, d, &launches);
+    }
+    STEP_TRY(launch_qk_norm_rope_append(s, ex->q, ex->k, ex->v, (const float*)t[kAttnQNorm].raw, (const float*)t[kAttnKNorm].raw, ex->inv_freq,
+                                        ex->meta.token_pos, ex->meta.token_slot, T, c.q_heads, c.kv_heads, c.head_dim, c.rms_eps, ck, cv));
+    return launch_attention(s, ex->q, ck, cv, ex->d_page_tables, ex->pages_per_sequence, ex->meta.token_seq, ex->meta.token_pos, T, c.q_heads,
+                            c.kv_heads, c.head_dim, 0, plan.max_keys, ex->scratch.attn_partial, ex->scratch.attn_partial_bytes, ex->attn,
+                            &launches, plan.run_first, plan.run_count);
+}
+
 cudaError_t run_layers_decode(ribn_b200_executor* ex, const StepPlan& plan, int& launches) {
     const ribn_b200_config& c = ex->cfg;
     cudaStream_t s = ex->stream;
@@ -382,36 +415,11 @@ cudaError_t run_layers_decode(ribn_b200_executor* ex, const StepPlan& plan, int&
     STEP_TRY(launch_gemv_mma(s, qkv_args(ex, 0, T), pdl));
     for (int l = 0; l < c.layers; ++l) {
         Tensor* t = &ex->lt(l, 0);
-        __half* ck = ex->cache_k + (long long)l * ex->layer_stride;
-        __half* cv = ex->cache_v + (long long)l * ex->layer_stride;
-        if (plan.n_rows == T && c.head_dim >= 64) {
-            // every row adds one token: norm, rotary, cache append, attention and operand form in one pass
-            DecodeAttention d{};
-            d.q = ex->q; d.k = ex->k; d.v = ex->v;
-            d.q_norm = (const float*)t[kAttnQNorm].raw; d.k_norm = (const float*)t[kAttnKNorm].raw;
-            d.inv_freq = ex->inv_freq; d.eps = c.rms_eps;
-            d.cache_k = ck; d.cache_v = cv;
-            d.page_tables = ex->d_page_tables; d.pages_per_sequence = ex->pages_per_sequence;
-            d.token_seq = ex->meta.token_seq; d.token_pos = ex->meta.token_pos; d.token_slot = ex->meta.token_slot;
-            d.n_tokens = T; d.q_heads = c.q_heads; d.kv_heads = c.kv_heads; d.head_dim = c.head_dim;
-            d.window = 0; d.max_keys = plan.max_keys;
-            d.partial = ex->scratch.attn_partial; d.partial_bytes = ex->scratch.attn_partial_bytes;
-            d.out = ex->attn; d.operand = ex->op_attn;
-            d.programmatic = pdl;
-            cudaError_t e = launch_attention_decode(s, d, &launches);
+        {
+            cudaError_t e = run_attention(ex, plan, l, pdl, ex->op_attn, launches);
             if (e != cudaSuccess) return e;
-        } else {
-            STEP_TRY(launch_qk_norm_rope_append(s, ex->q, ex->k, ex->v, (const float*)t[kAttnQNorm].raw,
-                                                (const float*)t[kAttnKNorm].raw, ex->inv_freq, ex->meta.token_pos,
-                                                ex->meta.token_slot, T, c.q_heads, c.kv_heads, c.head_dim,
-                                                c.rms_eps, ck, cv));
-            cudaError_t e = launch_attention(s, ex->q, ck, cv, ex->d_page_tables, ex->pages_per_sequence,
-                                             ex->meta.token_seq, ex->meta.token_pos, T, c.q_heads, c.kv_heads,
-                                             c.head_dim, 0, plan.max_keys, ex->scratch.attn_partial,
-                                             ex->scratch.attn_partial_bytes, ex->attn, &launches, plan.run_first, plan.run_count);
-            if (e != cudaSuccess) return e;
-            STEP_TRY(launch_to_operand(s, ex->attn, nullptr, nullptr, T, c.q_heads * c.head_dim, ex->op_attn));
         }
+        if (!fused_attention(ex, plan)) STEP_TRY(launch_to_operand(s, ex->attn, nullptr, nullptr, T, c.q_heads * c.head_dim, ex->op_attn));
         STEP_TRY(launch_gemv_mma(s, o_args(ex, l, T), pdl));
         if (ex->tp > 1) {
             cudaError_t e = tp_reduce_add(ex, T, launches);
@@ -441,7 +449,119 @@ cudaError_t run_layers_decode(ribn_b200_executor* ex, const StepPlan& plan, int&
     return cudaSuccess;
 }
 
-// ---- batch family: integer tensor-core GEMM over batch-operand activations (3+ tokens) --------
+// ---- a few rows (3 .. kFragStepRows): the fragment-order GEMM, its sums finished by the kernel that makes the next
+// projection's operand --------------------------------------------------------------------------------------------
+// The line: one launch's tensor-core time grows by a 32-row group at a time; from 33 rows on the tcgen05 kernels, whose
+// time hardly depends on the row count up to 64, are ahead.
+constexpr int kFragStepRows = 32;
+
+GemvSegment frag_segment(const Tensor& t, float* y) {
+    GemvSegment s = segment_of(t, y);
+    s.map = t.map;
+    return s;
+}
+FragGemm frag_base(ribn_b200_executor* ex, int k, int members, bool normed) {
+    FragGemm a{};
+    a.k = k;
+    a.members = members;
+    a.blocks = ex->op_frag.blocks;
+    a.ss = normed ? ex->op_frag.ss : nullptr;
+    a.eps = ex->cfg.rms_eps;
+    a.epilogue = kStore;
+    a.partial = ex->tc_partial;
+    a.error_flag = ex->d_error;
+    return a;
+}
+FragGemm frag_qkv(ribn_b200_executor* ex, int l, int m) {
+    Tensor* t = &ex->lt(l, 0);
+    FragGemm a = frag_base(ex, ex->cfg.hidden, m, true);
+    a.n_segments = 3;
+    a.seg[0] = frag_segment(t[kAttnQ], ex->q);
+    a.seg[1] = frag_segment(t[kAttnK], ex->k);
+    a.seg[2] = frag_segment(t[kAttnV], ex->v);
+    return a;
+}
+FragGemm frag_o(ribn_b200_executor* ex, int l, int m) {
+    FragGemm a = frag_base(ex, ex->cfg.q_heads * ex->cfg.head_dim, m, false);
+    a.n_segments = 1;
+    a.seg[0] = frag_segment(ex->lt(l, kAttnOutput), ex->hidden);
+    return a;
+}
+FragGemm frag_gate_up(ribn_b200_executor* ex, int l, int m) {
+    FragGemm a = frag_base(ex, ex->cfg.hidden, m, true);
+    a.n_segments = 2;
+    a.seg[0] = frag_segment(ex->lt(l, kFfnGate), ex->gate);
+    a.seg[1] = frag_segment(ex->lt(l, kFfnUp), ex->up);
+    return a;
+}
+FragGemm frag_down(ribn_b200_executor* ex, int l, int m) {
+    FragGemm a = frag_base(ex, ex->cfg.ffn, m, false);
+    a.n_segments = 1;
+    a.seg[0] = frag_segment(ex->lt(l, kFfnDown), ex->hidden);
+    return a;
+}
+
+cudaError_t run_layers_frag(ribn_b200_executor* ex, const StepPlan& plan, int& launches) {
+    const ribn_b200_config& c = ex->cfg;
+    cudaStream_t s = ex->stream;
+    const int T = plan.n_tokens, QD = c.q_heads * c.head_dim;
+    const bool pdl = !(c.flags & RIBN_B200_FLAG_NO_GRAPH);
+    FragOperand plain = ex->op_frag;   // an operand no norm follows
+    plain.ss = nullptr;
+    auto rows = [&](const float* x, const int32_t* index, const float* norm, int members, int k) -> cudaError_t {
+        FragFinish f{};
+        f.x = x; f.index = index; f.norm_weight = norm; f.members = members;
+        f.out = norm != nullptr ? ex->op_frag : plain;
+        return launch_frag_finish(s, kFragRows, nullptr, f, k, pdl);
+    };
+    STEP_TRY(rows(ex->hidden, nullptr, (const float*)ex->lt(0, kAttnNorm).raw, T, c.hidden));
+    for (int l = 0; l < c.layers; ++l) {
+        Tensor* t = &ex->lt(l, 0);
+        {
+            const FragGemm g = frag_qkv(ex, l, T);
+            STEP_TRY(launch_gemm_frag(s, g, pdl));
+            STEP_TRY(launch_frag_finish(s, kFragStore, &g, FragFinish{}, 0, pdl));
+        }
+        {
+            cudaError_t e = run_attention(ex, plan, l, pdl, ActOperand{}, launches);
+            if (e != cudaSuccess) return e;
+        }
+        STEP_TRY(rows(ex->attn, nullptr, nullptr, T, QD));
+        FragFinish f{};
+        {
+            const FragGemm g = frag_o(ex, l, T);
+            STEP_TRY(launch_gemm_frag(s, g, pdl));
+            f.norm_weight = (const float*)t[kFfnNorm].raw;
+            f.out = ex->op_frag;
+            STEP_TRY(launch_frag_finish(s, kFragResidual, &g, f, c.hidden, pdl));
+        }
+        {
+            const FragGemm g = frag_gate_up(ex, l, T);
+            STEP_TRY(launch_gemm_frag(s, g, pdl));
+            f.norm_weight = nullptr;
+            f.out = plain;
+            STEP_TRY(launch_frag_finish(s, kFragSwiGLU, &g, f, c.ffn, pdl));
+        }
+        {
+            const FragGemm g = frag_down(ex, l, T);
+            STEP_TRY(launch_gemm_frag(s, g, pdl));
+            f.norm_weight = l + 1 < c.layers ? (const float*)ex->lt(l + 1, kAttnNorm).raw : (const float*)ex->output_norm.raw;
+            f.out = ex->op_frag;
+            STEP_TRY(launch_frag_finish(s, kFragResidual, &g, f, c.hidden, pdl));
+        }
+    }
+    if (plan.n_sample > 0) {
+        if (plan.n_sample != T) STEP_TRY(rows(ex->hidden, ex->meta.sample_token, (const float*)ex->output_norm.raw, plan.n_sample, c.hidden));
+        FragGemm g = frag_base(ex, c.hidden, plan.n_sample, true);
+        g.n_segments = 1;
+        g.seg[0] = frag_segment(ex->output, ex->logits);
+        g.partial = nullptr;
+        STEP_TRY(launch_gemm_frag(s, g, pdl));
+    }
+    return cudaSuccess;
+}
+
+// ---- batch family: tensor-core GEMMs over batch-operand activations (more rows) --------
 // Tokens go through each projection in groups of up to kGemmMaxMembers; weights are read once per group.
 cudaError_t batch_project(ribn_b200_executor* ex, int& launches, const float* x, const int32_t* index,
                           const float* norm_weight, int tokens, int k, const Tensor* const* mats, float* const* ys,
@@ -451,6 +571,26 @@ cudaError_t batch_project(ribn_b200_executor* ex, int& launches, const float* x,
     GemvSegment probe[3];
     for (int i = 0; i < n_mats; ++i) probe[i] = GemvSegment{nullptr, mats[i]->type, 0, 0, nullptr};
     const bool kquant = tensor_memory && gemm_tc_kquant(probe, n_mats, 1);
+    if (tensor_memory && !kquant) {
+        // matrices with a Q8_0 member: the fragment-order kernel takes every row of the step in one launch
+        FragFinish f{};
+        f.x = x; f.index = index; f.norm_weight = norm_weight; f.members = tokens; f.out = ex->op_frag;
+        if (norm_weight == nullptr) f.out.ss = nullptr;
+        STEP_TRY(launch_frag_finish(s, kFragRows, nullptr, f, k, false));
+        FragGemm a{};
+        a.n_segments = n_mats;
+        for (int i = 0; i < n_mats; ++i) a.seg[i] = frag_segment(*mats[i], ys[i]);
+        a.k = k;
+        a.members = tokens;
+        a.blocks = ex->op_frag.blocks;
+        a.ss = f.out.ss;
+        a.eps = ex->cfg.rms_eps;
+        a.epilogue = epilogue == kSwiGLU ? kStore : epilogue;
+        a.error_flag = ex->d_error;
+        STEP_TRY(launch_gemm_frag(s, a, false));
+        if (epilogue == kSwiGLU) STEP_TRY(launch_silu_mul(s, ys[0], ys[1], (long long)tokens * mats[0]->rows, ys[0]));
+        return cudaSuccess;
+    }
     const int group = !tensor_memory ? kGemmMaxMembers : kquant ? 64 : kGemmTcMaxMembers;
     // K-quant form: one conversion of every row of the step, laid out as one operand per group
     const bool converted = kquant && tokens > group;
@@ -531,32 +671,8 @@ cudaError_t run_layers_batch(ribn_b200_executor* ex, const StepPlan& plan, int& 
                                           mats, ys, 3, kStore);
             if (e != cudaSuccess) return e;
         }
-        __half* ck = ex->cache_k + (long long)l * ex->layer_stride;
-        __half* cv = ex->cache_v + (long long)l * ex->layer_stride;
-        if (plan.n_rows == T && c.head_dim >= 64) {
-            DecodeAttention d{};
-            d.q = ex->q; d.k = ex->k; d.v = ex->v;
-            d.q_norm = (const float*)t[kAttnQNorm].raw; d.k_norm = (const float*)t[kAttnKNorm].raw;
-            d.inv_freq = ex->inv_freq; d.eps = c.rms_eps;
-            d.cache_k = ck; d.cache_v = cv;
-            d.page_tables = ex->d_page_tables; d.pages_per_sequence = ex->pages_per_sequence;
-            d.token_seq = ex->meta.token_seq; d.token_pos = ex->meta.token_pos; d.token_slot = ex->meta.token_slot;
-            d.n_tokens = T; d.q_heads = c.q_heads; d.kv_heads = c.kv_heads; d.head_dim = c.head_dim;
-            d.window = 0; d.max_keys = plan.max_keys;
-            d.partial = ex->scratch.attn_partial; d.partial_bytes = ex->scratch.attn_partial_bytes;
-            d.out = ex->attn;
-            d.programmatic = false;
-            cudaError_t e = launch_attention_decode(s, d, &launches);
-            if (e != cudaSuccess) return e;
-        } else {
-            STEP_TRY(launch_qk_norm_rope_append(s, ex->q, ex->k, ex->v, (const float*)t[kAttnQNorm].raw,
-                                                (const float*)t[kAttnKNorm].raw, ex->inv_freq, ex->meta.token_pos,
-                                                ex->meta.token_slot, T, c.q_heads, c.kv_heads, c.head_dim,
-                                                c.rms_eps, ck, cv));
-            cudaError_t e = launch_attention(s, ex->q, ck, cv, ex->d_page_tables, ex->pages_per_sequence,
-                                             ex->meta.token_seq, ex->meta.token_pos, T, c.q_heads, c.kv_heads,
-                                             c.head_dim, 0, plan.max_keys, ex->scratch.attn_partial,
-                                             ex->scratch.attn_partial_bytes, ex->attn, &launches, plan.run_first, plan.run_count);
+        {
+            cudaError_t e = run_attention(ex, plan, l, false, ActOperand{}, launches);
             if (e != cudaSuccess) return e;
         }
         {
@@ -605,6 +721,10 @@ bool decode_family_applies(const ribn_b200_executor* ex, const StepPlan& plan) {
     return plan.n_tokens <= kGemvMaxMembers && packed_family_applies(ex);
 }
 
+bool frag_family_applies(const ribn_b200_executor* ex, const StepPlan& plan) {
+    return plan.n_tokens <= kFragStepRows && ex->tp == 1 && !(ex->cfg.flags & RIBN_B200_FLAG_NO_TCGEN05) && packed_family_applies(ex);
+}
+
 cudaError_t run_step(ribn_b200_executor* ex, const StepPlan& plan, int& launches) {
     const ribn_b200_config& c = ex->cfg;
     cudaStream_t s = ex->stream;
@@ -615,6 +735,7 @@ cudaError_t run_step(ribn_b200_executor* ex, const StepPlan& plan, int& launches
     STEP_TRY(launch_embedding(s, ex->token_embd.type, ex->token_embd.raw, c.hidden, c.vocab, ex->meta.token_id, T,
                               ex->hidden));
     cudaError_t e = decode_family_applies(ex, plan) ? run_layers_decode(ex, plan, launches)
+                    : frag_family_applies(ex, plan)   ? run_layers_frag(ex, plan, launches)
                     : packed_family_applies(ex)     ? run_layers_batch(ex, plan, launches)
                                                     : run_layers_reference(ex, plan, launches);
     if (e != cudaSuccess) return e;
@@ -894,7 +1015,10 @@ int ribn_b200_finalize(ribn_b200_executor* ex) {
         mats.push_back(&ex->output);
         size_t largest = 0;
         for (Tensor* t : mats) if (packable(t->type, t->rows, t->cols)) largest = std::max(largest, t->bytes);
-        std::vector<unsigned char> raw(largest), packed;
+        std::vector<unsigned char> raw(largest), packed, maps(mats.size() * kTileMapBytes);
+        unsigned char* d_maps = nullptr;
+        CU_TRY(ex, dev_alloc(ex, &d_maps, maps.size()));
+        size_t map_index = 0;
         const int threads = (int)std::max(1u, std::min(32u, std::thread::hardware_concurrency()));
         for (Tensor* t : mats) {
             if (!packable(t->type, t->rows, t->cols)) continue;
@@ -908,6 +1032,8 @@ int ribn_b200_finalize(ribn_b200_executor* ex) {
             repack_host(t->type, raw.data(), t->rows, t->cols, packed.data(), threads);
             CU_TRY(ex, dev_alloc(ex, &p.data, p.bytes));
             CU_TRY(ex, cudaMemcpy(p.data, packed.data(), p.bytes, cudaMemcpyHostToDevice));
+            CU_TRY(ex, make_tile_map(t->type, p.data, t->rows, t->cols, maps.data() + map_index * kTileMapBytes));
+            t->map = d_maps + map_index++ * kTileMapBytes;
             // the tensor-memory GEMM's operands, converted once instead of on every use
             if ((c.flags & RIBN_B200_FLAG_OPERAND_CACHE) && !(c.flags & RIBN_B200_FLAG_NO_TCGEN05) &&
                 (t->type == kQ4_K || t->type == kQ6_K)) {
@@ -916,6 +1042,7 @@ int ribn_b200_finalize(ribn_b200_executor* ex) {
                 CU_TRY(ex, launch_tc_cache(ex->stream, t->type, p.data, t->rows, t->cols, t->op_a, t->op_meta));
             }
         }
+        CU_TRY(ex, cudaMemcpy(d_maps, maps.data(), maps.size(), cudaMemcpyHostToDevice));
         CU_TRY(ex, cudaStreamSynchronize(ex->stream));
     }
 
@@ -1010,8 +1137,17 @@ int ribn_b200_finalize(ribn_b200_executor* ex) {
                 CU_TRY(ex, dev_alloc(ex, (unsigned char**)&ex->op_tc.chunks,
                                      std::max(tc_operand_bytes(kGemmTcMaxMembers, kmax), tc_groups * tc_operand_bytes(64, kmax))));
                 CU_TRY(ex, dev_alloc(ex, &ex->op_tc.scale_in, tc_rows));
-                // room for four K slices of the widest fused projection at 64 rows
+                CU_TRY(ex, dev_alloc(ex, &ex->op_frag.blocks, std::max(frag_operand_bytes((int)T, kmax), frag_operand_bytes((int)S, c.hidden))));
+                CU_TRY(ex, dev_alloc(ex, &ex->op_frag.ss, std::max(T, S) * (size_t)(kmax / kTileCols)));
+                // room for four K slices of the widest fused projection at 64 rows, and for a split fragment-order launch
                 ex->tc_partial_floats = (size_t)4 * 64 * (size_t)std::max(std::max(2 * c.ffn, c.hidden), (c.q_heads + 2 * c.kv_heads) * c.head_dim);
+                if (packed_family_applies(ex)) {
+                    for (int m = 1; m <= std::min((int)T, kFragStepRows); ++m) {
+                        for (const FragGemm& g : {frag_qkv(ex, 0, m), frag_o(ex, 0, m), frag_gate_up(ex, 0, m), frag_down(ex, 0, m)}) {
+                            ex->tc_partial_floats = std::max(ex->tc_partial_floats, frag_partial_floats(g));
+                        }
+                    }
+                }
                 CU_TRY(ex, dev_alloc(ex, &ex->tc_partial, ex->tc_partial_floats));
                 CU_TRY(ex, dev_alloc(ex, &ex->op_tc.member_scale, tc_rows));
                 CU_TRY(ex, dev_alloc(ex, &ex->op_batch.member_scale, kGemmMaxMembers));

@@ -24,6 +24,7 @@ struct Tensor {
     PackedMatrix packed;           // tile-major repack for the fast kernels (matrices only)
     unsigned char* op_a = nullptr;     // K-quant matrices under RIBN_B200_FLAG_OPERAND_CACHE: tensor-core operand
     unsigned char* op_meta = nullptr;  // pieces and their per-k-tile records (launch_tc_cache)
+    unsigned char* map = nullptr;      // device copy of the packed matrix's tensor map (make_tile_map)
     bool loaded() const { return raw != nullptr; }
 };
 
@@ -120,7 +121,8 @@ struct ribn_b200_executor {
     ribn::ActOperand op_hidden, op_attn, op_act, op_head;
     ribn::BatchOperand op_batch;  // batch form, refilled before every batched projection
     ribn::TcOperand op_tc;        // tensor-memory form (the same, for the tcgen05 kernel)
-    float* tc_partial = nullptr;  // split-K sums of the tcgen05 kernel
+    ribn::FragOperand op_frag;    // fragment-order form (batches of a few rows; any batch of a Q8_0 model)
+    float* tc_partial = nullptr;  // split-K sums of the batched kernels
     size_t tc_partial_floats = 0;
     // Captured decode steps, keyed by (tokens, sampling rows, attention span bucket).
     struct StepGraph { cudaGraphExec_t exec = nullptr; int launches = 0; };

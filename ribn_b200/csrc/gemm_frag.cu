@@ -1,0 +1,896 @@
+// Dequant-GEMM in MMA-fragment order for batches of 3 and more rows, any packed block type.
+//
+//   y[m][n] = sum_k deq(W[n][k]) x[m][k]
+//
+// The packed tiles already hold, per lane, the bytes of its MMA A fragments, so a weight never passes through
+// shared memory a second time: a lane masks its bytes straight into binary16 SUBNORMALS (the bit pattern of a
+// small integer q is the number q 2^-24, which the tensor core multiplies exactly), one LOP3 per two weights, and
+// `mma.sync.m16n8k16` adds them against the activations' binary16 hi + lo pairs.  One group of inputs that shares a
+// block scale (32 inputs of Q4_K and Q8_0, 16 of Q6_K) is one chain of MMAs; its F32 sum is folded into the tile's
+// sum with the group's exact F32 scale, and the tile's (256 inputs) into the row's sum with the activations' power-
+// of-two scale, both round-to-nearest.  Offsets (Q4_K minima, Q6_K -32, Q8_0 -128) are one more MMA per tile against
+// the activations' group sums.
+//
+// Why not a tcgen05 pipeline that converts its A operand through shared memory: at these row counts its hand-offs
+// (packed ring -> registers -> shared memory -> MMA -> commit -> tensor memory -> registers) cost several
+// microseconds per 128 x 256 tile, whatever the row count.  Here a warp has no hand-off between the copy of a tile
+// and its sums.
+//
+// Execution: one persistent CTA per SM; a producer thread streams ring slots (the eight row tiles of a 128-row unit
+// at one k tile, one tensor copy, and the activations' block of that k tile), weights before the programmatic
+// dependency on the previous kernel resolves.  Two teams of four warps work on their own slots, a warp on two row
+// tiles (so that an activation fragment read from shared memory serves two).  The launch's slots are dealt out to
+// the teams in whole units when a unit's result is stored by this kernel, else evenly: a unit's partial sums are then
+// added in worker order by the kernel that consumes them.  Sums are ordered; a row's result does not depend on what it
+// is batched with.  Every wait is bounded and raises the caller's error word.
+#include <cuda.h>
+#include <cuda_fp16.h>
+#include <string.h>
+
+
+#include <algorithm>
+#include <type_traits>
+
+#include "blocks.cuh"
+#include "gemv.cuh"
+
+namespace ribn {
+
+namespace {
+
+constexpr int kUnitTiles = 8;                    // row tiles per unit: 128 output rows
+constexpr int kTeams = 2;
+constexpr int kTeamWarps = 4;                    // warps per team, two row tiles each
+constexpr int kWarps = kTeams * kTeamWarps;
+constexpr int kThreads = (kTeams + 1) * kTeamWarps * 32;
+constexpr int kSum16At = 16 * 512, kSum32At = kSum16At + 512, kScaleAt = kSum32At + 256;
+static_assert(kScaleAt + 32 == kFragBlockBytes, "operand block layout");
+constexpr uint32_t kSpinLimit = 1u << 22;
+constexpr size_t kSmemBudget = 220 * 1024;
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
+}
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* error_flag, int code, uint32_t limit) {
+    for (uint32_t i = 0; i < limit; ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        if (ok) return true;
+    }
+    if (error_flag != nullptr) atomicExch(error_flag, code);
+    return false;
+}
+__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+// The box of a packed matrix's tensor map at (k tile, first row tile): eight tiles, kUnitTiles x tile bytes.
+__device__ __forceinline__ void tiles_g2s(uint32_t dst, const void* map, int k_tile, int row_tile, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %2, %3, %4}], [%5];" ::"r"(dst),
+                 "l"(map), "r"(0), "r"(k_tile), "r"(row_tile), "r"(bar) : "memory");
+}
+__device__ __forceinline__ uint4 lds128(uint32_t addr) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ uint2 lds64(uint32_t addr) {
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ float2 lds64f(uint32_t addr) {
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ uint32_t lds16(uint32_t addr) {
+    uint32_t v;
+    asm volatile("{\n\t.reg .u16 t;\n\tld.shared.u16 t, [%1];\n\tcvt.u32.u16 %0, t;\n\t}" : "=r"(v) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ void sts128(uint32_t addr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+__device__ __forceinline__ void sts128f(uint32_t addr, float2 a, float2 b) {
+    asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y) : "memory");
+}
+__device__ __forceinline__ void sts32f(uint32_t addr, float a) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(a) : "memory"); }
+// D = A B (fresh accumulator) and D += A B
+__device__ __forceinline__ void mma_first(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.0f));
+}
+__device__ __forceinline__ void mma_next(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// (a & mask) | other in one LOP3
+__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t mask, uint32_t other) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(a), "r"(mask), "r"(other));
+    return r;
+}
+// bytes i and i + 1 of w as floats minus `bias` (exact), times f
+__device__ __forceinline__ float2 bytes_scaled(uint32_t w, int i, float bias, float2 f) {
+    const float2 raw = make_float2(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540u | (uint32_t)i)),
+                                   __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540u | (uint32_t)(i + 1))));
+    return __fmul2_rn(__fadd2_rn(raw, make_float2(-bias, -bias)), f);
+}
+__device__ __forceinline__ float half_low(uint32_t w) { return __half2float(__ushort_as_half((unsigned short)(w & 0xffffu))); }
+__device__ __forceinline__ float half_high(uint32_t w) { return __half2float(__ushort_as_half((unsigned short)(w >> 16))); }
+
+constexpr float kTwo24 = 16777216.0f, kTwo20 = 1048576.0f;   // an integer masked into binary16 is that integer times 2^-24
+
+// c: (row g, columns 2t, 2t + 1), (row g + 8, the same); s0 / s1: factors of rows g / g + 8
+__device__ __forceinline__ void fold(float (&acc)[4], const float (&c)[4], float s0, float s1) {
+    const float2 lo = __ffma2_rn(make_float2(s0, s0), make_float2(c[0], c[1]), make_float2(acc[0], acc[1]));
+    const float2 hi = __ffma2_rn(make_float2(s1, s1), make_float2(c[2], c[3]), make_float2(acc[2], acc[3]));
+    acc[0] = lo.x; acc[1] = lo.y; acc[2] = hi.x; acc[3] = hi.y;
+}
+
+// A fragments of one k16 step: registers 0 / 2 are row g's input pairs (4t, 4t + 2) and (4t + 1, 4t + 3), 1 / 3 row g + 8's.
+struct Frag { uint32_t r[4]; };
+
+// One scale group of both row tiles against every column group: lo parts first (the accumulator is still small), then
+// hi parts; the 2 NG chains advance side by side.
+template <int NG, int STEPS>
+__device__ __forceinline__ void group_mma(float (&d)[2][NG][4], const Frag (&a)[2][STEPS], const uint4 (&b)[STEPS][NG]) {
+#pragma unroll
+    for (int s = 0; s < STEPS; ++s) {
+#pragma unroll
+        for (int n = 0; n < NG; ++n) {
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                if (s == 0) mma_first(d[r][n], a[r][s].r[0], a[r][s].r[1], a[r][s].r[2], a[r][s].r[3], b[s][n].z, b[s][n].w);
+                else mma_next(d[r][n], a[r][s].r[0], a[r][s].r[1], a[r][s].r[2], a[r][s].r[3], b[s][n].z, b[s][n].w);
+            }
+        }
+    }
+#pragma unroll
+    for (int s = 0; s < STEPS; ++s) {
+#pragma unroll
+        for (int n = 0; n < NG; ++n) {
+#pragma unroll
+            for (int r = 0; r < 2; ++r) mma_next(d[r][n], a[r][s].r[0], a[r][s].r[1], a[r][s].r[2], a[r][s].r[3], b[s][n].x, b[s][n].y);
+        }
+    }
+}
+
+template <int NG>
+using TileSums = float[2][NG][4];
+
+// A warp's row records: its 32 rows' scales as F32 and its offsets' A operand, written by lane = row (decoding a row's
+// header once instead of in each of the four lanes that need it) and read back in fragment order.
+//   words 0..7 scales, 8..11 offset operand (binary16 pairs), 12 offset factor; a pitch of 20 words is conflict-free
+constexpr int kRecWords = 20;
+struct Record {
+    uint32_t wr, rd;   // this lane's row / row g of the warp's first row tile
+};
+__device__ __forceinline__ float2 rec_scales(const Record& rec, int r, int h, int pair) {   // scales 2 pair, 2 pair + 1
+    return lds64f(rec.rd + (uint32_t)((r * 16 + h * 8) * kRecWords + 2 * pair) * 4u);
+}
+__device__ __forceinline__ uint32_t rec_word(const Record& rec, int r, int h, int word) {
+    return lds32(rec.rd + (uint32_t)((r * 16 + h * 8) * kRecWords + word) * 4u);
+}
+
+// ---- Q4_K: w = d sc q - dmin m, groups of 32 --------------------------------------------------------------------
+template <int NG>
+__device__ __forceinline__ void slot_q4k(uint32_t tile, uint32_t b_at, const Record& rec, int lane, TileSums<NG>& sums) {
+    constexpr int kUnroll = NG <= 2 ? 2 : 1;
+    const int t = lane & 3;
+    {
+        const uint4 hd = lds128(tile + (lane >> 4) * 2304 + 2048 + (lane & 15) * 16);
+        const float d = half_low(hd.x);
+        const uint32_t s_lo = hd.y & 0x3F3F3F3Fu, s_hi = and_or(hd.w, 0x0F0F0F0Fu, (hd.y >> 2) & 0x30303030u);
+        const uint32_t m_lo = hd.z & 0x3F3F3F3Fu, m_hi = and_or(hd.w >> 4, 0x0F0F0F0Fu, (hd.z >> 2) & 0x30303030u);
+        const float2 dd = make_float2(d * kTwo24, d * kTwo20);   // odd groups: their nibbles sit 4 bits up
+        sts128f(rec.wr, bytes_scaled(s_lo, 0, 8388608.0f, dd), bytes_scaled(s_lo, 2, 8388608.0f, dd));
+        sts128f(rec.wr + 16, bytes_scaled(s_hi, 0, 8388608.0f, dd), bytes_scaled(s_hi, 2, 8388608.0f, dd));
+        sts128(rec.wr + 32, __byte_perm(m_lo, 0u, 0x4140), __byte_perm(m_lo, 0u, 0x4342), __byte_perm(m_hi, 0u, 0x4140), __byte_perm(m_hi, 0u, 0x4342));
+        sts32f(rec.wr + 48, half_high(hd.x) * -kTwo24);
+    }
+    __syncwarp();
+#pragma unroll kUnroll
+    for (int j = 0; j < 4; ++j) {
+        uint4 w[2];
+        float2 f[2][2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            w[r] = lds128(tile + r * 2304 + j * 512 + lane * 16);
+            f[r][0] = rec_scales(rec, r, 0, j);
+            f[r][1] = rec_scales(rec, r, 1, j);
+        }
+#pragma unroll
+        for (int odd = 0; odd < 2; ++odd) {
+            uint4 b[2][NG];
+#pragma unroll
+            for (int part = 0; part < 2; ++part) {
+#pragma unroll
+                for (int n = 0; n < NG; ++n) b[part][n] = lds128(b_at + n * kFragBlockBytes + (4 * j + 2 * odd + part) * 512 + lane * 16);
+            }
+            const uint32_t mask = odd ? 0x00F000F0u : 0x000F000Fu;
+            Frag a[2][2];
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+#pragma unroll
+                for (int part = 0; part < 2; ++part) {
+                    const uint32_t top = part == 0 ? w[r].x : w[r].y, bottom = part == 0 ? w[r].z : w[r].w;   // rows g, g + 8
+                    a[r][part].r[0] = top & mask; a[r][part].r[2] = (top >> 8) & mask;
+                    a[r][part].r[1] = bottom & mask; a[r][part].r[3] = (bottom >> 8) & mask;
+                }
+            }
+            float d[2][NG][4];
+            group_mma<NG, 2>(d, a, b);
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+#pragma unroll
+                for (int n = 0; n < NG; ++n) fold(sums[r][n], d[r][n], odd ? f[r][0].y : f[r][0].x, odd ? f[r][1].y : f[r][1].x);
+            }
+        }
+    }
+    // minima (groups 2t, 2t + 1) x group sums: hi sums in the operand's first eight rows, lo sums in its last
+#pragma unroll
+    for (int n = 0; n < NG; ++n) {
+        const uint2 s = lds64(b_at + n * kFragBlockBytes + kSum32At + lane * 8);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const uint32_t m0 = rec_word(rec, r, 0, 8 + t), m1 = rec_word(rec, r, 1, 8 + t);
+            float d[4];
+            mma_first(d, m0, m1, m0, m1, s.x, s.y);
+            fold(sums[r][n], d, __uint_as_float(rec_word(rec, r, 0, 12)), __uint_as_float(rec_word(rec, r, 1, 12)));
+        }
+    }
+    __syncwarp();   // the records are free again
+}
+
+// ---- Q8_0: w = d (u - 128), blocks of 32 ------------------------------------------------------------------------
+template <int NG>
+__device__ __forceinline__ void slot_q8_0(uint32_t tile, uint32_t b_at, const Record& rec, int lane, TileSums<NG>& sums) {
+    constexpr int kUnroll = NG <= 2 ? 2 : 1;
+    const int g = lane >> 2, t = lane & 3;
+    {
+        const uint4 hd = lds128(tile + (lane >> 4) * 4352 + 4096 + (lane & 15) * 16);
+        const float2 up = make_float2(kTwo24, kTwo24);
+        sts128f(rec.wr, __fmul2_rn(make_float2(half_low(hd.x), half_high(hd.x)), up), __fmul2_rn(make_float2(half_low(hd.y), half_high(hd.y)), up));
+        sts128f(rec.wr + 16, __fmul2_rn(make_float2(half_low(hd.z), half_high(hd.z)), up), __fmul2_rn(make_float2(half_low(hd.w), half_high(hd.w)), up));
+    }
+    __syncwarp();
+#pragma unroll kUnroll
+    for (int j = 0; j < 4; ++j) {
+        float2 f[2][2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) { f[r][0] = rec_scales(rec, r, 0, j); f[r][1] = rec_scales(rec, r, 1, j); }
+#pragma unroll
+        for (int odd = 0; odd < 2; ++odd) {
+            const int blk = 2 * j + odd;
+            uint4 b[2][NG];
+#pragma unroll
+            for (int part = 0; part < 2; ++part) {
+#pragma unroll
+                for (int n = 0; n < NG; ++n) b[part][n] = lds128(b_at + n * kFragBlockBytes + (2 * blk + part) * 512 + lane * 16);
+            }
+            Frag a[2][2];
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const uint4 w = lds128(tile + r * 4352 + blk * 512 + lane * 16);
+#pragma unroll
+                for (int part = 0; part < 2; ++part) {
+                    const uint32_t top = part == 0 ? w.x : w.y, bottom = part == 0 ? w.z : w.w;
+                    a[r][part].r[0] = top & 0x00FF00FFu; a[r][part].r[2] = (top >> 8) & 0x00FF00FFu;
+                    a[r][part].r[1] = bottom & 0x00FF00FFu; a[r][part].r[3] = (bottom >> 8) & 0x00FF00FFu;
+                }
+            }
+            float d[2][NG][4];
+            group_mma<NG, 2>(d, a, b);
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+#pragma unroll
+                for (int n = 0; n < NG; ++n) fold(sums[r][n], d[r][n], odd ? f[r][0].y : f[r][0].x, odd ? f[r][1].y : f[r][1].x);
+            }
+        }
+    }
+    // 128 x d of blocks 2t, 2t + 1 (as they lie in the tile) x block sums
+#pragma unroll
+    for (int n = 0; n < NG; ++n) {
+        const uint2 s = lds64(b_at + n * kFragBlockBytes + kSum32At + lane * 8);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const uint32_t at = tile + r * 4352 + 4096 + g * 16 + 4 * t;
+            const uint32_t d0 = lds32(at), d1 = lds32(at + 128);
+            float d[4];
+            mma_first(d, d0, d1, d0, d1, s.x, s.y);
+            fold(sums[r][n], d, -128.0f, -128.0f);
+        }
+    }
+    __syncwarp();
+}
+
+// ---- Q6_K: w = d sc (q - 32), one scale per 16 inputs -----------------------------------------------------------
+template <int NG>
+__device__ __forceinline__ void slot_q6k(uint32_t tile, uint32_t b_at, const Record& rec, int lane, TileSums<NG>& sums) {
+    const int g = lane >> 2, t = lane & 3;
+    const uint32_t own = tile + (lane >> 4) * 3360, own_scales = own + 3072 + (lane & 15) * 16;
+    const float d = half_low(lds16(own + 3328 + (lane & 15) * 2));
+#pragma unroll 1
+    for (int c = 0; c < 2; ++c) {
+        if (c == 1) __syncwarp();
+        {
+            // the eight 16-input scales of this half: variants 0, 1 (low nibbles), then 2, 3 (their nibbles sit 4 bits up)
+            uint2 sc = lds64(own_scales + c * 8);
+            sc.x ^= 0x80808080u; sc.y ^= 0x80808080u;
+            const float2 low = make_float2(d * kTwo24, d * kTwo24), high = make_float2(d * kTwo20, d * kTwo20);
+            sts128f(rec.wr, bytes_scaled(sc.x, 0, 8388736.0f, low), bytes_scaled(sc.x, 2, 8388736.0f, low));
+            sts128f(rec.wr + 16, bytes_scaled(sc.y, 0, 8388736.0f, high), bytes_scaled(sc.y, 2, 8388736.0f, high));
+            if (c == 0) sts32f(rec.wr + 48, -32.0f * d);
+        }
+        __syncwarp();
+        uint4 qh[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) qh[r] = lds128(tile + r * 3360 + 2048 + c * 512 + lane * 16);
+#pragma unroll
+        for (int kh = 0; kh < 2; ++kh) {       // inputs 0..15 / 16..31 of the groups
+            uint4 w[2];
+#pragma unroll
+            for (int r = 0; r < 2; ++r) w[r] = lds128(tile + r * 3360 + (c * 2 + kh) * 512 + lane * 16);
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+                uint4 b[1][NG];
+#pragma unroll
+                for (int n = 0; n < NG; ++n) b[0][n] = lds128(b_at + n * kFragBlockBytes + ((c * 4 + v) * 2 + kh) * 512 + lane * 16);
+                Frag a[2][1];
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const uint32_t low = h == 0 ? ((v & 1) ? w[r].y : w[r].x) : ((v & 1) ? w[r].w : w[r].z);
+                        const uint32_t high = h == 0 ? (kh == 0 ? qh[r].x : qh[r].z) : (kh == 0 ? qh[r].y : qh[r].w);
+                        // the variant's two high bits (bits 2v of each byte) go above its nibble
+                        const uint32_t up = (v & 1) ? high << 2 : high << 4, down = (v & 1) ? high >> 6 : high >> 4;
+                        const uint32_t lm = v < 2 ? 0x000F000Fu : 0x00F000F0u, hm = v < 2 ? 0x00300030u : 0x03000300u;
+                        a[r][0].r[h] = and_or(low, lm, up & hm);
+                        a[r][0].r[h + 2] = and_or(low >> 8, lm, down & hm);
+                    }
+                }
+                float dsum[2][NG][4];
+                group_mma<NG, 1>(dsum, a, b);
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    const uint32_t f0 = rec_word(rec, r, 0, v * 2 + kh), f1 = rec_word(rec, r, 1, v * 2 + kh);
+#pragma unroll
+                    for (int n = 0; n < NG; ++n) fold(sums[r][n], dsum[r][n], __uint_as_float(f0), __uint_as_float(f1));
+                }
+            }
+        }
+    }
+    // offset: the sixteen subs' scales x their input sums, times 32 d
+    uint32_t sa[2][4];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {   // fragment register i: row half i & 1, subs 2t + 8 (i >> 1), + 1
+            const uint32_t two = lds16(tile + r * 3360 + 3072 + (g + 8 * (i & 1)) * 16 + 2 * t + 8 * (i >> 1)) ^ 0x8080u;
+            const uint32_t x = __byte_perm(two, 0x64646464u, 0x4140);   // 1024 + (sc + 128)
+            const __half2 hv = __hsub2(*reinterpret_cast<const __half2*>(&x), __float2half2_rn(1152.0f));
+            sa[r][i] = *reinterpret_cast<const uint32_t*>(&hv);
+        }
+    }
+#pragma unroll
+    for (int n = 0; n < NG; ++n) {
+        const uint4 s = lds128(b_at + n * kFragBlockBytes + kSum16At + lane * 16);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            float dsum[4];
+            mma_first(dsum, sa[r][0], sa[r][1], sa[r][2], sa[r][3], s.z, s.w);
+            mma_next(dsum, sa[r][0], sa[r][1], sa[r][2], sa[r][3], s.x, s.y);
+            fold(sums[r][n], dsum, __uint_as_float(rec_word(rec, r, 0, 12)), __uint_as_float(rec_word(rec, r, 1, 12)));
+        }
+    }
+    __syncwarp();
+}
+
+// A slot: the tiles, then the activations' block; the tensor copy wants 128-byte aligned destinations.
+__host__ __device__ inline int frag_slot_bytes(int w_bytes, int ng) { return (w_bytes + ng * kFragBlockBytes + 127) & ~127; }
+
+struct UnitAt { int seg, rt0; };
+__device__ __forceinline__ UnitAt unit_at(const FragGemm& a, int u) {
+    UnitAt r{0, u * kUnitTiles};
+    while (r.seg + 1 < a.n_segments) {
+        const int tiles = (a.seg[r.seg].row_tiles + kUnitTiles - 1) / kUnitTiles * kUnitTiles;
+        if (r.rt0 < tiles) break;
+        r.rt0 -= tiles;
+        ++r.seg;
+    }
+    return r;
+}
+
+// RMSNorm factor of one row from the sums of squares of its k tiles (every lane of the warp gets it).
+__device__ __forceinline__ float norm_factor(const float* ss, int tiles, float eps, int lane) {
+    float sum = 0.0f;
+    for (int i = lane; i < tiles; i += 32) sum += ss[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    return 1.0f / sqrtf(sum / (float)(tiles * kTileCols) + eps);
+}
+
+// Register shares: the launch gives each of the 384 threads 168 registers (64,512 in all); the consumers' two warpgroups
+// then take what the producer's warpgroup (one working thread) hands back: 256 x 232 + 128 x 40 = 64,512.
+constexpr int kConsumerRegs = 232, kProducerRegs = 40;
+
+template <int NG>
+__global__ void __launch_bounds__(kThreads, 1) gemm_frag_kernel(const FragGemm a, const FragSplit split, const int depth, const int w_bytes) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    constexpr int kCols = 8 * NG;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t spin_limit = a.spin_limit ? a.spin_limit : kSpinLimit;
+    const int slot_bytes = frag_slot_bytes(w_bytes, NG), slots = kTeams * depth;   // team i's ring: slots i depth ..
+    const uint32_t records0 = smem_u32(smem + (size_t)slots * slot_bytes);
+    const uint32_t full = records0 + kWarps * 32 * kRecWords * 4, empty = full + 8 * slots;
+    const int k_tiles = split.k_tiles;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < slots; ++i) { mbar_init(full + 8 * i, 1); mbar_init(empty + 8 * i, kTeamWarps); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
+    if (warp >= kWarps) {
+        // ---------------- producer (one thread): the teams' rings in turn ----------------
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kProducerRegs));
+        if (warp > kWarps || lane != 0) return;
+        auto issue = [&](int s, int slot, bool weights, bool activations) {
+            const int item = s / k_tiles, kb = s - item * k_tiles;
+            const UnitAt at = unit_at(a, item / split.groups);
+            const GemvSegment& seg = a.seg[at.seg];
+            const uint32_t bar = full + 8 * slot;
+            unsigned char* base = smem + (size_t)slot * slot_bytes;
+            if (weights) {
+                mbar_expect_tx(bar, kUnitTiles * (uint32_t)packed_tile_bytes(seg.type) + NG * kFragBlockBytes);
+                tiles_g2s(smem_u32(base), seg.map, kb, at.rt0, bar);
+            }
+            if (activations) {
+                bulk_g2s(smem_u32(base + w_bytes), a.blocks + ((size_t)(item % split.groups) * k_tiles + kb) * (NG * kFragBlockBytes),
+                         NG * kFragBlockBytes, bar);
+            }
+        };
+        int begin[kTeams], end[kTeams], longest = 0;
+#pragma unroll
+        for (int i = 0; i < kTeams; ++i) {
+            begin[i] = split.begin((int)blockIdx.x * kTeams + i);
+            end[i] = split.begin((int)blockIdx.x * kTeams + i + 1);
+            longest = max(longest, end[i] - begin[i]);
+        }
+        for (int q = 0; q < min(depth, longest); ++q) {
+#pragma unroll
+            for (int i = 0; i < kTeams; ++i) if (begin[i] + q < end[i]) issue(begin[i] + q, i * depth + q, true, false);
+        }
+        asm volatile("griddepcontrol.wait;" ::: "memory");   // the activations come from the previous kernel
+        for (int q = 0; q < min(depth, longest); ++q) {
+#pragma unroll
+            for (int i = 0; i < kTeams; ++i) if (begin[i] + q < end[i]) issue(begin[i] + q, i * depth + q, false, true);
+        }
+        int slot = 0;
+        uint32_t parity = 0;
+        bool alive = true;
+        for (int q = depth; q < longest && alive; ++q) {
+#pragma unroll
+            for (int i = 0; i < kTeams; ++i) {
+                if (begin[i] + q >= end[i] || !alive) continue;
+                alive = mbar_wait(empty + 8 * (i * depth + slot), parity, a.error_flag, 81, spin_limit);
+                if (alive) issue(begin[i] + q, i * depth + slot, true, true);
+            }
+            if (++slot == depth) { slot = 0; parity ^= 1u; }
+        }
+        if (!alive) {
+            // the teams stop waiting too: let what is still in flight land before the block can end
+            for (int i = 0; i < slots; ++i) mbar_wait(full + 8 * i, 0, nullptr, 0, spin_limit);
+            for (int i = 0; i < slots; ++i) mbar_wait(full + 8 * i, 1, nullptr, 0, spin_limit);
+        }
+        return;
+    }
+
+    // ---------------- a team: four warps, each two of the unit's row tiles, over its own slots ----------------
+    // (its ring is its own too: its warps then see every phase of the ring's barriers; a one-bit parity wait for a phase
+    // that follows one the warp has not seen complete would pass too early)
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kConsumerRegs));
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int g = lane >> 2, t = lane & 3, team = warp / kTeamWarps, pair = warp % kTeamWarps;
+    const int worker = (int)blockIdx.x * kTeams + team;
+    const uint32_t records = records0 + (uint32_t)(warp * 32 * kRecWords * 4);
+    const Record rec{records + (uint32_t)lane * kRecWords * 4u, records + (uint32_t)g * kRecWords * 4u};
+    bool alive = true;
+    int slot = 0, inv_group = -1;
+    uint32_t parity = 0;
+    float inv[NG][2];
+#pragma unroll
+    for (int n = 0; n < NG; ++n) inv[n][0] = inv[n][1] = 1.0f;
+    const int s1 = split.begin(worker + 1);
+    for (int s = split.begin(worker); s < s1;) {
+        const int item = s / k_tiles, unit = item / split.groups, group = item - unit * split.groups;
+        const UnitAt at = unit_at(a, unit);
+        const GemvSegment& seg = a.seg[at.seg];
+        const int type = seg.type;
+        const bool present = at.rt0 + 2 * pair < seg.row_tiles;   // a pair's absent second tile reads as zeros and is never stored
+        const int end = min(s1, (item + 1) * k_tiles);
+        float acc[2][NG][4];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+#pragma unroll
+            for (int n = 0; n < NG; ++n) acc[r][n][0] = acc[r][n][1] = acc[r][n][2] = acc[r][n][3] = 0.0f;
+        }
+        for (; s < end; ++s) {
+            const uint32_t bar = 8 * (uint32_t)(team * depth + slot);
+            if (alive) alive = mbar_wait(full + bar, parity, a.error_flag, 82, spin_limit);
+            if (present) {
+                const uint32_t base = smem_u32(smem) + (uint32_t)((team * depth + slot) * slot_bytes), b_at = base + w_bytes;
+                TileSums<NG> sums;
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+#pragma unroll
+                    for (int n = 0; n < NG; ++n) sums[r][n][0] = sums[r][n][1] = sums[r][n][2] = sums[r][n][3] = 0.0f;
+                }
+                const uint32_t tile = base + (uint32_t)(2 * pair * packed_tile_bytes(type));
+                if (type == kQ4_K) slot_q4k<NG>(tile, b_at, rec, lane, sums);
+                else if (type == kQ6_K) slot_q6k<NG>(tile, b_at, rec, lane, sums);
+                else slot_q8_0<NG>(tile, b_at, rec, lane, sums);
+#pragma unroll
+                for (int n = 0; n < NG; ++n) {
+                    const float2 sx = lds64f(b_at + n * kFragBlockBytes + kScaleAt + 8 * t);
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {
+                        acc[r][n][0] = fmaf(sums[r][n][0], sx.x, acc[r][n][0]);
+                        acc[r][n][1] = fmaf(sums[r][n][1], sx.y, acc[r][n][1]);
+                        acc[r][n][2] = fmaf(sums[r][n][2], sx.x, acc[r][n][2]);
+                        acc[r][n][3] = fmaf(sums[r][n][3], sx.y, acc[r][n][3]);
+                    }
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(empty + bar);
+            if (++slot == depth) { slot = 0; parity ^= 1u; }
+        }
+        if (a.partial == nullptr && a.ss != nullptr && group != inv_group) {
+            // RMSNorm factors of this lane's columns: the eight lanes of a column share its k tiles' sums of squares
+            inv_group = group;
+#pragma unroll
+            for (int n = 0; n < NG; ++n) {
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    const int m = group * kCols + n * 8 + 2 * t + c;
+                    float sum = 0.0f;
+                    if (m < a.members) for (int i = g; i < k_tiles; i += 8) sum += a.ss[(size_t)m * k_tiles + i];
+#pragma unroll
+                    for (int o = 4; o < 32; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                    inv[n][c] = 1.0f / sqrtf(sum / (float)a.k + a.eps);
+                }
+            }
+        }
+        const int part = a.partial != nullptr ? worker - split.first_worker(item) : 0;
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int n_index = (at.rt0 + 2 * pair + r) * kTileRows + g + 8 * h;
+                if (n_index >= seg.n) continue;
+#pragma unroll
+                for (int n = 0; n < NG; ++n) {
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) {
+                        const int m = group * kCols + n * 8 + 2 * t + c;
+                        if (m >= a.members) continue;
+                        const float v = acc[r][n][2 * h + c];
+                        if (a.partial != nullptr) {
+                            a.partial[((size_t)part * a.members + m) * a.total_n + a.n_offset[at.seg] + n_index] = v;
+                        } else {
+                            float* y = seg.y + (size_t)m * seg.n + n_index;
+                            *y = a.epilogue == kResidual ? *y + v * inv[n][c] : v * inv[n][c];
+                        }
+                    }
+                }
+            }
+        }
+    }
+}
+
+// ---- consumers of partial sums, producers of operands -----------------------------------------------------------
+
+// Sum of the parts of outputs n .. n + 3 (inside segment `seg`) of member m, in worker order.
+__device__ __forceinline__ float4 part_sum(const FragFinish& a, int seg, int m, int n) {
+    const int unit = a.unit0[seg] + (n >> 7), item = unit * a.split.groups + m / a.split.group_members;
+    const int parts = a.split.last_worker(item) - a.split.first_worker(item) + 1;
+    const float* p = a.partial + (size_t)m * a.total_n + a.n_offset[seg] + n;
+    const size_t stride = (size_t)a.members * a.total_n;
+    float4 v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = i < parts ? *reinterpret_cast<const float4*>(p + i * stride) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4 s = v[0];
+#pragma unroll
+    for (int i = 1; i < 8; ++i) {
+        if (i < parts) { s.x += v[i].x; s.y += v[i].y; s.z += v[i].z; s.w += v[i].w; }
+    }
+    for (int i = 8; i < parts; ++i) {
+        const float4 w = *reinterpret_cast<const float4*>(p + i * stride);
+        s.x += w.x; s.y += w.y; s.z += w.z; s.w += w.w;
+    }
+    return s;
+}
+
+// One block: a k tile (256 values of the row) of eight members, 64 threads each, four neighbouring values per thread:
+// lane t of fragment step s holds inputs 16 s + 4 t .. + 3, so a thread writes its member's 16 bytes of the step.
+// MODE: where the values come from (FragFinishMode).
+template <int MODE>
+__global__ void __launch_bounds__(512) frag_finish_kernel(const FragFinish a) {
+    __shared__ float red[16], red_sq[16];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int kt = blockIdx.x, tid = threadIdx.x, g = tid >> 6, i = tid & 63, lane = tid & 31;
+    const int m = blockIdx.y * 8 + g, n = kt * kTileCols + 4 * i, k_tiles = gridDim.x, width = k_tiles * kTileCols;
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float square = 0.0f;
+    if (m < a.members) {
+        if (MODE == kFragRows) {
+            v = *reinterpret_cast<const float4*>(a.x + (size_t)(a.index ? a.index[m] : m) * width + n);
+        } else if (MODE == kFragResidual) {
+            float4* h = reinterpret_cast<float4*>(a.y[0] + (size_t)m * width + n);
+            const float4 before = *h, s = part_sum(a, 0, m, n);
+            v = make_float4(before.x + s.x, before.y + s.y, before.z + s.z, before.w + s.w);
+            *h = v;
+        } else {
+            const float inv = a.ss != nullptr ? norm_factor(a.ss + (size_t)m * a.split.k_tiles, a.split.k_tiles, a.eps, lane) : 1.0f;
+            const float4 gt = part_sum(a, 0, m, n), up = part_sum(a, 1, m, n);
+            auto act = [&](float x, float u) { x *= inv; return x / (1.0f + expf(-x)) * (u * inv); };
+            v = make_float4(act(gt.x, up.x), act(gt.y, up.y), act(gt.z, up.z), act(gt.w, up.w));
+        }
+        square = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w)));
+        if (a.norm_weight != nullptr) {
+            const float4 w = *reinterpret_cast<const float4*>(a.norm_weight + n);
+            v.x *= w.x; v.y *= w.y; v.z *= w.z; v.w *= w.w;
+        }
+    }
+    // the tile's largest magnitude and sum of squares over the member's 64 threads
+    float top = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+        square += __shfl_xor_sync(0xffffffffu, square, o);
+    }
+    if (lane == 0) { red[tid >> 5] = top; red_sq[tid >> 5] = square; }
+    __syncthreads();
+    top = fmaxf(red[2 * g], red[2 * g + 1]);
+    // a power of two that brings the largest value into [512, 1024): sums of 32 such values still fit binary16
+    int e = 0;
+    if (top > 0.0f && isfinite(top)) frexpf(top, &e);
+    e = max(-126, min(126, 10 - e));
+    const float scale = ldexpf(1.0f, e);
+    if (i == 0 && m < a.members && a.out.ss != nullptr) a.out.ss[(size_t)m * k_tiles + kt] = red_sq[2 * g] + red_sq[2 * g + 1];
+    const float s4[4] = {v.x * scale, v.y * scale, v.z * scale, v.w * scale};
+    __half hi[4], lo[4];
+    float sum = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        hi[j] = __float2half_rn(s4[j]);
+        lo[j] = __float2half_rn(s4[j] - __half2float(hi[j]));
+        sum += __half2float(hi[j]) + __half2float(lo[j]);   // what the tensor core will see
+    }
+    const int group = blockIdx.y / a.out.ng, ng = blockIdx.y - group * a.out.ng;
+    unsigned char* blk = a.out.blocks + (((size_t)group * k_tiles + kt) * a.out.ng + ng) * kFragBlockBytes;
+    auto pack = [](__half x, __half y) { const __half2 p = __halves2half2(x, y); return *reinterpret_cast<const uint32_t*>(&p); };
+    const int s = i >> 2, t = i & 3;
+    *reinterpret_cast<uint4*>(blk + s * 512 + (g * 4 + t) * 16) = make_uint4(pack(hi[0], hi[2]), pack(hi[1], hi[3]), pack(lo[0], lo[2]), pack(lo[1], lo[3]));
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    if (t == 0) {   // sub s: element s & 7 of lanes (g, (s & 7) / 2), register pair half s >> 3
+        const __half h = __float2half_rn(sum), l = __float2half_rn(sum - __half2float(h));
+        __half* at = reinterpret_cast<__half*>(blk + kSum16At + (g * 4 + ((s & 7) >> 1)) * 16 + (s >> 3) * 4) + (s & 1);
+        at[0] = h;
+        at[4] = l;
+    }
+    sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+    if ((i & 7) == 0) {
+        const int q = i >> 3;
+        const __half h = __float2half_rn(sum), l = __float2half_rn(sum - __half2float(h));
+        __half* at = reinterpret_cast<__half*>(blk + kSum32At + (g * 4 + (q >> 1)) * 8) + (q & 1);
+        at[0] = h;
+        at[2] = l;
+    }
+    if (i == 0) reinterpret_cast<float*>(blk + kScaleAt)[g] = ldexpf(1.0f, -e);
+}
+
+// Plain outputs of a split launch: y = (sum of the parts) x the RMSNorm factor, four values per thread; blockIdx.y = member.
+__global__ void __launch_bounds__(256) frag_store_kernel(const FragFinish a) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int m = blockIdx.y, lane = threadIdx.x & 31;
+    const float inv = a.ss != nullptr ? norm_factor(a.ss + (size_t)m * a.split.k_tiles, a.split.k_tiles, a.eps, lane) : 1.0f;
+    int n = 4 * (int)(blockIdx.x * blockDim.x + threadIdx.x), seg = 0;
+    while (seg < a.n_segments && n >= a.n[seg]) { n -= a.n[seg]; ++seg; }
+    if (seg >= a.n_segments) return;
+    const float4 s = part_sum(a, seg, m, n);
+    *reinterpret_cast<float4*>(a.y[seg] + (size_t)m * a.n[seg] + n) = make_float4(s.x * inv, s.y * inv, s.z * inv, s.w * inv);
+}
+
+int device_sms() {
+    static int counts[kMaxDevices] = {0};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 148;
+    if (counts[dev] == 0) {
+        if (cudaDeviceGetAttribute(&counts[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || counts[dev] <= 0) counts[dev] = 148;
+    }
+    return counts[dev];
+}
+
+template <typename... Params>
+cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t stream, bool programmatic,
+                       const std::common_type_t<Params>&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = programmatic ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+template <int NG>
+cudaError_t launch_variant(cudaStream_t stream, const FragGemm& a, int w_bytes, bool programmatic) {
+    static bool configured[kMaxDevices] = {false};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
+    if (!configured[dev]) {
+        e = cudaFuncSetAttribute(gemm_frag_kernel<NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget);
+        if (e != cudaSuccess) return e;
+        configured[dev] = true;
+    }
+    const int slot_bytes = frag_slot_bytes(w_bytes, NG);
+    const size_t fixed = (size_t)kWarps * 32 * kRecWords * sizeof(float);
+    const int depth = (int)std::min<size_t>(6, (kSmemBudget - fixed) / (slot_bytes + 16) / kTeams);
+    if (depth < 1) return cudaErrorInvalidValue;
+    const FragSplit split = frag_split(a, a.partial == nullptr);
+    return launch_pdl(gemm_frag_kernel<NG>, dim3((unsigned)((split.workers + kTeams - 1) / kTeams)), kThreads,
+                      fixed + (size_t)kTeams * depth * (slot_bytes + 16), stream, programmatic, a, split, depth, w_bytes);
+}
+
+}  // namespace
+
+FragShape frag_shape(int members) {
+    const int eights = (members + 7) / 8, groups = (eights + kFragMaxGroup - 1) / kFragMaxGroup;
+    return FragShape{groups, (eights + groups - 1) / groups};
+}
+
+size_t frag_operand_bytes(int members, int k) {
+    const FragShape s = frag_shape(members);
+    return (size_t)s.groups * s.ng * (size_t)(k / kTileCols) * kFragBlockBytes;
+}
+
+cudaError_t make_tile_map(int type, const unsigned char* packed, long long rows, long long cols, void* host_map) {
+    static_assert(sizeof(CUtensorMap) == kTileMapBytes, "tensor map size");
+    if (!packable(type, rows, cols) || ((uintptr_t)packed & 15) != 0) return cudaErrorInvalidValue;
+    using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                                const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static Encode encode = nullptr;
+    if (encode == nullptr) {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        cudaError_t e = cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &found);
+        if (e != cudaSuccess) return e;
+        if (found != cudaDriverEntryPointSuccess || fn == nullptr) return cudaErrorNotSupported;
+        encode = (Encode)fn;
+    }
+    // a tile as lines of 224 (Q6_K) or 256 bytes: box dimensions are limited to 256 elements of 8 bytes
+    const cuuint64_t tile = (cuuint64_t)packed_tile_bytes(type), line = type == kQ6_K ? 224 : 256;
+    const cuuint64_t k_tiles = (cuuint64_t)(cols / kTileCols), row_tiles = (cuuint64_t)((rows + kTileRows - 1) / kTileRows);
+    const cuuint64_t dims[4] = {line / 8, tile / line, k_tiles, row_tiles};
+    const cuuint64_t strides[3] = {line, tile, tile * k_tiles};
+    const cuuint32_t box[4] = {(cuuint32_t)(line / 8), (cuuint32_t)(tile / line), 1, kUnitTiles}, steps[4] = {1, 1, 1, 1};
+    CUtensorMap map;
+    const CUresult r = encode(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, (void*)packed, dims, strides, box, steps, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
+    memcpy(host_map, &map, sizeof(map));
+    return cudaSuccess;
+}
+
+FragSplit frag_split(const FragGemm& a, bool whole_items) {
+    const FragShape shape = frag_shape(a.members);
+    FragSplit s{};
+    s.k_tiles = a.k / kTileCols;
+    s.groups = shape.groups;
+    s.group_members = shape.ng * 8;
+    for (int i = 0; i < a.n_segments; ++i) s.items += (a.seg[i].row_tiles + kUnitTiles - 1) / kUnitTiles * shape.groups;
+    s.whole = whole_items ? 1 : 0;
+    s.workers = std::min(device_sms() * kTeams, whole_items ? s.items : s.items * s.k_tiles);
+    return s;
+}
+
+size_t frag_partial_floats(const FragGemm& a) {
+    const FragSplit s = frag_split(a, false);
+    int parts = 1;
+    for (int i = 0; i < s.items; ++i) parts = std::max(parts, s.last_worker(i) - s.first_worker(i) + 1);
+    size_t total_n = 0;
+    for (int i = 0; i < a.n_segments; ++i) total_n += a.seg[i].n;
+    return (size_t)parts * a.members * total_n;
+}
+
+cudaError_t launch_gemm_frag(cudaStream_t stream, const FragGemm& args, bool programmatic) {
+    if (args.members < 1 || args.k % kTileCols != 0 || args.blocks == nullptr) return cudaErrorInvalidValue;
+    if (args.epilogue != kStore && args.epilogue != kResidual) return cudaErrorInvalidValue;
+    FragGemm a = args;
+    int w_bytes = 0;
+    a.total_n = 0;
+    for (int i = 0; i < a.n_segments; ++i) {
+        const int b = packed_tile_bytes(a.seg[i].type);
+        if (b == 0 || a.seg[i].map == nullptr) return cudaErrorInvalidValue;
+        w_bytes = std::max(w_bytes, kUnitTiles * b);
+        a.n_offset[i] = a.total_n;
+        a.total_n += a.seg[i].n;
+    }
+    if (a.total_n <= 0) return cudaSuccess;
+    switch (frag_shape(a.members).ng) {
+        case 1: return launch_variant<1>(stream, a, w_bytes, programmatic);
+        case 2: return launch_variant<2>(stream, a, w_bytes, programmatic);
+        case 3: return launch_variant<3>(stream, a, w_bytes, programmatic);
+        default: return launch_variant<4>(stream, a, w_bytes, programmatic);
+    }
+}
+
+cudaError_t launch_frag_finish(cudaStream_t stream, int mode, const FragGemm* gemm, FragFinish a, int width, bool programmatic) {
+    a.n_segments = 0;
+    if (gemm != nullptr) {
+        a.split = frag_split(*gemm, false);
+        a.partial = gemm->partial;
+        a.members = gemm->members;
+        a.n_segments = gemm->n_segments;
+        a.ss = gemm->ss;
+        a.eps = gemm->eps;
+        int units = 0;
+        a.total_n = 0;
+        for (int i = 0; i < gemm->n_segments; ++i) {
+            a.y[i] = gemm->seg[i].y;
+            a.n[i] = gemm->seg[i].n;
+            a.unit0[i] = units;
+            a.n_offset[i] = a.total_n;
+            units += (gemm->seg[i].row_tiles + kUnitTiles - 1) / kUnitTiles;
+            a.total_n += gemm->seg[i].n;
+            if (gemm->seg[i].n % 4 != 0) return cudaErrorInvalidValue;
+        }
+    }
+    if (a.members < 1) return cudaErrorInvalidValue;
+    if (mode == kFragStore) {
+        return launch_pdl(frag_store_kernel, dim3((unsigned)((a.total_n / 4 + 255) / 256), (unsigned)a.members), 256, 0, stream, programmatic, a);
+    }
+    if (width % kTileCols != 0) return cudaErrorInvalidValue;
+    const FragShape shape = frag_shape(a.members);
+    a.out.ng = shape.ng;
+    const dim3 grid((unsigned)(width / kTileCols), (unsigned)(shape.groups * shape.ng));
+    switch (mode) {
+        case kFragRows: return launch_pdl(frag_finish_kernel<kFragRows>, grid, 512, 0, stream, programmatic, a);
+        case kFragResidual: return launch_pdl(frag_finish_kernel<kFragResidual>, grid, 512, 0, stream, programmatic, a);
+        case kFragSwiGLU: return launch_pdl(frag_finish_kernel<kFragSwiGLU>, grid, 512, 0, stream, programmatic, a);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+}  // namespace ribn

@@ -99,6 +99,7 @@ struct GemvSegment {
     // tensor-memory GEMM then copies operand stages instead of converting packed tiles
     const unsigned char* op_a = nullptr;
     const unsigned char* op_meta = nullptr;
+    const void* map = nullptr;  // device copy of the matrix's tensor map (launch_gemm_frag)
 };
 
 enum GemvEpilogue : int {
@@ -228,6 +229,84 @@ cudaError_t launch_unpack_packed(cudaStream_t stream, int type, const unsigned c
                                  float* out);
 // Kernels the calling thread's last launch_gemm_tc enqueued (2 when a split-K launch adds its ordered reduction).
 int gemm_tc_last_launches();
+
+// ---- fragment-order form (mma.sync, any packed type, any number of rows) ------------------------------
+// Activations as the B fragments of `mma.sync.m16n8k16`: per k tile (256 inputs) and eight rows one block of
+//   [16 steps][lane] 16 bytes   hi pairs (4t, 4t + 2), (4t + 1, 4t + 3) of the step's 16 inputs of row lane / 4, then lo pairs
+//   [lane] 16 bytes             sums of the sixteen 16-input subs as an operand pair (hi, then lo)
+//   [lane] 8 bytes              sums of the eight 32-input groups: hi in the first eight operand rows, lo in the last eight
+//   [8] F32                     the rows' power-of-two scales (the stored pair is x / scale)
+// Rows are taken in `groups` of 8 * ng (at most 32); blocks are ordered [group][k tile][ng].  `ss` holds, per row and k
+// tile, the sum of squares of the values before the norm weight, for the RMSNorm factor of the consumer.
+constexpr int kFragBlockBytes = 16 * 512 + 512 + 256 + 32;
+constexpr int kFragMaxGroup = 4;   // eights of rows per group
+
+struct FragOperand {
+    unsigned char* blocks = nullptr;
+    float* ss = nullptr;   // [members][k tiles]
+    int ng = 0;            // filled in by the launcher
+};
+struct FragShape { int groups, ng; };
+FragShape frag_shape(int members);
+size_t frag_operand_bytes(int members, int k);
+
+struct FragGemm {
+    GemvSegment seg[3];
+    int n_segments;
+    int k;
+    int members;
+    const unsigned char* blocks;   // FragOperand::blocks
+    const float* ss;               // optional: multiply the results by the RMSNorm factor of these sums of squares
+    float eps;
+    int epilogue;                  // kStore or kResidual (when partial is null)
+    float* partial;                // not null: leave partial sums [part][member][rows of all segments] for launch_frag_finish
+    int* error_flag;
+    uint32_t spin_limit;
+    int n_offset[3], total_n;      // filled in by the launcher
+};
+// How a launch's (item, k tile) slots are dealt to its workers (the CTAs' teams of warps): in whole items, or evenly, an
+// item's slots then lying with consecutive workers first_worker(item) .. last_worker(item).  It depends on the matrices
+// and the row groups only.
+struct FragSplit {
+    int k_tiles, groups, group_members, items, workers, whole;
+    __host__ __device__ int begin(int w) const {   // workers past the last one have nothing
+        w = w < workers ? w : workers;
+        return whole ? (int)((long long)w * items / workers) * k_tiles : (int)((long long)w * items * k_tiles / workers);
+    }
+    __host__ __device__ int first_worker(int item) const { return (int)((((long long)item * k_tiles + 1) * workers - 1) / ((long long)items * k_tiles)); }
+    __host__ __device__ int last_worker(int item) const { return (int)(((long long)(item + 1) * k_tiles * workers - 1) / ((long long)items * k_tiles)); }
+};
+FragSplit frag_split(const FragGemm& a, bool whole_items);
+// A packed matrix as a rank-4 tensor map (128 bytes, to be copied to device memory, 64-byte aligned): one copy then
+// brings a unit's eight row tiles at one k tile; row tiles past the end read zeros.
+constexpr size_t kTileMapBytes = 128;
+cudaError_t make_tile_map(int type, const unsigned char* packed, long long rows, long long cols, void* host_map);
+size_t frag_partial_floats(const FragGemm& a);   // scratch a split launch of these arguments needs
+cudaError_t launch_gemm_frag(cudaStream_t stream, const FragGemm& args, bool programmatic);
+
+// What follows a split launch (or stands alone), writing the operand form of its values:
+//   kFragRows      rows of x (through `index`)
+//   kFragResidual  y[0] += sums; operand of y[0] * norm_weight
+//   kFragSwiGLU    silu(gate) * up of the two segments' sums
+//   kFragStore     y = sums * RMSNorm factor, no operand
+enum FragFinishMode : int { kFragRows = 0, kFragResidual = 1, kFragSwiGLU = 2, kFragStore = 3 };
+struct FragFinish {
+    const float* x;
+    const int32_t* index;
+    const float* norm_weight;
+    int members;
+    FragOperand out;
+    // from the launch's FragGemm, filled in by the launcher
+    FragSplit split;
+    const float* partial;
+    const float* ss;
+    float eps;
+    int n_segments, total_n;
+    float* y[3];
+    int n[3], unit0[3], n_offset[3];
+};
+// `gemm`: the split launch whose sums are finished (null for kFragRows); `width`: values per row of the operand.
+cudaError_t launch_frag_finish(cudaStream_t stream, int mode, const FragGemm* gemm, FragFinish args, int width, bool programmatic);
 
 // Scratch shared by the step kernels: per-span attention accumulators.
 struct StepScratch {

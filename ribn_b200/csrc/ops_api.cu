@@ -324,6 +324,29 @@ int ribn_b200_op_gemv(int32_t device, int32_t type, const void* weights, int64_t
                 a.partial_floats = partial_floats;
                 OP_TRY(launch_gemm_tc(s.stream, a));
             }
+        } else if (variant == 6) {
+            // the fragment-order kernel: partial sums finished by a second kernel where a step of a few rows does so
+            alignas(64) unsigned char map[kTileMapBytes];
+            OP_TRY(make_tile_map(type, d_w, rows, cols, map));
+            FragFinish f{};
+            f.x = d_x;
+            f.members = members;
+            f.out.blocks = s.alloc<unsigned char>(frag_operand_bytes(members, (int)cols));
+            FragGemm g{};
+            g.n_segments = 1;
+            g.seg[0] = GemvSegment{d_w, type, (int)rows, (int)((rows + kTileRows - 1) / kTileRows), d_y};
+            g.seg[0].map = s.upload(map, sizeof(map));
+            g.k = (int)cols;
+            g.members = members;
+            g.blocks = f.out.blocks;
+            g.epilogue = kStore;
+            g.error_flag = d_err;
+            const bool split = members <= 64 && rows % 4 == 0;
+            if (split) { g.partial = s.alloc<float>(frag_partial_floats(g)); OP_PTR(g.partial); }
+            OP_PTR(f.out.blocks); OP_PTR(g.seg[0].map);
+            OP_TRY(launch_frag_finish(s.stream, kFragRows, nullptr, f, (int)cols, false));
+            OP_TRY(launch_gemm_frag(s.stream, g, false));
+            if (split) OP_TRY(launch_frag_finish(s.stream, kFragStore, &g, FragFinish{}, 0, false));
         } else if (variant == 2) {
             // the batched kernel, in groups of up to kGemmMaxMembers members
             BatchOperand bop;
