@@ -449,114 +449,120 @@ cudaError_t run_layers_decode(ribn_b200_executor* ex, const StepPlan& plan, int&
     return cudaSuccess;
 }
 
-// ---- a few rows (3 .. kFragStepRows): the fragment-order GEMM, its sums finished by the kernel that makes the next
-// projection's operand --------------------------------------------------------------------------------------------
-// The line: one launch's tensor-core time grows by a 32-row group at a time; from 33 rows on the tcgen05 kernels, whose
-// time hardly depends on the row count up to 64, are ahead.
-constexpr int kFragStepRows = 32;
+// ---- a few rows (3 .. kStepRows): one GEMM launch per projection over the whole step, its partial sums finished by the
+// kernel that makes the next projection's operand -------------------------------------------------------------------
+constexpr int kStepRows = 64;
 
-GemvSegment frag_segment(const Tensor& t, float* y) {
+// The block form of a step's activations, which selects its GEMM kernel.  A projection of the 8B model (gate | up, 57 MB)
+// takes 19 / 27 / 38 / 55 / 99 us in fragment order at 8 / 16 / 24 / 32 / 64 rows and 33 / 33 / 34 / 35 / 47 us with
+// tensor-memory conversion, so the line lies at 24 rows; Q8_0 matrices are taken in fragment order only.
+int step_form(const ribn_b200_executor* ex, int members) { return ex->kquant && members > 24 ? kColumnForm : kFragmentForm; }
+
+GemvSegment step_segment(const Tensor& t, float* y) {
     GemvSegment s = segment_of(t, y);
     s.map = t.map;
     return s;
 }
-FragGemm frag_base(ribn_b200_executor* ex, int k, int members, bool normed) {
-    FragGemm a{};
+StepGemm step_base(ribn_b200_executor* ex, int k, int members, bool normed) {
+    StepGemm a{};
+    a.form = step_form(ex, members);
     a.k = k;
     a.members = members;
-    a.blocks = ex->op_frag.blocks;
-    a.ss = normed ? ex->op_frag.ss : nullptr;
+    a.blocks = ex->op_step.blocks;
+    a.ss = normed ? ex->op_step.ss : nullptr;
     a.eps = ex->cfg.rms_eps;
     a.epilogue = kStore;
     a.partial = ex->tc_partial;
     a.error_flag = ex->d_error;
     return a;
 }
-FragGemm frag_qkv(ribn_b200_executor* ex, int l, int m) {
+StepGemm step_qkv(ribn_b200_executor* ex, int l, int m) {
     Tensor* t = &ex->lt(l, 0);
-    FragGemm a = frag_base(ex, ex->cfg.hidden, m, true);
+    StepGemm a = step_base(ex, ex->cfg.hidden, m, true);
     a.n_segments = 3;
-    a.seg[0] = frag_segment(t[kAttnQ], ex->q);
-    a.seg[1] = frag_segment(t[kAttnK], ex->k);
-    a.seg[2] = frag_segment(t[kAttnV], ex->v);
+    a.seg[0] = step_segment(t[kAttnQ], ex->q);
+    a.seg[1] = step_segment(t[kAttnK], ex->k);
+    a.seg[2] = step_segment(t[kAttnV], ex->v);
     return a;
 }
-FragGemm frag_o(ribn_b200_executor* ex, int l, int m) {
-    FragGemm a = frag_base(ex, ex->cfg.q_heads * ex->cfg.head_dim, m, false);
+StepGemm step_o(ribn_b200_executor* ex, int l, int m) {
+    StepGemm a = step_base(ex, ex->cfg.q_heads * ex->cfg.head_dim, m, false);
     a.n_segments = 1;
-    a.seg[0] = frag_segment(ex->lt(l, kAttnOutput), ex->hidden);
+    a.seg[0] = step_segment(ex->lt(l, kAttnOutput), ex->hidden);
     return a;
 }
-FragGemm frag_gate_up(ribn_b200_executor* ex, int l, int m) {
-    FragGemm a = frag_base(ex, ex->cfg.hidden, m, true);
+StepGemm step_gate_up(ribn_b200_executor* ex, int l, int m) {
+    StepGemm a = step_base(ex, ex->cfg.hidden, m, true);
     a.n_segments = 2;
-    a.seg[0] = frag_segment(ex->lt(l, kFfnGate), ex->gate);
-    a.seg[1] = frag_segment(ex->lt(l, kFfnUp), ex->up);
+    a.seg[0] = step_segment(ex->lt(l, kFfnGate), ex->gate);
+    a.seg[1] = step_segment(ex->lt(l, kFfnUp), ex->up);
     return a;
 }
-FragGemm frag_down(ribn_b200_executor* ex, int l, int m) {
-    FragGemm a = frag_base(ex, ex->cfg.ffn, m, false);
+StepGemm step_down(ribn_b200_executor* ex, int l, int m) {
+    StepGemm a = step_base(ex, ex->cfg.ffn, m, false);
     a.n_segments = 1;
-    a.seg[0] = frag_segment(ex->lt(l, kFfnDown), ex->hidden);
+    a.seg[0] = step_segment(ex->lt(l, kFfnDown), ex->hidden);
     return a;
 }
 
-cudaError_t run_layers_frag(ribn_b200_executor* ex, const StepPlan& plan, int& launches) {
+cudaError_t run_layers_step(ribn_b200_executor* ex, const StepPlan& plan, int& launches) {
     const ribn_b200_config& c = ex->cfg;
     cudaStream_t s = ex->stream;
     const int T = plan.n_tokens, QD = c.q_heads * c.head_dim;
     const bool pdl = !(c.flags & RIBN_B200_FLAG_NO_GRAPH);
-    FragOperand plain = ex->op_frag;   // an operand no norm follows
+    StepOperand normed = ex->op_step, plain = ex->op_step;   // operands a norm's consumer reads / no norm follows
+    normed.form = plain.form = step_form(ex, T);
     plain.ss = nullptr;
     auto rows = [&](const float* x, const int32_t* index, const float* norm, int members, int k) -> cudaError_t {
-        FragFinish f{};
+        StepFinish f{};
         f.x = x; f.index = index; f.norm_weight = norm; f.members = members;
-        f.out = norm != nullptr ? ex->op_frag : plain;
-        return launch_frag_finish(s, kFragRows, nullptr, f, k, pdl);
+        f.out = norm != nullptr ? normed : plain;
+        f.out.form = step_form(ex, members);
+        return launch_step_finish(s, kFinishRows, nullptr, f, k, pdl);
     };
     STEP_TRY(rows(ex->hidden, nullptr, (const float*)ex->lt(0, kAttnNorm).raw, T, c.hidden));
     for (int l = 0; l < c.layers; ++l) {
         Tensor* t = &ex->lt(l, 0);
         {
-            const FragGemm g = frag_qkv(ex, l, T);
-            STEP_TRY(launch_gemm_frag(s, g, pdl));
-            STEP_TRY(launch_frag_finish(s, kFragStore, &g, FragFinish{}, 0, pdl));
+            const StepGemm g = step_qkv(ex, l, T);
+            STEP_TRY(launch_step_gemm(s, g, pdl));
+            STEP_TRY(launch_step_finish(s, kFinishStore, &g, StepFinish{}, 0, pdl));
         }
         {
             cudaError_t e = run_attention(ex, plan, l, pdl, ActOperand{}, launches);
             if (e != cudaSuccess) return e;
         }
         STEP_TRY(rows(ex->attn, nullptr, nullptr, T, QD));
-        FragFinish f{};
+        StepFinish f{};
         {
-            const FragGemm g = frag_o(ex, l, T);
-            STEP_TRY(launch_gemm_frag(s, g, pdl));
+            const StepGemm g = step_o(ex, l, T);
+            STEP_TRY(launch_step_gemm(s, g, pdl));
             f.norm_weight = (const float*)t[kFfnNorm].raw;
-            f.out = ex->op_frag;
-            STEP_TRY(launch_frag_finish(s, kFragResidual, &g, f, c.hidden, pdl));
+            f.out = normed;
+            STEP_TRY(launch_step_finish(s, kFinishResidual, &g, f, c.hidden, pdl));
         }
         {
-            const FragGemm g = frag_gate_up(ex, l, T);
-            STEP_TRY(launch_gemm_frag(s, g, pdl));
+            const StepGemm g = step_gate_up(ex, l, T);
+            STEP_TRY(launch_step_gemm(s, g, pdl));
             f.norm_weight = nullptr;
             f.out = plain;
-            STEP_TRY(launch_frag_finish(s, kFragSwiGLU, &g, f, c.ffn, pdl));
+            STEP_TRY(launch_step_finish(s, kFinishSwiGLU, &g, f, c.ffn, pdl));
         }
         {
-            const FragGemm g = frag_down(ex, l, T);
-            STEP_TRY(launch_gemm_frag(s, g, pdl));
+            const StepGemm g = step_down(ex, l, T);
+            STEP_TRY(launch_step_gemm(s, g, pdl));
             f.norm_weight = l + 1 < c.layers ? (const float*)ex->lt(l + 1, kAttnNorm).raw : (const float*)ex->output_norm.raw;
-            f.out = ex->op_frag;
-            STEP_TRY(launch_frag_finish(s, kFragResidual, &g, f, c.hidden, pdl));
+            f.out = normed;
+            STEP_TRY(launch_step_finish(s, kFinishResidual, &g, f, c.hidden, pdl));
         }
     }
     if (plan.n_sample > 0) {
         if (plan.n_sample != T) STEP_TRY(rows(ex->hidden, ex->meta.sample_token, (const float*)ex->output_norm.raw, plan.n_sample, c.hidden));
-        FragGemm g = frag_base(ex, c.hidden, plan.n_sample, true);
+        StepGemm g = step_base(ex, c.hidden, plan.n_sample, true);
         g.n_segments = 1;
-        g.seg[0] = frag_segment(ex->output, ex->logits);
+        g.seg[0] = step_segment(ex->output, ex->logits);
         g.partial = nullptr;
-        STEP_TRY(launch_gemm_frag(s, g, pdl));
+        STEP_TRY(launch_step_gemm(s, g, pdl));
     }
     return cudaSuccess;
 }
@@ -573,21 +579,22 @@ cudaError_t batch_project(ribn_b200_executor* ex, int& launches, const float* x,
     const bool kquant = tensor_memory && gemm_tc_kquant(probe, n_mats, 1);
     if (tensor_memory && !kquant) {
         // matrices with a Q8_0 member: the fragment-order kernel takes every row of the step in one launch
-        FragFinish f{};
-        f.x = x; f.index = index; f.norm_weight = norm_weight; f.members = tokens; f.out = ex->op_frag;
+        StepFinish f{};
+        f.x = x; f.index = index; f.norm_weight = norm_weight; f.members = tokens; f.out = ex->op_step;
+        f.out.form = kFragmentForm;
         if (norm_weight == nullptr) f.out.ss = nullptr;
-        STEP_TRY(launch_frag_finish(s, kFragRows, nullptr, f, k, false));
-        FragGemm a{};
+        STEP_TRY(launch_step_finish(s, kFinishRows, nullptr, f, k, false));
+        StepGemm a{};
         a.n_segments = n_mats;
-        for (int i = 0; i < n_mats; ++i) a.seg[i] = frag_segment(*mats[i], ys[i]);
+        for (int i = 0; i < n_mats; ++i) a.seg[i] = step_segment(*mats[i], ys[i]);
         a.k = k;
         a.members = tokens;
-        a.blocks = ex->op_frag.blocks;
+        a.blocks = ex->op_step.blocks;
         a.ss = f.out.ss;
         a.eps = ex->cfg.rms_eps;
         a.epilogue = epilogue == kSwiGLU ? kStore : epilogue;
         a.error_flag = ex->d_error;
-        STEP_TRY(launch_gemm_frag(s, a, false));
+        STEP_TRY(launch_step_gemm(s, a, false));
         if (epilogue == kSwiGLU) STEP_TRY(launch_silu_mul(s, ys[0], ys[1], (long long)tokens * mats[0]->rows, ys[0]));
         return cudaSuccess;
     }
@@ -721,8 +728,8 @@ bool decode_family_applies(const ribn_b200_executor* ex, const StepPlan& plan) {
     return plan.n_tokens <= kGemvMaxMembers && packed_family_applies(ex);
 }
 
-bool frag_family_applies(const ribn_b200_executor* ex, const StepPlan& plan) {
-    return plan.n_tokens <= kFragStepRows && ex->tp == 1 && !(ex->cfg.flags & RIBN_B200_FLAG_NO_TCGEN05) && packed_family_applies(ex);
+bool step_family_applies(const ribn_b200_executor* ex, const StepPlan& plan) {
+    return plan.n_tokens <= kStepRows && ex->tp == 1 && !(ex->cfg.flags & RIBN_B200_FLAG_NO_TCGEN05) && packed_family_applies(ex);
 }
 
 cudaError_t run_step(ribn_b200_executor* ex, const StepPlan& plan, int& launches) {
@@ -735,7 +742,7 @@ cudaError_t run_step(ribn_b200_executor* ex, const StepPlan& plan, int& launches
     STEP_TRY(launch_embedding(s, ex->token_embd.type, ex->token_embd.raw, c.hidden, c.vocab, ex->meta.token_id, T,
                               ex->hidden));
     cudaError_t e = decode_family_applies(ex, plan) ? run_layers_decode(ex, plan, launches)
-                    : frag_family_applies(ex, plan)   ? run_layers_frag(ex, plan, launches)
+                    : step_family_applies(ex, plan)   ? run_layers_step(ex, plan, launches)
                     : packed_family_applies(ex)     ? run_layers_batch(ex, plan, launches)
                                                     : run_layers_reference(ex, plan, launches);
     if (e != cudaSuccess) return e;
@@ -1042,6 +1049,8 @@ int ribn_b200_finalize(ribn_b200_executor* ex) {
                 CU_TRY(ex, launch_tc_cache(ex->stream, t->type, p.data, t->rows, t->cols, t->op_a, t->op_meta));
             }
         }
+        ex->kquant = true;
+        for (Tensor* t : mats) ex->kquant = ex->kquant && (t->type == kQ4_K || t->type == kQ6_K);
         CU_TRY(ex, cudaMemcpy(d_maps, maps.data(), maps.size(), cudaMemcpyHostToDevice));
         CU_TRY(ex, cudaStreamSynchronize(ex->stream));
     }
@@ -1137,14 +1146,18 @@ int ribn_b200_finalize(ribn_b200_executor* ex) {
                 CU_TRY(ex, dev_alloc(ex, (unsigned char**)&ex->op_tc.chunks,
                                      std::max(tc_operand_bytes(kGemmTcMaxMembers, kmax), tc_groups * tc_operand_bytes(64, kmax))));
                 CU_TRY(ex, dev_alloc(ex, &ex->op_tc.scale_in, tc_rows));
-                CU_TRY(ex, dev_alloc(ex, &ex->op_frag.blocks, std::max(frag_operand_bytes((int)T, kmax), frag_operand_bytes((int)S, c.hidden))));
-                CU_TRY(ex, dev_alloc(ex, &ex->op_frag.ss, std::max(T, S) * (size_t)(kmax / kTileCols)));
+                size_t step_bytes = 0;
+                const int few = std::min((int)std::max(T, S), kStepRows);
+                for (int m = 1; m <= few; ++m) step_bytes = std::max(step_bytes, step_operand_bytes(m, kmax, step_form(ex, m)));
+                if (!ex->kquant) step_bytes = std::max(step_bytes, step_operand_bytes((int)std::max(T, S), kmax, kFragmentForm));
+                CU_TRY(ex, dev_alloc(ex, &ex->op_step.blocks, step_bytes));
+                CU_TRY(ex, dev_alloc(ex, &ex->op_step.ss, std::max(T, S) * (size_t)(kmax / kTileCols)));
                 // room for four K slices of the widest fused projection at 64 rows, and for a split fragment-order launch
                 ex->tc_partial_floats = (size_t)4 * 64 * (size_t)std::max(std::max(2 * c.ffn, c.hidden), (c.q_heads + 2 * c.kv_heads) * c.head_dim);
                 if (packed_family_applies(ex)) {
-                    for (int m = 1; m <= std::min((int)T, kFragStepRows); ++m) {
-                        for (const FragGemm& g : {frag_qkv(ex, 0, m), frag_o(ex, 0, m), frag_gate_up(ex, 0, m), frag_down(ex, 0, m)}) {
-                            ex->tc_partial_floats = std::max(ex->tc_partial_floats, frag_partial_floats(g));
+                    for (int m = 1; m <= std::min((int)T, kStepRows); ++m) {
+                        for (const StepGemm& g : {step_qkv(ex, 0, m), step_o(ex, 0, m), step_gate_up(ex, 0, m), step_down(ex, 0, m)}) {
+                            ex->tc_partial_floats = std::max(ex->tc_partial_floats, step_partial_floats(g));
                         }
                     }
                 }

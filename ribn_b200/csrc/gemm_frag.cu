@@ -23,13 +23,9 @@
 // the teams in whole units when a unit's result is stored by this kernel, else evenly: a unit's partial sums are then
 // added in worker order by the kernel that consumes them.  Sums are ordered; a row's result does not depend on what it
 // is batched with.  Every wait is bounded and raises the caller's error word.
-#include <cuda.h>
 #include <cuda_fp16.h>
-#include <string.h>
-
 
 #include <algorithm>
-#include <type_traits>
 
 #include "blocks.cuh"
 #include "gemv.cuh"
@@ -39,7 +35,7 @@ namespace ribn {
 namespace {
 
 constexpr int kUnitTiles = 8;                    // row tiles per unit: 128 output rows
-constexpr int kTeams = 2;
+constexpr int kTeams = kFragTeams;
 constexpr int kTeamWarps = 4;                    // warps per team, two row tiles each
 constexpr int kWarps = kTeams * kTeamWarps;
 constexpr int kThreads = (kTeams + 1) * kTeamWarps * 32;
@@ -409,7 +405,7 @@ __device__ __forceinline__ void slot_q6k(uint32_t tile, uint32_t b_at, const Rec
 __host__ __device__ inline int frag_slot_bytes(int w_bytes, int ng) { return (w_bytes + ng * kFragBlockBytes + 127) & ~127; }
 
 struct UnitAt { int seg, rt0; };
-__device__ __forceinline__ UnitAt unit_at(const FragGemm& a, int u) {
+__device__ __forceinline__ UnitAt unit_at(const StepGemm& a, int u) {
     UnitAt r{0, u * kUnitTiles};
     while (r.seg + 1 < a.n_segments) {
         const int tiles = (a.seg[r.seg].row_tiles + kUnitTiles - 1) / kUnitTiles * kUnitTiles;
@@ -420,21 +416,12 @@ __device__ __forceinline__ UnitAt unit_at(const FragGemm& a, int u) {
     return r;
 }
 
-// RMSNorm factor of one row from the sums of squares of its k tiles (every lane of the warp gets it).
-__device__ __forceinline__ float norm_factor(const float* ss, int tiles, float eps, int lane) {
-    float sum = 0.0f;
-    for (int i = lane; i < tiles; i += 32) sum += ss[i];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    return 1.0f / sqrtf(sum / (float)(tiles * kTileCols) + eps);
-}
-
 // Register shares: the launch gives each of the 384 threads 168 registers (64,512 in all); the consumers' two warpgroups
 // then take what the producer's warpgroup (one working thread) hands back: 256 x 232 + 128 x 40 = 64,512.
 constexpr int kConsumerRegs = 232, kProducerRegs = 40;
 
 template <int NG>
-__global__ void __launch_bounds__(kThreads, 1) gemm_frag_kernel(const FragGemm a, const FragSplit split, const int depth, const int w_bytes) {
+__global__ void __launch_bounds__(kThreads, 1) gemm_frag_kernel(const StepGemm a, const StepSplit split, const int depth, const int w_bytes) {
     extern __shared__ __align__(128) unsigned char smem[];
     constexpr int kCols = 8 * NG;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -609,151 +596,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_frag_kernel(const FragGemm a
     }
 }
 
-// ---- consumers of partial sums, producers of operands -----------------------------------------------------------
-
-// Sum of the parts of outputs n .. n + 3 (inside segment `seg`) of member m, in worker order.
-__device__ __forceinline__ float4 part_sum(const FragFinish& a, int seg, int m, int n) {
-    const int unit = a.unit0[seg] + (n >> 7), item = unit * a.split.groups + m / a.split.group_members;
-    const int parts = a.split.last_worker(item) - a.split.first_worker(item) + 1;
-    const float* p = a.partial + (size_t)m * a.total_n + a.n_offset[seg] + n;
-    const size_t stride = (size_t)a.members * a.total_n;
-    float4 v[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = i < parts ? *reinterpret_cast<const float4*>(p + i * stride) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    float4 s = v[0];
-#pragma unroll
-    for (int i = 1; i < 8; ++i) {
-        if (i < parts) { s.x += v[i].x; s.y += v[i].y; s.z += v[i].z; s.w += v[i].w; }
-    }
-    for (int i = 8; i < parts; ++i) {
-        const float4 w = *reinterpret_cast<const float4*>(p + i * stride);
-        s.x += w.x; s.y += w.y; s.z += w.z; s.w += w.w;
-    }
-    return s;
-}
-
-// One block: a k tile (256 values of the row) of eight members, 64 threads each, four neighbouring values per thread:
-// lane t of fragment step s holds inputs 16 s + 4 t .. + 3, so a thread writes its member's 16 bytes of the step.
-// MODE: where the values come from (FragFinishMode).
-template <int MODE>
-__global__ void __launch_bounds__(512) frag_finish_kernel(const FragFinish a) {
-    __shared__ float red[16], red_sq[16];
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int kt = blockIdx.x, tid = threadIdx.x, g = tid >> 6, i = tid & 63, lane = tid & 31;
-    const int m = blockIdx.y * 8 + g, n = kt * kTileCols + 4 * i, k_tiles = gridDim.x, width = k_tiles * kTileCols;
-    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    float square = 0.0f;
-    if (m < a.members) {
-        if (MODE == kFragRows) {
-            v = *reinterpret_cast<const float4*>(a.x + (size_t)(a.index ? a.index[m] : m) * width + n);
-        } else if (MODE == kFragResidual) {
-            float4* h = reinterpret_cast<float4*>(a.y[0] + (size_t)m * width + n);
-            const float4 before = *h, s = part_sum(a, 0, m, n);
-            v = make_float4(before.x + s.x, before.y + s.y, before.z + s.z, before.w + s.w);
-            *h = v;
-        } else {
-            const float inv = a.ss != nullptr ? norm_factor(a.ss + (size_t)m * a.split.k_tiles, a.split.k_tiles, a.eps, lane) : 1.0f;
-            const float4 gt = part_sum(a, 0, m, n), up = part_sum(a, 1, m, n);
-            auto act = [&](float x, float u) { x *= inv; return x / (1.0f + expf(-x)) * (u * inv); };
-            v = make_float4(act(gt.x, up.x), act(gt.y, up.y), act(gt.z, up.z), act(gt.w, up.w));
-        }
-        square = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w)));
-        if (a.norm_weight != nullptr) {
-            const float4 w = *reinterpret_cast<const float4*>(a.norm_weight + n);
-            v.x *= w.x; v.y *= w.y; v.z *= w.z; v.w *= w.w;
-        }
-    }
-    // the tile's largest magnitude and sum of squares over the member's 64 threads
-    float top = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-        square += __shfl_xor_sync(0xffffffffu, square, o);
-    }
-    if (lane == 0) { red[tid >> 5] = top; red_sq[tid >> 5] = square; }
-    __syncthreads();
-    top = fmaxf(red[2 * g], red[2 * g + 1]);
-    // a power of two that brings the largest value into [512, 1024): sums of 32 such values still fit binary16
-    int e = 0;
-    if (top > 0.0f && isfinite(top)) frexpf(top, &e);
-    e = max(-126, min(126, 10 - e));
-    const float scale = ldexpf(1.0f, e);
-    if (i == 0 && m < a.members && a.out.ss != nullptr) a.out.ss[(size_t)m * k_tiles + kt] = red_sq[2 * g] + red_sq[2 * g + 1];
-    const float s4[4] = {v.x * scale, v.y * scale, v.z * scale, v.w * scale};
-    __half hi[4], lo[4];
-    float sum = 0.0f;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        hi[j] = __float2half_rn(s4[j]);
-        lo[j] = __float2half_rn(s4[j] - __half2float(hi[j]));
-        sum += __half2float(hi[j]) + __half2float(lo[j]);   // what the tensor core will see
-    }
-    const int group = blockIdx.y / a.out.ng, ng = blockIdx.y - group * a.out.ng;
-    unsigned char* blk = a.out.blocks + (((size_t)group * k_tiles + kt) * a.out.ng + ng) * kFragBlockBytes;
-    auto pack = [](__half x, __half y) { const __half2 p = __halves2half2(x, y); return *reinterpret_cast<const uint32_t*>(&p); };
-    const int s = i >> 2, t = i & 3;
-    *reinterpret_cast<uint4*>(blk + s * 512 + (g * 4 + t) * 16) = make_uint4(pack(hi[0], hi[2]), pack(hi[1], hi[3]), pack(lo[0], lo[2]), pack(lo[1], lo[3]));
-    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-    if (t == 0) {   // sub s: element s & 7 of lanes (g, (s & 7) / 2), register pair half s >> 3
-        const __half h = __float2half_rn(sum), l = __float2half_rn(sum - __half2float(h));
-        __half* at = reinterpret_cast<__half*>(blk + kSum16At + (g * 4 + ((s & 7) >> 1)) * 16 + (s >> 3) * 4) + (s & 1);
-        at[0] = h;
-        at[4] = l;
-    }
-    sum += __shfl_xor_sync(0xffffffffu, sum, 4);
-    if ((i & 7) == 0) {
-        const int q = i >> 3;
-        const __half h = __float2half_rn(sum), l = __float2half_rn(sum - __half2float(h));
-        __half* at = reinterpret_cast<__half*>(blk + kSum32At + (g * 4 + (q >> 1)) * 8) + (q & 1);
-        at[0] = h;
-        at[2] = l;
-    }
-    if (i == 0) reinterpret_cast<float*>(blk + kScaleAt)[g] = ldexpf(1.0f, -e);
-}
-
-// Plain outputs of a split launch: y = (sum of the parts) x the RMSNorm factor, four values per thread; blockIdx.y = member.
-__global__ void __launch_bounds__(256) frag_store_kernel(const FragFinish a) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int m = blockIdx.y, lane = threadIdx.x & 31;
-    const float inv = a.ss != nullptr ? norm_factor(a.ss + (size_t)m * a.split.k_tiles, a.split.k_tiles, a.eps, lane) : 1.0f;
-    int n = 4 * (int)(blockIdx.x * blockDim.x + threadIdx.x), seg = 0;
-    while (seg < a.n_segments && n >= a.n[seg]) { n -= a.n[seg]; ++seg; }
-    if (seg >= a.n_segments) return;
-    const float4 s = part_sum(a, seg, m, n);
-    *reinterpret_cast<float4*>(a.y[seg] + (size_t)m * a.n[seg] + n) = make_float4(s.x * inv, s.y * inv, s.z * inv, s.w * inv);
-}
-
-int device_sms() {
-    static int counts[kMaxDevices] = {0};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 148;
-    if (counts[dev] == 0) {
-        if (cudaDeviceGetAttribute(&counts[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || counts[dev] <= 0) counts[dev] = 148;
-    }
-    return counts[dev];
-}
-
-template <typename... Params>
-cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t stream, bool programmatic,
-                       const std::common_type_t<Params>&... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = programmatic ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 template <int NG>
-cudaError_t launch_variant(cudaStream_t stream, const FragGemm& a, int w_bytes, bool programmatic) {
+cudaError_t launch_variant(cudaStream_t stream, const StepGemm& a, int w_bytes, bool programmatic) {
     static bool configured[kMaxDevices] = {false};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -768,128 +612,28 @@ cudaError_t launch_variant(cudaStream_t stream, const FragGemm& a, int w_bytes, 
     const size_t fixed = (size_t)kWarps * 32 * kRecWords * sizeof(float);
     const int depth = (int)std::min<size_t>(6, (kSmemBudget - fixed) / (slot_bytes + 16) / kTeams);
     if (depth < 1) return cudaErrorInvalidValue;
-    const FragSplit split = frag_split(a, a.partial == nullptr);
-    return launch_pdl(gemm_frag_kernel<NG>, dim3((unsigned)((split.workers + kTeams - 1) / kTeams)), kThreads,
-                      fixed + (size_t)kTeams * depth * (slot_bytes + 16), stream, programmatic, a, split, depth, w_bytes);
+    const StepSplit split = step_split(a, a.partial == nullptr);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((split.workers + kTeams - 1) / kTeams));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = fixed + (size_t)kTeams * depth * (slot_bytes + 16);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = programmatic ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, gemm_frag_kernel<NG>, a, split, depth, w_bytes);
 }
 
 }  // namespace
 
-FragShape frag_shape(int members) {
-    const int eights = (members + 7) / 8, groups = (eights + kFragMaxGroup - 1) / kFragMaxGroup;
-    return FragShape{groups, (eights + groups - 1) / groups};
-}
-
-size_t frag_operand_bytes(int members, int k) {
-    const FragShape s = frag_shape(members);
-    return (size_t)s.groups * s.ng * (size_t)(k / kTileCols) * kFragBlockBytes;
-}
-
-cudaError_t make_tile_map(int type, const unsigned char* packed, long long rows, long long cols, void* host_map) {
-    static_assert(sizeof(CUtensorMap) == kTileMapBytes, "tensor map size");
-    if (!packable(type, rows, cols) || ((uintptr_t)packed & 15) != 0) return cudaErrorInvalidValue;
-    using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    static Encode encode = nullptr;
-    if (encode == nullptr) {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult found;
-        cudaError_t e = cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &found);
-        if (e != cudaSuccess) return e;
-        if (found != cudaDriverEntryPointSuccess || fn == nullptr) return cudaErrorNotSupported;
-        encode = (Encode)fn;
-    }
-    // a tile as lines of 224 (Q6_K) or 256 bytes: box dimensions are limited to 256 elements of 8 bytes
-    const cuuint64_t tile = (cuuint64_t)packed_tile_bytes(type), line = type == kQ6_K ? 224 : 256;
-    const cuuint64_t k_tiles = (cuuint64_t)(cols / kTileCols), row_tiles = (cuuint64_t)((rows + kTileRows - 1) / kTileRows);
-    const cuuint64_t dims[4] = {line / 8, tile / line, k_tiles, row_tiles};
-    const cuuint64_t strides[3] = {line, tile, tile * k_tiles};
-    const cuuint32_t box[4] = {(cuuint32_t)(line / 8), (cuuint32_t)(tile / line), 1, kUnitTiles}, steps[4] = {1, 1, 1, 1};
-    CUtensorMap map;
-    const CUresult r = encode(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, (void*)packed, dims, strides, box, steps, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
-    memcpy(host_map, &map, sizeof(map));
-    return cudaSuccess;
-}
-
-FragSplit frag_split(const FragGemm& a, bool whole_items) {
-    const FragShape shape = frag_shape(a.members);
-    FragSplit s{};
-    s.k_tiles = a.k / kTileCols;
-    s.groups = shape.groups;
-    s.group_members = shape.ng * 8;
-    for (int i = 0; i < a.n_segments; ++i) s.items += (a.seg[i].row_tiles + kUnitTiles - 1) / kUnitTiles * shape.groups;
-    s.whole = whole_items ? 1 : 0;
-    s.workers = std::min(device_sms() * kTeams, whole_items ? s.items : s.items * s.k_tiles);
-    return s;
-}
-
-size_t frag_partial_floats(const FragGemm& a) {
-    const FragSplit s = frag_split(a, false);
-    int parts = 1;
-    for (int i = 0; i < s.items; ++i) parts = std::max(parts, s.last_worker(i) - s.first_worker(i) + 1);
-    size_t total_n = 0;
-    for (int i = 0; i < a.n_segments; ++i) total_n += a.seg[i].n;
-    return (size_t)parts * a.members * total_n;
-}
-
-cudaError_t launch_gemm_frag(cudaStream_t stream, const FragGemm& args, bool programmatic) {
-    if (args.members < 1 || args.k % kTileCols != 0 || args.blocks == nullptr) return cudaErrorInvalidValue;
-    if (args.epilogue != kStore && args.epilogue != kResidual) return cudaErrorInvalidValue;
-    FragGemm a = args;
-    int w_bytes = 0;
-    a.total_n = 0;
-    for (int i = 0; i < a.n_segments; ++i) {
-        const int b = packed_tile_bytes(a.seg[i].type);
-        if (b == 0 || a.seg[i].map == nullptr) return cudaErrorInvalidValue;
-        w_bytes = std::max(w_bytes, kUnitTiles * b);
-        a.n_offset[i] = a.total_n;
-        a.total_n += a.seg[i].n;
-    }
-    if (a.total_n <= 0) return cudaSuccess;
-    switch (frag_shape(a.members).ng) {
+cudaError_t launch_gemm_frag(cudaStream_t stream, const StepGemm& a, int w_bytes, bool programmatic) {
+    switch (step_shape(a.members, kFragmentForm).ng) {
         case 1: return launch_variant<1>(stream, a, w_bytes, programmatic);
         case 2: return launch_variant<2>(stream, a, w_bytes, programmatic);
         case 3: return launch_variant<3>(stream, a, w_bytes, programmatic);
         default: return launch_variant<4>(stream, a, w_bytes, programmatic);
-    }
-}
-
-cudaError_t launch_frag_finish(cudaStream_t stream, int mode, const FragGemm* gemm, FragFinish a, int width, bool programmatic) {
-    a.n_segments = 0;
-    if (gemm != nullptr) {
-        a.split = frag_split(*gemm, false);
-        a.partial = gemm->partial;
-        a.members = gemm->members;
-        a.n_segments = gemm->n_segments;
-        a.ss = gemm->ss;
-        a.eps = gemm->eps;
-        int units = 0;
-        a.total_n = 0;
-        for (int i = 0; i < gemm->n_segments; ++i) {
-            a.y[i] = gemm->seg[i].y;
-            a.n[i] = gemm->seg[i].n;
-            a.unit0[i] = units;
-            a.n_offset[i] = a.total_n;
-            units += (gemm->seg[i].row_tiles + kUnitTiles - 1) / kUnitTiles;
-            a.total_n += gemm->seg[i].n;
-            if (gemm->seg[i].n % 4 != 0) return cudaErrorInvalidValue;
-        }
-    }
-    if (a.members < 1) return cudaErrorInvalidValue;
-    if (mode == kFragStore) {
-        return launch_pdl(frag_store_kernel, dim3((unsigned)((a.total_n / 4 + 255) / 256), (unsigned)a.members), 256, 0, stream, programmatic, a);
-    }
-    if (width % kTileCols != 0) return cudaErrorInvalidValue;
-    const FragShape shape = frag_shape(a.members);
-    a.out.ng = shape.ng;
-    const dim3 grid((unsigned)(width / kTileCols), (unsigned)(shape.groups * shape.ng));
-    switch (mode) {
-        case kFragRows: return launch_pdl(frag_finish_kernel<kFragRows>, grid, 512, 0, stream, programmatic, a);
-        case kFragResidual: return launch_pdl(frag_finish_kernel<kFragResidual>, grid, 512, 0, stream, programmatic, a);
-        case kFragSwiGLU: return launch_pdl(frag_finish_kernel<kFragSwiGLU>, grid, 512, 0, stream, programmatic, a);
-        default: return cudaErrorInvalidValue;
     }
 }
 

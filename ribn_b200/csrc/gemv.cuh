@@ -99,7 +99,7 @@ struct GemvSegment {
     // tensor-memory GEMM then copies operand stages instead of converting packed tiles
     const unsigned char* op_a = nullptr;
     const unsigned char* op_meta = nullptr;
-    const void* map = nullptr;  // device copy of the matrix's tensor map (launch_gemm_frag)
+    const void* map = nullptr;  // device copy of the matrix's tensor map (launch_step_gemm)
 };
 
 enum GemvEpilogue : int {
@@ -230,36 +230,45 @@ cudaError_t launch_unpack_packed(cudaStream_t stream, int type, const unsigned c
 // Kernels the calling thread's last launch_gemm_tc enqueued (2 when a split-K launch adds its ordered reduction).
 int gemm_tc_last_launches();
 
-// ---- fragment-order form (mma.sync, any packed type, any number of rows) ------------------------------
-// Activations as the B fragments of `mma.sync.m16n8k16`: per k tile (256 inputs) and eight rows one block of
-//   [16 steps][lane] 16 bytes   hi pairs (4t, 4t + 2), (4t + 1, 4t + 3) of the step's 16 inputs of row lane / 4, then lo pairs
-//   [lane] 16 bytes             sums of the sixteen 16-input subs as an operand pair (hi, then lo)
-//   [lane] 8 bytes              sums of the eight 32-input groups: hi in the first eight operand rows, lo in the last eight
-//   [8] F32                     the rows' power-of-two scales (the stored pair is x / scale)
-// Rows are taken in `groups` of 8 * ng (at most 32); blocks are ordered [group][k tile][ng].  `ss` holds, per row and k
-// tile, the sum of squares of the values before the norm weight, for the RMSNorm factor of the consumer.
+// ---- GEMMs of a step of a few rows ---------------------------------------------------------------------
+// Activations per k tile (256 inputs) and group of rows, as binary16 hi + lo pairs of x / scale with one power-of-two scale
+// per row and k tile, in one of two block forms:
+//   kFragmentForm (gemm_frag.cu, mma.sync, any packed type): groups of 8 ng rows (at most 32), ng blocks of eight rows each
+//     [16 steps][lane] 16 bytes   hi pairs (4t, 4t + 2), (4t + 1, 4t + 3) of the step's 16 inputs of row lane / 4, then lo pairs
+//     [lane] 16 bytes             sums of the sixteen 16-input subs as an operand pair (hi, then lo)
+//     [lane] 8 bytes              sums of the eight 32-input groups: hi in the first eight operand rows, lo in the last eight
+//     [8] F32                     the rows' scales
+//   kColumnForm (gemm_ta.cu, tcgen05, Q4_K / Q6_K): groups of mp = 8 ng rows (at most 64), one block
+//     [32][2 mp] 16 bytes         K-major core matrices: input 16 s + 4 t + i + 2 e is element 2 t + e of 8-input block 2 s + i;
+//                                 columns: hi parts, then lo parts
+//     [2][max(16, mp to 16)] 16 bytes   sums of the eight 32-input groups: hi, then lo
+//     [mp] F32                    the rows' scales
+// Blocks are ordered [group][k tile](ng).  `ss` holds, per row and k tile, the sum of squares of the values before the
+// norm weight, for the RMSNorm factor of the consumer.
+enum StepForm : int { kFragmentForm = 0, kColumnForm = 1 };
 constexpr int kFragBlockBytes = 16 * 512 + 512 + 256 + 32;
-constexpr int kFragMaxGroup = 4;   // eights of rows per group
 
-struct FragOperand {
+struct StepOperand {
     unsigned char* blocks = nullptr;
     float* ss = nullptr;   // [members][k tiles]
+    int form = kFragmentForm;
     int ng = 0;            // filled in by the launcher
 };
-struct FragShape { int groups, ng; };
-FragShape frag_shape(int members);
-size_t frag_operand_bytes(int members, int k);
+struct StepShape { int groups, ng; };
+StepShape step_shape(int members, int form);
+size_t step_operand_bytes(int members, int k, int form);
 
-struct FragGemm {
+struct StepGemm {
     GemvSegment seg[3];
     int n_segments;
     int k;
     int members;
-    const unsigned char* blocks;   // FragOperand::blocks
+    const unsigned char* blocks;   // StepOperand::blocks
+    int form;                      // StepForm of the blocks; selects the kernel
     const float* ss;               // optional: multiply the results by the RMSNorm factor of these sums of squares
     float eps;
     int epilogue;                  // kStore or kResidual (when partial is null)
-    float* partial;                // not null: leave partial sums [part][member][rows of all segments] for launch_frag_finish
+    float* partial;                // not null: leave partial sums [part][member][rows of all segments] for launch_step_finish
     int* error_flag;
     uint32_t spin_limit;
     int n_offset[3], total_n;      // filled in by the launcher
@@ -267,7 +276,7 @@ struct FragGemm {
 // How a launch's (item, k tile) slots are dealt to its workers (the CTAs' teams of warps): in whole items, or evenly, an
 // item's slots then lying with consecutive workers first_worker(item) .. last_worker(item).  It depends on the matrices
 // and the row groups only.
-struct FragSplit {
+struct StepSplit {
     int k_tiles, groups, group_members, items, workers, whole;
     __host__ __device__ int begin(int w) const {   // workers past the last one have nothing
         w = w < workers ? w : workers;
@@ -276,28 +285,32 @@ struct FragSplit {
     __host__ __device__ int first_worker(int item) const { return (int)((((long long)item * k_tiles + 1) * workers - 1) / ((long long)items * k_tiles)); }
     __host__ __device__ int last_worker(int item) const { return (int)(((long long)(item + 1) * k_tiles * workers - 1) / ((long long)items * k_tiles)); }
 };
-FragSplit frag_split(const FragGemm& a, bool whole_items);
+StepSplit step_split(const StepGemm& a, bool whole_items);
 // A packed matrix as a rank-4 tensor map (128 bytes, to be copied to device memory, 64-byte aligned): one copy then
 // brings a unit's eight row tiles at one k tile; row tiles past the end read zeros.
 constexpr size_t kTileMapBytes = 128;
 cudaError_t make_tile_map(int type, const unsigned char* packed, long long rows, long long cols, void* host_map);
-size_t frag_partial_floats(const FragGemm& a);   // scratch a split launch of these arguments needs
-cudaError_t launch_gemm_frag(cudaStream_t stream, const FragGemm& args, bool programmatic);
+size_t step_partial_floats(const StepGemm& a);   // scratch a split launch of these arguments needs
+cudaError_t launch_step_gemm(cudaStream_t stream, const StepGemm& args, bool programmatic);
+// The two kernels, for launch_step_gemm: `w_bytes` is the largest unit's bytes at one k tile.
+constexpr int kFragTeams = 2;   // independent workers per CTA of the fragment-order kernel
+cudaError_t launch_gemm_frag(cudaStream_t stream, const StepGemm& a, int w_bytes, bool programmatic);
+cudaError_t launch_gemm_ta(cudaStream_t stream, const StepGemm& a, int w_bytes, bool programmatic);
 
 // What follows a split launch (or stands alone), writing the operand form of its values:
-//   kFragRows      rows of x (through `index`)
-//   kFragResidual  y[0] += sums; operand of y[0] * norm_weight
-//   kFragSwiGLU    silu(gate) * up of the two segments' sums
-//   kFragStore     y = sums * RMSNorm factor, no operand
-enum FragFinishMode : int { kFragRows = 0, kFragResidual = 1, kFragSwiGLU = 2, kFragStore = 3 };
-struct FragFinish {
+//   kFinishRows      rows of x (through `index`)
+//   kFinishResidual  y[0] += sums; operand of y[0] * norm_weight
+//   kFinishSwiGLU    silu(gate) * up of the two segments' sums
+//   kFinishStore     y = sums * RMSNorm factor, no operand
+enum StepFinishMode : int { kFinishRows = 0, kFinishResidual = 1, kFinishSwiGLU = 2, kFinishStore = 3 };
+struct StepFinish {
     const float* x;
     const int32_t* index;
     const float* norm_weight;
     int members;
-    FragOperand out;
-    // from the launch's FragGemm, filled in by the launcher
-    FragSplit split;
+    StepOperand out;
+    // from the launch's StepGemm, filled in by the launcher
+    StepSplit split;
     const float* partial;
     const float* ss;
     float eps;
@@ -305,8 +318,8 @@ struct FragFinish {
     float* y[3];
     int n[3], unit0[3], n_offset[3];
 };
-// `gemm`: the split launch whose sums are finished (null for kFragRows); `width`: values per row of the operand.
-cudaError_t launch_frag_finish(cudaStream_t stream, int mode, const FragGemm* gemm, FragFinish args, int width, bool programmatic);
+// `gemm`: the split launch whose sums are finished (null for kFinishRows); `width`: values per row of the operand.
+cudaError_t launch_step_finish(cudaStream_t stream, int mode, const StepGemm* gemm, StepFinish args, int width, bool programmatic);
 
 // Scratch shared by the step kernels: per-span attention accumulators.
 struct StepScratch {

@@ -324,15 +324,19 @@ int ribn_b200_op_gemv(int32_t device, int32_t type, const void* weights, int64_t
                 a.partial_floats = partial_floats;
                 OP_TRY(launch_gemm_tc(s.stream, a));
             }
-        } else if (variant == 6) {
-            // the fragment-order kernel: partial sums finished by a second kernel where a step of a few rows does so
+        } else if (variant == 6 || variant == 7) {
+            // the kernels of a step of a few rows, in fragment order or with tensor-memory conversion: partial sums finished by a second kernel where a step of a few rows does so
+            const int form = variant == 7 ? kColumnForm : kFragmentForm;
+            if (variant == 7 && type == kQ8_0) return op_fail("gemv: the tensor-memory conversion kernel takes Q4_K and Q6_K matrices only", cudaSuccess);
             alignas(64) unsigned char map[kTileMapBytes];
             OP_TRY(make_tile_map(type, d_w, rows, cols, map));
-            FragFinish f{};
+            StepFinish f{};
             f.x = d_x;
             f.members = members;
-            f.out.blocks = s.alloc<unsigned char>(frag_operand_bytes(members, (int)cols));
-            FragGemm g{};
+            f.out.blocks = s.alloc<unsigned char>(step_operand_bytes(members, (int)cols, form));
+            f.out.form = form;
+            StepGemm g{};
+            g.form = form;
             g.n_segments = 1;
             g.seg[0] = GemvSegment{d_w, type, (int)rows, (int)((rows + kTileRows - 1) / kTileRows), d_y};
             g.seg[0].map = s.upload(map, sizeof(map));
@@ -342,11 +346,11 @@ int ribn_b200_op_gemv(int32_t device, int32_t type, const void* weights, int64_t
             g.epilogue = kStore;
             g.error_flag = d_err;
             const bool split = members <= 64 && rows % 4 == 0;
-            if (split) { g.partial = s.alloc<float>(frag_partial_floats(g)); OP_PTR(g.partial); }
+            if (split) { g.partial = s.alloc<float>(step_partial_floats(g)); OP_PTR(g.partial); }
             OP_PTR(f.out.blocks); OP_PTR(g.seg[0].map);
-            OP_TRY(launch_frag_finish(s.stream, kFragRows, nullptr, f, (int)cols, false));
-            OP_TRY(launch_gemm_frag(s.stream, g, false));
-            if (split) OP_TRY(launch_frag_finish(s.stream, kFragStore, &g, FragFinish{}, 0, false));
+            OP_TRY(launch_step_finish(s.stream, kFinishRows, nullptr, f, (int)cols, false));
+            OP_TRY(launch_step_gemm(s.stream, g, false));
+            if (split) OP_TRY(launch_step_finish(s.stream, kFinishStore, &g, StepFinish{}, 0, false));
         } else if (variant == 2) {
             // the batched kernel, in groups of up to kGemmMaxMembers members
             BatchOperand bop;

@@ -242,19 +242,33 @@ def test_operand_cache_refuses_other_types(ops):
         ops.gemv(H.Q8_0, enc, 128, 256, np.ones((4, 256), np.float32), variant=5)
 
 
-@pytest.mark.parametrize("kind", [H.Q8_0, H.Q4_K, H.Q6_K])
-@pytest.mark.parametrize("rows,cols,members", [(4, 256, 1), (40, 512, 3), (132, 768, 8), (272, 1024, 9), (128, 2048, 32), (260, 1024, 33),
-                                               (30, 512, 5), (144, 768, 70)])
-def test_fragment_order_kernel_tile_and_group_edges(ops, kind, rows, cols, members):
-    # row tiles, pairs and 128-row units cut short; row groups of 1..4 eights and several groups; split and direct results
+@pytest.mark.parametrize("kind,variant", [(H.Q8_0, 6), (H.Q4_K, 6), (H.Q6_K, 6), (H.Q4_K, 7), (H.Q6_K, 7)])
+@pytest.mark.parametrize("rows,cols,members", [(4, 256, 1), (40, 512, 3), (132, 768, 8), (272, 1024, 9), (128, 2048, 32), (260, 1024, 33), (384, 512, 24),
+                                               (136, 1024, 64), (30, 512, 5), (144, 768, 70)])
+def test_step_gemm_tile_and_group_edges(ops, kind, variant, rows, cols, members):
+    # row tiles and 128-row units cut short; every operand width, one and several row groups; split and direct results
     rng = np.random.default_rng(rows + 3 * cols + 7 * members + kind)
     enc = H.quantize(kind, rng.normal(0, 0.02, size=(rows, cols)).astype(np.float32))
     xs = (rng.normal(0, 1, (members, cols)) * 10.0 ** rng.uniform(-3, 3, (members, 1))).astype(np.float32)
     xs[:, : cols // 2] *= np.float32(1e-4)       # k tiles of very different magnitude
     xs[members // 2, 256 * (cols // 512):] = 0.0
     want = np.stack([orc.gemv(kind, enc, cols, rows, x) for x in xs])
-    got = ops.gemv(kind, enc, rows, cols, xs, variant=6)
+    got = ops.gemv(kind, enc, rows, cols, xs, variant=variant)
     scale = np.max(np.abs(want), axis=1, keepdims=True) + 1e-30
     assert np.max(np.abs(got - want) / scale) < 3e-6
     if members <= 32:   # one row group: a row's bits do not depend on what it is batched with
-        assert np.array_equal(ops.gemv(kind, enc, rows, cols, xs[:1], variant=6)[0].view(np.uint32), got[0].view(np.uint32))
+        assert np.array_equal(ops.gemv(kind, enc, rows, cols, xs[:1], variant=variant)[0].view(np.uint32), got[0].view(np.uint32))
+
+
+@pytest.mark.parametrize("kind,variant", [(H.Q8_0, 6), (H.Q4_K, 6), (H.Q6_K, 6), (H.Q4_K, 7), (H.Q6_K, 7)])
+def test_step_gemm_random_bytes(ops, kind, variant):
+    rng = np.random.default_rng(kind + 31)
+    elems, size = H.BLOCK[kind]
+    rows, cols = 272, 1024
+    blocks = rng.integers(0, 256, size=(rows * cols // elems, size), dtype=np.uint8)
+    for off in ([0] if kind == H.Q8_0 else [0, 2] if kind == H.Q4_K else [208]):
+        blocks[:, off + 1] = (blocks[:, off + 1] & 0x83) | 0x10
+    xs = rng.normal(0, 1, (21, cols)).astype(np.float32)
+    want = np.stack([orc.gemv(kind, blocks, cols, rows, x) for x in xs])
+    got = ops.gemv(kind, blocks, rows, cols, xs, variant=variant)
+    assert np.max(np.abs(got - want)) / np.max(np.abs(want)) < 3e-6
