@@ -149,54 +149,55 @@ __device__ __forceinline__ int token_spans(const AttnArgs& a, int pos) {
     return (pos + 1 - first + span_keys - 1) / span_keys;
 }
 
-// One warp merges the spans of one (token, q head) in span order:
-// out = sum_s acc_s e^(m_s - M) / sum_s l_s e^(m_s - M).  Lane = dimension lane + 32 i.  The first
-// group of spans' values is requested together with the maxima, so a short context costs one round trip.
+// Four warps merge the spans of one (token, q head): out = sum_s acc_s e^(m_s - M) / sum_s l_s e^(m_s - M).  Warp w
+// takes spans w, w + 4, .. in order, then the warps' sums are added in warp order.  Lane = dimension lane + 32 i.  A
+// group's values are requested together with the maxima, so up to sixteen spans cost one round trip.
 template <int HD>
-__device__ __forceinline__ void merge_head(const AttnArgs& a, int t, int qh, int spans, int lane) {
+__device__ __forceinline__ void merge_head(const AttnArgs& a, int t, int qh, int spans, int warp, int lane, float (*sums)[HD + 1]) {
     constexpr int DPL = HD / 32;
     constexpr int REC = HD + 2;
-    constexpr int GROUP = DPL <= 4 ? 16 : 8;  // spans whose values are in flight together
+    constexpr int GROUP = 4;  // spans of a warp whose values are in flight together
     const float* pp = a.partial + ((long long)(t - a.token_base) * a.q_heads + qh) * a.max_spans * REC;
-    float v[GROUP][DPL];
-#pragma unroll
-    for (int u = 0; u < GROUP; ++u) {
-#pragma unroll
-        for (int i = 0; i < DPL; ++i) v[u][i] = u < spans ? __ldcg(pp + u * REC + lane + 32 * i) : 0.0f;
-    }
-    float top = -INFINITY;
-    float denom = 0.0f;  // per-lane partial sums in span order, folded in a fixed shuffle order
-    for (int s = lane; s < spans; s += 32) top = fmaxf(top, __ldcg(pp + s * REC + HD));
-    top = warp_max(top);
-    for (int s = lane; s < spans; s += 32) denom = fmaf(__ldcg(pp + s * REC + HD + 1), __expf(__ldcg(pp + s * REC + HD) - top), denom);
-    denom = warp_sum(denom);
-    float sum[DPL];
-#pragma unroll
-    for (int i = 0; i < DPL; ++i) sum[i] = 0.0f;
-    for (int s0 = 0; s0 < spans; s0 += GROUP) {
-        const float mine = s0 + lane < spans ? __expf(__ldcg(pp + (s0 + lane) * REC + HD) - top) : 0.0f;
-        if (s0 > 0) {
-#pragma unroll
-            for (int u = 0; u < GROUP; ++u) {
-#pragma unroll
-                for (int i = 0; i < DPL; ++i) v[u][i] = s0 + u < spans ? __ldcg(pp + (s0 + u) * REC + lane + 32 * i) : 0.0f;
-            }
-        }
+    float v[GROUP][DPL], mx[GROUP], l[GROUP];
+    auto fetch = [&](int s0) {
 #pragma unroll
         for (int u = 0; u < GROUP; ++u) {
-            const float w = __shfl_sync(0xffffffffu, mine, u);
-            if (s0 + u < spans) {
+            const int s = s0 + 4 * u;
+            const float* rec = pp + (long long)s * REC;
 #pragma unroll
-                for (int i = 0; i < DPL; ++i) sum[i] = fmaf(v[u][i], w, sum[i]);
-            }
+            for (int i = 0; i < DPL; ++i) v[u][i] = s < spans ? __ldcg(rec + lane + 32 * i) : 0.0f;
+            mx[u] = s < spans ? __ldcg(rec + HD) : -INFINITY;
+            l[u] = s < spans ? __ldcg(rec + HD + 1) : 0.0f;
+        }
+    };
+    fetch(warp);
+    float top = -INFINITY;   // every warp needs the maximum over all spans
+    for (int s = lane; s < spans; s += 32) top = fmaxf(top, __ldcg(pp + (long long)s * REC + HD));
+    top = warp_max(top);
+    float sum[DPL], denom = 0.0f;
+#pragma unroll
+    for (int i = 0; i < DPL; ++i) sum[i] = 0.0f;
+    for (int s0 = warp; s0 < spans; s0 += 4 * GROUP) {
+        if (s0 != warp) fetch(s0);
+#pragma unroll
+        for (int u = 0; u < GROUP; ++u) {
+            const float w = __expf(mx[u] - top);   // 0 past the last span
+            denom = fmaf(l[u], w, denom);
+#pragma unroll
+            for (int i = 0; i < DPL; ++i) sum[i] = fmaf(v[u][i], w, sum[i]);
         }
     }
+#pragma unroll
+    for (int i = 0; i < DPL; ++i) sums[warp][lane + 32 * i] = sum[i];
+    if (lane == 0) sums[warp][HD] = denom;
+    __syncthreads();
     ActOperand op = a.operand;
     op.ss32 = nullptr;
-#pragma unroll
-    for (int i = 0; i < DPL; ++i) {
-        const float value = sum[i] / denom;
-        a.out[((long long)t * a.q_heads + qh) * HD + lane + 32 * i] = value;
+    const float total = ((sums[0][HD] + sums[1][HD]) + sums[2][HD]) + sums[3][HD];
+    for (int i = warp; i < DPL; i += 4) {
+        const int d = lane + 32 * i;
+        const float value = (((sums[0][d] + sums[1][d]) + sums[2][d]) + sums[3][d]) / total;
+        a.out[((long long)t * a.q_heads + qh) * HD + d] = value;
         if (op.dig != nullptr) operand_store_span(op, t - a.token_base, a.q_heads * HD, (qh * HD) / 32 + i, lane, value, 0.0f);
     }
 }
@@ -332,8 +333,11 @@ __global__ void __launch_bounds__(kMmaWarps * 32, HD <= 128 && NT == 1 ? 3 : 1) 
     // this one began, so they may be read before the programmatic dependency resolves.
     auto next_item = [&](int& id, SpanItem& it) -> bool {
         for (id += gridDim.x; id < total_items; id += gridDim.x) {
-            it.span = id % a.max_spans;
-            const int tk = id / a.max_spans;
+            // spans outermost: every token has a span 0, so the CTAs' shares stay even when contexts are ragged (with
+            // spans innermost a CTA's stride can land on the same, longer or empty, span every time)
+            const int per_span = n_tokens * a.kv_heads;
+            it.span = id / per_span;
+            const int tk = id - it.span * per_span;
             it.kvh = tk % a.kv_heads;
             const int local = tk / a.kv_heads;
             it.t = a.token_base + local;
@@ -757,18 +761,17 @@ __global__ void __launch_bounds__(kMmaWarps * 32) attention_prefill_mma_kernel(c
     }
 }
 
-// The merge: one warp per (token, q head).  A launch of its own, so that the span CTAs retire as soon as their
-// sums are stored and the next projection's weight stream can start under the merge.
+// The merge: one block of four warps per (token, q head).  A launch of its own, so that the span CTAs retire as soon as
+// their sums are stored and the next projection's weight stream can start under the merge.
 template <int HD>
-__global__ void __launch_bounds__(kMmaWarps * 32) attention_merge_kernel(const AttnArgs a, const int n_tokens) {
+__global__ void __launch_bounds__(kMmaWarps * 32) attention_merge_kernel(const AttnArgs a) {
+    __shared__ float sums[kMmaWarps][HD + 1];
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const int pair = blockIdx.x * kMmaWarps + (threadIdx.x >> 5);
-    if (pair >= n_tokens * a.q_heads) return;
-    const int t = a.token_base + pair / a.q_heads, qh = pair % a.q_heads;
+    const int t = a.token_base + (int)blockIdx.x / a.q_heads, qh = (int)blockIdx.x % a.q_heads;
     const int spans = token_spans(a, a.token_pos[t]);
     if (spans <= 1) return;  // written directly by the span kernel
-    merge_head<HD>(a, t, qh, spans, threadIdx.x & 31);
+    merge_head<HD>(a, t, qh, spans, threadIdx.x >> 5, threadIdx.x & 31, sums);
 }
 
 int attn_sm_count() {
@@ -836,14 +839,22 @@ cudaError_t launch_spans_hd(cudaStream_t stream, AttnArgs a, bool fused, int fir
     const int q_per_kv = a.q_heads / a.kv_heads;
     const int max_tiles = (max_keys + kAttnSpanKeys - 1) / kAttnSpanKeys;
     if (max_tiles > kAttnMaxSpans) return cudaErrorInvalidValue;
-    // Tiles per span: as many as leave sixteen CTAs per SM's worth of spans (the per-item set-up and the
-    // merge are paid once per span); a launch that cannot fill the GPU keeps one tile per span.
     // Prefill-sized launches: up to 16 / group-size consecutive tokens of a sequence are the columns of one item
     // and share its staged K / V rows (a token's bits do not depend on the grouping).
     a.run_tokens = (!fused && a.window <= 0 && a.operand.dig == nullptr && n_tokens >= 16) ? std::max(1, 16 / q_per_kv) : 1;
     const long long item_tokens = (n_tokens + a.run_tokens - 1) / a.run_tokens;
+    // Tiles per span: the fewest tile-times on the busiest of the resident CTAs (three per SM), an item's set-up and fold
+    // counted as one tile and a span's share of the merge as a quarter.  (One tile per span while that did not fill the
+    // GPU sixteen times over left two rows at 6,144 keys with 104 spans: 24 us of spans and 18 us of merge per layer.)
+    const long long ctas = 3ll * attn_sm_count();
+    float best = 0.0f;
     a.tiles = 1;
-    while (a.tiles < 8 && item_tokens * a.kv_heads * ((max_tiles + 2 * a.tiles - 1) / (2 * a.tiles)) >= 16 * 148) a.tiles *= 2;
+    for (int tiles = 1; tiles <= std::min(16, max_tiles); ++tiles) {
+        const int spans = (max_tiles + tiles - 1) / tiles;
+        const long long waves = (item_tokens * a.kv_heads * spans + ctas - 1) / ctas;
+        const float cost = (float)waves * (float)(tiles + 1) + 0.25f * (float)spans;
+        if (tiles == 1 || cost < best) { best = cost; a.tiles = tiles; }
+    }
     a.max_spans = (max_tiles + a.tiles - 1) / a.tiles;
     const size_t per_token = (size_t)a.q_heads * a.max_spans * (HD + 2) * sizeof(float);
     int chunk = n_tokens;
@@ -894,8 +905,7 @@ cudaError_t launch_spans_hd(cudaStream_t stream, AttnArgs a, bool fused, int fir
         if (e != cudaSuccess) return e;
         if (launches) ++*launches;
         if (a.max_spans > 1) {
-            e = launch_pdl(stream, attention_merge_kernel<HD>, dim3((n * a.q_heads + kMmaWarps - 1) / kMmaWarps), kMmaWarps * 32, 0, a,
-                           programmatic, n);
+            e = launch_pdl(stream, attention_merge_kernel<HD>, dim3(n * a.q_heads), kMmaWarps * 32, 0, a, programmatic);
             if (e != cudaSuccess) return e;
             if (launches) ++*launches;
         }
