@@ -454,9 +454,9 @@ cudaError_t run_layers_decode(ribn_b200_executor* ex, const StepPlan& plan, int&
 constexpr int kStepRows = 64;
 
 // The block form of a step's activations, which selects its GEMM kernel.  A projection of the 8B model (gate | up, 57 MB)
-// takes 19 / 27 / 38 / 55 / 99 us in fragment order at 8 / 16 / 24 / 32 / 64 rows and 33 / 33 / 34 / 35 / 47 us with
-// tensor-memory conversion, so the line lies at 24 rows; Q8_0 matrices are taken in fragment order only.
-int step_form(const ribn_b200_executor* ex, int members) { return ex->kquant && members > 24 ? kColumnForm : kFragmentForm; }
+// takes 19 / 27 / 38 / 55 / 99 us in fragment order at 8 / 16 / 24 / 32 / 64 rows and 25 / 26 / 29 / 30 / 40 us with
+// tensor-memory conversion, so the line lies at 16 rows; Q8_0 matrices are taken in fragment order only.
+int step_form(const ribn_b200_executor* ex, int members) { return ex->kquant && members > 16 ? kColumnForm : kFragmentForm; }
 
 GemvSegment step_segment(const Tensor& t, float* y) {
     GemvSegment s = segment_of(t, y);
