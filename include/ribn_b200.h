@@ -91,9 +91,11 @@ enum {
     RIBN_B200_FLAG_NO_TCGEN05 = 8,    /* batches of 3+ rows on the integer mma.sync kernel instead of tcgen05 */
     RIBN_B200_FLAG_KV_ON_DEMAND = 16, /* admit reserves the prompt's KV pages only; prepare takes the pages a row's
                                          range needs and defers the rows the arena cannot serve */
-    RIBN_B200_FLAG_OPERAND_CACHE = 32 /* finalize also keeps every Q4_K / Q6_K matrix as tcgen05 operands (binary16
-                                         integers, 2 or 4 bytes of HBM per weight); steps of 3+ rows then copy operand
-                                         stages instead of converting packed tiles.  Same results bit for bit. */
+    RIBN_B200_FLAG_OPERAND_CACHE = 32 /* tensor-parallel executors: finalize also keeps every Q4_K / Q6_K matrix as tcgen05
+                                         operands (binary16 integers, 2 or 4 bytes of HBM per weight); steps of 3+ rows
+                                         then copy operand stages instead of converting packed tiles.  Same results bit
+                                         for bit.  Elsewhere the flag changes nothing: the kernels that convert as they
+                                         go are the faster ones. */
 };
 
 /* GenerationLimits (crates/runtime/src/executor.rs:43-51). */
@@ -340,7 +342,7 @@ RIBN_B200_API int ribn_b200_op_embedding(int32_t device, int32_t ggml_type, cons
  * 5 = the K-quant form over operands converted once (what RIBN_B200_FLAG_OPERAND_CACHE
  * runs; Q4_K / Q6_K only; bit-identical to variant 3), 6 = the fragment-order mma.sync kernel (steps of a
  * few rows with Q8_0 matrices, and every batch of them), 7 = the tcgen05 kernel that converts weights into
- * tensor memory (steps of a few rows; Q4_K / Q6_K only). */
+ * tensor memory (steps of a few rows; Q4_K / Q6_K only), 8 = its wide form for prefill-sized steps. */
 RIBN_B200_API int ribn_b200_op_gemv(int32_t device, int32_t ggml_type, const void* weights,
                                     int64_t rows, int64_t cols, const float* x, int32_t members,
                                     float* y, int32_t variant);

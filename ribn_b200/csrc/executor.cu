@@ -449,14 +449,19 @@ cudaError_t run_layers_decode(ribn_b200_executor* ex, const StepPlan& plan, int&
     return cudaSuccess;
 }
 
-// ---- a few rows (3 .. kStepRows): one GEMM launch per projection over the whole step, its partial sums finished by the
-// kernel that makes the next projection's operand -------------------------------------------------------------------
-constexpr int kStepRows = 64;
-
+// ---- three rows and more: one GEMM launch per projection over the whole step, its partial sums finished by the kernel
+// that makes the next projection's operand -----------------------------------------------------------------------------
 // The block form of a step's activations, which selects its GEMM kernel.  A projection of the 8B model (gate | up, 57 MB)
-// takes 19 / 27 / 38 / 55 / 99 us in fragment order at 8 / 16 / 24 / 32 / 64 rows and 25 / 26 / 29 / 30 / 40 us with
-// tensor-memory conversion, so the line lies at 16 rows; Q8_0 matrices are taken in fragment order only.
-int step_form(const ribn_b200_executor* ex, int members) { return ex->kquant && members > 16 ? kColumnForm : kFragmentForm; }
+// takes 19 / 27 / 38 / 55 / 99 us in fragment order at 8 / 16 / 24 / 32 / 64 rows, 25 / 26 / 29 / 30 / 34 us with
+// tensor-memory conversion (61 us for two groups of 64) and 48 us in the wide form at 65 to 128 rows: the lines lie at 16
+// and at 64 rows.  Q8_0 matrices are taken in fragment order only.
+int step_form(const ribn_b200_executor* ex, int members) {
+    if (!ex->kquant || members <= 16) return kFragmentForm;
+    return members <= 64 ? kColumnForm : kWideForm;
+}
+
+// Tensor-parallel executors reduce between projections (run_layers_batch), and NO_TCGEN05 asks for the integer kernels.
+bool step_gemms(const ribn_b200_executor* ex) { return ex->tp == 1 && !(ex->cfg.flags & RIBN_B200_FLAG_NO_TCGEN05); }
 
 GemvSegment step_segment(const Tensor& t, float* y) {
     GemvSegment s = segment_of(t, y);
@@ -567,7 +572,7 @@ cudaError_t run_layers_step(ribn_b200_executor* ex, const StepPlan& plan, int& l
     return cudaSuccess;
 }
 
-// ---- batch family: tensor-core GEMMs over batch-operand activations (more rows) --------
+// ---- batch family (tensor parallelism, or without tcgen05): tensor-core GEMMs over batch-operand activations --------
 // Tokens go through each projection in groups of up to kGemmMaxMembers; weights are read once per group.
 cudaError_t batch_project(ribn_b200_executor* ex, int& launches, const float* x, const int32_t* index,
                           const float* norm_weight, int tokens, int k, const Tensor* const* mats, float* const* ys,
@@ -728,8 +733,8 @@ bool decode_family_applies(const ribn_b200_executor* ex, const StepPlan& plan) {
     return plan.n_tokens <= kGemvMaxMembers && packed_family_applies(ex);
 }
 
-bool step_family_applies(const ribn_b200_executor* ex, const StepPlan& plan) {
-    return plan.n_tokens <= kStepRows && ex->tp == 1 && !(ex->cfg.flags & RIBN_B200_FLAG_NO_TCGEN05) && packed_family_applies(ex);
+bool step_family_applies(const ribn_b200_executor* ex) {
+    return step_gemms(ex) && packed_family_applies(ex);
 }
 
 cudaError_t run_step(ribn_b200_executor* ex, const StepPlan& plan, int& launches) {
@@ -742,7 +747,7 @@ cudaError_t run_step(ribn_b200_executor* ex, const StepPlan& plan, int& launches
     STEP_TRY(launch_embedding(s, ex->token_embd.type, ex->token_embd.raw, c.hidden, c.vocab, ex->meta.token_id, T,
                               ex->hidden));
     cudaError_t e = decode_family_applies(ex, plan) ? run_layers_decode(ex, plan, launches)
-                    : step_family_applies(ex, plan)   ? run_layers_step(ex, plan, launches)
+                    : step_family_applies(ex)       ? run_layers_step(ex, plan, launches)
                     : packed_family_applies(ex)     ? run_layers_batch(ex, plan, launches)
                                                     : run_layers_reference(ex, plan, launches);
     if (e != cudaSuccess) return e;
@@ -1041,8 +1046,9 @@ int ribn_b200_finalize(ribn_b200_executor* ex) {
             CU_TRY(ex, cudaMemcpy(p.data, packed.data(), p.bytes, cudaMemcpyHostToDevice));
             CU_TRY(ex, make_tile_map(t->type, p.data, t->rows, t->cols, maps.data() + map_index * kTileMapBytes));
             t->map = d_maps + map_index++ * kTileMapBytes;
-            // the tensor-memory GEMM's operands, converted once instead of on every use
-            if ((c.flags & RIBN_B200_FLAG_OPERAND_CACHE) && !(c.flags & RIBN_B200_FLAG_NO_TCGEN05) &&
+            // the batched tensor-memory GEMM's operands, converted once instead of on every use (the step GEMMs convert
+            // under their copies and products, and are faster without)
+            if ((c.flags & RIBN_B200_FLAG_OPERAND_CACHE) && !(c.flags & RIBN_B200_FLAG_NO_TCGEN05) && !step_gemms(ex) &&
                 (t->type == kQ4_K || t->type == kQ6_K)) {
                 CU_TRY(ex, dev_alloc(ex, &t->op_a, tc_cache_a_bytes(t->type, t->rows, t->cols)));
                 CU_TRY(ex, dev_alloc(ex, &t->op_meta, tc_cache_meta_bytes(t->rows, t->cols)));
@@ -1139,32 +1145,37 @@ int ribn_b200_finalize(ribn_b200_executor* ex) {
         {
             const int kmax = std::max(std::max(c.hidden, c.ffn), c.q_heads * c.head_dim);
             if (kmax % 256 == 0) {
-                CU_TRY(ex, dev_alloc(ex, &ex->op_batch.chunks, batch_operand_bytes(kGemmMaxMembers, kmax)));
-                // room for every 64-row group of the largest step (one conversion per projection), or one 128-row operand
-                const size_t tc_groups = ((size_t)c.max_batch_tokens + 63) / 64;
-                const size_t tc_rows = std::max<size_t>(tc_groups * 64, kGemmTcMaxMembers);
-                CU_TRY(ex, dev_alloc(ex, (unsigned char**)&ex->op_tc.chunks,
-                                     std::max(tc_operand_bytes(kGemmTcMaxMembers, kmax), tc_groups * tc_operand_bytes(64, kmax))));
-                CU_TRY(ex, dev_alloc(ex, &ex->op_tc.scale_in, tc_rows));
+                const int most = (int)std::max(T, S);
                 size_t step_bytes = 0;
-                const int few = std::min((int)std::max(T, S), kStepRows);
-                for (int m = 1; m <= few; ++m) step_bytes = std::max(step_bytes, step_operand_bytes(m, kmax, step_form(ex, m)));
-                if (!ex->kquant) step_bytes = std::max(step_bytes, step_operand_bytes((int)std::max(T, S), kmax, kFragmentForm));
+                for (int m = 1; m <= most; ++m) step_bytes = std::max(step_bytes, step_operand_bytes(m, kmax, step_form(ex, m)));
+                if (!ex->kquant) step_bytes = std::max(step_bytes, step_operand_bytes(most, kmax, kFragmentForm));
                 CU_TRY(ex, dev_alloc(ex, &ex->op_step.blocks, step_bytes));
-                CU_TRY(ex, dev_alloc(ex, &ex->op_step.ss, std::max(T, S) * (size_t)(kmax / kTileCols)));
-                // room for four K slices of the widest fused projection at 64 rows, and for a split fragment-order launch
-                ex->tc_partial_floats = (size_t)4 * 64 * (size_t)std::max(std::max(2 * c.ffn, c.hidden), (c.q_heads + 2 * c.kv_heads) * c.head_dim);
-                if (packed_family_applies(ex)) {
-                    for (int m = 1; m <= std::min((int)T, kStepRows); ++m) {
-                        for (const StepGemm& g : {step_qkv(ex, 0, m), step_o(ex, 0, m), step_gate_up(ex, 0, m), step_down(ex, 0, m)}) {
-                            ex->tc_partial_floats = std::max(ex->tc_partial_floats, step_partial_floats(g));
+                CU_TRY(ex, dev_alloc(ex, &ex->op_step.ss, (size_t)most * (size_t)(kmax / kTileCols)));
+                if (step_gemms(ex)) {
+                    // partial sums of every row count a step can have (their number of parts changes with the row groups)
+                    if (packed_family_applies(ex)) {
+                        for (int m = 1; m <= (int)T; ++m) {
+                            if (m > 64 && m % 8 != 0 && m != (int)T) continue;
+                            for (const StepGemm& g : {step_qkv(ex, 0, m), step_o(ex, 0, m), step_gate_up(ex, 0, m), step_down(ex, 0, m)}) {
+                                ex->tc_partial_floats = std::max(ex->tc_partial_floats, step_partial_floats(g));
+                            }
                         }
                     }
+                } else {
+                    // room for every 64-row group of the largest step (one conversion per projection), or one 128-row operand
+                    const size_t tc_groups = ((size_t)c.max_batch_tokens + 63) / 64;
+                    const size_t tc_rows = std::max<size_t>(tc_groups * 64, kGemmTcMaxMembers);
+                    CU_TRY(ex, dev_alloc(ex, (unsigned char**)&ex->op_tc.chunks,
+                                         std::max(tc_operand_bytes(kGemmTcMaxMembers, kmax), tc_groups * tc_operand_bytes(64, kmax))));
+                    CU_TRY(ex, dev_alloc(ex, &ex->op_tc.scale_in, tc_rows));
+                    CU_TRY(ex, dev_alloc(ex, &ex->op_tc.member_scale, tc_rows));
+                    CU_TRY(ex, dev_alloc(ex, &ex->op_batch.chunks, batch_operand_bytes(kGemmMaxMembers, kmax)));
+                    CU_TRY(ex, dev_alloc(ex, &ex->op_batch.member_scale, kGemmMaxMembers));
+                    CU_TRY(ex, dev_alloc(ex, &ex->op_batch.digit_inv, kGemmMaxMembers));
+                    // room for four K slices of the widest fused projection at 64 rows
+                    ex->tc_partial_floats = (size_t)4 * 64 * (size_t)std::max(std::max(2 * c.ffn, c.hidden), (c.q_heads + 2 * c.kv_heads) * c.head_dim);
                 }
                 CU_TRY(ex, dev_alloc(ex, &ex->tc_partial, ex->tc_partial_floats));
-                CU_TRY(ex, dev_alloc(ex, &ex->op_tc.member_scale, tc_rows));
-                CU_TRY(ex, dev_alloc(ex, &ex->op_batch.member_scale, kGemmMaxMembers));
-                CU_TRY(ex, dev_alloc(ex, &ex->op_batch.digit_inv, kGemmMaxMembers));
             }
         }
         CU_TRY(ex, dev_alloc(ex, &ex->d_error, 1));

@@ -243,9 +243,10 @@ int gemm_tc_last_launches();
 //                                 columns: hi parts, then lo parts
 //     [2][max(16, mp to 16)] 16 bytes   sums of the eight 32-input groups: hi, then lo
 //     [mp] F32                    the rows' scales
+//   kWideForm (gemm_pf.cu, tcgen05, Q4_K / Q6_K): the column form with mp = 128
 // Blocks are ordered [group][k tile](ng).  `ss` holds, per row and k tile, the sum of squares of the values before the
 // norm weight, for the RMSNorm factor of the consumer.
-enum StepForm : int { kFragmentForm = 0, kColumnForm = 1 };
+enum StepForm : int { kFragmentForm = 0, kColumnForm = 1, kWideForm = 2 };
 constexpr int kFragBlockBytes = 16 * 512 + 512 + 256 + 32;
 
 struct StepOperand {
@@ -273,17 +274,41 @@ struct StepGemm {
     uint32_t spin_limit;
     int n_offset[3], total_n;      // filled in by the launcher
 };
-// How a launch's (item, k tile) slots are dealt to its workers (the CTAs' teams of warps): in whole items, or evenly, an
-// item's slots then lying with consecutive workers first_worker(item) .. last_worker(item).  It depends on the matrices
-// and the row groups only.
+// An item is one group of rows of a unit of weight rows (128; 256 in the wide form).  How a launch's (item, k tile) slots are
+// dealt to its workers (CTAs, or a CTA's teams of warps): in whole items, or evenly, an item's slots then lying with
+// consecutive workers.  The wide form takes whole items in rounds, neighbouring workers the same activations side by side,
+// and deals out only the last, incomplete round evenly.  It depends on the matrices and the row groups only.
+struct StepRun { int item, begin, end, part; };   // k tiles [begin, end) of an item, whose sums are its part `part`
 struct StepSplit {
-    int k_tiles, groups, group_members, items, workers, whole;
-    __host__ __device__ int begin(int w) const {   // workers past the last one have nothing
+    int k_tiles, groups, group_members, items, workers, whole, unit_shift;   // unit_shift: log2 of a unit's weight rows
+    int rounds;                                                              // wide form: rounds of whole items
+    __host__ __device__ int even() const { return items - rounds * workers; }   // items dealt out evenly
+    __host__ __device__ int begin(int w) const {   // first even slot of worker w; workers past the last one have nothing
         w = w < workers ? w : workers;
-        return whole ? (int)((long long)w * items / workers) * k_tiles : (int)((long long)w * items * k_tiles / workers);
+        return whole ? (int)((long long)w * even() / workers) * k_tiles : (int)((long long)w * even() * k_tiles / workers);
     }
-    __host__ __device__ int first_worker(int item) const { return (int)((((long long)item * k_tiles + 1) * workers - 1) / ((long long)items * k_tiles)); }
-    __host__ __device__ int last_worker(int item) const { return (int)(((long long)(item + 1) * k_tiles * workers - 1) / ((long long)items * k_tiles)); }
+    __host__ __device__ int first_worker(int item) const {
+        item -= rounds * workers;
+        return (int)((((long long)item * k_tiles + 1) * workers - 1) / ((long long)even() * k_tiles));
+    }
+    __host__ __device__ int last_worker(int item) const {
+        item -= rounds * workers;
+        return (int)(((long long)(item + 1) * k_tiles * workers - 1) / ((long long)even() * k_tiles));
+    }
+    __host__ __device__ int parts(int item) const {
+        return whole || item < rounds * workers ? 1 : last_worker(item) - first_worker(item) + 1;
+    }
+    // worker w's runs: its whole items, then the items its even slots touch
+    __host__ __device__ int runs(int w) const {
+        const int b = begin(w), e = begin(w + 1);
+        return rounds + (e > b ? (e - 1) / k_tiles - b / k_tiles + 1 : 0);
+    }
+    __host__ __device__ StepRun run(int w, int r) const {
+        if (r < rounds) return StepRun{r * workers + w, 0, k_tiles, 0};
+        const int b = begin(w), e = begin(w + 1), i = b / k_tiles + (r - rounds), item = rounds * workers + i;
+        const int lo = b > i * k_tiles ? b - i * k_tiles : 0, hi = e < (i + 1) * k_tiles ? e - i * k_tiles : k_tiles;
+        return StepRun{item, lo, hi, whole ? 0 : w - first_worker(item)};
+    }
 };
 StepSplit step_split(const StepGemm& a, bool whole_items);
 // A packed matrix as a rank-4 tensor map (128 bytes, to be copied to device memory, 64-byte aligned): one copy then
@@ -292,10 +317,11 @@ constexpr size_t kTileMapBytes = 128;
 cudaError_t make_tile_map(int type, const unsigned char* packed, long long rows, long long cols, void* host_map);
 size_t step_partial_floats(const StepGemm& a);   // scratch a split launch of these arguments needs
 cudaError_t launch_step_gemm(cudaStream_t stream, const StepGemm& args, bool programmatic);
-// The two kernels, for launch_step_gemm: `w_bytes` is the largest unit's bytes at one k tile.
+// The kernels, for launch_step_gemm: `w_bytes` is the largest bytes of eight row tiles at one k tile.
 constexpr int kFragTeams = 2;   // independent workers per CTA of the fragment-order kernel
 cudaError_t launch_gemm_frag(cudaStream_t stream, const StepGemm& a, int w_bytes, bool programmatic);
 cudaError_t launch_gemm_ta(cudaStream_t stream, const StepGemm& a, int w_bytes, bool programmatic);
+cudaError_t launch_gemm_pf(cudaStream_t stream, const StepGemm& a, int w_bytes, bool programmatic);
 
 // What follows a split launch (or stands alone), writing the operand form of its values:
 //   kFinishRows      rows of x (through `index`)

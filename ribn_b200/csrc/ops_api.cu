@@ -324,10 +324,10 @@ int ribn_b200_op_gemv(int32_t device, int32_t type, const void* weights, int64_t
                 a.partial_floats = partial_floats;
                 OP_TRY(launch_gemm_tc(s.stream, a));
             }
-        } else if (variant == 6 || variant == 7) {
+        } else if (variant >= 6 && variant <= 8) {
             // the kernels of a step of a few rows, in fragment order or with tensor-memory conversion: partial sums finished by a second kernel where a step of a few rows does so
-            const int form = variant == 7 ? kColumnForm : kFragmentForm;
-            if (variant == 7 && type == kQ8_0) return op_fail("gemv: the tensor-memory conversion kernel takes Q4_K and Q6_K matrices only", cudaSuccess);
+            const int form = variant == 8 ? kWideForm : variant == 7 ? kColumnForm : kFragmentForm;
+            if (variant != 6 && type == kQ8_0) return op_fail("gemv: the tensor-memory conversion kernels take Q4_K and Q6_K matrices only", cudaSuccess);
             alignas(64) unsigned char map[kTileMapBytes];
             OP_TRY(make_tile_map(type, d_w, rows, cols, map));
             StepFinish f{};
@@ -345,7 +345,7 @@ int ribn_b200_op_gemv(int32_t device, int32_t type, const void* weights, int64_t
             g.blocks = f.out.blocks;
             g.epilogue = kStore;
             g.error_flag = d_err;
-            const bool split = members <= 64 && rows % 4 == 0;
+            const bool split = (members <= 64 || variant == 8) && rows % 4 == 0;
             if (split) { g.partial = s.alloc<float>(step_partial_floats(g)); OP_PTR(g.partial); }
             OP_PTR(f.out.blocks); OP_PTR(g.seg[0].map);
             OP_TRY(launch_step_finish(s.stream, kFinishRows, nullptr, f, (int)cols, false));

@@ -1,4 +1,4 @@
-// Around the GEMMs of a step of a few rows (gemm_frag.cu, gemm_ta.cu): how their work is dealt out, the tensor maps of the
+// Around the GEMMs of a step (gemm_frag.cu, gemm_ta.cu, gemm_pf.cu): how their work is dealt out, the tensor maps of the
 // packed matrices, and the kernels that finish a split launch's partial sums (residual add, SwiGLU) and write the next
 // projection's operand in the same pass.
 #include <cuda.h>
@@ -15,7 +15,7 @@ namespace ribn {
 
 namespace {
 
-constexpr int kUnitTiles = 8;   // row tiles per unit of both GEMM kernels: 128 output rows
+constexpr int kUnitTiles = 8;   // row tiles per tensor copy and per unit: 128 output rows (two units make one of the wide form)
 constexpr int kSum16At = 16 * 512, kSum32At = kSum16At + 512, kScaleAt = kSum32At + 256;   // fragment-form block
 
 // RMSNorm factor of one row from the sums of squares of its k tiles (every lane of the warp gets it).
@@ -31,8 +31,8 @@ __device__ __forceinline__ float norm_factor(const float* ss, int tiles, float e
 
 // Sum of the parts of outputs n .. n + 3 (inside segment `seg`) of member m, in worker order.
 __device__ __forceinline__ float4 part_sum(const StepFinish& a, int seg, int m, int n) {
-    const int unit = a.unit0[seg] + (n >> 7), item = unit * a.split.groups + m / a.split.group_members;
-    const int parts = a.split.last_worker(item) - a.split.first_worker(item) + 1;
+    const int unit = a.unit0[seg] + (n >> a.split.unit_shift), item = unit * a.split.groups + m / a.split.group_members;
+    const int parts = a.split.parts(item);
     const float* p = a.partial + (size_t)m * a.total_n + a.n_offset[seg] + n;
     const size_t stride = (size_t)a.members * a.total_n;
     float4 v[8];
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(512) step_finish_kernel(const StepFinish a) {
     auto pack = [](__half x, __half y) { const __half2 p = __halves2half2(x, y); return *reinterpret_cast<const uint32_t*>(&p); };
     const int s = i >> 2, t = i & 3;
     const float inv_scale = ldexpf(1.0f, -e);
-    if (a.out.form == kColumnForm) {
+    if (a.out.form != kFragmentForm) {
         const int mp = 8 * a.out.ng, sum_cols = max(16, (mp + 15) / 16 * 16), col = ng * 8 + g;
         unsigned char* blk = a.out.blocks + ((size_t)group * k_tiles + kt) * (1028 * mp + 32 * sum_cols);
         uint32_t* at = reinterpret_cast<uint32_t*>(blk + ((size_t)(2 * s) * 2 * mp + col) * 16 + 4 * t);
@@ -194,6 +194,7 @@ cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, int threads, size_t
 
 StepShape step_shape(int members, int form) {
     const int eights = (members + 7) / 8;
+    if (form == kWideForm) return StepShape{(eights + 15) / 16, 16};
     if (form == kColumnForm) {
         // one group of up to 64 rows: 8, 16, 24, 32, 48 or 64 columns
         if (eights <= 4) return StepShape{1, eights};
@@ -209,7 +210,7 @@ size_t column_block_bytes(int mp) { return (size_t)1028 * mp + 32 * (size_t)(mp 
 
 size_t step_operand_bytes(int members, int k, int form) {
     const StepShape s = step_shape(members, form);
-    return (size_t)s.groups * (size_t)(k / kTileCols) * (form == kColumnForm ? column_block_bytes(8 * s.ng) : (size_t)s.ng * kFragBlockBytes);
+    return (size_t)s.groups * (size_t)(k / kTileCols) * (form != kFragmentForm ? column_block_bytes(8 * s.ng) : (size_t)s.ng * kFragBlockBytes);
 }
 
 cudaError_t make_tile_map(int type, const unsigned char* packed, long long rows, long long cols, void* host_map) {
@@ -243,19 +244,23 @@ cudaError_t make_tile_map(int type, const unsigned char* packed, long long rows,
 StepSplit step_split(const StepGemm& a, bool whole_items) {
     const StepShape shape = step_shape(a.members, a.form);
     StepSplit s{};
+    const int tiles = a.form == kWideForm ? 2 * kUnitTiles : kUnitTiles;
+    s.unit_shift = a.form == kWideForm ? 8 : 7;
     s.k_tiles = a.k / kTileCols;
     s.groups = shape.groups;
     s.group_members = shape.ng * 8;
-    for (int i = 0; i < a.n_segments; ++i) s.items += (a.seg[i].row_tiles + kUnitTiles - 1) / kUnitTiles * shape.groups;
+    for (int i = 0; i < a.n_segments; ++i) s.items += (a.seg[i].row_tiles + tiles - 1) / tiles * shape.groups;
     s.whole = whole_items ? 1 : 0;
-    s.workers = std::min(device_sms() * (a.form == kColumnForm ? 1 : kFragTeams), whole_items ? s.items : s.items * s.k_tiles);
+    s.workers = std::min(device_sms() * (a.form == kFragmentForm ? kFragTeams : 1), whole_items ? s.items : s.items * s.k_tiles);
+    s.rounds = a.form == kWideForm ? s.items / s.workers : 0;
+    if (s.rounds * s.workers == s.items && s.rounds > 0) s.whole = 1;   // nothing is left to deal out evenly
     return s;
 }
 
 size_t step_partial_floats(const StepGemm& a) {
     const StepSplit s = step_split(a, false);
     int parts = 1;
-    for (int i = 0; i < s.items; ++i) parts = std::max(parts, s.last_worker(i) - s.first_worker(i) + 1);
+    for (int i = 0; i < s.items; ++i) parts = std::max(parts, s.parts(i));
     size_t total_n = 0;
     for (int i = 0; i < a.n_segments; ++i) total_n += a.seg[i].n;
     return (size_t)parts * a.members * total_n;
@@ -269,12 +274,13 @@ cudaError_t launch_step_gemm(cudaStream_t stream, const StepGemm& args, bool pro
     a.total_n = 0;
     for (int i = 0; i < a.n_segments; ++i) {
         const int b = packed_tile_bytes(a.seg[i].type);
-        if (b == 0 || a.seg[i].map == nullptr || (a.form == kColumnForm && a.seg[i].type == kQ8_0)) return cudaErrorInvalidValue;
+        if (b == 0 || a.seg[i].map == nullptr || (a.form != kFragmentForm && a.seg[i].type == kQ8_0)) return cudaErrorInvalidValue;
         w_bytes = std::max(w_bytes, kUnitTiles * b);
         a.n_offset[i] = a.total_n;
         a.total_n += a.seg[i].n;
     }
     if (a.total_n <= 0) return cudaSuccess;
+    if (a.form == kWideForm) return launch_gemm_pf(stream, a, w_bytes, programmatic);
     return a.form == kColumnForm ? launch_gemm_ta(stream, a, w_bytes, programmatic) : launch_gemm_frag(stream, a, w_bytes, programmatic);
 }
 
@@ -294,7 +300,7 @@ cudaError_t launch_step_finish(cudaStream_t stream, int mode, const StepGemm* ge
             a.n[i] = gemm->seg[i].n;
             a.unit0[i] = units;
             a.n_offset[i] = a.total_n;
-            units += (gemm->seg[i].row_tiles + kUnitTiles - 1) / kUnitTiles;
+            units += (gemm->seg[i].n + (1 << a.split.unit_shift) - 1) >> a.split.unit_shift;
             a.total_n += gemm->seg[i].n;
             if (gemm->seg[i].n % 4 != 0) return cudaErrorInvalidValue;
         }

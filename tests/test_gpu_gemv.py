@@ -242,9 +242,9 @@ def test_operand_cache_refuses_other_types(ops):
         ops.gemv(H.Q8_0, enc, 128, 256, np.ones((4, 256), np.float32), variant=5)
 
 
-@pytest.mark.parametrize("kind,variant", [(H.Q8_0, 6), (H.Q4_K, 6), (H.Q6_K, 6), (H.Q4_K, 7), (H.Q6_K, 7)])
+@pytest.mark.parametrize("kind,variant", [(H.Q8_0, 6), (H.Q4_K, 6), (H.Q6_K, 6), (H.Q4_K, 7), (H.Q6_K, 7), (H.Q4_K, 8), (H.Q6_K, 8)])
 @pytest.mark.parametrize("rows,cols,members", [(4, 256, 1), (40, 512, 3), (132, 768, 8), (272, 1024, 9), (128, 2048, 32), (260, 1024, 33), (384, 512, 24),
-                                               (136, 1024, 64), (30, 512, 5), (144, 768, 70)])
+                                               (136, 1024, 64), (30, 512, 5), (144, 768, 70), (520, 768, 200), (257, 512, 129), (19200, 256, 300)])
 def test_step_gemm_tile_and_group_edges(ops, kind, variant, rows, cols, members):
     # row tiles and 128-row units cut short; every operand width, one and several row groups; split and direct results
     rng = np.random.default_rng(rows + 3 * cols + 7 * members + kind)
@@ -255,12 +255,12 @@ def test_step_gemm_tile_and_group_edges(ops, kind, variant, rows, cols, members)
     want = np.stack([orc.gemv(kind, enc, cols, rows, x) for x in xs])
     got = ops.gemv(kind, enc, rows, cols, xs, variant=variant)
     scale = np.max(np.abs(want), axis=1, keepdims=True) + 1e-30
-    assert np.max(np.abs(got - want) / scale) < 3e-6
+    assert np.max(np.abs(got - want) / scale) < (3e-6 if rows < 1000 else 8e-6)   # the largest of 5.8 million errors
     if members <= 32:   # one row group: a row's bits do not depend on what it is batched with
         assert np.array_equal(ops.gemv(kind, enc, rows, cols, xs[:1], variant=variant)[0].view(np.uint32), got[0].view(np.uint32))
 
 
-@pytest.mark.parametrize("kind,variant", [(H.Q8_0, 6), (H.Q4_K, 6), (H.Q6_K, 6), (H.Q4_K, 7), (H.Q6_K, 7)])
+@pytest.mark.parametrize("kind,variant", [(H.Q8_0, 6), (H.Q4_K, 6), (H.Q6_K, 6), (H.Q4_K, 7), (H.Q6_K, 7), (H.Q4_K, 8), (H.Q6_K, 8)])
 def test_step_gemm_random_bytes(ops, kind, variant):
     rng = np.random.default_rng(kind + 31)
     elems, size = H.BLOCK[kind]
