@@ -58,9 +58,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const uint32_t spin_limit = a.spin_limit ? a.spin_limit : kSpinLimit;
     const uint32_t b_ring = smem_u32(smem), tails = b_ring + 2 * kChunkBytes, a2_buf = tails + 2 * kTailBytes, scales = a2_buf + 2 * kA2Bytes,
-                   inv_at = scales + 4 * kUnitRows * 4, tmem_slot = inv_at + kCols * 4, bars = tmem_slot + 16, w_ring = (bars + 192 + 127) & ~127u;
+                   inv_at = scales + 4 * kUnitRows * 4, tmem_slot = inv_at + kCols * 4, bars = tmem_slot + 16, w_ring = (bars + 200 + 127) & ~127u;
     const uint32_t w_full = bars, w_empty = bars + 32, b_full = bars + 64, b_empty = bars + 80, a_full = bars + 96, a_free = bars + 112,
-                   d_full = bars + 128, d_free = bars + 144, t_full = bars + 160, t_empty = bars + 176, min_free = tmem_slot + 8;
+                   d_full = bars + 128, d_free = bars + 144, t_full = bars + 160, t_empty = bars + 176, min_full = bars + 192, min_free = tmem_slot + 8;
     const int k_tiles = split.k_tiles, groups = split.groups, runs = split.runs((int)blockIdx.x);   // item = pair of units * groups + group
 
     if (threadIdx.x == 0) {
@@ -72,6 +72,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
             mbar_init(t_full + 8 * i, 1); mbar_init(t_empty + 8 * i, kFoldWarps);
         }
         mbar_init(min_free, kFoldWarps);
+        mbar_init(min_full, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kMmaWarp) {
@@ -158,28 +159,30 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
                             if (alive) alive = mbar_wait(a_full + 8 * u, uses & 1u, a.error_flag, 106, spin_limit);
                             tc_fence_after();
                             if (q4k) {
-                                if (leader) {
 #pragma unroll
-                                    for (int i = 0; i < 8; ++i) umma_ts(d_main, a_at + 8 * i, b_desc + kLo + i * kStep, idesc, (uint32_t)(h | i));
+                                for (int i = 0; i < 8; ++i) umma_ts_if(leader, d_main, a_at + 8 * i, b_desc + kLo + i * kStep, idesc, (uint32_t)(h | i));
 #pragma unroll
-                                    for (int i = 0; i < 8; ++i) umma_ts(d_main, a_at + 8 * i, b_desc + i * kStep, idesc, 1u);
-                                }
-                                if (last) {
-                                    // minima x group sums, once the previous fold has read its minima sums
+                                for (int i = 0; i < 8; ++i) umma_ts_if(leader, d_main, a_at + 8 * i, b_desc + i * kStep, idesc, 1u);
+                                if (h == u) {
+                                    // minima x group sums: unit 0's with its first stage, so that they are folded by the time
+                                    // unit 1's, with its last stage, need the columns
                                     if (u == 0 && alive) alive = mbar_wait(t_full + 8 * (n & 1u), (n >> 1) & 1u, a.error_flag, 107, spin_limit);
                                     if (mins >= 1 && alive) alive = mbar_wait(min_free, (mins - 1u) & 1u, a.error_flag, 108, spin_limit);
                                     tc_fence_after();
-                                    if (leader) umma_ss(tmem + 256, a2_desc0 + u * (kA2Bytes >> 4), sum_desc0 + (n & 1u) * (kTailBytes >> 4), idesc, 0u);
+                                    if (leader) {
+                                        umma_ss(tmem + 256, a2_desc0 + u * (kA2Bytes >> 4), sum_desc0 + (n & 1u) * (kTailBytes >> 4), idesc, 0u);
+                                        umma_commit(min_full);
+                                    }
                                     ++mins;
                                 }
-                            } else if (leader) {
+                            } else {
                                 // position i of the stage holds step 2 (i & 1) + (i >> 1) of its 64 inputs; p2 x lo is below F32's resolution
 #pragma unroll
-                                for (int i = 0; i < 4; ++i) umma_ts(d_main, a_at + 8 * i, b_desc + kLo + (2 * (i & 1) + (i >> 1)) * kStep, idesc, (uint32_t)(h | i));
+                                for (int i = 0; i < 4; ++i) umma_ts_if(leader, d_main, a_at + 8 * i, b_desc + kLo + (2 * (i & 1) + (i >> 1)) * kStep, idesc, (uint32_t)(h | i));
 #pragma unroll
-                                for (int i = 0; i < 4; ++i) umma_ts(d_main, a_at + 32 + 8 * i, b_desc + (2 * (i & 1) + (i >> 1)) * kStep, idesc, 1u);
+                                for (int i = 0; i < 4; ++i) umma_ts_if(leader, d_main, a_at + 32 + 8 * i, b_desc + (2 * (i & 1) + (i >> 1)) * kStep, idesc, 1u);
 #pragma unroll
-                                for (int i = 0; i < 4; ++i) umma_ts(d_main, a_at + 8 * i, b_desc + (2 * (i & 1) + (i >> 1)) * kStep, idesc, 1u);
+                                for (int i = 0; i < 4; ++i) umma_ts_if(leader, d_main, a_at + 8 * i, b_desc + (2 * (i & 1) + (i >> 1)) * kStep, idesc, 1u);
                             }
                             if (leader) {
                                 umma_commit(a_free + 8 * u);
@@ -240,7 +243,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
         const int quadrant = warp & 3, col0 = kMine * (warp >> 2), row = quadrant * 32 + lane;
         bool alive = true;
         int inv_group = -1;
-        uint32_t n = 0;
+        uint32_t n = 0, mins = 0;
         float* inv = reinterpret_cast<float*>(smem + (inv_at - b_ring));
         for (int r = 0; r < runs; ++r) {
             const StepRun run = split.run((int)blockIdx.x, r);
@@ -259,11 +262,16 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
                 if (alive) alive = mbar_wait(t_full + 8 * p, (n >> 1) & 1u, a.error_flag, 111, spin_limit);
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
-                    if (alive) alive = mbar_wait(d_full + 8 * u, n & 1u, a.error_flag, 112, spin_limit);
+                    if (q4k) {
+                        if (alive) alive = mbar_wait(min_full, mins & 1u, a.error_flag, 113, spin_limit);
+                        ++mins;
+                    } else {
+                        if (alive) alive = mbar_wait(d_full + 8 * u, n & 1u, a.error_flag, 112, spin_limit);
+                    }
                     tc_fence_after();
                     const float2 d = __half22float2(as_half2(lds32(scales + (2 * p + u) * (kUnitRows * 4) + row * 4)));
                     const uint32_t t_at = tmem + ((uint32_t)(quadrant * 32) << 16) + col0;
-                    if (q4k) {   // the minima sums first: the other unit's follow in the same columns
+                    if (q4k) {
 #pragma unroll
                         for (int c = 0; c < kMine; c += 8) {
                             float x[8];
@@ -273,6 +281,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
                             if (c == kMine - 8) { tc_fence_before(); __syncwarp(); if (lane == 0) mbar_arrive(min_free); }
                             fold8(&acc[u][c], x, -d.y, sx_at + c * 4);
                         }
+                        if (alive) alive = mbar_wait(d_full + 8 * u, n & 1u, a.error_flag, 112, spin_limit);
+                        tc_fence_after();
                     }
 #pragma unroll
                     for (int c = 0; c < kMine; c += 8) {
@@ -345,7 +355,7 @@ cudaError_t launch_gemm_pf(cudaStream_t stream, const StepGemm& a, int w_bytes, 
         configured[dev] = true;
     }
     w_bytes = (w_bytes + 127) & ~127;
-    const int fixed = 2 * kChunkBytes + 2 * kTailBytes + 2 * kA2Bytes + 4 * kUnitRows * 4 + kCols * 4 + 16 + 192 + 127;
+    const int fixed = 2 * kChunkBytes + 2 * kTailBytes + 2 * kA2Bytes + 4 * kUnitRows * 4 + kCols * 4 + 16 + 200 + 127;
     const int nw = std::min(kWStages, (kSmemMost - fixed) / w_bytes);
     if (nw < 2) return cudaErrorInvalidValue;
     const StepSplit split = step_split(a, a.partial == nullptr);

@@ -29,32 +29,38 @@ __device__ __forceinline__ float norm_factor(const float* ss, int tiles, float e
 
 // ---- consumers of partial sums, producers of operands -----------------------------------------------------------
 
-// Sum of the parts of outputs n .. n + 3 (inside segment `seg`) of member m, in worker order.
-__device__ __forceinline__ float4 part_sum(const StepFinish& a, int seg, int m, int n) {
+// The parts of outputs n .. n + 3 (inside segment `seg`) of member m: where the first lies, and how many there are.
+struct Parts { const float* at; int count; };
+__device__ __forceinline__ Parts parts_of(const StepFinish& a, int seg, int m, int n) {
     const int unit = a.unit0[seg] + (n >> a.split.unit_shift), item = unit * a.split.groups + m / a.split.group_members;
-    const int parts = a.split.parts(item);
-    const float* p = a.partial + (size_t)m * a.total_n + a.n_offset[seg] + n;
+    return Parts{a.partial + (size_t)m * a.total_n + a.n_offset[seg] + n, a.split.parts(item)};
+}
+// Their sum in worker order, `s` holding the first, BATCH at a time in flight.  Prefill-sized launches have one or two parts
+// and want threads (two in flight: 40 registers, SwiGLU of 2,048 x 12,288 in 124 us; eight: 199 us), small ones up to a
+// dozen and want the round trips back (eight in flight: 3.5 us against 5.4).
+template <int BATCH>
+__device__ __forceinline__ float4 add_parts(const StepFinish& a, const Parts& p, float4 s) {
     const size_t stride = (size_t)a.members * a.total_n;
-    float4 v[8];
+    for (int i = 1; i < p.count; i += BATCH) {
+        float4 v[BATCH];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = i < parts ? *reinterpret_cast<const float4*>(p + i * stride) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    float4 s = v[0];
+        for (int j = 0; j < BATCH; ++j) v[j] = i + j < p.count ? *reinterpret_cast<const float4*>(p.at + (i + j) * stride) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
-    for (int i = 1; i < 8; ++i) {
-        if (i < parts) { s.x += v[i].x; s.y += v[i].y; s.z += v[i].z; s.w += v[i].w; }
-    }
-    for (int i = 8; i < parts; ++i) {
-        const float4 w = *reinterpret_cast<const float4*>(p + i * stride);
-        s.x += w.x; s.y += w.y; s.z += w.z; s.w += w.w;
+        for (int j = 0; j < BATCH; ++j) {
+            if (i + j < p.count) { s.x += v[j].x; s.y += v[j].y; s.z += v[j].z; s.w += v[j].w; }
+        }
     }
     return s;
 }
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+// 2^k, k in [-126, 127]
+__device__ __forceinline__ float power2(int k) { return __int_as_float((k + 127) << 23); }
 
 // One block: a k tile (256 values of the row) of eight members, 64 threads each, four neighbouring values per thread:
 // lane t of fragment step s holds inputs 16 s + 4 t .. + 3, so a thread writes its member's 16 bytes of the step.
 // MODE: where the values come from (StepFinishMode).
-template <int MODE>
-__global__ void __launch_bounds__(512) step_finish_kernel(const StepFinish a) {
+template <int MODE, int BATCH>
+__global__ void __launch_bounds__(512, BATCH > 2 ? 1 : 3) step_finish_kernel(const StepFinish a) {
     __shared__ float red[16], red_sq[16];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -67,12 +73,15 @@ __global__ void __launch_bounds__(512) step_finish_kernel(const StepFinish a) {
             v = *reinterpret_cast<const float4*>(a.x + (size_t)(a.index ? a.index[m] : m) * width + n);
         } else if (MODE == kFinishResidual) {
             float4* h = reinterpret_cast<float4*>(a.y[0] + (size_t)m * width + n);
-            const float4 before = *h, s = part_sum(a, 0, m, n);
+            const Parts p = parts_of(a, 0, m, n);
+            const float4 before = *h, first = load4(p.at), s = add_parts<BATCH>(a, p, first);
             v = make_float4(before.x + s.x, before.y + s.y, before.z + s.z, before.w + s.w);
             *h = v;
         } else {
+            const Parts pg = parts_of(a, 0, m, n), pu = parts_of(a, 1, m, n);
+            const float4 first_g = load4(pg.at), first_u = load4(pu.at);
             const float inv = a.ss != nullptr ? norm_factor(a.ss + (size_t)m * a.split.k_tiles, a.split.k_tiles, a.eps, lane) : 1.0f;
-            const float4 gt = part_sum(a, 0, m, n), up = part_sum(a, 1, m, n);
+            const float4 gt = add_parts<BATCH>(a, pg, first_g), up = add_parts<BATCH>(a, pu, first_u);
             auto act = [&](float x, float u) { x *= inv; return x / (1.0f + expf(-x)) * (u * inv); };
             v = make_float4(act(gt.x, up.x), act(gt.y, up.y), act(gt.z, up.z), act(gt.w, up.w));
         }
@@ -93,10 +102,9 @@ __global__ void __launch_bounds__(512) step_finish_kernel(const StepFinish a) {
     __syncthreads();
     top = fmaxf(red[2 * g], red[2 * g + 1]);
     // a power of two that brings the largest value into [512, 1024): sums of 32 such values still fit binary16
-    int e = 0;
-    if (top > 0.0f && isfinite(top)) frexpf(top, &e);
-    e = max(-126, min(126, 10 - e));
-    const float scale = ldexpf(1.0f, e);
+    const int biased = (int)(__float_as_uint(top) >> 23);   // top is not negative
+    const int e = biased == 255 ? 10 : max(-126, min(126, 136 - biased));
+    const float scale = power2(e);
     if (i == 0 && m < a.members && a.out.ss != nullptr) a.out.ss[(size_t)m * k_tiles + kt] = red_sq[2 * g] + red_sq[2 * g + 1];
     const float s4[4] = {v.x * scale, v.y * scale, v.z * scale, v.w * scale};
     __half hi[4], lo[4];
@@ -110,15 +118,25 @@ __global__ void __launch_bounds__(512) step_finish_kernel(const StepFinish a) {
     const int group = blockIdx.y / a.out.ng, ng = blockIdx.y - group * a.out.ng;
     auto pack = [](__half x, __half y) { const __half2 p = __halves2half2(x, y); return *reinterpret_cast<const uint32_t*>(&p); };
     const int s = i >> 2, t = i & 3;
-    const float inv_scale = ldexpf(1.0f, -e);
+    const float inv_scale = power2(-e);
     if (a.out.form != kFragmentForm) {
         const int mp = 8 * a.out.ng, sum_cols = max(16, (mp + 15) / 16 * 16), col = ng * 8 + g;
         unsigned char* blk = a.out.blocks + ((size_t)group * k_tiles + kt) * (1028 * mp + 32 * sum_cols);
-        uint32_t* at = reinterpret_cast<uint32_t*>(blk + ((size_t)(2 * s) * 2 * mp + col) * 16 + 4 * t);
-        at[0] = pack(hi[0], hi[2]);
-        at[8 * mp] = pack(hi[1], hi[3]);          // the next 8-input block: 2 mp columns of 16 bytes on
-        at[4 * mp] = pack(lo[0], lo[2]);          // the lo columns
-        at[12 * mp] = pack(lo[1], lo[3]);
+        // The eight members' 16-byte pieces of an 8-input block lie side by side: through shared memory, so that a warp's
+        // stores are whole 128-byte lines.  staged[8-input block][hi, lo][member ^ step % 8]: conflict-free both ways.
+        __shared__ uint4 staged[32][2][8];
+        {
+            uint32_t* at = reinterpret_cast<uint32_t*>(&staged[2 * s][0][g ^ (s & 7)]) + t;
+            at[0] = pack(hi[0], hi[2]);
+            at[32] = pack(lo[0], lo[2]);
+            at[64] = pack(hi[1], hi[3]);          // the next 8-input block
+            at[96] = pack(lo[1], lo[3]);
+        }
+        __syncthreads();
+        {
+            const int kb = tid >> 4, half = (tid >> 3) & 1, member = tid & 7;
+            *reinterpret_cast<uint4*>(blk + ((size_t)kb * 2 * mp + half * mp + ng * 8 + member) * 16) = staged[kb][half][member ^ ((kb >> 1) & 7)];
+        }
 #pragma unroll
         for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
         if ((i & 7) == 0) {
@@ -160,7 +178,8 @@ __global__ void __launch_bounds__(256) step_store_kernel(const StepFinish a) {
     int n = 4 * (int)(blockIdx.x * blockDim.x + threadIdx.x), seg = 0;
     while (seg < a.n_segments && n >= a.n[seg]) { n -= a.n[seg]; ++seg; }
     if (seg >= a.n_segments) return;
-    const float4 s = part_sum(a, seg, m, n);
+    const Parts p = parts_of(a, seg, m, n);
+    const float4 s = add_parts<4>(a, p, load4(p.at));
     *reinterpret_cast<float4*>(a.y[seg] + (size_t)m * a.n[seg] + n) = make_float4(s.x * inv, s.y * inv, s.z * inv, s.w * inv);
 }
 
@@ -250,6 +269,7 @@ StepSplit step_split(const StepGemm& a, bool whole_items) {
     s.groups = shape.groups;
     s.group_members = shape.ng * 8;
     for (int i = 0; i < a.n_segments; ++i) s.items += (a.seg[i].row_tiles + tiles - 1) / tiles * shape.groups;
+    if ((unsigned long long)s.items * s.k_tiles * (device_sms() * kFragTeams) >> 32) whole_items = true;
     s.whole = whole_items ? 1 : 0;
     s.workers = std::min(device_sms() * (a.form == kFragmentForm ? kFragTeams : 1), whole_items ? s.items : s.items * s.k_tiles);
     s.rounds = a.form == kWideForm ? s.items / s.workers : 0;
@@ -313,10 +333,14 @@ cudaError_t launch_step_finish(cudaStream_t stream, int mode, const StepGemm* ge
     const StepShape shape = step_shape(a.members, a.out.form);
     a.out.ng = shape.ng;
     const dim3 grid((unsigned)(width / kTileCols), (unsigned)(shape.groups * shape.ng));
+    // as many parts as an evenly dealt item can have
+    const bool deep = mode != kFinishRows && !a.split.whole && a.split.workers > 2 * a.split.even();
     switch (mode) {
-        case kFinishRows: return launch_pdl(step_finish_kernel<kFinishRows>, grid, 512, 0, stream, programmatic, a);
-        case kFinishResidual: return launch_pdl(step_finish_kernel<kFinishResidual>, grid, 512, 0, stream, programmatic, a);
-        case kFinishSwiGLU: return launch_pdl(step_finish_kernel<kFinishSwiGLU>, grid, 512, 0, stream, programmatic, a);
+        case kFinishRows: return launch_pdl(step_finish_kernel<kFinishRows, 2>, grid, 512, 0, stream, programmatic, a);
+        case kFinishResidual:
+            return launch_pdl(deep ? step_finish_kernel<kFinishResidual, 7> : step_finish_kernel<kFinishResidual, 2>, grid, 512, 0, stream, programmatic, a);
+        case kFinishSwiGLU:
+            return launch_pdl(deep ? step_finish_kernel<kFinishSwiGLU, 7> : step_finish_kernel<kFinishSwiGLU, 2>, grid, 512, 0, stream, programmatic, a);
         default: return cudaErrorInvalidValue;
     }
 }
