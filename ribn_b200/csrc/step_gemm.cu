@@ -333,8 +333,8 @@ cudaError_t launch_step_finish(cudaStream_t stream, int mode, const StepGemm* ge
     const StepShape shape = step_shape(a.members, a.out.form);
     a.out.ng = shape.ng;
     const dim3 grid((unsigned)(width / kTileCols), (unsigned)(shape.groups * shape.ng));
-    // as many parts as an evenly dealt item can have
-    const bool deep = mode != kFinishRows && !a.split.whole && a.split.workers > 2 * a.split.even();
+    // small launches, all of whose items are cut into several parts
+    const bool deep = mode != kFinishRows && !a.split.whole && a.split.rounds == 0 && a.split.workers > 2 * a.split.even();
     switch (mode) {
         case kFinishRows: return launch_pdl(step_finish_kernel<kFinishRows, 2>, grid, 512, 0, stream, programmatic, a);
         case kFinishResidual:
