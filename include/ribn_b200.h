@@ -341,8 +341,8 @@ RIBN_B200_API int ribn_b200_op_embedding(int32_t device, int32_t ggml_type, cons
  * decode-and-split form for Q8_0), 4 = the decode-and-split form for every type,
  * 5 = the K-quant form over operands converted once (what RIBN_B200_FLAG_OPERAND_CACHE
  * runs; Q4_K / Q6_K only; bit-identical to variant 3), 6 = the fragment-order mma.sync kernel (steps of a
- * few rows with Q8_0 matrices, and every batch of them), 7 = the tcgen05 kernel that converts weights into
- * tensor memory (steps of a few rows; Q4_K / Q6_K only), 8 = its wide form for prefill-sized steps. */
+ * few rows), 7 = the tcgen05 kernel that converts weights into tensor memory (steps of up to 64 rows), 8 = its wide
+ * form for prefill-sized steps. */
 RIBN_B200_API int ribn_b200_op_gemv(int32_t device, int32_t ggml_type, const void* weights,
                                     int64_t rows, int64_t cols, const float* x, int32_t members,
                                     float* y, int32_t variant);

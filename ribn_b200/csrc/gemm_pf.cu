@@ -1,4 +1,4 @@
-// Dequant-GEMM over Q4_K / Q6_K weights for prefill-sized steps: 256 weight rows x 128 activation rows per work item, the
+// Dequant-GEMM for prefill-sized steps: 256 weight rows x 128 activation rows per work item, the
 // converted weights in tensor memory (the arithmetic of gemm_ta.cu).
 //
 // What bounds it.  An activation is four bytes (a binary16 hi + lo pair) per input, so a 128-row unit that multiplies T
@@ -7,7 +7,7 @@
 // clocks of products per k tile), and the chunk meets the packed weights' conversion once per 128 activation rows.
 //
 // Tensor memory: main sums of unit u at columns 128 u (one accumulator for hi and lo parts, lo first), minima sums at 256
-// (shared by the units in turn), A stages at 384 + 64 u: 128 inputs of Q4_K's one plane, 64 inputs of Q6_K's two.  The
+// (shared by the units in turn), A stages at 384 + 64 u: 128 inputs of Q4_K's one plane, 64 inputs of the others' two.  The
 // units alternate stage by stage, so a unit's conversion hides under the other unit's products, and so does the fold of
 // its sums once per k tile.  The F32 sums of a work item (2 x 128 x 128) live in the registers of sixteen warps.
 // Roles of the 28 warps: 0..15 fold and store (one row of each unit and 32 columns per thread), 16..23 convert (two row
@@ -220,8 +220,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
                         if (type == kQ4_K) {
                             convert_q4k(tile, 2 * h + part, a_at + 32 * part, sc, a2_buf + u * kA2Bytes, 32 * quadrant, lane);
                             if (h == 0) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the minima operand
-                        } else {
+                        } else if (type == kQ6_K) {
                             convert_q6k(tile, h >> 1, part + 2 * (h & 1), a_at + 16 * part, 32, sc, 32 * quadrant, lane);
+                        } else {
+                            convert_q8_0(tile, h >> 1, part + 2 * (h & 1), a_at + 16 * part, 32, sc, 32 * quadrant, lane);
                         }
                         tmem_wait_st();
                         tc_fence_before();

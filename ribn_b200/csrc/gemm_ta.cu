@@ -1,10 +1,10 @@
-// Dequant-GEMM over Q4_K / Q6_K weights with the converted weights in TENSOR MEMORY (tcgen05, A operand in TMEM).
+// Dequant-GEMM with the converted weights in TENSOR MEMORY (tcgen05, A operand in TMEM).
 //
 //   y[m][n] = sum_k deq(W[n][k]) x[m][k]
 //
 // The tensor core multiplies the blocks' exact integers, as binary16, by the activations' binary16 hi + lo pairs:
 // sc q (at most 945) for Q4_K, sc (q - 32) (up to 4096 in magnitude, as p1 = its value rounded to binary16 and the exact
-// rest p2) for Q6_K.  Per 256 inputs the F32 sums leave tensor memory and are folded into F32 registers with the row's
+// rest p2) for Q6_K; d q (d scaled by a power of two per row and 256 inputs, again in two parts) for Q8_0.  Per 256 inputs the F32 sums leave tensor memory and are folded into F32 registers with the row's
 // super-block scale d and the activations' power-of-two tile scale, round-to-nearest, in order; the Q4_K minima are one
 // more K = 16 MMA per 256 inputs against the activations' group sums.
 //
@@ -23,7 +23,7 @@
 // a k tile has ONE commit (two for Q6_K, whose A operand fills two stages), which frees its A stage and starts its fold; one
 // arrival per fold warp frees the sums and the activations' slot.
 // Tensor memory: main sums of k tile parity p at columns 64 p, minima sums at 128 + 64 p, A stages at 256 + 128 s (256
-// inputs of Q4_K's one plane, 128 inputs of Q6_K's two).  Slots (unit, row group, k tile) are dealt to the CTAs evenly
+// inputs of Q4_K's one plane, 128 inputs of the others' two).  Slots (unit, row group, k tile) are dealt to the CTAs evenly
 // when another kernel finishes the sums, in whole items otherwise (StepSplit).  Every wait is bounded.
 #include <cuda_fp16.h>
 
@@ -233,7 +233,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ta_kernel(const StepGemm a, 
                         for (int c = 2 * part; c < 2 * part + 2; ++c) convert_q4k(tile, c, a_at + 32 * c, scales, a2_buf + st * kA2Bytes, 32 * quadrant, lane);
                     } else {
 #pragma unroll 1
-                        for (int hi = 0; hi < 2; ++hi) convert_q6k(tile, half, part + 2 * hi, a_at + 16 * (part + 2 * hi), 64, scales, 32 * quadrant, lane);
+                        for (int hi = 0; hi < 2; ++hi) {
+                            if (type == kQ6_K) convert_q6k(tile, half, part + 2 * hi, a_at + 16 * (part + 2 * hi), 64, scales, 32 * quadrant, lane);
+                            else convert_q8_0(tile, half, part + 2 * hi, a_at + 16 * (part + 2 * hi), 64, scales, 32 * quadrant, lane);
+                        }
                     }
                     tmem_wait_st();
                     tc_fence_before();

@@ -327,7 +327,6 @@ int ribn_b200_op_gemv(int32_t device, int32_t type, const void* weights, int64_t
         } else if (variant >= 6 && variant <= 8) {
             // the kernels of a step of a few rows, in fragment order or with tensor-memory conversion: partial sums finished by a second kernel where a step of a few rows does so
             const int form = variant == 8 ? kWideForm : variant == 7 ? kColumnForm : kFragmentForm;
-            if (variant != 6 && type == kQ8_0) return op_fail("gemv: the tensor-memory conversion kernels take Q4_K and Q6_K matrices only", cudaSuccess);
             alignas(64) unsigned char map[kTileMapBytes];
             OP_TRY(make_tile_map(type, d_w, rows, cols, map));
             StepFinish f{};

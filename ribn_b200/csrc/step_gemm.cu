@@ -294,7 +294,7 @@ cudaError_t launch_step_gemm(cudaStream_t stream, const StepGemm& args, bool pro
     a.total_n = 0;
     for (int i = 0; i < a.n_segments; ++i) {
         const int b = packed_tile_bytes(a.seg[i].type);
-        if (b == 0 || a.seg[i].map == nullptr || (a.form != kFragmentForm && a.seg[i].type == kQ8_0)) return cudaErrorInvalidValue;
+        if (b == 0 || a.seg[i].map == nullptr) return cudaErrorInvalidValue;
         w_bytes = std::max(w_bytes, kUnitTiles * b);
         a.n_offset[i] = a.total_n;
         a.total_n += a.seg[i].n;

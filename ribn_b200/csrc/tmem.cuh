@@ -1,5 +1,5 @@
 // What the tcgen05 GEMMs with a tensor-memory A operand share: barriers, copies, tensor-memory accesses, and the
-// conversion of packed Q4_K / Q6_K tiles to operand columns.
+// conversion of packed Q4_K / Q6_K / Q8_0 tiles to operand columns.
 #pragma once
 #include <cuda_fp16.h>
 
@@ -224,6 +224,47 @@ __device__ __forceinline__ void convert_q6k(uint32_t tile, int cc, int c, uint32
                 for (int i = 0; i < 2; ++i) {
                     const uint32_t x = and_or(i ? low >> 8 : low, lm, and_or(i ? down : up, hm, 0x64006400u));
                     const __half2 v = __hfma2(as_half2(x), mul, bias), p = __hmul2(sc, v);
+                    p1[(2 * vv + i) * 2 + h] = as_bits(p);
+                    p2[(2 * vv + i) * 2 + h] = as_bits(__hfma2(sc, v, __hneg2(p)));
+                }
+            }
+        }
+        tmem_st_x4(a_tmem + ((uint32_t)(16 * r) << 16), p1);
+        tmem_st_x4(a_tmem + ((uint32_t)(16 * r) << 16) + plane, p2);
+    }
+}
+
+// The same quarter of a Q8_0 half: p = d' q with d' = d 2^s, s the power of two that brings the largest of the row's eight d
+// of this tile into [128, 256) (so p stays below 65,504, and what binary16 cannot hold of the rest lies 2^-39 below the
+// largest p); the row's scale for the fold is 2^-s.
+__device__ __forceinline__ void convert_q8_0(uint32_t tile, int cc, int c, uint32_t a_tmem, uint32_t plane, uint32_t scales, int row0, int lane) {
+    const int g = lane >> 2, t = lane & 3, kh = c & 1, hi = c >> 1;
+    const __half2 bias = __float2half2_rn(1152.0f);   // 1024 + 128
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const uint32_t at = tile + r * 4352;
+        uint32_t p1[8], p2[8];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int row = g + 8 * h;
+            const uint4 d8 = lds128(at + 4096 + row * 16);
+            uint32_t top = __vmaxu2(__vmaxu2(d8.x & 0x7FFF7FFFu, d8.y & 0x7FFF7FFFu), __vmaxu2(d8.z & 0x7FFF7FFFu, d8.w & 0x7FFF7FFFu));
+            top = max(top & 0xffffu, top >> 16);
+            const int s = 22 - (int)(top >> 10);
+            if (cc == 0 && c == 0 && t == 0) {
+                const uint32_t back = s <= 14 ? (uint32_t)(15 - s) << 10 : 1u << (24 - s);   // 2^-s as binary16
+                asm volatile("st.shared.u32 [%0], %1;" ::"r"(scales + (row0 + r * 16 + row) * 4), "r"(back) : "memory");
+            }
+            const uint32_t two = cc == 0 ? (hi ? d8.y : d8.x) : (hi ? d8.w : d8.z);          // d of blocks 4 cc + 2 hi, + 1
+            const float up = __int_as_float((s + 127) << 23);
+            const float2 df = __half22float2(as_half2(two));
+#pragma unroll
+            for (int vv = 0; vv < 2; ++vv) {
+                const __half2 sc = __float2half2_rn((vv ? df.y : df.x) * up);
+                const uint32_t word = lds32(at + (cc * 4 + 2 * hi + vv) * 512 + lane * 16 + 8 * h + 4 * kh);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const __half2 v = __hsub2(as_half2(and_or(i ? word >> 8 : word, 0x00FF00FFu, 0x64006400u)), bias), p = __hmul2(sc, v);
                     p1[(2 * vv + i) * 2 + h] = as_bits(p);
                     p2[(2 * vv + i) * 2 + h] = as_bits(__hfma2(sc, v, __hneg2(p)));
                 }

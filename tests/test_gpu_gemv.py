@@ -242,7 +242,7 @@ def test_operand_cache_refuses_other_types(ops):
         ops.gemv(H.Q8_0, enc, 128, 256, np.ones((4, 256), np.float32), variant=5)
 
 
-@pytest.mark.parametrize("kind,variant", [(H.Q8_0, 6), (H.Q4_K, 6), (H.Q6_K, 6), (H.Q4_K, 7), (H.Q6_K, 7), (H.Q4_K, 8), (H.Q6_K, 8)])
+@pytest.mark.parametrize("kind,variant", [(H.Q8_0, 6), (H.Q4_K, 6), (H.Q6_K, 6), (H.Q4_K, 7), (H.Q6_K, 7), (H.Q4_K, 8), (H.Q6_K, 8), (H.Q8_0, 7), (H.Q8_0, 8)])
 @pytest.mark.parametrize("rows,cols,members", [(4, 256, 1), (40, 512, 3), (132, 768, 8), (272, 1024, 9), (128, 2048, 32), (260, 1024, 33), (384, 512, 24),
                                                (136, 1024, 64), (30, 512, 5), (144, 768, 70), (520, 768, 200), (257, 512, 129), (19200, 256, 300)])
 def test_step_gemm_tile_and_group_edges(ops, kind, variant, rows, cols, members):
@@ -260,7 +260,7 @@ def test_step_gemm_tile_and_group_edges(ops, kind, variant, rows, cols, members)
         assert np.array_equal(ops.gemv(kind, enc, rows, cols, xs[:1], variant=variant)[0].view(np.uint32), got[0].view(np.uint32))
 
 
-@pytest.mark.parametrize("kind,variant", [(H.Q8_0, 6), (H.Q4_K, 6), (H.Q6_K, 6), (H.Q4_K, 7), (H.Q6_K, 7), (H.Q4_K, 8), (H.Q6_K, 8)])
+@pytest.mark.parametrize("kind,variant", [(H.Q8_0, 6), (H.Q4_K, 6), (H.Q6_K, 6), (H.Q4_K, 7), (H.Q6_K, 7), (H.Q4_K, 8), (H.Q6_K, 8), (H.Q8_0, 7), (H.Q8_0, 8)])
 def test_step_gemm_random_bytes(ops, kind, variant):
     rng = np.random.default_rng(kind + 31)
     elems, size = H.BLOCK[kind]
