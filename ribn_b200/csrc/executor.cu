@@ -452,12 +452,13 @@ cudaError_t run_layers_decode(ribn_b200_executor* ex, const StepPlan& plan, int&
 // ---- three rows and more: one GEMM launch per projection over the whole step, its partial sums finished by the kernel
 // that makes the next projection's operand -----------------------------------------------------------------------------
 // The block form of a step's activations, which selects its GEMM kernel.  A projection of the 8B model (gate | up, 57 MB)
-// takes 19 / 27 / 38 / 55 / 99 us in fragment order at 8 / 16 / 24 / 32 / 64 rows, 25 / 26 / 29 / 30 / 34 us with
-// tensor-memory conversion (61 us for two groups of 64) and 48 us in the wide form at 65 to 128 rows: the lines lie at 16
-// and at 64 rows.  Q8_0 matrices are taken in fragment order only.
-int step_form(const ribn_b200_executor* ex, int members) {
-    if (!ex->kquant || members <= 16) return kFragmentForm;
-    return members <= 64 ? kColumnForm : kWideForm;
+// takes 19 / 27 / 38 / 55 / 99 us in fragment order at 8 / 16 / 24 / 32 / 64 rows, 23 / 24 / 26 / 27 / 31 us with
+// tensor-memory conversion (58 us for two groups of 64) and 47 us in the wide form at 65 to 128 rows: the lines lie at 16
+// (at 16 the smaller projections decide) and at 64 rows.  Q8_0 (0.6B, a layer's four projections): 21 / 33 us in fragment
+// order at 16 / 32 rows against 20 / 24 us; 43 us at 128 rows in two groups of 64 against 47 us in the wide form, 98 us
+// against 167 us at 777.
+int step_form(int members) {
+    return members <= 16 ? kFragmentForm : members <= 64 ? kColumnForm : kWideForm;
 }
 
 // Tensor-parallel executors reduce between projections (run_layers_batch), and NO_TCGEN05 asks for the integer kernels.
@@ -470,7 +471,7 @@ GemvSegment step_segment(const Tensor& t, float* y) {
 }
 StepGemm step_base(ribn_b200_executor* ex, int k, int members, bool normed) {
     StepGemm a{};
-    a.form = step_form(ex, members);
+    a.form = step_form(members);
     a.k = k;
     a.members = members;
     a.blocks = ex->op_step.blocks;
@@ -516,13 +517,13 @@ cudaError_t run_layers_step(ribn_b200_executor* ex, const StepPlan& plan, int& l
     const int T = plan.n_tokens, QD = c.q_heads * c.head_dim;
     const bool pdl = !(c.flags & RIBN_B200_FLAG_NO_GRAPH);
     StepOperand normed = ex->op_step, plain = ex->op_step;   // operands a norm's consumer reads / no norm follows
-    normed.form = plain.form = step_form(ex, T);
+    normed.form = plain.form = step_form(T);
     plain.ss = nullptr;
     auto rows = [&](const float* x, const int32_t* index, const float* norm, int members, int k) -> cudaError_t {
         StepFinish f{};
         f.x = x; f.index = index; f.norm_weight = norm; f.members = members;
         f.out = norm != nullptr ? normed : plain;
-        f.out.form = step_form(ex, members);
+        f.out.form = step_form(members);
         return launch_step_finish(s, kFinishRows, nullptr, f, k, pdl);
     };
     STEP_TRY(rows(ex->hidden, nullptr, (const float*)ex->lt(0, kAttnNorm).raw, T, c.hidden));
@@ -1055,8 +1056,6 @@ int ribn_b200_finalize(ribn_b200_executor* ex) {
                 CU_TRY(ex, launch_tc_cache(ex->stream, t->type, p.data, t->rows, t->cols, t->op_a, t->op_meta));
             }
         }
-        ex->kquant = true;
-        for (Tensor* t : mats) ex->kquant = ex->kquant && (t->type == kQ4_K || t->type == kQ6_K);
         CU_TRY(ex, cudaMemcpy(d_maps, maps.data(), maps.size(), cudaMemcpyHostToDevice));
         CU_TRY(ex, cudaStreamSynchronize(ex->stream));
     }
@@ -1147,8 +1146,8 @@ int ribn_b200_finalize(ribn_b200_executor* ex) {
             if (kmax % 256 == 0) {
                 const int most = (int)std::max(T, S);
                 size_t step_bytes = 0;
-                for (int m = 1; m <= most; ++m) step_bytes = std::max(step_bytes, step_operand_bytes(m, kmax, step_form(ex, m)));
-                if (!ex->kquant) step_bytes = std::max(step_bytes, step_operand_bytes(most, kmax, kFragmentForm));
+                for (int m = 1; m <= most; ++m) step_bytes = std::max(step_bytes, step_operand_bytes(m, kmax, step_form(m)));
+                if (!step_gemms(ex)) step_bytes = std::max(step_bytes, step_operand_bytes(most, kmax, kFragmentForm));
                 CU_TRY(ex, dev_alloc(ex, &ex->op_step.blocks, step_bytes));
                 CU_TRY(ex, dev_alloc(ex, &ex->op_step.ss, (size_t)most * (size_t)(kmax / kTileCols)));
                 if (step_gemms(ex)) {

@@ -122,7 +122,6 @@ struct ribn_b200_executor {
     ribn::BatchOperand op_batch;  // batch form, refilled before every batched projection
     ribn::TcOperand op_tc;        // tensor-memory form (the same, for the tcgen05 kernel)
     ribn::StepOperand op_step;    // operand of the step GEMMs (batches of a few rows; any batch of a Q8_0 model)
-    bool kquant = false;          // every packed matrix is Q4_K or Q6_K
     float* tc_partial = nullptr;  // split-K sums of the batched kernels
     size_t tc_partial_floats = 0;
     // Captured decode steps, keyed by (tokens, sampling rows, attention span bucket).

@@ -53,6 +53,7 @@ __device__ __forceinline__ void fold8(float* acc, const float (&x)[8], float f, 
     }
 }
 
+template <int TYPE>
 __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, const StepSplit split, const int w_bytes, const int nw) {
     extern __shared__ __align__(128) unsigned char smem[];
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
@@ -96,7 +97,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
                 const StepRun run = split.run((int)blockIdx.x, r);
                 const UnitAt at = unit_at(a, run.item / groups, 2 * kUnitTiles);
                 const GemvSegment& seg = a.seg[at.seg];
-                const uint32_t bytes = kUnitTiles * (uint32_t)packed_tile_bytes(seg.type);
+                const uint32_t bytes = kUnitTiles * (uint32_t)packed_tile_bytes(type_of<TYPE>(seg));
                 for (int kb = run.begin; kb < run.end && alive; ++kb) {
                     for (int u = 0; u < 2 && alive; ++u) {
                         if (filled == nw) alive = mbar_wait(w_empty + 8 * ws, parity, a.error_flag, 101, spin_limit);
@@ -143,7 +144,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
             for (int r = 0; r < runs; ++r) {
                 const StepRun run = split.run((int)blockIdx.x, r);
                 // broadcast, so that the loop below stays on uniform registers
-                const bool q4k = __shfl_sync(0xffffffffu, a.seg[unit_at(a, run.item / groups, 2 * kUnitTiles).seg].type, 0) == kQ4_K;
+                const bool q4k = (TYPE >= 0 ? TYPE : __shfl_sync(0xffffffffu, a.seg[unit_at(a, run.item / groups, 2 * kUnitTiles).seg].type, 0)) == kQ4_K;
                 const int stages = q4k ? 2 : 4, stop = __shfl_sync(0xffffffffu, (int)n + run.end - run.begin, 0);
                 for (; (int)n < stop; ++n) {
 #pragma unroll 1
@@ -202,7 +203,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
         uint32_t uses = 0, n = 0, ws0 = 0, wp0 = 0;   // ws0 / wp0: ring place and phase of the k tile's first unit
         for (int r = 0; r < runs; ++r) {
             const StepRun run = split.run((int)blockIdx.x, r);
-            const int type = a.seg[unit_at(a, run.item / groups, 2 * kUnitTiles).seg].type;
+            const int type = type_of<TYPE>(a.seg[unit_at(a, run.item / groups, 2 * kUnitTiles).seg]);
             const int stages = type == kQ4_K ? 2 : 4;
             const uint32_t row_bytes = 2 * quadrant * packed_tile_bytes(type);
             for (int kb = run.begin; kb < run.end; ++kb, ++n) {
@@ -220,7 +221,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
                         if (type == kQ4_K) {
                             convert_q4k(tile, 2 * h + part, a_at + 32 * part, sc, a2_buf + u * kA2Bytes, 32 * quadrant, lane);
                             if (h == 0) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the minima operand
-                        } else if (type == kQ6_K) {
+                        } else if (TYPE == kKQuants || type == kQ6_K) {
                             convert_q6k(tile, h >> 1, part + 2 * (h & 1), a_at + 16 * part, 32, sc, 32 * quadrant, lane);
                         } else {
                             convert_q8_0(tile, h >> 1, part + 2 * (h & 1), a_at + 16 * part, 32, sc, 32 * quadrant, lane);
@@ -252,7 +253,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
             const int group = run.item % groups;
             const UnitAt at = unit_at(a, run.item / groups, 2 * kUnitTiles);
             const GemvSegment& seg = a.seg[at.seg];
-            const bool q4k = seg.type == kQ4_K;
+            const bool q4k = type_of<TYPE>(seg) == kQ4_K;
             float acc[2][kMine];
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
@@ -343,16 +344,15 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
     }
 }
 
-}  // namespace
-
-cudaError_t launch_gemm_pf(cudaStream_t stream, const StepGemm& a, int w_bytes, bool programmatic) {
+template <int TYPE>
+cudaError_t launch_typed(cudaStream_t stream, const StepGemm& a, int w_bytes, bool programmatic) {
     static bool configured[kMaxDevices] = {false};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
     if (!configured[dev]) {
-        e = cudaFuncSetAttribute(gemm_pf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost);
+        e = cudaFuncSetAttribute(gemm_pf_kernel<TYPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost);
         if (e != cudaSuccess) return e;
         configured[dev] = true;
     }
@@ -371,7 +371,19 @@ cudaError_t launch_gemm_pf(cudaStream_t stream, const StepGemm& a, int w_bytes, 
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = programmatic ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, gemm_pf_kernel, a, split, w_bytes, nw);
+    return cudaLaunchKernelEx(&cfg, gemm_pf_kernel<TYPE>, a, split, w_bytes, nw);
+}
+
+}  // namespace
+
+cudaError_t launch_gemm_pf(cudaStream_t stream, const StepGemm& a, int w_bytes, bool programmatic) {
+    switch (common_type(a)) {
+        case kQ6_K: return launch_typed<kQ6_K>(stream, a, w_bytes, programmatic);
+        case kQ8_0: return launch_typed<kQ8_0>(stream, a, w_bytes, programmatic);
+        case kQ4_K:   // compiled for Q4_K alone, the fold's registers spill (o_proj 105 -> 111 us at 2,048 rows)
+        case kKQuants: return launch_typed<kKQuants>(stream, a, w_bytes, programmatic);
+        default: return launch_typed<kAnyType>(stream, a, w_bytes, programmatic);
+    }
 }
 
 }  // namespace ribn

@@ -56,7 +56,7 @@ struct Cols {
 
 struct TaRings { int w_stages, b_stages, w_bytes; };
 
-template <int MP>
+template <int MP, int TYPE>
 __global__ void __launch_bounds__(kThreads, 1) gemm_ta_kernel(const StepGemm a, const StepSplit split, const TaRings rings) {
     using C = Cols<MP>;
     constexpr int kBBytes = (C::kBlock + 127) & ~127;
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ta_kernel(const StepGemm a, 
                 const int item = s / k_tiles, end = min(s1, (item + 1) * k_tiles);
                 const UnitAt at = unit_at(a, item / split.groups, kUnitTiles);
                 const GemvSegment& seg = a.seg[at.seg];
-                const uint32_t bytes = kUnitTiles * (uint32_t)packed_tile_bytes(seg.type);
+                const uint32_t bytes = kUnitTiles * (uint32_t)packed_tile_bytes(type_of<TYPE>(seg));
                 for (int kb = s - item * k_tiles; s < end; ++s, ++kb) {
                     if (filled == nw) alive = mbar_wait(w_empty + 8 * ws, parity, a.error_flag, 91, spin_limit);
                     else ++filled;
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ta_kernel(const StepGemm a, 
             uint32_t b_parity = 0, fold_parity = 0, a_count = 0, kt = 0, q6_count = 0;
             for (int s = s0; s < s1;) {
                 const int item = s / k_tiles, end = min(s1, (item + 1) * k_tiles);
-                const bool q4k = a.seg[unit_at(a, item / split.groups, kUnitTiles).seg].type == kQ4_K;
+                const bool q4k = type_of<TYPE>(a.seg[unit_at(a, item / split.groups, kUnitTiles).seg]) == kQ4_K;
                 for (; s < end; ++s, ++kt) {
                     const uint32_t p = kt & 1u, d_main = tmem + 64 * p, d_min = tmem + 128 + 64 * p;
                     if (kt >= 2) {   // the fold of k tile kt - 2 has left these sums
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ta_kernel(const StepGemm a, 
         };
         for (int s = s0; s < s1;) {
             const int item = s / k_tiles, end = min(s1, (item + 1) * k_tiles);
-            const int type = a.seg[unit_at(a, item / split.groups, kUnitTiles).seg].type;
+            const int type = type_of<TYPE>(a.seg[unit_at(a, item / split.groups, kUnitTiles).seg]);
             for (; s < end; ++s, ++kt) {
                 if (alive) alive = mbar_wait(w_full + 8 * ws, parity, a.error_flag, 96, spin_limit);
                 const uint32_t tile = w_ring + ws * rings.w_bytes + 2 * quadrant * packed_tile_bytes(type);
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ta_kernel(const StepGemm a, 
                     } else {
 #pragma unroll 1
                         for (int hi = 0; hi < 2; ++hi) {
-                            if (type == kQ6_K) convert_q6k(tile, half, part + 2 * hi, a_at + 16 * (part + 2 * hi), 64, scales, 32 * quadrant, lane);
+                            if (TYPE == kKQuants || type == kQ6_K) convert_q6k(tile, half, part + 2 * hi, a_at + 16 * (part + 2 * hi), 64, scales, 32 * quadrant, lane);
                             else convert_q8_0(tile, half, part + 2 * hi, a_at + 16 * (part + 2 * hi), 64, scales, 32 * quadrant, lane);
                         }
                     }
@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ta_kernel(const StepGemm a, 
             const int item = s / k_tiles, unit = item / split.groups, group = item - unit * split.groups;
             const UnitAt at = unit_at(a, unit, kUnitTiles);
             const GemvSegment& seg = a.seg[at.seg];
-            const bool q4k = seg.type == kQ4_K;
+            const bool q4k = type_of<TYPE>(seg) == kQ4_K;
             const int end = min(s1, (item + 1) * k_tiles);
             float acc[kChunks][8];
 #pragma unroll
@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ta_kernel(const StepGemm a, 
     }
 }
 
-template <int MP>
+template <int MP, int TYPE>
 cudaError_t launch_variant(cudaStream_t stream, const StepGemm& a, int w_bytes, bool programmatic) {
     static bool configured[kMaxDevices] = {false};
     int dev = 0;
@@ -368,7 +368,7 @@ cudaError_t launch_variant(cudaStream_t stream, const StepGemm& a, int w_bytes, 
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
     if (!configured[dev]) {
-        e = cudaFuncSetAttribute(gemm_ta_kernel<MP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget);
+        e = cudaFuncSetAttribute(gemm_ta_kernel<MP, TYPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget);
         if (e != cudaSuccess) return e;
         configured[dev] = true;
     }
@@ -389,19 +389,30 @@ cudaError_t launch_variant(cudaStream_t stream, const StepGemm& a, int w_bytes, 
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = programmatic ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, gemm_ta_kernel<MP>, a, split, rings);
+    return cudaLaunchKernelEx(&cfg, gemm_ta_kernel<MP, TYPE>, a, split, rings);
+}
+
+template <int TYPE>
+cudaError_t launch_typed(cudaStream_t stream, const StepGemm& a, int w_bytes, bool programmatic) {
+    switch (step_shape(a.members, kColumnForm).ng) {
+        case 1: return launch_variant<8, TYPE>(stream, a, w_bytes, programmatic);
+        case 2: return launch_variant<16, TYPE>(stream, a, w_bytes, programmatic);
+        case 3: return launch_variant<24, TYPE>(stream, a, w_bytes, programmatic);
+        case 4: return launch_variant<32, TYPE>(stream, a, w_bytes, programmatic);
+        case 6: return launch_variant<48, TYPE>(stream, a, w_bytes, programmatic);
+        default: return launch_variant<64, TYPE>(stream, a, w_bytes, programmatic);
+    }
 }
 
 }  // namespace
 
 cudaError_t launch_gemm_ta(cudaStream_t stream, const StepGemm& a, int w_bytes, bool programmatic) {
-    switch (step_shape(a.members, kColumnForm).ng) {
-        case 1: return launch_variant<8>(stream, a, w_bytes, programmatic);
-        case 2: return launch_variant<16>(stream, a, w_bytes, programmatic);
-        case 3: return launch_variant<24>(stream, a, w_bytes, programmatic);
-        case 4: return launch_variant<32>(stream, a, w_bytes, programmatic);
-        case 6: return launch_variant<48>(stream, a, w_bytes, programmatic);
-        default: return launch_variant<64>(stream, a, w_bytes, programmatic);
+    switch (common_type(a)) {
+        case kQ4_K: return launch_typed<kQ4_K>(stream, a, w_bytes, programmatic);
+        case kQ6_K: return launch_typed<kQ6_K>(stream, a, w_bytes, programmatic);
+        case kQ8_0: return launch_typed<kQ8_0>(stream, a, w_bytes, programmatic);
+        case kKQuants: return launch_typed<kKQuants>(stream, a, w_bytes, programmatic);
+        default: return launch_typed<kAnyType>(stream, a, w_bytes, programmatic);
     }
 }
 

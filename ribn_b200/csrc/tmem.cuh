@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_fp16.h>
 
+#include "blocks.cuh"
 #include "gemv.cuh"
 
 namespace ribn {
@@ -136,6 +137,20 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_tie(float (&x)[8]) {
     asm volatile("" : "+f"(x[0]), "+f"(x[1]), "+f"(x[2]), "+f"(x[3]), "+f"(x[4]), "+f"(x[5]), "+f"(x[6]), "+f"(x[7]) :: "memory");
+}
+
+// The block type of a launch's matrices where it is one for all (the kernels are compiled for each: without the other types'
+// branches they run 5 to 15 % faster), else kKQuants or kAnyType.
+constexpr int kAnyType = -1, kKQuants = -2;
+template <int TYPE>
+__device__ __forceinline__ int type_of(const GemvSegment& s) { return TYPE < 0 ? s.type : TYPE; }
+inline int common_type(const StepGemm& a) {
+    bool same = true, k_quants = true;
+    for (int i = 0; i < a.n_segments; ++i) {
+        same = same && a.seg[i].type == a.seg[0].type;
+        k_quants = k_quants && (a.seg[i].type == kQ4_K || a.seg[i].type == kQ6_K);
+    }
+    return same ? a.seg[0].type : k_quants ? kKQuants : kAnyType;
 }
 
 struct UnitAt { int seg, rt0; };
