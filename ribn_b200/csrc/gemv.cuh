@@ -282,19 +282,20 @@ struct StepRun { int item, begin, end, part; };   // k tiles [begin, end) of an 
 struct StepSplit {
     int k_tiles, groups, group_members, items, workers, whole, unit_shift;   // unit_shift: log2 of a unit's weight rows
     int rounds;                                                              // wide form: rounds of whole items
+    int spread;   // workers that share the even slots: never more than there are slots, so that an item's parts have no gaps
     __host__ __device__ int even() const { return items - rounds * workers; }   // items dealt out evenly
     // (32-bit arithmetic: step_split deals out whole items where slots x workers would not fit)
     __host__ __device__ int begin(int w) const {   // first even slot of worker w; workers past the last one have nothing
-        const uint32_t v = (uint32_t)(w < workers ? w : workers) * (uint32_t)even(), n = (uint32_t)workers;
+        const uint32_t v = (uint32_t)(w < spread ? w : spread) * (uint32_t)even(), n = (uint32_t)spread;
         return (int)(whole ? v / n * (uint32_t)k_tiles : v * (uint32_t)k_tiles / n);
     }
     __host__ __device__ int first_worker(int item) const {
         const uint32_t slot = (uint32_t)(item - rounds * workers) * (uint32_t)k_tiles;
-        return (int)(((slot + 1) * (uint32_t)workers - 1) / (uint32_t)(even() * k_tiles));
+        return (int)(((slot + 1) * (uint32_t)spread - 1) / (uint32_t)(even() * k_tiles));
     }
     __host__ __device__ int last_worker(int item) const {
         const uint32_t slot = (uint32_t)(item + 1 - rounds * workers) * (uint32_t)k_tiles;
-        return (int)((slot * (uint32_t)workers - 1) / (uint32_t)(even() * k_tiles));
+        return (int)((slot * (uint32_t)spread - 1) / (uint32_t)(even() * k_tiles));
     }
     __host__ __device__ int parts(int item) const {
         return whole || item < rounds * workers ? 1 : last_worker(item) - first_worker(item) + 1;

@@ -274,6 +274,7 @@ StepSplit step_split(const StepGemm& a, bool whole_items) {
     s.workers = std::min(device_sms() * (a.form == kFragmentForm ? kFragTeams : 1), whole_items ? s.items : s.items * s.k_tiles);
     s.rounds = a.form == kWideForm ? s.items / s.workers : 0;
     if (s.rounds * s.workers == s.items && s.rounds > 0) s.whole = 1;   // nothing is left to deal out evenly
+    s.spread = std::max(1, s.whole ? std::min(s.workers, s.even()) : std::min(s.workers, s.even() * s.k_tiles));
     return s;
 }
 

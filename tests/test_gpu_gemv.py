@@ -244,7 +244,7 @@ def test_operand_cache_refuses_other_types(ops):
 
 @pytest.mark.parametrize("kind,variant", [(H.Q8_0, 6), (H.Q4_K, 6), (H.Q6_K, 6), (H.Q4_K, 7), (H.Q6_K, 7), (H.Q4_K, 8), (H.Q6_K, 8), (H.Q8_0, 7), (H.Q8_0, 8)])
 @pytest.mark.parametrize("rows,cols,members", [(4, 256, 1), (40, 512, 3), (132, 768, 8), (272, 1024, 9), (128, 2048, 32), (260, 1024, 33), (384, 512, 24),
-                                               (136, 1024, 64), (30, 512, 5), (144, 768, 70), (520, 768, 200), (257, 512, 129), (19200, 256, 300)])
+                                               (136, 1024, 64), (30, 512, 5), (144, 768, 70), (520, 768, 200), (257, 512, 129), (19200, 256, 300), (6144, 1024, 800)])
 def test_step_gemm_tile_and_group_edges(ops, kind, variant, rows, cols, members):
     # row tiles and 128-row units cut short; every operand width, one and several row groups; split and direct results
     rng = np.random.default_rng(rows + 3 * cols + 7 * members + kind)
