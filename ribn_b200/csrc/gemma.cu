@@ -119,30 +119,42 @@ __global__ void gm_embed_kernel(const uint32_t* tokens, const bf16_t* embed, con
 }
 
 // ---------------------------------------------------------------------------------------------
-// Projection: out[r][n] = bf16(sum_k in[r][k] * w[n][k]) (linear.rs:23-66), the sum in k order.  One warp
-// per block; a thread owns one output column for a tile of RT rows and keeps RT independent accumulation
-// chains.  Weights and input rows arrive in 256-input tiles through a two- or three-stage cp.async pipeline: the
-// warp copies 32 weight-row segments of 512 bytes each (coalesced, L2-only) plus the RT input segments,
-// then each thread walks its own row of the tile in shared memory (rows are pitched by 528 bytes, so the
-// 128-bit reads of a quarter-warp fall in distinct banks; the input segment is a broadcast read).
+// Projection: out[r][n] = bf16(sum_k in[r][k] * w[n][k]) (linear.rs:23-66), the sum in k order.  A block is a
+// feeder warp and a consumer warp.  The consumer owns 32 output columns for R rows: a thread walks one weight row
+// and keeps R independent accumulation chains, rows packed in pairs (`fma.rn.f32x2` rounds each half as `fmaf`
+// does).  The feeder brings weight tiles by cp.async into a ring of stages (rows pitched 16 bytes apart from a
+// multiple of 128, so the 128-bit reads of a quarter-warp fall in distinct banks) and writes the input rows
+// expanded to FP32, in the order the consumer reads them.  Named barriers hand the stages over.
+//
+// What bounds it: the chain of dependent additions, 4 cycles per input (14.4 us for the 6,912 inputs of a down
+// projection), or, with several warps per scheduler, the instructions issued per input.  A warp that did its own
+// copying and four rows took 24 cycles per input; see `project_rows` for how R is chosen.
 // ---------------------------------------------------------------------------------------------
-constexpr int kProjectCols = 32;                        // output columns (= threads) per block
-// 16-byte chunks per row per tile: 256 inputs, or 128 for eight-row tiles (prefill), whose stages then fit eight
-// blocks per SM: those tiles are bound by instruction issue and want two warps per scheduler
-__host__ __device__ constexpr int project_tile_chunks(int rt) { return rt >= 8 ? 16 : 32; }
-__host__ __device__ constexpr int project_stages(int rt) { return rt >= 8 ? 2 : 3; }  // an 8-row tile spends longer per stage
-__host__ __device__ constexpr int project_row_pitch(int rt) { return project_tile_chunks(rt) * 16 + 16; }  // bytes between weight rows of a tile
-
-__host__ __device__ constexpr int project_stage_bytes(int rt) {
-    return rt * project_tile_chunks(rt) * 16 + kProjectCols * project_row_pitch(rt);
-}
-// all stages, then the current tile's input rows expanded to FP32 (one conversion per value instead of one per column)
-__host__ __device__ constexpr int project_smem_bytes(int rt) {
-    return project_stages(rt) * project_stage_bytes(rt) + rt * project_tile_chunks(rt) * 32;
+constexpr int kProjectCols = 32;                        // output columns per block
+constexpr int kProjectThreads = 64;
+constexpr int kProjectMaxStages = 6;
+// inputs per tile: 256, or 128 for eight-row tiles (prefill), whose stages then leave room for more blocks per SM
+__host__ __device__ constexpr int project_tile(int r) { return r >= 8 ? 128 : 256; }
+__host__ __device__ constexpr int project_pitch(int r) { return project_tile(r) * 2 + 16; }  // bytes between weight rows of a tile
+// floats between groups of eight inputs of the expanded rows: padded so that the feeder's stores fall in distinct banks
+__host__ __device__ constexpr int project_x_pitch(int r) { return r == 1 ? 8 : r == 2 ? 20 : 9 * r; }
+__host__ __device__ constexpr int project_stage_bytes(int r) {
+    return kProjectCols * project_pitch(r) + project_tile(r) / 8 * project_x_pitch(r) * 4;
 }
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void named_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kProjectThreads) : "memory"); }
+__device__ __forceinline__ void named_arrive(int id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(kProjectThreads) : "memory"); }
+__device__ __forceinline__ unsigned long long fma_pair(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ float bf_half(const uint4& v, int e) {   // value e of eight BF16 values; e is a constant after unrolling
+    const uint32_t w = e < 2 ? v.x : e < 4 ? v.y : e < 6 ? v.z : v.w;
+    return __uint_as_float(e & 1 ? w & 0xffff0000u : w << 16);
 }
 
 // Up to three matrices that read the same input rows share one launch (q | k | v, gate | up): their
@@ -155,109 +167,174 @@ struct ProjectTargets {
     int count;
 };
 
-template <int RT>
-__global__ void __launch_bounds__(kProjectCols) gm_project_kernel(const bf16_t* __restrict__ in,
-                                                                  const int* __restrict__ row_index, int rows,
-                                                                  const ProjectTargets targets, int k) {
+template <int R>
+__global__ void __launch_bounds__(kProjectThreads) gm_project_kernel(const bf16_t* __restrict__ in,
+                                                                     const int* __restrict__ row_index, int rows,
+                                                                     const ProjectTargets targets, int k, int stages) {
     extern __shared__ __align__(16) unsigned char project_smem[];
-    constexpr int kStageBytes = project_stage_bytes(RT);
-    constexpr int kProjectStages = project_stages(RT);
-    constexpr int kTileChunks = project_tile_chunks(RT);
-    constexpr int kRowPitch = project_row_pitch(RT);
-    constexpr int kRowsPerIssue = 32 / kTileChunks;  // rows one warp-wide copy instruction covers
-    const int lane = threadIdx.x;
-    const int piece = lane % kTileChunks, sub_row = lane / kTileChunks;
+    constexpr int kTile = project_tile(R), kTileChunks = kTile / 8, kPitch = project_pitch(R), kXPitch = project_x_pitch(R);
+    constexpr int kStageBytes = project_stage_bytes(R), kXOffset = kProjectCols * kPitch;
+    constexpr int kRowsPerIssue = 32 / kTileChunks;      // weight rows one warp-wide copy instruction covers
+    constexpr int kPieces = R * kTileChunks / 32;        // 16-byte pieces of the input rows per lane and tile
+    const int lane = threadIdx.x & 31;
     int which = 0;
     if (targets.count > 1 && (int)blockIdx.x >= targets.first_block[1]) which = 1;
     if (targets.count > 2 && (int)blockIdx.x >= targets.first_block[2]) which = 2;
-    const bf16_t* __restrict__ w = targets.w[which];
-    bf16_t* __restrict__ out = targets.out[which];
     const int n = targets.n[which];
-    const int col0 = ((int)blockIdx.x - targets.first_block[which]) * kProjectCols, col = col0 + lane;
-    const int r0 = blockIdx.y * RT;
+    const int col0 = ((int)blockIdx.x - targets.first_block[which]) * kProjectCols;
+    const int r0 = blockIdx.y * R;
     const int live_cols = min(kProjectCols, n - col0);
-    const uint4* x[RT];
-#pragma unroll
-    for (int r = 0; r < RT; ++r) {
-        const int row = min(r0 + r, rows - 1);
-        x[r] = reinterpret_cast<const uint4*>(in + (size_t)(row_index ? row_index[row] : row) * k);
-    }
-    const uint4* wbase = reinterpret_cast<const uint4*>(w + (size_t)col0 * k);
-    const int chunks = k / 8, row_chunks = chunks;  // 16-byte chunks per weight row
+    const int chunks = k / 8;  // 16-byte chunks per weight row
     const int tiles = (chunks + kTileChunks - 1) / kTileChunks;
-    const uint32_t smem = (uint32_t)__cvta_generic_to_shared(project_smem);
+    // named barriers: 1 + stage when a stage is filled, 1 + stages + stage when it has been read
 
-    auto issue = [&](int tile) {
-        if (tile < tiles) {
-            const int c = tile * kTileChunks + piece;  // this lane's chunk of its row segments
-            if (c < chunks) {
-                const uint32_t stage = smem + (uint32_t)((tile % kProjectStages) * kStageBytes);
-#pragma unroll
-                for (int r = 0; r < RT; ++r) {  // static indices keep the row pointers in registers
-                    if (r % kRowsPerIssue == sub_row) cp_async16(stage + (uint32_t)(r * kTileChunks * 16 + piece * 16), x[r] + c);
-                }
-                uint32_t wdst = stage + (uint32_t)(RT * kTileChunks * 16 + sub_row * kRowPitch + piece * 16);
-                const uint4* src = wbase + (size_t)sub_row * row_chunks + c;
-                for (int j = sub_row; j < live_cols; j += kRowsPerIssue, wdst += kRowsPerIssue * kRowPitch,
-                         src += (size_t)kRowsPerIssue * row_chunks) {
-                    cp_async16(wdst, src);
+    if (threadIdx.x < 32) {   // feeder
+        const int piece = lane % kTileChunks, sub_row = lane / kTileChunks;
+        const uint4* wsrc = reinterpret_cast<const uint4*>(targets.w[which] + (size_t)(col0 + sub_row) * k) + piece;
+        const uint32_t wdst = (uint32_t)__cvta_generic_to_shared(project_smem) + (uint32_t)(sub_row * kPitch + piece * 16);
+        auto copy = [&](int tile, int slot) {
+            const int c = tile * kTileChunks;
+            if (tile < tiles && c + piece < chunks) {
+                const uint4* src = wsrc + c;
+                uint32_t dst = wdst + (uint32_t)(slot * kStageBytes);
+#pragma unroll 8
+                for (int j = sub_row; j < live_cols; j += kRowsPerIssue, dst += kRowsPerIssue * kPitch, src += (size_t)kRowsPerIssue * chunks) {
+                    cp_async16(dst, src);
                 }
             }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-
-    float acc[RT];
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        // a lane's pieces of the input rows: row lane % R, chunk lane / R and every 32 / R after it
+        const int row = min(r0 + lane % R, rows - 1), first_chunk = lane / R;
+        const uint4* xsrc = reinterpret_cast<const uint4*>(in + (size_t)(row_index ? row_index[row] : row) * k);
+        uint4 x[kPieces];
+        auto read = [&](int tile) {
 #pragma unroll
-    for (int r = 0; r < RT; ++r) acc[r] = 0.0f;
-#pragma unroll
-    for (int s = 0; s < kProjectStages - 1; ++s) issue(s);
-    for (int tile = 0; tile < tiles; ++tile) {
-        issue(tile + kProjectStages - 1);
-        asm volatile("cp.async.wait_group %0;" ::"n"(kProjectStages - 1) : "memory");
-        __syncwarp();
-        const unsigned char* stage = project_smem + (size_t)(tile % kProjectStages) * kStageBytes;
-        const uint4* ws = reinterpret_cast<const uint4*>(stage + RT * kTileChunks * 16 + lane * kRowPitch);
-        const int count = min(kTileChunks, chunks - tile * kTileChunks);
-        // lane l expands chunk l of every input row to FP32
-        float4* xf = reinterpret_cast<float4*>(project_smem + kProjectStages * kStageBytes);
-        if (lane < count) {
-#pragma unroll
-            for (int r = 0; r < RT; ++r) {
-                const uint4 xv = reinterpret_cast<const uint4*>(stage)[r * kTileChunks + lane];
-                xf[(r * kTileChunks + lane) * 2] = make_float4(__uint_as_float(xv.x << 16), __uint_as_float(xv.x & 0xffff0000u),
-                                                               __uint_as_float(xv.y << 16), __uint_as_float(xv.y & 0xffff0000u));
-                xf[(r * kTileChunks + lane) * 2 + 1] = make_float4(__uint_as_float(xv.z << 16), __uint_as_float(xv.z & 0xffff0000u),
-                                                                   __uint_as_float(xv.w << 16), __uint_as_float(xv.w & 0xffff0000u));
+            for (int i = 0; i < kPieces; ++i) {
+                const int c = tile * kTileChunks + first_chunk + i * (32 / R);
+                x[i] = c < chunks ? xsrc[c] : make_uint4(0, 0, 0, 0);
             }
+        };
+        for (int t = 0; t < stages - 1; ++t) copy(t, t);
+        read(0);
+        int slot = 0, ahead = stages - 1;   // slots of tile t and of tile t + stages - 1
+        for (int t = 0; t < tiles; ++t) {
+            // the input rows first: they need nothing but the slot, which was free when its weights were requested
+            float* xf = reinterpret_cast<float*>(project_smem + (size_t)slot * kStageBytes + kXOffset);
+#pragma unroll
+            for (int i = 0; i < kPieces; ++i) {
+                float* dst = xf + (first_chunk + i * (32 / R)) * kXPitch;
+                if constexpr (R == 1) {
+                    reinterpret_cast<float4*>(dst)[0] = make_float4(bf_half(x[i], 0), bf_half(x[i], 1), bf_half(x[i], 2), bf_half(x[i], 3));
+                    reinterpret_cast<float4*>(dst)[1] = make_float4(bf_half(x[i], 4), bf_half(x[i], 5), bf_half(x[i], 6), bf_half(x[i], 7));
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) dst[e * R + lane % R] = bf_half(x[i], e);
+                }
+            }
+            read(t + 1);
+            // at most stages - 2 younger copies stay in flight behind tile t's
+            switch (stages) {
+                case 2: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
+                case 3: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
+                case 4: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
+                case 5: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
+                default: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
+            }
+            __syncwarp();
+            named_arrive(1 + slot);
+            if (t > 0 && t - 1 + stages < tiles) named_sync(1 + stages + ahead);   // the consumer has left tile t - 1
+            copy(t + stages - 1, ahead);
+            slot = slot + 1 == stages ? 0 : slot + 1;
+            ahead = ahead + 1 == stages ? 0 : ahead + 1;
         }
-        __syncwarp();
-        if (lane < live_cols) {
+        return;
+    }
+
+    using Pair = unsigned long long;
+    constexpr int kPairs = R == 1 ? 1 : R / 2;
+    Pair acc[kPairs];
+    float sum = 0.0f;
+#pragma unroll
+    for (int p = 0; p < kPairs; ++p) acc[p] = 0;
+    int slot = 0;
+    for (int t = 0; t < tiles; ++t) {
+        named_sync(1 + slot);
+        const unsigned char* stage = project_smem + (size_t)slot * kStageBytes;
+        const uint4* ws = reinterpret_cast<const uint4*>(stage + lane * kPitch);
+        const float* xf = reinterpret_cast<const float*>(stage + kXOffset);
+        const int count = min(kTileChunks, chunks - t * kTileChunks);
+        auto chunk = [&](int i) {
+            const uint4 wv = ws[i];
+            const float* x = xf + i * kXPitch;
+            if constexpr (R == 1) {
+                const float4 a = reinterpret_cast<const float4*>(x)[0], b = reinterpret_cast<const float4*>(x)[1];
+                sum = fmaf(a.x, bf_half(wv, 0), sum); sum = fmaf(a.y, bf_half(wv, 1), sum);
+                sum = fmaf(a.z, bf_half(wv, 2), sum); sum = fmaf(a.w, bf_half(wv, 3), sum);
+                sum = fmaf(b.x, bf_half(wv, 4), sum); sum = fmaf(b.y, bf_half(wv, 5), sum);
+                sum = fmaf(b.z, bf_half(wv, 6), sum); sum = fmaf(b.w, bf_half(wv, 7), sum);
+            } else {
+                const ulonglong2* pairs = reinterpret_cast<const ulonglong2*>(x);   // rows 0 .. R - 1 of input 0, of input 1, ...
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const float w = bf_half(wv, e);
+                    Pair ww;
+                    asm("mov.b64 %0, {%1, %1};" : "=l"(ww) : "f"(w));
+                    if constexpr (R == 2) {
+                        const ulonglong2 v = pairs[e / 2];
+                        acc[0] = fma_pair(e & 1 ? v.y : v.x, ww, acc[0]);
+                    } else {
+#pragma unroll
+                        for (int p = 0; p < kPairs; p += 2) {
+                            const ulonglong2 v = pairs[e * (R / 4) + p / 2];
+                            acc[p] = fma_pair(v.x, ww, acc[p]);
+                            acc[p + 1] = fma_pair(v.y, ww, acc[p + 1]);
+                        }
+                    }
+                }
+            }
+        };
+        if (count == kTileChunks) {
 #pragma unroll 4
-            for (int i = 0; i < count; ++i) {
-                const uint4 wv = ws[i];
-                const float w0 = __uint_as_float(wv.x << 16), w1 = __uint_as_float(wv.x & 0xffff0000u);
-                const float w2 = __uint_as_float(wv.y << 16), w3 = __uint_as_float(wv.y & 0xffff0000u);
-                const float w4 = __uint_as_float(wv.z << 16), w5 = __uint_as_float(wv.z & 0xffff0000u);
-                const float w6 = __uint_as_float(wv.w << 16), w7 = __uint_as_float(wv.w & 0xffff0000u);
-#pragma unroll
-                for (int r = 0; r < RT; ++r) {
-                    const float4 a = xf[(r * kTileChunks + i) * 2], b = xf[(r * kTileChunks + i) * 2 + 1];
-                    acc[r] = fmaf(a.x, w0, acc[r]); acc[r] = fmaf(a.y, w1, acc[r]);
-                    acc[r] = fmaf(a.z, w2, acc[r]); acc[r] = fmaf(a.w, w3, acc[r]);
-                    acc[r] = fmaf(b.x, w4, acc[r]); acc[r] = fmaf(b.y, w5, acc[r]);
-                    acc[r] = fmaf(b.z, w6, acc[r]); acc[r] = fmaf(b.w, w7, acc[r]);
-                }
-            }
+            for (int i = 0; i < kTileChunks; ++i) chunk(i);
+        } else {
+            for (int i = 0; i < count; ++i) chunk(i);
         }
-        __syncwarp();  // every lane has left this stage (and the expanded rows) before they are overwritten
+        if (t + stages < tiles) named_arrive(1 + stages + slot);
+        slot = slot + 1 == stages ? 0 : slot + 1;
     }
     if (lane < live_cols) {
+        bf16_t* out = targets.out[which] + col0 + lane;
+        if constexpr (R == 1) {
+            out[(size_t)r0 * n] = bf_round(sum);
+        } else {
 #pragma unroll
-        for (int r = 0; r < RT; ++r) {
-            if (r0 + r < rows) out[(size_t)(r0 + r) * n + col] = bf_round(acc[r]);
+            for (int p = 0; p < kPairs; ++p) {
+                float lo, hi;
+                asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc[p]));
+                if (r0 + 2 * p < rows) out[(size_t)(r0 + 2 * p) * n] = bf_round(lo);
+                if (r0 + 2 * p + 1 < rows) out[(size_t)(r0 + 2 * p + 1) * n] = bf_round(hi);
+            }
         }
     }
+}
+
+// Rows per consumer warp.  A warp alone on its scheduler advances one input per 4 cycles (the addition's latency) or
+// per the instructions it issues for an input; warps that share a scheduler add up.  Fewer rows per warp spread a
+// narrow projection of a few rows over the SMs (a 1,152-column one of four rows: 144 warps instead of 36), more rows
+// per warp issue less per product and read the weights fewer times.
+int project_rows(int col_blocks, int rows, int sms) {
+    constexpr int kRows[4] = {8, 4, 2, 1};
+    constexpr float kIssue[4] = {8.3f, 5.3f, 3.8f, 2.6f};   // instructions per input, counted from the loop above
+    int best = 0;
+    float best_cost = 0.0f;
+    for (int i = 0; i < 4; ++i) {
+        if (kRows[i] >= 2 * rows) continue;
+        const int warps = col_blocks * ((rows + kRows[i] - 1) / kRows[i]);
+        const float cost = std::max(4.0f, kIssue[i] * (float)((warps + 4 * sms - 1) / (4 * sms)));
+        if (best == 0 || cost < best_cost) { best = kRows[i]; best_cost = cost; }
+    }
+    return best;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -772,6 +849,7 @@ struct ribn_b200_gemma {
     int *h_slot = nullptr, *h_position = nullptr, *h_out_rows = nullptr;
     uint32_t* h_choice = nullptr;
     int max_outputs = 0;
+    int sms = 1;
     std::string error;
     float last_ms = 0.0f;
     uint32_t last_launches = 0;
@@ -1068,11 +1146,12 @@ RIBN_B200_API int ribn_b200_gemma_finalize(ribn_b200_gemma* m) {
         GM_CUDA(m, cudaMemcpy(m->sine[kind], sn.data(), sizeof(bf16_t) * sn.size(), cudaMemcpyHostToDevice));
     }
     {
+        GM_CUDA(m, cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, m->cfg.device));
         const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
-        GM_CUDA(m, cudaFuncSetAttribute(gm_project_kernel<1>, at, project_smem_bytes(1)));
-        GM_CUDA(m, cudaFuncSetAttribute(gm_project_kernel<2>, at, project_smem_bytes(2)));
-        GM_CUDA(m, cudaFuncSetAttribute(gm_project_kernel<4>, at, project_smem_bytes(4)));
-        GM_CUDA(m, cudaFuncSetAttribute(gm_project_kernel<8>, at, project_smem_bytes(8)));
+        GM_CUDA(m, cudaFuncSetAttribute(gm_project_kernel<1>, at, kProjectMaxStages * project_stage_bytes(1)));
+        GM_CUDA(m, cudaFuncSetAttribute(gm_project_kernel<2>, at, kProjectMaxStages * project_stage_bytes(2)));
+        GM_CUDA(m, cudaFuncSetAttribute(gm_project_kernel<4>, at, kProjectMaxStages * project_stage_bytes(4)));
+        GM_CUDA(m, cudaFuncSetAttribute(gm_project_kernel<8>, at, kProjectMaxStages * project_stage_bytes(8)));
     }
     const size_t attention_bytes = attention_smem_bytes(c.context, c.head_dim > c.global_head_dim ? c.head_dim : c.global_head_dim);
     if (attention_bytes > 48 * 1024) {
@@ -1114,10 +1193,20 @@ struct Pass {
             ++launches;
             return;
         }
-        if (n_rows <= 1) gm_project_kernel<1><<<dim3(col_blocks, 1), block, project_smem_bytes(1), s>>>(in, row_index, n_rows, t, k);
-        else if (n_rows <= 2) gm_project_kernel<2><<<dim3(col_blocks, 1), block, project_smem_bytes(2), s>>>(in, row_index, n_rows, t, k);
-        else if (n_rows <= 4) gm_project_kernel<4><<<dim3(col_blocks, 1), block, project_smem_bytes(4), s>>>(in, row_index, n_rows, t, k);
-        else gm_project_kernel<8><<<dim3(col_blocks, (unsigned)((n_rows + 7) / 8)), block, project_smem_bytes(8), s>>>(in, row_index, n_rows, t, k);
+        switch (project_rows((int)col_blocks, n_rows, m->sms)) {
+            case 1: launch_project<1>(in, row_index, n_rows, t, col_blocks, k); break;
+            case 2: launch_project<2>(in, row_index, n_rows, t, col_blocks, k); break;
+            case 4: launch_project<4>(in, row_index, n_rows, t, col_blocks, k); break;
+            default: launch_project<8>(in, row_index, n_rows, t, col_blocks, k); break;
+        }
+    }
+    template <int R>
+    void launch_project(const bf16_t* in, const int* row_index, int n_rows, const ProjectTargets& t, unsigned col_blocks, int k) {
+        const dim3 grid(col_blocks, (unsigned)((n_rows + R - 1) / R));
+        // as many stages as the blocks that share an SM leave room for: few blocks need more bytes in flight each
+        const int per_sm = ((int)(grid.x * grid.y) + m->sms - 1) / m->sms;
+        const int stages = std::max(2, std::min(kProjectMaxStages, 220 * 1024 / (per_sm * (project_stage_bytes(R) + 1024))));
+        gm_project_kernel<R><<<grid, kProjectThreads, (size_t)stages * project_stage_bytes(R), m->stream>>>(in, row_index, n_rows, t, k, stages);
         ++launches;
     }
     void project(const bf16_t* in, const int* row_index, int n_rows, const bf16_t* w, int n, int k, bf16_t* out) {
