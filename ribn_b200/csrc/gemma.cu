@@ -120,33 +120,45 @@ __global__ void gm_embed_kernel(const uint32_t* tokens, const bf16_t* embed, con
 
 // ---------------------------------------------------------------------------------------------
 // Projection: out[r][n] = bf16(sum_k in[r][k] * w[n][k]) (linear.rs:23-66), the sum in k order.  A block is a
-// feeder warp and a consumer warp.  The consumer owns 32 output columns for R rows: a thread walks one weight row
-// and keeps R independent accumulation chains, rows packed in pairs (`fma.rn.f32x2` rounds each half as `fmaf`
+// feeder warp and G consumer warps.  A consumer owns 32 * C output columns for R rows: a thread walks C weight rows
+// and keeps R * C independent accumulation chains, rows packed in pairs (`fma.rn.f32x2` rounds each half as `fmaf`
 // does).  The feeder brings weight tiles by cp.async into a ring of stages (rows pitched 16 bytes apart from a
 // multiple of 128, so the 128-bit reads of a quarter-warp fall in distinct banks) and writes the input rows
-// expanded to FP32, in the order the consumer reads them.  Named barriers hand the stages over.
+// expanded to FP32, in the order the consumers read them.  Named barriers hand the stages over; their ids are
+// constants because an SM has 64 barriers and a block whose ids are computed is given 16 of them.
 //
 // What bounds it: the chain of dependent additions, 4 cycles per input (14.4 us for the 6,912 inputs of a down
-// projection), or, with several warps per scheduler, the instructions issued per input.  A warp that did its own
-// copying and four rows took 24 cycles per input; see `project_rows` for how R is chosen.
+// projection), or, with several warps per scheduler, the instructions issued per input and the broadcast reads of
+// the input rows, which cost shared memory as much as distinct ones: two columns per thread halve them.
 // ---------------------------------------------------------------------------------------------
-constexpr int kProjectCols = 32;                        // output columns per block
-constexpr int kProjectThreads = 64;
-constexpr int kProjectMaxStages = 6;
-// inputs per tile: 256, or 128 for eight-row tiles (prefill), whose stages then leave room for more blocks per SM
-__host__ __device__ constexpr int project_tile(int r) { return r >= 8 ? 128 : 256; }
-__host__ __device__ constexpr int project_pitch(int r) { return project_tile(r) * 2 + 16; }  // bytes between weight rows of a tile
-// floats between groups of eight inputs of the expanded rows: padded so that the feeder's stores fall in distinct banks
-__host__ __device__ constexpr int project_x_pitch(int r) { return r == 1 ? 8 : r == 2 ? 20 : 9 * r; }
-__host__ __device__ constexpr int project_stage_bytes(int r) {
-    return kProjectCols * project_pitch(r) + project_tile(r) / 8 * project_x_pitch(r) * 4;
-}
+struct ProjectNarrow { static constexpr int R = 1, C = 1, G = 1, tile = 256, stages = 4; };   // a few rows: chains spread over blocks
+struct ProjectRows4 { static constexpr int R = 4, C = 1, G = 1, tile = 256, stages = 3; };    // a few rows of a wide projection
+struct ProjectChunk { static constexpr int R = 4, C = 2, G = 2, tile = 128, stages = 2; };    // prefill
+template <typename V>
+struct ProjectShape {
+    static constexpr int cols = 32 * V::C, rows = V::R * V::G, threads = 32 * (1 + V::G);
+    static constexpr int chunks = V::tile / 8, pitch = V::tile * 2 + 16;        // 16-byte chunks, and bytes between weight rows of a tile
+    // floats of eight inputs of a consumer's rows: padded so that the feeder's stores fall in distinct banks
+    static constexpr int x_warp = V::R == 1 ? 8 : 9 * V::R, x_pitch = x_warp * V::G;
+    static constexpr int x_offset = cols * pitch, stage_bytes = x_offset + chunks * x_pitch * 4, smem_bytes = V::stages * stage_bytes;
+};
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
-__device__ __forceinline__ void named_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kProjectThreads) : "memory"); }
-__device__ __forceinline__ void named_arrive(int id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(kProjectThreads) : "memory"); }
+// Barrier of stage `slot`: 1 + slot when it is filled, 1 + STAGES + slot when it has been read.
+template <int ID, int THREADS>
+__device__ __forceinline__ void stage_barrier(bool wait) {
+    if (wait) asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(THREADS) : "memory");
+    else asm volatile("bar.arrive %0, %1;" ::"n"(ID), "n"(THREADS) : "memory");
+}
+template <int FIRST, int STAGES, int THREADS>
+__device__ __forceinline__ void stage_barrier(int slot, bool wait) {
+    if (slot == 0) stage_barrier<FIRST, THREADS>(wait);
+    else if (STAGES <= 2 || slot == 1) stage_barrier<FIRST + 1, THREADS>(wait);
+    else if (STAGES <= 3 || slot == 2) stage_barrier<FIRST + (STAGES > 2 ? 2 : 0), THREADS>(wait);
+    else stage_barrier<FIRST + (STAGES > 3 ? 3 : 0), THREADS>(wait);
+}
 __device__ __forceinline__ unsigned long long fma_pair(unsigned long long a, unsigned long long b, unsigned long long c) {
     unsigned long long d;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
@@ -167,172 +179,184 @@ struct ProjectTargets {
     int count;
 };
 
-template <int R>
-__global__ void __launch_bounds__(kProjectThreads) gm_project_kernel(const bf16_t* __restrict__ in,
-                                                                     const int* __restrict__ row_index, int rows,
-                                                                     const ProjectTargets targets, int k, int stages) {
+template <typename V>
+__global__ void __launch_bounds__(ProjectShape<V>::threads) gm_project_kernel(const bf16_t* __restrict__ in,
+                                                                              const int* __restrict__ row_index, int rows,
+                                                                              const ProjectTargets targets, int k) {
     extern __shared__ __align__(16) unsigned char project_smem[];
-    constexpr int kTile = project_tile(R), kTileChunks = kTile / 8, kPitch = project_pitch(R), kXPitch = project_x_pitch(R);
-    constexpr int kStageBytes = project_stage_bytes(R), kXOffset = kProjectCols * kPitch;
-    constexpr int kRowsPerIssue = 32 / kTileChunks;      // weight rows one warp-wide copy instruction covers
-    constexpr int kPieces = R * kTileChunks / 32;        // 16-byte pieces of the input rows per lane and tile
+    using S = ProjectShape<V>;
+    constexpr int R = V::R, C = V::C, kStages = V::stages, kThreads = S::threads;
+    constexpr int kRowsPerIssue = 32 / S::chunks;              // weight rows one warp-wide copy instruction covers
+    constexpr int kPieces = S::rows * S::chunks / 32;          // 16-byte pieces of the input rows per lane and tile
     const int lane = threadIdx.x & 31;
     int which = 0;
     if (targets.count > 1 && (int)blockIdx.x >= targets.first_block[1]) which = 1;
     if (targets.count > 2 && (int)blockIdx.x >= targets.first_block[2]) which = 2;
     const int n = targets.n[which];
-    const int col0 = ((int)blockIdx.x - targets.first_block[which]) * kProjectCols;
-    const int r0 = blockIdx.y * R;
-    const int live_cols = min(kProjectCols, n - col0);
+    const int col0 = ((int)blockIdx.x - targets.first_block[which]) * S::cols;
+    const int r0 = blockIdx.y * S::rows;
+    const int live_cols = min(S::cols, n - col0);
     const int chunks = k / 8;  // 16-byte chunks per weight row
-    const int tiles = (chunks + kTileChunks - 1) / kTileChunks;
-    // named barriers: 1 + stage when a stage is filled, 1 + stages + stage when it has been read
+    const int tiles = (chunks + S::chunks - 1) / S::chunks;
 
     if (threadIdx.x < 32) {   // feeder
-        const int piece = lane % kTileChunks, sub_row = lane / kTileChunks;
+        const int piece = lane % S::chunks, sub_row = lane / S::chunks;
         const uint4* wsrc = reinterpret_cast<const uint4*>(targets.w[which] + (size_t)(col0 + sub_row) * k) + piece;
-        const uint32_t wdst = (uint32_t)__cvta_generic_to_shared(project_smem) + (uint32_t)(sub_row * kPitch + piece * 16);
+        const uint32_t wdst = (uint32_t)__cvta_generic_to_shared(project_smem) + (uint32_t)(sub_row * S::pitch + piece * 16);
         auto copy = [&](int tile, int slot) {
-            const int c = tile * kTileChunks;
+            const int c = tile * S::chunks;
             if (tile < tiles && c + piece < chunks) {
                 const uint4* src = wsrc + c;
-                uint32_t dst = wdst + (uint32_t)(slot * kStageBytes);
+                uint32_t dst = wdst + (uint32_t)(slot * S::stage_bytes);
 #pragma unroll 8
-                for (int j = sub_row; j < live_cols; j += kRowsPerIssue, dst += kRowsPerIssue * kPitch, src += (size_t)kRowsPerIssue * chunks) {
+                for (int j = sub_row; j < live_cols; j += kRowsPerIssue, dst += kRowsPerIssue * S::pitch, src += (size_t)kRowsPerIssue * chunks) {
                     cp_async16(dst, src);
                 }
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
-        // a lane's pieces of the input rows: row lane % R, chunk lane / R and every 32 / R after it
-        const int row = min(r0 + lane % R, rows - 1), first_chunk = lane / R;
+        // a lane's pieces of the input rows: one row, chunk lane / rows and every 32 / rows after it
+        const int own = lane % S::rows, row = min(r0 + own, rows - 1), first_chunk = lane / S::rows;
         const uint4* xsrc = reinterpret_cast<const uint4*>(in + (size_t)(row_index ? row_index[row] : row) * k);
         uint4 x[kPieces];
         auto read = [&](int tile) {
 #pragma unroll
             for (int i = 0; i < kPieces; ++i) {
-                const int c = tile * kTileChunks + first_chunk + i * (32 / R);
+                const int c = tile * S::chunks + first_chunk + i * (32 / S::rows);
                 x[i] = c < chunks ? xsrc[c] : make_uint4(0, 0, 0, 0);
             }
         };
-        for (int t = 0; t < stages - 1; ++t) copy(t, t);
+#pragma unroll
+        for (int t = 0; t < kStages - 1; ++t) copy(t, t);
         read(0);
-        int slot = 0, ahead = stages - 1;   // slots of tile t and of tile t + stages - 1
+        int slot = 0, ahead = kStages - 1;   // slots of tile t and of tile t + kStages - 1
         for (int t = 0; t < tiles; ++t) {
             // the input rows first: they need nothing but the slot, which was free when its weights were requested
-            float* xf = reinterpret_cast<float*>(project_smem + (size_t)slot * kStageBytes + kXOffset);
+            float* xf = reinterpret_cast<float*>(project_smem + (size_t)slot * S::stage_bytes + S::x_offset) + own / R * S::x_warp;
 #pragma unroll
             for (int i = 0; i < kPieces; ++i) {
-                float* dst = xf + (first_chunk + i * (32 / R)) * kXPitch;
+                float* dst = xf + (first_chunk + i * (32 / S::rows)) * S::x_pitch;
                 if constexpr (R == 1) {
                     reinterpret_cast<float4*>(dst)[0] = make_float4(bf_half(x[i], 0), bf_half(x[i], 1), bf_half(x[i], 2), bf_half(x[i], 3));
                     reinterpret_cast<float4*>(dst)[1] = make_float4(bf_half(x[i], 4), bf_half(x[i], 5), bf_half(x[i], 6), bf_half(x[i], 7));
                 } else {
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) dst[e * R + lane % R] = bf_half(x[i], e);
+                    for (int e = 0; e < 8; ++e) dst[e * R + own % R] = bf_half(x[i], e);
                 }
             }
             read(t + 1);
-            // at most stages - 2 younger copies stay in flight behind tile t's
-            switch (stages) {
-                case 2: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
-                case 3: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
-                case 4: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
-                case 5: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
-                default: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
-            }
+            asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");   // tile t; younger copies stay in flight
             __syncwarp();
-            named_arrive(1 + slot);
-            if (t > 0 && t - 1 + stages < tiles) named_sync(1 + stages + ahead);   // the consumer has left tile t - 1
-            copy(t + stages - 1, ahead);
-            slot = slot + 1 == stages ? 0 : slot + 1;
-            ahead = ahead + 1 == stages ? 0 : ahead + 1;
+            stage_barrier<1, kStages, kThreads>(slot, false);
+            if (t > 0 && t - 1 + kStages < tiles) stage_barrier<1 + kStages, kStages, kThreads>(ahead, true);   // the consumers have left tile t - 1
+            copy(t + kStages - 1, ahead);
+            slot = slot + 1 == kStages ? 0 : slot + 1;
+            ahead = ahead + 1 == kStages ? 0 : ahead + 1;
         }
         return;
     }
 
+    const int g = (int)threadIdx.x / 32 - 1;
     using Pair = unsigned long long;
-    constexpr int kPairs = R == 1 ? 1 : R / 2;
-    Pair acc[kPairs];
+    // eight inputs: C weight rows' values and the R rows' inputs, read one group ahead of their use
+    constexpr int kAhead = R == 1 ? 2 : 1, kXVectors = 2 * R;
+    struct Group { uint4 w[C]; ulonglong2 x[kXVectors]; };
+    Pair acc[C][R == 1 ? 1 : R / 2];
     float sum = 0.0f;
 #pragma unroll
-    for (int p = 0; p < kPairs; ++p) acc[p] = 0;
+    for (int c = 0; c < C; ++c) {
+#pragma unroll
+        for (int q = 0; q < (R == 1 ? 1 : R / 2); ++q) acc[c][q] = 0;
+    }
     int slot = 0;
     for (int t = 0; t < tiles; ++t) {
-        named_sync(1 + slot);
-        const unsigned char* stage = project_smem + (size_t)slot * kStageBytes;
-        const uint4* ws = reinterpret_cast<const uint4*>(stage + lane * kPitch);
-        const float* xf = reinterpret_cast<const float*>(stage + kXOffset);
-        const int count = min(kTileChunks, chunks - t * kTileChunks);
-        auto chunk = [&](int i) {
-            const uint4 wv = ws[i];
-            const float* x = xf + i * kXPitch;
-            if constexpr (R == 1) {
-                const float4 a = reinterpret_cast<const float4*>(x)[0], b = reinterpret_cast<const float4*>(x)[1];
-                sum = fmaf(a.x, bf_half(wv, 0), sum); sum = fmaf(a.y, bf_half(wv, 1), sum);
-                sum = fmaf(a.z, bf_half(wv, 2), sum); sum = fmaf(a.w, bf_half(wv, 3), sum);
-                sum = fmaf(b.x, bf_half(wv, 4), sum); sum = fmaf(b.y, bf_half(wv, 5), sum);
-                sum = fmaf(b.z, bf_half(wv, 6), sum); sum = fmaf(b.w, bf_half(wv, 7), sum);
-            } else {
-                const ulonglong2* pairs = reinterpret_cast<const ulonglong2*>(x);   // rows 0 .. R - 1 of input 0, of input 1, ...
+        stage_barrier<1, kStages, kThreads>(slot, true);
+        const unsigned char* stage = project_smem + (size_t)slot * S::stage_bytes;
+        const unsigned char* ws = stage + lane * S::pitch;
+        const float* xf = reinterpret_cast<const float*>(stage + S::x_offset) + g * S::x_warp;
+        const int count = min(S::chunks, chunks - t * S::chunks);
+        auto fetch = [&](Group& to, int i) {
 #pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    const float w = bf_half(wv, e);
-                    Pair ww;
-                    asm("mov.b64 %0, {%1, %1};" : "=l"(ww) : "f"(w));
-                    if constexpr (R == 2) {
-                        const ulonglong2 v = pairs[e / 2];
-                        acc[0] = fma_pair(e & 1 ? v.y : v.x, ww, acc[0]);
-                    } else {
+            for (int c = 0; c < C; ++c) to.w[c] = *reinterpret_cast<const uint4*>(ws + c * 32 * S::pitch + i * 16);
 #pragma unroll
-                        for (int p = 0; p < kPairs; p += 2) {
-                            const ulonglong2 v = pairs[e * (R / 4) + p / 2];
-                            acc[p] = fma_pair(v.x, ww, acc[p]);
-                            acc[p + 1] = fma_pair(v.y, ww, acc[p + 1]);
+            for (int v = 0; v < kXVectors; ++v) to.x[v] = reinterpret_cast<const ulonglong2*>(xf + i * S::x_pitch)[v];
+        };
+        auto add = [&](const Group& from) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                if constexpr (R == 1) {
+                    const Pair two = e % 4 < 2 ? from.x[e / 4].x : from.x[e / 4].y;
+                    float lo, hi;
+                    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(two));
+                    sum = fmaf(e & 1 ? hi : lo, bf_half(from.w[0], e), sum);
+                } else {
+#pragma unroll
+                    for (int c = 0; c < C; ++c) {
+                        const float w = bf_half(from.w[c], e);
+                        Pair ww;
+                        asm("mov.b64 %0, {%1, %1};" : "=l"(ww) : "f"(w));
+#pragma unroll
+                        for (int q = 0; q < R / 2; ++q) {
+                            const ulonglong2 v = from.x[e * (R / 4) + q / 2];
+                            acc[c][q] = fma_pair(q & 1 ? v.y : v.x, ww, acc[c][q]);
                         }
                     }
                 }
             }
         };
-        if (count == kTileChunks) {
-#pragma unroll 4
-            for (int i = 0; i < kTileChunks; ++i) chunk(i);
+        if (count == S::chunks) {
+            Group now[kAhead], next[kAhead];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) fetch(now[u], u);
+#pragma unroll 2
+            for (int i = 0; i < S::chunks; i += kAhead) {
+#pragma unroll
+                for (int u = 0; u < kAhead; ++u) fetch(next[u], min(i + kAhead + u, S::chunks - 1));
+#pragma unroll
+                for (int u = 0; u < kAhead; ++u) add(now[u]);
+#pragma unroll
+                for (int u = 0; u < kAhead; ++u) now[u] = next[u];
+            }
         } else {
-            for (int i = 0; i < count; ++i) chunk(i);
+            for (int i = 0; i < count; ++i) { Group one; fetch(one, i); add(one); }
         }
-        if (t + stages < tiles) named_arrive(1 + stages + slot);
-        slot = slot + 1 == stages ? 0 : slot + 1;
+        if (t + kStages < tiles) stage_barrier<1 + kStages, kStages, kThreads>(slot, false);
+        slot = slot + 1 == kStages ? 0 : slot + 1;
     }
-    if (lane < live_cols) {
-        bf16_t* out = targets.out[which] + col0 + lane;
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        if (lane + 32 * c >= live_cols) break;
+        bf16_t* out = targets.out[which] + col0 + lane + 32 * c;
+        const int first = r0 + g * R;
         if constexpr (R == 1) {
-            out[(size_t)r0 * n] = bf_round(sum);
+            out[(size_t)first * n] = bf_round(sum);
         } else {
 #pragma unroll
-            for (int p = 0; p < kPairs; ++p) {
+            for (int q = 0; q < R / 2; ++q) {
                 float lo, hi;
-                asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc[p]));
-                if (r0 + 2 * p < rows) out[(size_t)(r0 + 2 * p) * n] = bf_round(lo);
-                if (r0 + 2 * p + 1 < rows) out[(size_t)(r0 + 2 * p + 1) * n] = bf_round(hi);
+                asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc[c][q]));
+                if (first + 2 * q < rows) out[(size_t)(first + 2 * q) * n] = bf_round(lo);
+                if (first + 2 * q + 1 < rows) out[(size_t)(first + 2 * q + 1) * n] = bf_round(hi);
             }
         }
     }
 }
 
-// Rows per consumer warp.  A warp alone on its scheduler advances one input per 4 cycles (the addition's latency) or
-// per the instructions it issues for an input; warps that share a scheduler add up.  Fewer rows per warp spread a
-// narrow projection of a few rows over the SMs (a 1,152-column one of four rows: 144 warps instead of 36), more rows
-// per warp issue less per product and read the weights fewer times.
-int project_rows(int col_blocks, int rows, int sms) {
-    constexpr int kRows[4] = {8, 4, 2, 1};
-    constexpr float kIssue[4] = {8.3f, 5.3f, 3.8f, 2.6f};   // instructions per input, counted from the loop above
+// Which variant: the one whose busiest scheduler finishes first.  A warp alone on its scheduler advances one input
+// per 4 cycles (the addition's latency) or per the instructions it issues for an input; warps that share a scheduler
+// add up.  So a narrow projection of a few rows goes to one warp per row and 32 columns (1,152 columns x four rows:
+// 144 warps), and many rows or columns to the variants that issue less per product and read the weights fewer times.
+int project_variant(const int* n, int count, int rows, int sms) {
+    constexpr int kCols[3] = {64, 32, 32}, kRows[3] = {4, 4, 1};
+    constexpr float kIssue[3] = {9.5f, 5.3f, 2.6f};   // per input of a consumer warp, counted from the loop above
     int best = 0;
     float best_cost = 0.0f;
-    for (int i = 0; i < 4; ++i) {
-        if (kRows[i] >= 2 * rows) continue;
-        const int warps = col_blocks * ((rows + kRows[i] - 1) / kRows[i]);
-        const float cost = std::max(4.0f, kIssue[i] * (float)((warps + 4 * sms - 1) / (4 * sms)));
-        if (best == 0 || cost < best_cost) { best = kRows[i]; best_cost = cost; }
+    for (int v = 0; v < 3; ++v) {
+        int warps = 0;
+        for (int i = 0; i < count; ++i) warps += (n[i] + kCols[v] - 1) / kCols[v];
+        warps *= (rows + kRows[v] - 1) / kRows[v];
+        const float cost = std::max(4.0f, kIssue[v] * (float)((warps + 4 * sms - 1) / (4 * sms)));
+        if (v == 0 || cost < best_cost) { best = v; best_cost = cost; }
     }
     return best;
 }
@@ -563,47 +587,29 @@ __global__ void __launch_bounds__(256) gm_head_kernel(const bf16_t* q_in, const 
 }
 
 // ---------------------------------------------------------------------------------------------
-// Attention (attention.rs:203-277).  One block per (row, query head).  Keys and values pass through shared
-// memory in tiles of 64 positions, copied by the whole block with coalesced 128-bit loads (many loads in
-// flight per thread: the kernel is bound by load latency, not by arithmetic).  Scores: one thread per key,
-// the dot product in channel order, BF16 rounded, scaling 1.0.  Softmax in FP32 with the total added in key
-// order; weights rounded to BF16; the output accumulates weight x value in FP32 over the keys in position
-// order, one thread per channel.  window 0 = full attention.
-// Dynamic shared memory: one float per visible key (rounded up to 16 bytes), then the tile.
+// Attention (attention.rs:203-277).  One block per (row, query head).  Keys, then values, pass through two shared
+// memory tiles of TILE positions: while a tile is used, cp.async brings the next one (the first values arrive during
+// the softmax).  Scores: one thread per key, the dot product in channel order, BF16 rounded, scaling 1.0.  Softmax in
+// FP32 with the total added in key order; weights rounded to BF16; the output accumulates weight x value in FP32 over
+// the keys in position order, one thread per channel.  window 0 = full attention.
+// Bound by chains of dependent additions: the channels of a score once per tile, the keys of the total and of the
+// output.  A step of a few rows takes tiles of 128 positions, so that the scores of 128 keys run side by side; more
+// blocks than SMs take 64, which leaves room for three blocks per SM.  Tiles of 64 loaded between barriers, with
+// nothing in flight while a tile was used, took 36 us for 331 keys of four rows.
+// Dynamic shared memory: one float per visible key (rounded up to 16 bytes), then the tiles.
 // ---------------------------------------------------------------------------------------------
-constexpr int kAttnTile = 64;
+constexpr size_t kAttnSmemLimit = 200 * 1024;
 
-__host__ __device__ inline size_t attention_smem_bytes(int visible, int width) {
-    return (((size_t)visible * sizeof(float) + 15) & ~(size_t)15) + (size_t)kAttnTile * ((size_t)width * 2 + 16);
+__host__ __device__ inline size_t attention_smem_bytes(int tile, int visible, int width) {
+    return (((size_t)visible * sizeof(float) + 15) & ~(size_t)15) + 2 * (size_t)tile * ((size_t)width * 2 + 16);
+}
+// Tiles of 32 positions are for contexts whose scores leave no room for more.
+inline int attention_tile(int visible, int width, int blocks, int sms) {
+    if (blocks <= sms && attention_smem_bytes(128, visible, width) <= kAttnSmemLimit) return 128;
+    return attention_smem_bytes(64, visible, width) <= kAttnSmemLimit ? 64 : 32;
 }
 
-// Copies rows [t0, t0 + count) of a cache (row stride `stride` elements, `chunks` 16-byte chunks used per
-// row) into the tile, whose rows are pitched by 16 extra bytes.
-__device__ __forceinline__ void attention_load_tile(const bf16_t* base, size_t stride, int t0, int count, int chunks,
-                                                    unsigned char* tile, int pitch) {
-    const int total = count * chunks;
-    for (int first = 0; first < total; first += 8 * 256) {
-        // eight requests per thread leave before the first value is stored
-        uint4 v[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int idx = first + u * 256 + (int)threadIdx.x;
-            if (idx < total) {
-                const int key = idx / chunks, c = idx - key * chunks;
-                v[u] = __ldg(reinterpret_cast<const uint4*>(base + (size_t)(t0 + key) * stride) + c);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int idx = first + u * 256 + (int)threadIdx.x;
-            if (idx < total) {
-                const int key = idx / chunks, c = idx - key * chunks;
-                *reinterpret_cast<uint4*>(tile + (size_t)key * pitch + (size_t)c * 16) = v[u];
-            }
-        }
-    }
-}
-
+template <int TILE>
 __global__ void __launch_bounds__(256, 1) gm_attention_kernel(const bf16_t* q, const int* slot, const int* position,
                                                               const bf16_t* key_cache, const bf16_t* value_cache, int heads,
                                                               int kv_heads, int width, int window, int context, bf16_t* out) {
@@ -616,33 +622,63 @@ __global__ void __launch_bounds__(256, 1) gm_attention_kernel(const bf16_t* q, c
     const int last = pos, first = window > 0 ? max(0, pos - (window - 1)) : 0;
     const int visible = last - first + 1;
     float* scores = reinterpret_cast<float*>(attention_smem);
-    unsigned char* tile = attention_smem + (((size_t)visible * sizeof(float) + 15) & ~(size_t)15);
+    unsigned char* tiles = attention_smem + (((size_t)visible * sizeof(float) + 15) & ~(size_t)15);
     const int pitch = width * 2 + 16;
     const size_t stride = (size_t)kv_heads * width;
     const bf16_t* kbase = key_cache + ((size_t)slot[row] * context + first) * stride + (size_t)kv_head * width;
     const bf16_t* vbase = value_cache + ((size_t)slot[row] * context + first) * stride + (size_t)kv_head * width;
-    const int chunks = width / 8;
+    const int chunks = width / 8, steps = (visible + TILE - 1) / TILE;
+    // steps 0 .. steps - 1 bring the keys, the next as many the values; a warp copies whole positions
+    auto copy = [&](int step) {
+        if (step < 2 * steps) {
+            const int t0 = (step < steps ? step : step - steps) * TILE, count = min(TILE, visible - t0);
+            const bf16_t* base = (step < steps ? kbase : vbase) + (size_t)t0 * stride;
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(tiles) + (uint32_t)((step & 1) * TILE * pitch);
+#pragma unroll 4
+            for (int key = (int)threadIdx.x / 32; key < count; key += 8) {
+                for (int c = (int)threadIdx.x % 32; c < chunks; c += 32) {
+                    cp_async16(dst + (uint32_t)(key * pitch + c * 16), reinterpret_cast<const uint4*>(base + (size_t)key * stride) + c);
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // the tile of `step` is in place and the one before it, whose place step + 1 takes, has been used
+    auto next_tile = [&](int step) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        copy(step + 1);
+        return tiles + (size_t)(step & 1) * TILE * pitch;
+    };
+    copy(0);
     for (int i = threadIdx.x; i < chunks; i += blockDim.x) {
         query[i] = reinterpret_cast<const uint4*>(q + ((size_t)row * heads + h) * width)[i];
     }
     float maximum = -INFINITY;
-    for (int t0 = 0; t0 < visible; t0 += kAttnTile) {
-        const int count = min(kAttnTile, visible - t0);
-        __syncthreads();  // the previous tile has been consumed (and the query is in place)
-        attention_load_tile(kbase, stride, t0, count, chunks, tile, pitch);
-        __syncthreads();
-        if ((int)threadIdx.x < count) {
+    for (int step = 0; step < steps; ++step) {
+        const unsigned char* tile = next_tile(step);
+        const int t0 = step * TILE;
+        if ((int)threadIdx.x < min(TILE, visible - t0)) {
             const uint4* key = reinterpret_cast<const uint4*>(tile + (size_t)threadIdx.x * pitch);
             float sum = 0.0f;
-#pragma unroll 4
-            for (int i = 0; i < chunks; ++i) {
-                const uint4 kv = key[i];
-                const uint4 qq = query[i];
-                const uint32_t kk[4] = {kv.x, kv.y, kv.z, kv.w}, q4[4] = {qq.x, qq.y, qq.z, qq.w};
+            uint4 kv[2] = {key[0], key[min(1, chunks - 1)]}, qq[2] = {query[0], query[min(1, chunks - 1)]};
+#pragma unroll 2
+            for (int i = 0; i < chunks; i += 2) {   // two chunks read ahead of the two in use
+                uint4 next_k[2], next_q[2];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    sum = fmaf(__uint_as_float(q4[j] << 16), __uint_as_float(kk[j] << 16), sum);
-                    sum = fmaf(__uint_as_float(q4[j] & 0xffff0000u), __uint_as_float(kk[j] & 0xffff0000u), sum);
+                for (int u = 0; u < 2; ++u) {
+                    const int at = min(i + 2 + u, chunks - 1);
+                    next_k[u] = key[at];
+                    next_q[u] = query[at];
+                }
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    if (i + u < chunks) {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) sum = fmaf(bf_half(qq[u], e), bf_half(kv[u], e), sum);
+                    }
+                    kv[u] = next_k[u];
+                    qq[u] = next_q[u];
                 }
             }
             const float score = bf_load(bf_round(sum));
@@ -669,17 +705,15 @@ __global__ void __launch_bounds__(256, 1) gm_attention_kernel(const bf16_t* q, c
     for (int t = threadIdx.x; t < visible; t += blockDim.x) scores[t] = bf_load(bf_round(scores[t] / total));
     // weight x value, two channels per thread at most (width <= 512)
     float acc[2] = {0.0f, 0.0f};
-    for (int t0 = 0; t0 < visible; t0 += kAttnTile) {
-        const int count = min(kAttnTile, visible - t0);
-        __syncthreads();  // weights are final; the previous tile has been consumed
-        attention_load_tile(vbase, stride, t0, count, chunks, tile, pitch);
-        __syncthreads();
+    for (int step = 0; step < steps; ++step) {
+        const unsigned char* tile = next_tile(steps + step);   // its barrier also follows the last write of a weight
+        const int t0 = step * TILE, count = min(TILE, visible - t0);
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
             const int c = threadIdx.x + u * 256;
             if (c < width) {
                 const bf16_t* column = reinterpret_cast<const bf16_t*>(tile) + c;
-#pragma unroll 8
+#pragma unroll 16
                 for (int t = 0; t < count; ++t) acc[u] = fmaf(scores[t0 + t], bf_load(column[(size_t)t * (pitch / 2)]), acc[u]);
             }
         }
@@ -1148,16 +1182,17 @@ RIBN_B200_API int ribn_b200_gemma_finalize(ribn_b200_gemma* m) {
     {
         GM_CUDA(m, cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, m->cfg.device));
         const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
-        GM_CUDA(m, cudaFuncSetAttribute(gm_project_kernel<1>, at, kProjectMaxStages * project_stage_bytes(1)));
-        GM_CUDA(m, cudaFuncSetAttribute(gm_project_kernel<2>, at, kProjectMaxStages * project_stage_bytes(2)));
-        GM_CUDA(m, cudaFuncSetAttribute(gm_project_kernel<4>, at, kProjectMaxStages * project_stage_bytes(4)));
-        GM_CUDA(m, cudaFuncSetAttribute(gm_project_kernel<8>, at, kProjectMaxStages * project_stage_bytes(8)));
+        GM_CUDA(m, cudaFuncSetAttribute(gm_project_kernel<ProjectNarrow>, at, ProjectShape<ProjectNarrow>::smem_bytes));
+        GM_CUDA(m, cudaFuncSetAttribute(gm_project_kernel<ProjectRows4>, at, ProjectShape<ProjectRows4>::smem_bytes));
+        GM_CUDA(m, cudaFuncSetAttribute(gm_project_kernel<ProjectChunk>, at, ProjectShape<ProjectChunk>::smem_bytes));
     }
-    const size_t attention_bytes = attention_smem_bytes(c.context, c.head_dim > c.global_head_dim ? c.head_dim : c.global_head_dim);
-    if (attention_bytes > 48 * 1024) {
-        if (attention_bytes > 200 * 1024) return fail(m, RIBN_B200_ERROR, "context %d exceeds the attention kernel's score buffer", c.context);
-        GM_CUDA(m, cudaFuncSetAttribute(gm_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attention_bytes));
+    const int widest = c.head_dim > c.global_head_dim ? c.head_dim : c.global_head_dim;
+    if (attention_smem_bytes(32, c.context, widest) > kAttnSmemLimit) {
+        return fail(m, RIBN_B200_ERROR, "context %d exceeds the attention kernel's score buffer", c.context);
     }
+    GM_CUDA(m, cudaFuncSetAttribute(gm_attention_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAttnSmemLimit));
+    GM_CUDA(m, cudaFuncSetAttribute(gm_attention_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAttnSmemLimit));
+    GM_CUDA(m, cudaFuncSetAttribute(gm_attention_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAttnSmemLimit));
     m->finalized = true;
     return RIBN_B200_OK;
 }
@@ -1175,13 +1210,7 @@ struct Pass {
                       const int* n, bf16_t* const* out) {
         ProjectTargets t{};
         t.count = count;
-        unsigned col_blocks = 0;
-        for (int i = 0; i < count; ++i) {
-            t.w[i] = w[i]; t.out[i] = out[i]; t.n[i] = n[i];
-            t.first_block[i] = (int)col_blocks;
-            col_blocks += (unsigned)((n[i] + kProjectCols - 1) / kProjectCols);
-        }
-        const dim3 block(kProjectCols);
+        for (int i = 0; i < count; ++i) { t.w[i] = w[i]; t.out[i] = out[i]; t.n[i] = n[i]; }
         cudaStream_t s = m->stream;
         if ((m->cfg.flags & RIBN_B200_GEMMA_FLAG_TENSOR_CORE_PREFILL) && n_rows >= 16 && k % kMmaStageK == 0) {
             unsigned tile_blocks = 0;
@@ -1193,20 +1222,21 @@ struct Pass {
             ++launches;
             return;
         }
-        switch (project_rows((int)col_blocks, n_rows, m->sms)) {
-            case 1: launch_project<1>(in, row_index, n_rows, t, col_blocks, k); break;
-            case 2: launch_project<2>(in, row_index, n_rows, t, col_blocks, k); break;
-            case 4: launch_project<4>(in, row_index, n_rows, t, col_blocks, k); break;
-            default: launch_project<8>(in, row_index, n_rows, t, col_blocks, k); break;
+        switch (project_variant(n, count, n_rows, m->sms)) {
+            case 0: launch_project<ProjectChunk>(in, row_index, n_rows, t, k); break;
+            case 1: launch_project<ProjectRows4>(in, row_index, n_rows, t, k); break;
+            default: launch_project<ProjectNarrow>(in, row_index, n_rows, t, k); break;
         }
     }
-    template <int R>
-    void launch_project(const bf16_t* in, const int* row_index, int n_rows, const ProjectTargets& t, unsigned col_blocks, int k) {
-        const dim3 grid(col_blocks, (unsigned)((n_rows + R - 1) / R));
-        // as many stages as the blocks that share an SM leave room for: few blocks need more bytes in flight each
-        const int per_sm = ((int)(grid.x * grid.y) + m->sms - 1) / m->sms;
-        const int stages = std::max(2, std::min(kProjectMaxStages, 220 * 1024 / (per_sm * (project_stage_bytes(R) + 1024))));
-        gm_project_kernel<R><<<grid, kProjectThreads, (size_t)stages * project_stage_bytes(R), m->stream>>>(in, row_index, n_rows, t, k, stages);
+    template <typename V>
+    void launch_project(const bf16_t* in, const int* row_index, int n_rows, ProjectTargets& t, int k) {
+        using S = ProjectShape<V>;
+        unsigned col_blocks = 0;
+        for (int i = 0; i < t.count; ++i) {
+            t.first_block[i] = (int)col_blocks;
+            col_blocks += (unsigned)((t.n[i] + S::cols - 1) / S::cols);
+        }
+        gm_project_kernel<V><<<dim3(col_blocks, (unsigned)((n_rows + S::rows - 1) / S::rows)), S::threads, S::smem_bytes, m->stream>>>(in, row_index, n_rows, t, k);
         ++launches;
     }
     void project(const bf16_t* in, const int* row_index, int n_rows, const bf16_t* w, int n, int k, bf16_t* out) {
@@ -1263,7 +1293,9 @@ int enqueue_pass(ribn_b200_gemma* m, int rows, int n_out, int max_position, uint
         ++p.launches;
         const int window = kind ? 0 : c.window;
         const int visible = window > 0 && window < max_position + 1 ? window : max_position + 1;
-        gm_attention_kernel<<<dim3((unsigned)rows, (unsigned)c.heads), 256, attention_smem_bytes(visible, w), s>>>(
+        const int tile = attention_tile(visible, w, rows * c.heads, m->sms);
+        const auto attention = tile == 128 ? gm_attention_kernel<128> : tile == 64 ? gm_attention_kernel<64> : gm_attention_kernel<32>;
+        attention<<<dim3((unsigned)rows, (unsigned)c.heads), 256, attention_smem_bytes(tile, visible, w), s>>>(
             m->q2, m->d_slot, m->d_position, m->key_cache[(size_t)cache], m->value_cache[(size_t)cache], c.heads, c.kv_heads, w,
             window, c.context, m->attended);
         ++p.launches;
