@@ -57,6 +57,19 @@ __host__ __device__ __forceinline__ bf16_t bf_round(float value) {
 // equals the reference's multiply-then-add.  Transcendentals are evaluated in double and rounded once,
 // which is what the host libm's float routines return in all but rare cases.
 
+__device__ __forceinline__ float bf_half(const uint4& v, int e) {   // value e of eight BF16 values; e is a constant after unrolling
+    const uint32_t w = e < 2 ? v.x : e < 4 ? v.y : e < 6 ? v.z : v.w;
+    return __uint_as_float(e & 1 ? w & 0xffff0000u : w << 16);
+}
+
+// The kernels of a pass are launched so that each may start while the one before it ends: its blocks take their places
+// and fetch what no kernel writes (weights), then wait here for everything before them.  Every kernel of a pass waits,
+// so a kernel that has finished waiting follows all earlier ones.
+__device__ __forceinline__ void wait_for_previous() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 __device__ __forceinline__ float block_max(float v, float* scratch) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = (blockDim.x + 31) >> 5;
 #pragma unroll
@@ -106,13 +119,16 @@ __device__ __forceinline__ bf16_t gelu_round(bf16_t v) {
 // Embedding rows: hidden = bf16(embed[token] * sqrt(H) as BF16), identity = bf16(ple_embed[token] * sqrt(P) as BF16)
 // (decoder.rs:346-360).  One block per row.
 // ---------------------------------------------------------------------------------------------
-__global__ void gm_embed_kernel(const uint32_t* tokens, const bf16_t* embed, const bf16_t* ple_embed, int hidden, int packed,
-                                float embed_scale, float ple_scale, bf16_t* out_hidden, bf16_t* out_identity) {
+__global__ void gm_embed_kernel(const uint32_t* tokens, const bf16_t* __restrict__ embed, const bf16_t* __restrict__ ple_embed, int hidden, int packed,
+                                float embed_scale, float ple_scale, bf16_t* __restrict__ out_hidden, bf16_t* __restrict__ out_identity) {
+    wait_for_previous();
     const int row = blockIdx.x;
     const size_t token = tokens[row];
+#pragma unroll 4
     for (int i = threadIdx.x; i < hidden; i += blockDim.x) {
         out_hidden[(size_t)row * hidden + i] = bf_round(bf_load(embed[token * hidden + i]) * embed_scale);
     }
+#pragma unroll 4
     for (int i = threadIdx.x; i < packed; i += blockDim.x) {
         out_identity[(size_t)row * packed + i] = bf_round(bf_load(ple_embed[token * packed + i]) * ple_scale);
     }
@@ -121,26 +137,25 @@ __global__ void gm_embed_kernel(const uint32_t* tokens, const bf16_t* embed, con
 // ---------------------------------------------------------------------------------------------
 // Projection: out[r][n] = bf16(sum_k in[r][k] * w[n][k]) (linear.rs:23-66), the sum in k order.  A block is a
 // feeder warp and G consumer warps.  A consumer owns 32 * C output columns for R rows: a thread walks C weight rows
-// and keeps R * C independent accumulation chains, rows packed in pairs (`fma.rn.f32x2` rounds each half as `fmaf`
-// does).  The feeder brings weight tiles by cp.async into a ring of stages (rows pitched 16 bytes apart from a
-// multiple of 128, so the 128-bit reads of a quarter-warp fall in distinct banks) and writes the input rows
-// expanded to FP32, in the order the consumers read them.  Named barriers hand the stages over; their ids are
-// constants because an SM has 64 barriers and a block whose ids are computed is given 16 of them.
+// and keeps R * C independent accumulation chains.  The feeder brings tiles of the weights and of the blocks' input
+// rows by cp.async into a ring of stages (rows pitched 16 bytes apart from a multiple of 128, so the 128-bit reads of
+// a quarter-warp fall in distinct banks).  Named barriers hand the stages over; their ids are constants because an
+// SM has 64 barriers and a block whose ids are computed is given 16 of them.
 //
 // What bounds it: the chain of dependent additions, 4 cycles per input (14.4 us for the 6,912 inputs of a down
-// projection), or, with several warps per scheduler, the instructions issued per input and the broadcast reads of
-// the input rows, which cost shared memory as much as distinct ones: two columns per thread halve them.
+// projection), or, with several chains per scheduler, the instructions issued per input and the shared-memory reads.
+// A scheduler's reads return 64 bytes per cycle, broadcast or not, so the input rows stay BF16 (expanded to FP32 in
+// shared memory they cost twice the reads: 14 instead of 10 cycles per input at four rows).
 // ---------------------------------------------------------------------------------------------
 struct ProjectNarrow { static constexpr int R = 1, C = 1, G = 1, tile = 256, stages = 4; };   // a few rows: chains spread over blocks
-struct ProjectRows4 { static constexpr int R = 4, C = 1, G = 1, tile = 256, stages = 3; };    // a few rows of a wide projection
-struct ProjectChunk { static constexpr int R = 4, C = 2, G = 2, tile = 128, stages = 2; };    // prefill
+struct ProjectWide { static constexpr int R = 4, C = 1, G = 1, tile = 256, stages = 3; };     // a few rows of a wide projection
+struct ProjectRows { static constexpr int R = 4, C = 1, G = 4, tile = 256, stages = 3; };     // a few tens of rows
+struct ProjectChunk { static constexpr int R = 4, C = 2, G = 4, tile = 128, stages = 3; };    // prefill
 template <typename V>
 struct ProjectShape {
     static constexpr int cols = 32 * V::C, rows = V::R * V::G, threads = 32 * (1 + V::G);
-    static constexpr int chunks = V::tile / 8, pitch = V::tile * 2 + 16;        // 16-byte chunks, and bytes between weight rows of a tile
-    // floats of eight inputs of a consumer's rows: padded so that the feeder's stores fall in distinct banks
-    static constexpr int x_warp = V::R == 1 ? 8 : 9 * V::R, x_pitch = x_warp * V::G;
-    static constexpr int x_offset = cols * pitch, stage_bytes = x_offset + chunks * x_pitch * 4, smem_bytes = V::stages * stage_bytes;
+    static constexpr int chunks = V::tile / 8, pitch = V::tile * 2 + 16;        // 16-byte chunks, and bytes between rows of a tile
+    static constexpr int stage_bytes = (cols + rows) * pitch, smem_bytes = V::stages * stage_bytes;
 };
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
@@ -159,15 +174,6 @@ __device__ __forceinline__ void stage_barrier(int slot, bool wait) {
     else if (STAGES <= 3 || slot == 2) stage_barrier<FIRST + (STAGES > 2 ? 2 : 0), THREADS>(wait);
     else stage_barrier<FIRST + (STAGES > 3 ? 3 : 0), THREADS>(wait);
 }
-__device__ __forceinline__ unsigned long long fma_pair(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ float bf_half(const uint4& v, int e) {   // value e of eight BF16 values; e is a constant after unrolling
-    const uint32_t w = e < 2 ? v.x : e < 4 ? v.y : e < 6 ? v.z : v.w;
-    return __uint_as_float(e & 1 ? w & 0xffff0000u : w << 16);
-}
 
 // Up to three matrices that read the same input rows share one launch (q | k | v, gate | up): their
 // column blocks are laid side by side in the grid.
@@ -180,14 +186,11 @@ struct ProjectTargets {
 };
 
 template <typename V>
-__global__ void __launch_bounds__(ProjectShape<V>::threads) gm_project_kernel(const bf16_t* __restrict__ in,
-                                                                              const int* __restrict__ row_index, int rows,
-                                                                              const ProjectTargets targets, int k) {
+__global__ void __launch_bounds__(ProjectShape<V>::threads) gm_project_kernel(const bf16_t* __restrict__ in, int rows,
+                                                                              const __grid_constant__ ProjectTargets targets, int k) {
     extern __shared__ __align__(16) unsigned char project_smem[];
     using S = ProjectShape<V>;
     constexpr int R = V::R, C = V::C, kStages = V::stages, kThreads = S::threads;
-    constexpr int kRowsPerIssue = 32 / S::chunks;              // weight rows one warp-wide copy instruction covers
-    constexpr int kPieces = S::rows * S::chunks / 32;          // 16-byte pieces of the input rows per lane and tile
     const int lane = threadIdx.x & 31;
     int which = 0;
     if (targets.count > 1 && (int)blockIdx.x >= targets.first_block[1]) which = 1;
@@ -196,129 +199,91 @@ __global__ void __launch_bounds__(ProjectShape<V>::threads) gm_project_kernel(co
     const int col0 = ((int)blockIdx.x - targets.first_block[which]) * S::cols;
     const int r0 = blockIdx.y * S::rows;
     const int live_cols = min(S::cols, n - col0);
-    const int chunks = k / 8;  // 16-byte chunks per weight row
+    const int chunks = k / 8;  // 16-byte chunks per row
     const int tiles = (chunks + S::chunks - 1) / S::chunks;
 
     if (threadIdx.x < 32) {   // feeder
+        constexpr int kRowsPerIssue = 32 / S::chunks;              // rows one warp-wide copy instruction covers
         const int piece = lane % S::chunks, sub_row = lane / S::chunks;
         const uint4* wsrc = reinterpret_cast<const uint4*>(targets.w[which] + (size_t)(col0 + sub_row) * k) + piece;
+        const uint4* xsrc = reinterpret_cast<const uint4*>(in) + piece;
         const uint32_t wdst = (uint32_t)__cvta_generic_to_shared(project_smem) + (uint32_t)(sub_row * S::pitch + piece * 16);
-        auto copy = [&](int tile, int slot) {
+        auto copy_weights = [&](int tile, int slot) {
             const int c = tile * S::chunks;
-            if (tile < tiles && c + piece < chunks) {
-                const uint4* src = wsrc + c;
-                uint32_t dst = wdst + (uint32_t)(slot * S::stage_bytes);
+            if (tile >= tiles || c + piece >= chunks) return;
+            const uint4* src = wsrc + c;
+            uint32_t dst = wdst + (uint32_t)(slot * S::stage_bytes);
 #pragma unroll 8
-                for (int j = sub_row; j < live_cols; j += kRowsPerIssue, dst += kRowsPerIssue * S::pitch, src += (size_t)kRowsPerIssue * chunks) {
-                    cp_async16(dst, src);
-                }
+            for (int j = sub_row; j < live_cols; j += kRowsPerIssue, dst += kRowsPerIssue * S::pitch, src += (size_t)kRowsPerIssue * chunks) {
+                cp_async16(dst, src);
             }
+        };
+        auto copy_rows = [&](int tile, int slot) {
+            const int c = tile * S::chunks;
+            if (tile >= tiles || c + piece >= chunks) return;
+            const uint32_t dst = wdst + (uint32_t)(slot * S::stage_bytes + S::cols * S::pitch);
+#pragma unroll
+            for (int j = 0; j < S::rows; j += kRowsPerIssue) {
+                if (j + sub_row < S::rows) cp_async16(dst + (uint32_t)(j * S::pitch), xsrc + (size_t)min(r0 + j + sub_row, rows - 1) * chunks + c);
+            }
+        };
+#pragma unroll
+        for (int t = 0; t < kStages - 1; ++t) copy_weights(t, t);   // weights need nothing of the kernel before this one
+        wait_for_previous();
+#pragma unroll
+        for (int t = 0; t < kStages - 1; ++t) {
+            copy_rows(t, t);
             asm volatile("cp.async.commit_group;" ::: "memory");
-        };
-        // a lane's pieces of the input rows: one row, chunk lane / rows and every 32 / rows after it
-        const int own = lane % S::rows, row = min(r0 + own, rows - 1), first_chunk = lane / S::rows;
-        const uint4* xsrc = reinterpret_cast<const uint4*>(in + (size_t)(row_index ? row_index[row] : row) * k);
-        uint4 x[kPieces];
-        auto read = [&](int tile) {
-#pragma unroll
-            for (int i = 0; i < kPieces; ++i) {
-                const int c = tile * S::chunks + first_chunk + i * (32 / S::rows);
-                x[i] = c < chunks ? xsrc[c] : make_uint4(0, 0, 0, 0);
-            }
-        };
-#pragma unroll
-        for (int t = 0; t < kStages - 1; ++t) copy(t, t);
-        read(0);
+        }
         int slot = 0, ahead = kStages - 1;   // slots of tile t and of tile t + kStages - 1
         for (int t = 0; t < tiles; ++t) {
-            // the input rows first: they need nothing but the slot, which was free when its weights were requested
-            float* xf = reinterpret_cast<float*>(project_smem + (size_t)slot * S::stage_bytes + S::x_offset) + own / R * S::x_warp;
-#pragma unroll
-            for (int i = 0; i < kPieces; ++i) {
-                float* dst = xf + (first_chunk + i * (32 / S::rows)) * S::x_pitch;
-                if constexpr (R == 1) {
-                    reinterpret_cast<float4*>(dst)[0] = make_float4(bf_half(x[i], 0), bf_half(x[i], 1), bf_half(x[i], 2), bf_half(x[i], 3));
-                    reinterpret_cast<float4*>(dst)[1] = make_float4(bf_half(x[i], 4), bf_half(x[i], 5), bf_half(x[i], 6), bf_half(x[i], 7));
-                } else {
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) dst[e * R + own % R] = bf_half(x[i], e);
-                }
-            }
-            read(t + 1);
             asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");   // tile t; younger copies stay in flight
             __syncwarp();
             stage_barrier<1, kStages, kThreads>(slot, false);
             if (t > 0 && t - 1 + kStages < tiles) stage_barrier<1 + kStages, kStages, kThreads>(ahead, true);   // the consumers have left tile t - 1
-            copy(t + kStages - 1, ahead);
+            copy_weights(t + kStages - 1, ahead);
+            copy_rows(t + kStages - 1, ahead);
+            asm volatile("cp.async.commit_group;" ::: "memory");
             slot = slot + 1 == kStages ? 0 : slot + 1;
             ahead = ahead + 1 == kStages ? 0 : ahead + 1;
         }
         return;
     }
 
+    wait_for_previous();
     const int g = (int)threadIdx.x / 32 - 1;
-    using Pair = unsigned long long;
-    // eight inputs: C weight rows' values and the R rows' inputs, read one group ahead of their use
-    constexpr int kAhead = R == 1 ? 2 : 1, kXVectors = 2 * R;
-    struct Group { uint4 w[C]; ulonglong2 x[kXVectors]; };
-    Pair acc[C][R == 1 ? 1 : R / 2];
-    float sum = 0.0f;
+    float sum[C][R];
 #pragma unroll
     for (int c = 0; c < C; ++c) {
 #pragma unroll
-        for (int q = 0; q < (R == 1 ? 1 : R / 2); ++q) acc[c][q] = 0;
+        for (int r = 0; r < R; ++r) sum[c][r] = 0.0f;
     }
     int slot = 0;
     for (int t = 0; t < tiles; ++t) {
         stage_barrier<1, kStages, kThreads>(slot, true);
-        const unsigned char* stage = project_smem + (size_t)slot * S::stage_bytes;
-        const unsigned char* ws = stage + lane * S::pitch;
-        const float* xf = reinterpret_cast<const float*>(stage + S::x_offset) + g * S::x_warp;
+        const unsigned char* ws = project_smem + (size_t)slot * S::stage_bytes + lane * S::pitch;
+        const unsigned char* xs = project_smem + (size_t)slot * S::stage_bytes + (S::cols + g * R) * S::pitch;
         const int count = min(S::chunks, chunks - t * S::chunks);
-        auto fetch = [&](Group& to, int i) {
+        auto chunk = [&](int i) {
+            uint4 wv[C], xv[R];
 #pragma unroll
-            for (int c = 0; c < C; ++c) to.w[c] = *reinterpret_cast<const uint4*>(ws + c * 32 * S::pitch + i * 16);
+            for (int c = 0; c < C; ++c) wv[c] = *reinterpret_cast<const uint4*>(ws + c * 32 * S::pitch + i * 16);
 #pragma unroll
-            for (int v = 0; v < kXVectors; ++v) to.x[v] = reinterpret_cast<const ulonglong2*>(xf + i * S::x_pitch)[v];
-        };
-        auto add = [&](const Group& from) {
+            for (int r = 0; r < R; ++r) xv[r] = *reinterpret_cast<const uint4*>(xs + r * S::pitch + i * 16);
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-                if constexpr (R == 1) {
-                    const Pair two = e % 4 < 2 ? from.x[e / 4].x : from.x[e / 4].y;
-                    float lo, hi;
-                    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(two));
-                    sum = fmaf(e & 1 ? hi : lo, bf_half(from.w[0], e), sum);
-                } else {
 #pragma unroll
-                    for (int c = 0; c < C; ++c) {
-                        const float w = bf_half(from.w[c], e);
-                        Pair ww;
-                        asm("mov.b64 %0, {%1, %1};" : "=l"(ww) : "f"(w));
+                for (int c = 0; c < C; ++c) {
 #pragma unroll
-                        for (int q = 0; q < R / 2; ++q) {
-                            const ulonglong2 v = from.x[e * (R / 4) + q / 2];
-                            acc[c][q] = fma_pair(q & 1 ? v.y : v.x, ww, acc[c][q]);
-                        }
-                    }
+                    for (int r = 0; r < R; ++r) sum[c][r] = fmaf(bf_half(xv[r], e), bf_half(wv[c], e), sum[c][r]);
                 }
             }
         };
         if (count == S::chunks) {
-            Group now[kAhead], next[kAhead];
-#pragma unroll
-            for (int u = 0; u < kAhead; ++u) fetch(now[u], u);
-#pragma unroll 2
-            for (int i = 0; i < S::chunks; i += kAhead) {
-#pragma unroll
-                for (int u = 0; u < kAhead; ++u) fetch(next[u], min(i + kAhead + u, S::chunks - 1));
-#pragma unroll
-                for (int u = 0; u < kAhead; ++u) add(now[u]);
-#pragma unroll
-                for (int u = 0; u < kAhead; ++u) now[u] = next[u];
-            }
+#pragma unroll(R == 1 ? 8 : 4)
+            for (int i = 0; i < S::chunks; ++i) chunk(i);
         } else {
-            for (int i = 0; i < count; ++i) { Group one; fetch(one, i); add(one); }
+            for (int i = 0; i < count; ++i) chunk(i);
         }
         if (t + kStages < tiles) stage_barrier<1 + kStages, kStages, kThreads>(slot, false);
         slot = slot + 1 == kStages ? 0 : slot + 1;
@@ -327,17 +292,10 @@ __global__ void __launch_bounds__(ProjectShape<V>::threads) gm_project_kernel(co
     for (int c = 0; c < C; ++c) {
         if (lane + 32 * c >= live_cols) break;
         bf16_t* out = targets.out[which] + col0 + lane + 32 * c;
-        const int first = r0 + g * R;
-        if constexpr (R == 1) {
-            out[(size_t)first * n] = bf_round(sum);
-        } else {
 #pragma unroll
-            for (int q = 0; q < R / 2; ++q) {
-                float lo, hi;
-                asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc[c][q]));
-                if (first + 2 * q < rows) out[(size_t)(first + 2 * q) * n] = bf_round(lo);
-                if (first + 2 * q + 1 < rows) out[(size_t)(first + 2 * q + 1) * n] = bf_round(hi);
-            }
+        for (int r = 0; r < R; ++r) {
+            const int row = r0 + g * R + r;
+            if (row < rows) out[(size_t)row * n] = bf_round(sum[c][r]);
         }
     }
 }
@@ -347,15 +305,16 @@ __global__ void __launch_bounds__(ProjectShape<V>::threads) gm_project_kernel(co
 // add up.  So a narrow projection of a few rows goes to one warp per row and 32 columns (1,152 columns x four rows:
 // 144 warps), and many rows or columns to the variants that issue less per product and read the weights fewer times.
 int project_variant(const int* n, int count, int rows, int sms) {
-    constexpr int kCols[3] = {64, 32, 32}, kRows[3] = {4, 4, 1};
-    constexpr float kIssue[3] = {9.5f, 5.3f, 2.6f};   // per input of a consumer warp, counted from the loop above
+    constexpr int kCols[4] = {64, 32, 32, 32}, kRows[4] = {16, 16, 4, 1}, kWarps[4] = {4, 4, 1, 1};
+    constexpr float kIssue[4] = {15.0f, 9.8f, 9.8f, 3.4f};   // per input of a consumer warp, counted from the loop above
     int best = 0;
     float best_cost = 0.0f;
-    for (int v = 0; v < 3; ++v) {
-        int warps = 0;
-        for (int i = 0; i < count; ++i) warps += (n[i] + kCols[v] - 1) / kCols[v];
-        warps *= (rows + kRows[v] - 1) / kRows[v];
-        const float cost = std::max(4.0f, kIssue[v] * (float)((warps + 4 * sms - 1) / (4 * sms)));
+    for (int v = 0; v < 4; ++v) {
+        int blocks = 0;
+        for (int i = 0; i < count; ++i) blocks += (n[i] + kCols[v] - 1) / kCols[v];
+        blocks *= (rows + kRows[v] - 1) / kRows[v];
+        const int per_sm = (blocks + sms - 1) / sms, per_scheduler = (per_sm * kWarps[v] + 3) / 4;
+        const float cost = std::max(4.0f, kIssue[v] * (float)per_scheduler);
         if (v == 0 || cost < best_cost) { best = v; best_cost = cost; }
     }
     return best;
@@ -465,60 +424,59 @@ __global__ void __launch_bounds__(128) gm_project_mma_kernel(const bf16_t* __res
 //   mode 0: out = bf16(x * inverse * scale)
 //   mode 1: out = bf16(residual + mode 0)                         (post-norm + residual add)
 //   mode 2: out = bf16(mode 1 * scalar)                           (end of a layer: layer scalar)
-// row_index gathers input rows (the rows that want logits).  Dynamic shared memory: width floats.
+// row_index gathers input rows (the rows that want logits).  With `next_scale` the block goes on to normalise the row
+// that it has just written (mode 0, into next_out): the norm that follows a post-norm needs no launch of its own.
+// Bound by the ordered sum, 4 cycles per value.  Dynamic shared memory: width floats.
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) gm_rms_kernel(const bf16_t* in, const int* row_index, int width, float eps,
                                                      const bf16_t* scale, const bf16_t* residual, const bf16_t* scalar,
-                                                     int mode, bf16_t* out) {
+                                                     int mode, bf16_t* out, const bf16_t* next_scale, bf16_t* next_out) {
     extern __shared__ __align__(16) float squares[];
     __shared__ float slot;
+    wait_for_previous();
     const int row = blockIdx.x;
     const uint4* x = reinterpret_cast<const uint4*>(in + (size_t)(row_index ? row_index[row] : row) * width);
-    const uint4* sc = reinterpret_cast<const uint4*>(scale);
     const uint4* res = reinterpret_cast<const uint4*>(residual + (mode >= 1 ? (size_t)row * width : 0));
     uint4* dst = reinterpret_cast<uint4*>(out + (size_t)row * width);
     const int chunks = width / 8;
-    // Eight values per thread per trip; everything a trip needs is requested before the sum starts.
-    for (int c0 = 0; c0 < chunks; c0 += blockDim.x) {
-        const int c = c0 + threadIdx.x;
-        if (c < chunks) {
-            const uint4 v = __ldg(x + c);
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    const float factor = mode == 2 ? bf_load(scalar[0]) : 1.0f;
+    for (int pass = 0; pass < (next_scale ? 2 : 1); ++pass) {
+        const uint4* sc = reinterpret_cast<const uint4*>(pass ? next_scale : scale);
+        if (pass) { x = dst; dst = reinterpret_cast<uint4*>(next_out + (size_t)row * width); }   // a thread reads back what it wrote
+        const int how = pass ? 0 : mode;
+        // Eight values per thread per trip; everything a trip needs is requested before the sum starts.
+        for (int c = threadIdx.x; c < chunks; c += blockDim.x) {
+            const uint4 v = x[c];
+            float4* to = reinterpret_cast<float4*>(squares + c * 8);
+            float f[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] = bf_half(v, e) * bf_half(v, e);
+            to[0] = make_float4(f[0], f[1], f[2], f[3]);
+            to[1] = make_float4(f[4], f[5], f[6], f[7]);
+        }
+        const float energy = ordered_energy(squares, width, &slot);
+        const float inverse = inverse_root(energy / (float)width + eps);
+        for (int c = threadIdx.x; c < chunks; c += blockDim.x) {
+            const uint4 v = x[c];
+            const uint4 sv = sc ? __ldg(sc + c) : make_uint4(0, 0, 0, 0);
+            const uint4 rv = how >= 1 ? res[c] : make_uint4(0, 0, 0, 0);
+            uint32_t ow[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const float lo = __uint_as_float(w[j] << 16), hi = __uint_as_float(w[j] & 0xffff0000u);
-                squares[c * 8 + 2 * j] = lo * lo;
-                squares[c * 8 + 2 * j + 1] = hi * hi;
-            }
-        }
-    }
-    const float energy = ordered_energy(squares, width, &slot);
-    const float inverse = inverse_root(energy / (float)width + eps);
-    const float factor = mode == 2 ? bf_load(scalar[0]) : 1.0f;
-    for (int c0 = 0; c0 < chunks; c0 += blockDim.x) {
-        const int c = c0 + threadIdx.x;
-        if (c >= chunks) continue;
-        const uint4 v = __ldg(x + c);
-        const uint4 sv = scale ? __ldg(sc + c) : make_uint4(0, 0, 0, 0);
-        const uint4 rv = mode >= 1 ? res[c] : make_uint4(0, 0, 0, 0);
-        const uint32_t xw[4] = {v.x, v.y, v.z, v.w}, sw[4] = {sv.x, sv.y, sv.z, sv.w}, rw[4] = {rv.x, rv.y, rv.z, rv.w};
-        uint32_t ow[4];
+                bf16_t pair[2];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            bf16_t pair[2];
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const bf16_t xb = (bf16_t)(e ? xw[j] >> 16 : xw[j] & 0xffffu);
-                float value = bf_load(xb) * inverse;
-                if (scale) value *= bf_load((bf16_t)(e ? sw[j] >> 16 : sw[j] & 0xffffu));
-                bf16_t r = bf_round(value);
-                if (mode >= 1) r = bf_round(bf_load((bf16_t)(e ? rw[j] >> 16 : rw[j] & 0xffffu)) + bf_load(r));
-                if (mode == 2) r = bf_round(bf_load(r) * factor);
-                pair[e] = r;
+                for (int e = 0; e < 2; ++e) {
+                    float value = bf_half(v, 2 * j + e) * inverse;
+                    if (sc) value *= bf_half(sv, 2 * j + e);
+                    bf16_t r = bf_round(value);
+                    if (how >= 1) r = bf_round(bf_half(rv, 2 * j + e) + bf_load(r));
+                    if (how == 2) r = bf_round(bf_load(r) * factor);
+                    pair[e] = r;
+                }
+                ow[j] = (uint32_t)pair[0] | ((uint32_t)pair[1] << 16);
             }
-            ow[j] = (uint32_t)pair[0] | ((uint32_t)pair[1] << 16);
+            dst[c] = make_uint4(ow[0], ow[1], ow[2], ow[3]);
         }
-        dst[c] = make_uint4(ow[0], ow[1], ow[2], ow[3]);
     }
 }
 
@@ -538,6 +496,7 @@ __global__ void __launch_bounds__(256) gm_head_kernel(const bf16_t* q_in, const 
     __shared__ __align__(16) float squares[512];
     __shared__ float energy_slot;
     __shared__ bf16_t normed[512];
+    wait_for_previous();
     const int row = blockIdx.x, h = blockIdx.y, half = width / 2, pos = position[row];
     const bf16_t* x;
     const bf16_t* scale = nullptr;
@@ -617,6 +576,7 @@ __global__ void __launch_bounds__(256, 1) gm_attention_kernel(const bf16_t* q, c
     __shared__ float scratch[8];
     __shared__ float total_slot;
     __shared__ uint4 query[64];  // up to 512 BF16 channels
+    wait_for_previous();
     const int row = blockIdx.x, h = blockIdx.y, pos = position[row];
     const int kv_head = h / (heads / kv_heads);
     const int last = pos, first = window > 0 ? max(0, pos - (window - 1)) : 0;
@@ -727,6 +687,7 @@ __global__ void __launch_bounds__(256, 1) gm_attention_kernel(const bf16_t* q, c
 
 // out = bf16(bf16(gelu(gate)) * other)   (decoder.rs:592-593 and 608-609)
 __global__ void gm_gelu_mul_kernel(const bf16_t* gate, const bf16_t* other, size_t n, bf16_t* out) {
+    wait_for_previous();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = bf_round(bf_load(gelu_round(gate[i])) * bf_load(other[i]));
 }
@@ -740,6 +701,7 @@ __global__ void __launch_bounds__(256) gm_ple_kernel(const bf16_t* projection, c
     __shared__ __align__(16) float squares[1024];
     __shared__ float energy_slot;
     __shared__ bf16_t scaled[1024];
+    wait_for_previous();
     const int row = blockIdx.x, layer = blockIdx.y;
     const bf16_t* p = projection + (size_t)row * packed + (size_t)layer * ple;
     const bf16_t* id = identity + (size_t)row * packed + (size_t)layer * ple;
@@ -762,6 +724,7 @@ __global__ void __launch_bounds__(256) gm_ple_kernel(const bf16_t* projection, c
 
 // Soft cap (elementwise.rs:85-107): divide, tanh, multiply, each rounded.
 __global__ void gm_softcap_kernel(bf16_t* logits, size_t n, float cap) {
+    wait_for_previous();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const bf16_t divided = bf_round(__fdiv_rn(bf_load(logits[i]), cap));
@@ -774,6 +737,7 @@ __global__ void gm_softcap_kernel(bf16_t* logits, size_t n, float cap) {
 __global__ void __launch_bounds__(1024) gm_argmax_kernel(const bf16_t* logits, int vocab, uint32_t* out) {
     __shared__ float best_value[32];
     __shared__ int best_index[32];
+    wait_for_previous();
     const bf16_t* x = logits + (size_t)blockIdx.x * vocab;
     const float head = bf_load(x[0]);
     if (head != head) {  // nothing compares greater than a NaN incumbent
@@ -782,7 +746,18 @@ __global__ void __launch_bounds__(1024) gm_argmax_kernel(const bf16_t* logits, i
     }
     float value = -INFINITY;
     int index = 0x7fffffff;
-    for (int i = threadIdx.x; i < vocab; i += blockDim.x) {
+    // four 128-bit loads in flight per thread (one value at a time took 20 us for 32,768)
+    const int vectors = vocab % 8 == 0 ? vocab / 8 : 0;
+#pragma unroll 4
+    for (int c = threadIdx.x; c < vectors; c += blockDim.x) {
+        const uint4 eight = reinterpret_cast<const uint4*>(x)[c];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const float v = bf_half(eight, e);
+            if (v > value || (v == value && c * 8 + e < index)) { value = v; index = c * 8 + e; }
+        }
+    }
+    for (int i = vectors * 8 + threadIdx.x; i < vocab; i += blockDim.x) {
         const float v = bf_load(x[i]);
         if (v > value || (v == value && i < index)) { value = v; index = i; }
     }
@@ -1183,7 +1158,8 @@ RIBN_B200_API int ribn_b200_gemma_finalize(ribn_b200_gemma* m) {
         GM_CUDA(m, cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, m->cfg.device));
         const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
         GM_CUDA(m, cudaFuncSetAttribute(gm_project_kernel<ProjectNarrow>, at, ProjectShape<ProjectNarrow>::smem_bytes));
-        GM_CUDA(m, cudaFuncSetAttribute(gm_project_kernel<ProjectRows4>, at, ProjectShape<ProjectRows4>::smem_bytes));
+        GM_CUDA(m, cudaFuncSetAttribute(gm_project_kernel<ProjectWide>, at, ProjectShape<ProjectWide>::smem_bytes));
+        GM_CUDA(m, cudaFuncSetAttribute(gm_project_kernel<ProjectRows>, at, ProjectShape<ProjectRows>::smem_bytes));
         GM_CUDA(m, cudaFuncSetAttribute(gm_project_kernel<ProjectChunk>, at, ProjectShape<ProjectChunk>::smem_bytes));
     }
     const int widest = c.head_dim > c.global_head_dim ? c.head_dim : c.global_head_dim;
@@ -1206,50 +1182,65 @@ struct Pass {
     int rows;
     uint32_t launches = 0;
 
-    void project_many(const bf16_t* in, const int* row_index, int n_rows, int k, int count, const bf16_t* const* w,
+    // A launch that may begin while the kernel before it ends (`wait_for_previous`).
+    template <typename... Params, typename... Args>
+    void launch(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, Args... args) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = grid;
+        cfg.blockDim = dim3((unsigned)threads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = m->stream;
+        cudaLaunchAttribute attribute{};
+        attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attribute.val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = &attribute;
+        cfg.numAttrs = launches > 0 ? 1 : 0;   // the first kernel follows the copies of the pass's rows
+        cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);   // its error is read at the end of the pass
+        ++launches;
+    }
+    void project_many(const bf16_t* in, int n_rows, int k, int count, const bf16_t* const* w,
                       const int* n, bf16_t* const* out) {
         ProjectTargets t{};
         t.count = count;
         for (int i = 0; i < count; ++i) { t.w[i] = w[i]; t.out[i] = out[i]; t.n[i] = n[i]; }
-        cudaStream_t s = m->stream;
         if ((m->cfg.flags & RIBN_B200_GEMMA_FLAG_TENSOR_CORE_PREFILL) && n_rows >= 16 && k % kMmaStageK == 0) {
             unsigned tile_blocks = 0;
             for (int i = 0; i < count; ++i) {
                 t.first_block[i] = (int)tile_blocks;
                 tile_blocks += (unsigned)((n[i] + kMmaTile - 1) / kMmaTile);
             }
-            gm_project_mma_kernel<<<dim3(tile_blocks, (unsigned)((n_rows + kMmaTile - 1) / kMmaTile)), 128, 0, s>>>(in, row_index, n_rows, t, k);
+            gm_project_mma_kernel<<<dim3(tile_blocks, (unsigned)((n_rows + kMmaTile - 1) / kMmaTile)), 128, 0, m->stream>>>(in, nullptr, n_rows, t, k);
             ++launches;
             return;
         }
         switch (project_variant(n, count, n_rows, m->sms)) {
-            case 0: launch_project<ProjectChunk>(in, row_index, n_rows, t, k); break;
-            case 1: launch_project<ProjectRows4>(in, row_index, n_rows, t, k); break;
-            default: launch_project<ProjectNarrow>(in, row_index, n_rows, t, k); break;
+            case 0: launch_project<ProjectChunk>(in, n_rows, t, k); break;
+            case 1: launch_project<ProjectRows>(in, n_rows, t, k); break;
+            case 2: launch_project<ProjectWide>(in, n_rows, t, k); break;
+            default: launch_project<ProjectNarrow>(in, n_rows, t, k); break;
         }
     }
     template <typename V>
-    void launch_project(const bf16_t* in, const int* row_index, int n_rows, ProjectTargets& t, int k) {
+    void launch_project(const bf16_t* in, int n_rows, ProjectTargets& t, int k) {
         using S = ProjectShape<V>;
         unsigned col_blocks = 0;
         for (int i = 0; i < t.count; ++i) {
             t.first_block[i] = (int)col_blocks;
             col_blocks += (unsigned)((t.n[i] + S::cols - 1) / S::cols);
         }
-        gm_project_kernel<V><<<dim3(col_blocks, (unsigned)((n_rows + S::rows - 1) / S::rows)), S::threads, S::smem_bytes, m->stream>>>(in, row_index, n_rows, t, k);
-        ++launches;
+        launch(gm_project_kernel<V>, dim3(col_blocks, (unsigned)((n_rows + S::rows - 1) / S::rows)), S::threads, S::smem_bytes, in, n_rows,
+               (const ProjectTargets)t, k);
     }
-    void project(const bf16_t* in, const int* row_index, int n_rows, const bf16_t* w, int n, int k, bf16_t* out) {
-        project_many(in, row_index, n_rows, k, 1, &w, &n, &out);
+    void project(const bf16_t* in, int n_rows, const bf16_t* w, int n, int k, bf16_t* out) {
+        project_many(in, n_rows, k, 1, &w, &n, &out);
     }
     void rms(const bf16_t* in, const int* row_index, int n_rows, int width, const bf16_t* scale, const bf16_t* residual,
-             const bf16_t* scalar, int mode, bf16_t* out) {
-        gm_rms_kernel<<<(unsigned)n_rows, 256, sizeof(float) * (size_t)width, m->stream>>>(in, row_index, width, m->cfg.eps, scale, residual, scalar, mode, out);
-        ++launches;
+             const bf16_t* scalar, int mode, bf16_t* out, const bf16_t* next_scale = nullptr, bf16_t* next_out = nullptr) {
+        launch(gm_rms_kernel, dim3((unsigned)n_rows), 256, sizeof(float) * (size_t)width, in, row_index, width, m->cfg.eps, scale, residual,
+               scalar, mode, out, next_scale, next_out);
     }
     void gelu_mul(const bf16_t* gate, const bf16_t* other, size_t n, bf16_t* out) {
-        gm_gelu_mul_kernel<<<(unsigned)((n + 255) / 256), 256, 0, m->stream>>>(gate, other, n, out);
-        ++launches;
+        launch(gm_gelu_mul_kernel, dim3((unsigned)((n + 255) / 256)), 256, 0, gate, other, n, out);
     }
 };
 
@@ -1268,64 +1259,59 @@ int enqueue_pass(ribn_b200_gemma* m, int rows, int n_out, int max_position, uint
     const float embed_scale = bf_load(bf_round(sqrtf((float)H)));
     const float ple_scale = bf_load(bf_round(sqrtf((float)P)));
     const float projection_scale = 1.0f / sqrtf((float)H);
-    gm_embed_kernel<<<(unsigned)rows, 256, 0, s>>>(m->d_tokens, m->g[G_EMBED].data, m->g[G_PLE_EMBED].data, H, packed,
+    p.launch(gm_embed_kernel, dim3((unsigned)rows), 256, 0, m->d_tokens, m->g[G_EMBED].data, m->g[G_PLE_EMBED].data, H, packed,
                                                     embed_scale, ple_scale, m->hidden, m->identity);
-    ++p.launches;
-    p.project(m->hidden, nullptr, rows, m->g[G_PLE_PROJ].data, packed, H, m->projection);
-    gm_ple_kernel<<<dim3((unsigned)rows, (unsigned)c.layers), 256, 0, s>>>(m->projection, m->identity, m->g[G_PLE_NORM].data, rows,
+    p.project(m->hidden, rows, m->g[G_PLE_PROJ].data, packed, H, m->projection);
+    p.launch(gm_ple_kernel, dim3((unsigned)rows, (unsigned)c.layers), 256, 0, m->projection, m->identity, m->g[G_PLE_NORM].data, rows,
                                                                            P, packed, projection_scale, c.eps, m->per_layer);
-    ++p.launches;
     for (int l = 0; l < c.layers; ++l) {
         Tensor* L = m->l[l];
         const int w = width_of(c, l), kind = c.full[l] ? 1 : 0, owner = m->owner[l], cache = m->cache_of[owner];
         const bool owns = owner == l;
-        p.rms(m->hidden, nullptr, rows, H, L[L_IN].data, nullptr, nullptr, 0, m->normed);
+        if (l == 0) p.rms(m->hidden, nullptr, rows, H, L[L_IN].data, nullptr, nullptr, 0, m->normed);   // later layers: with the layer before
         {
             const bf16_t* ws[3] = {L[L_Q].data, L[L_K].data, L[L_V].data};
             const int ns[3] = {c.heads * w, c.kv_heads * w, c.kv_heads * w};
             bf16_t* outs[3] = {m->q, m->k, m->v};
-            p.project_many(m->normed, nullptr, rows, H, owns ? 3 : 1, ws, ns, outs);
+            p.project_many(m->normed, rows, H, owns ? 3 : 1, ws, ns, outs);
         }
-        gm_head_kernel<<<dim3((unsigned)rows, (unsigned)(c.heads + (owns ? 2 * c.kv_heads : 0))), 128, 0, s>>>(
+        p.launch(gm_head_kernel, dim3((unsigned)rows, (unsigned)(c.heads + (owns ? 2 * c.kv_heads : 0))), 128, 0,
             m->q, m->k, m->v, L[L_QNORM].data, owns ? L[L_KNORM].data : nullptr, m->d_slot, m->d_position, m->cosine[kind],
             m->sine[kind], c.heads, c.kv_heads, w, c.eps, c.context, m->q2, m->key_cache[(size_t)cache],
             m->value_cache[(size_t)cache]);
-        ++p.launches;
         const int window = kind ? 0 : c.window;
         const int visible = window > 0 && window < max_position + 1 ? window : max_position + 1;
         const int tile = attention_tile(visible, w, rows * c.heads, m->sms);
         const auto attention = tile == 128 ? gm_attention_kernel<128> : tile == 64 ? gm_attention_kernel<64> : gm_attention_kernel<32>;
-        attention<<<dim3((unsigned)rows, (unsigned)c.heads), 256, attention_smem_bytes(tile, visible, w), s>>>(
+        p.launch(attention, dim3((unsigned)rows, (unsigned)c.heads), 256, attention_smem_bytes(tile, visible, w),
             m->q2, m->d_slot, m->d_position, m->key_cache[(size_t)cache], m->value_cache[(size_t)cache], c.heads, c.kv_heads, w,
             window, c.context, m->attended);
-        ++p.launches;
-        p.project(m->attended, nullptr, rows, L[L_O].data, H, c.heads * w, m->projected);
-        p.rms(m->projected, nullptr, rows, H, L[L_POST_ATTN].data, m->hidden, nullptr, 1, m->mid);
+        p.project(m->attended, rows, L[L_O].data, H, c.heads * w, m->projected);
+        p.rms(m->projected, nullptr, rows, H, L[L_POST_ATTN].data, m->hidden, nullptr, 1, m->mid, L[L_PRE_FFN].data, m->normed);
         // feed-forward (decoder.rs:570-600)
-        p.rms(m->mid, nullptr, rows, H, L[L_PRE_FFN].data, nullptr, nullptr, 0, m->normed);
         {
             const bf16_t* ws[2] = {L[L_GATE].data, L[L_UP].data};
             const int ns[2] = {c.ffn, c.ffn};
             bf16_t* outs[2] = {m->gate, m->up};
-            p.project_many(m->normed, nullptr, rows, H, 2, ws, ns, outs);
+            p.project_many(m->normed, rows, H, 2, ws, ns, outs);
         }
         p.gelu_mul(m->gate, m->up, (size_t)rows * c.ffn, m->gate);
-        p.project(m->gate, nullptr, rows, L[L_DOWN].data, H, c.ffn, m->projected);
+        p.project(m->gate, rows, L[L_DOWN].data, H, c.ffn, m->projected);
         p.rms(m->projected, nullptr, rows, H, L[L_POST_FFN].data, m->mid, nullptr, 1, m->hidden);
         // per-layer embedding gate, layer scalar (decoder.rs:602-626)
-        p.project(m->hidden, nullptr, rows, L[L_PLE_GATE].data, P, H, m->ple_gate);
+        p.project(m->hidden, rows, L[L_PLE_GATE].data, P, H, m->ple_gate);
         p.gelu_mul(m->ple_gate, m->per_layer + (size_t)l * rows * P, (size_t)rows * P, m->ple_gate);
-        p.project(m->ple_gate, nullptr, rows, L[L_PLE_PROJ].data, H, P, m->projected);
-        p.rms(m->projected, nullptr, rows, H, L[L_POST_PLE].data, m->hidden, L[L_SCALAR].data, 2, m->hidden);
+        p.project(m->ple_gate, rows, L[L_PLE_PROJ].data, H, P, m->projected);
+        p.rms(m->projected, nullptr, rows, H, L[L_POST_PLE].data, m->hidden, L[L_SCALAR].data, 2, m->hidden,
+              l + 1 < c.layers ? m->l[l + 1][L_IN].data : nullptr, m->normed);
     }
     if (n_out > 0) {
         // decoder.rs:410-428: final norm, tied head, soft cap; then the greedy choice
         p.rms(m->hidden, m->d_out_rows, n_out, H, m->g[G_NORM].data, nullptr, nullptr, 0, m->normed);
-        p.project(m->normed, nullptr, n_out, m->g[G_EMBED].data, c.vocab, H, m->logits);
+        p.project(m->normed, n_out, m->g[G_EMBED].data, c.vocab, H, m->logits);
         const size_t n = (size_t)n_out * c.vocab;
-        gm_softcap_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(m->logits, n, c.softcap);
-        gm_argmax_kernel<<<(unsigned)n_out, 1024, 0, s>>>(m->logits, c.vocab, m->d_choice);
-        p.launches += 2;
+        p.launch(gm_softcap_kernel, dim3((unsigned)((n + 255) / 256)), 256, 0, m->logits, n, c.softcap);
+        p.launch(gm_argmax_kernel, dim3((unsigned)n_out), 1024, 0, m->logits, c.vocab, m->d_choice);
         GM_CUDA(m, cudaMemcpyAsync(m->h_choice, m->d_choice, sizeof(uint32_t) * (size_t)n_out, cudaMemcpyDeviceToHost, s));
     }
     GM_CUDA(m, cudaGetLastError());
