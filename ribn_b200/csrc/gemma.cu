@@ -62,14 +62,6 @@ __device__ __forceinline__ float bf_half(const uint4& v, int e) {   // value e o
     return __uint_as_float(e & 1 ? w & 0xffff0000u : w << 16);
 }
 
-// The kernels of a pass are launched so that each may start while the one before it ends: its blocks take their places
-// and fetch what no kernel writes (weights), then wait here for everything before them.  Every kernel of a pass waits,
-// so a kernel that has finished waiting follows all earlier ones.
-__device__ __forceinline__ void wait_for_previous() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
 __device__ __forceinline__ float block_max(float v, float* scratch) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = (blockDim.x + 31) >> 5;
 #pragma unroll
@@ -121,7 +113,6 @@ __device__ __forceinline__ bf16_t gelu_round(bf16_t v) {
 // ---------------------------------------------------------------------------------------------
 __global__ void gm_embed_kernel(const uint32_t* tokens, const bf16_t* __restrict__ embed, const bf16_t* __restrict__ ple_embed, int hidden, int packed,
                                 float embed_scale, float ple_scale, bf16_t* __restrict__ out_hidden, bf16_t* __restrict__ out_identity) {
-    wait_for_previous();
     const int row = blockIdx.x;
     const size_t token = tokens[row];
 #pragma unroll 4
@@ -228,10 +219,8 @@ __global__ void __launch_bounds__(ProjectShape<V>::threads) gm_project_kernel(co
             }
         };
 #pragma unroll
-        for (int t = 0; t < kStages - 1; ++t) copy_weights(t, t);   // weights need nothing of the kernel before this one
-        wait_for_previous();
-#pragma unroll
         for (int t = 0; t < kStages - 1; ++t) {
+            copy_weights(t, t);
             copy_rows(t, t);
             asm volatile("cp.async.commit_group;" ::: "memory");
         }
@@ -250,7 +239,6 @@ __global__ void __launch_bounds__(ProjectShape<V>::threads) gm_project_kernel(co
         return;
     }
 
-    wait_for_previous();
     const int g = (int)threadIdx.x / 32 - 1;
     float sum[C][R];
 #pragma unroll
@@ -433,7 +421,6 @@ __global__ void __launch_bounds__(256) gm_rms_kernel(const bf16_t* in, const int
                                                      int mode, bf16_t* out, const bf16_t* next_scale, bf16_t* next_out) {
     extern __shared__ __align__(16) float squares[];
     __shared__ float slot;
-    wait_for_previous();
     const int row = blockIdx.x;
     const uint4* x = reinterpret_cast<const uint4*>(in + (size_t)(row_index ? row_index[row] : row) * width);
     const uint4* res = reinterpret_cast<const uint4*>(residual + (mode >= 1 ? (size_t)row * width : 0));
@@ -496,7 +483,6 @@ __global__ void __launch_bounds__(256) gm_head_kernel(const bf16_t* q_in, const 
     __shared__ __align__(16) float squares[512];
     __shared__ float energy_slot;
     __shared__ bf16_t normed[512];
-    wait_for_previous();
     const int row = blockIdx.x, h = blockIdx.y, half = width / 2, pos = position[row];
     const bf16_t* x;
     const bf16_t* scale = nullptr;
@@ -576,7 +562,6 @@ __global__ void __launch_bounds__(256, 1) gm_attention_kernel(const bf16_t* q, c
     __shared__ float scratch[8];
     __shared__ float total_slot;
     __shared__ uint4 query[64];  // up to 512 BF16 channels
-    wait_for_previous();
     const int row = blockIdx.x, h = blockIdx.y, pos = position[row];
     const int kv_head = h / (heads / kv_heads);
     const int last = pos, first = window > 0 ? max(0, pos - (window - 1)) : 0;
@@ -687,7 +672,6 @@ __global__ void __launch_bounds__(256, 1) gm_attention_kernel(const bf16_t* q, c
 
 // out = bf16(bf16(gelu(gate)) * other)   (decoder.rs:592-593 and 608-609)
 __global__ void gm_gelu_mul_kernel(const bf16_t* gate, const bf16_t* other, size_t n, bf16_t* out) {
-    wait_for_previous();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = bf_round(bf_load(gelu_round(gate[i])) * bf_load(other[i]));
 }
@@ -701,7 +685,6 @@ __global__ void __launch_bounds__(256) gm_ple_kernel(const bf16_t* projection, c
     __shared__ __align__(16) float squares[1024];
     __shared__ float energy_slot;
     __shared__ bf16_t scaled[1024];
-    wait_for_previous();
     const int row = blockIdx.x, layer = blockIdx.y;
     const bf16_t* p = projection + (size_t)row * packed + (size_t)layer * ple;
     const bf16_t* id = identity + (size_t)row * packed + (size_t)layer * ple;
@@ -724,7 +707,6 @@ __global__ void __launch_bounds__(256) gm_ple_kernel(const bf16_t* projection, c
 
 // Soft cap (elementwise.rs:85-107): divide, tanh, multiply, each rounded.
 __global__ void gm_softcap_kernel(bf16_t* logits, size_t n, float cap) {
-    wait_for_previous();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const bf16_t divided = bf_round(__fdiv_rn(bf_load(logits[i]), cap));
@@ -737,7 +719,6 @@ __global__ void gm_softcap_kernel(bf16_t* logits, size_t n, float cap) {
 __global__ void __launch_bounds__(1024) gm_argmax_kernel(const bf16_t* logits, int vocab, uint32_t* out) {
     __shared__ float best_value[32];
     __shared__ int best_index[32];
-    wait_for_previous();
     const bf16_t* x = logits + (size_t)blockIdx.x * vocab;
     const float head = bf_load(x[0]);
     if (head != head) {  // nothing compares greater than a NaN incumbent
@@ -1182,20 +1163,9 @@ struct Pass {
     int rows;
     uint32_t launches = 0;
 
-    // A launch that may begin while the kernel before it ends (`wait_for_previous`).
     template <typename... Params, typename... Args>
     void launch(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, Args... args) {
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = grid;
-        cfg.blockDim = dim3((unsigned)threads);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = m->stream;
-        cudaLaunchAttribute attribute{};
-        attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attribute.val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = &attribute;
-        cfg.numAttrs = launches > 0 ? 1 : 0;   // the first kernel follows the copies of the pass's rows
-        cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);   // its error is read at the end of the pass
+        kernel<<<grid, threads, smem, m->stream>>>(static_cast<Params>(args)...);   // its error is read at the end of the pass
         ++launches;
     }
     void project_many(const bf16_t* in, int n_rows, int k, int count, const bf16_t* const* w,
