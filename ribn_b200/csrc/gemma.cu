@@ -127,26 +127,33 @@ __global__ void gm_embed_kernel(const uint32_t* tokens, const bf16_t* __restrict
 
 // ---------------------------------------------------------------------------------------------
 // Projection: out[r][n] = bf16(sum_k in[r][k] * w[n][k]) (linear.rs:23-66), the sum in k order.  A block is a
-// feeder warp and G consumer warps.  A consumer owns 32 * C output columns for R rows: a thread walks C weight rows
-// and keeps R * C independent accumulation chains.  The feeder brings tiles of the weights and of the blocks' input
-// rows by cp.async into a ring of stages (rows pitched 16 bytes apart from a multiple of 128, so the 128-bit reads of
-// a quarter-warp fall in distinct banks).  Named barriers hand the stages over; their ids are constants because an
-// SM has 64 barriers and a block whose ids are computed is given 16 of them.
+// feeder warp and GR x GC consumer warps.  A consumer owns 32 * C output columns for R rows: a thread walks C weight
+// rows and keeps R * C independent accumulation chains, pairs of rows packed (`fma.rn.f32x2` rounds each half as
+// `fmaf` does).  The feeder brings weight tiles by cp.async into a ring of stages (rows pitched 16 bytes apart from a
+// multiple of 128, so the 128-bit reads of a quarter-warp fall in distinct banks) and the input rows beside them: one
+// row as it is, four rows expanded to FP32 and interleaved as the consumers' packed operands.  Named barriers hand
+// the stages over; their ids are constants because an SM has 64 barriers and a block whose ids are computed is given
+// 16 of them.  Four consumer warps per block fall on the four schedulers; two-warp blocks leave two without one.
 //
 // What bounds it: the chain of dependent additions, 4 cycles per input (14.4 us for the 6,912 inputs of a down
-// projection), or, with several chains per scheduler, the instructions issued per input and the shared-memory reads.
-// A scheduler's reads return 64 bytes per cycle, broadcast or not, so the input rows stay BF16 (expanded to FP32 in
-// shared memory they cost twice the reads: 14 instead of 10 cycles per input at four rows).
+// projection), or, with several chains per scheduler, issue and the shared-memory reads (a 128-bit read occupies a
+// scheduler's return path about 12 cycles, broadcast or not).  Measured per input of a consumer warp, alone and with
+// others on its scheduler: one row 5.6 and 4, 4 rows x 1 column 14.5 and 10.2, 4 x 2 19.5 and 13.8 cycles; 4 x 2 with
+// BF16 input rows 28.
 // ---------------------------------------------------------------------------------------------
-struct ProjectNarrow { static constexpr int R = 1, C = 1, G = 1, tile = 256, stages = 4; };   // a few rows: chains spread over blocks
-struct ProjectWide { static constexpr int R = 4, C = 1, G = 1, tile = 256, stages = 3; };     // a few rows of a wide projection
-struct ProjectRows { static constexpr int R = 4, C = 1, G = 4, tile = 256, stages = 3; };     // a few tens of rows
-struct ProjectChunk { static constexpr int R = 4, C = 2, G = 4, tile = 128, stages = 3; };    // prefill
+struct ProjectNarrow { static constexpr int R = 1, C = 1, GR = 1, GC = 1, tile = 256, stages = 4; };   // a few rows: chains spread over blocks
+struct ProjectWide { static constexpr int R = 4, C = 1, GR = 1, GC = 4, tile = 128, stages = 3; };     // up to four rows of a wide projection
+struct ProjectRows { static constexpr int R = 4, C = 1, GR = 4, GC = 1, tile = 128, stages = 3; };     // a few tens of rows
+struct ProjectChunk { static constexpr int R = 4, C = 2, GR = 4, GC = 1, tile = 128, stages = 2; };    // prefill
 template <typename V>
 struct ProjectShape {
-    static constexpr int cols = 32 * V::C, rows = V::R * V::G, threads = 32 * (1 + V::G);
+    static constexpr int consumers = V::GR * V::GC, threads = 32 * (1 + consumers);
+    static constexpr int cols = 32 * V::C * V::GC, rows = V::R * V::GR;
     static constexpr int chunks = V::tile / 8, pitch = V::tile * 2 + 16;        // 16-byte chunks, and bytes between rows of a tile
-    static constexpr int stage_bytes = (cols + rows) * pitch, smem_bytes = V::stages * stage_bytes;
+    // floats of eight inputs of R expanded rows: padded so that the feeder's stores fall in distinct banks
+    static constexpr int x_group = 9 * V::R, x_pitch = x_group * V::GR;
+    static constexpr int x_offset = cols * pitch, x_bytes = V::R == 1 ? rows * pitch : chunks * x_pitch * 4;
+    static constexpr int stage_bytes = x_offset + x_bytes, smem_bytes = V::stages * stage_bytes;
 };
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
@@ -166,6 +173,12 @@ __device__ __forceinline__ void stage_barrier(int slot, bool wait) {
     else stage_barrier<FIRST + (STAGES > 3 ? 3 : 0), THREADS>(wait);
 }
 
+__device__ __forceinline__ unsigned long long fma_pair(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
 // Up to three matrices that read the same input rows share one launch (q | k | v, gate | up): their
 // column blocks are laid side by side in the grid.
 struct ProjectTargets {
@@ -177,7 +190,7 @@ struct ProjectTargets {
 };
 
 template <typename V>
-__global__ void __launch_bounds__(ProjectShape<V>::threads) gm_project_kernel(const bf16_t* __restrict__ in, int rows,
+__global__ void __launch_bounds__(ProjectShape<V>::threads, 4) gm_project_kernel(const bf16_t* __restrict__ in, int rows,
                                                                               const __grid_constant__ ProjectTargets targets, int k) {
     extern __shared__ __align__(16) unsigned char project_smem[];
     using S = ProjectShape<V>;
@@ -197,7 +210,6 @@ __global__ void __launch_bounds__(ProjectShape<V>::threads) gm_project_kernel(co
         constexpr int kRowsPerIssue = 32 / S::chunks;              // rows one warp-wide copy instruction covers
         const int piece = lane % S::chunks, sub_row = lane / S::chunks;
         const uint4* wsrc = reinterpret_cast<const uint4*>(targets.w[which] + (size_t)(col0 + sub_row) * k) + piece;
-        const uint4* xsrc = reinterpret_cast<const uint4*>(in) + piece;
         const uint32_t wdst = (uint32_t)__cvta_generic_to_shared(project_smem) + (uint32_t)(sub_row * S::pitch + piece * 16);
         auto copy_weights = [&](int tile, int slot) {
             const int c = tile * S::chunks;
@@ -209,66 +221,100 @@ __global__ void __launch_bounds__(ProjectShape<V>::threads) gm_project_kernel(co
                 cp_async16(dst, src);
             }
         };
-        auto copy_rows = [&](int tile, int slot) {
+        // one row: copied like the weights
+        auto copy_row = [&](int tile, int slot) {
             const int c = tile * S::chunks;
-            if (tile >= tiles || c + piece >= chunks) return;
-            const uint32_t dst = wdst + (uint32_t)(slot * S::stage_bytes + S::cols * S::pitch);
+            if (R > 1 || tile >= tiles || c + piece >= chunks || sub_row > 0) return;
+            cp_async16(wdst + (uint32_t)(slot * S::stage_bytes + S::x_offset), reinterpret_cast<const uint4*>(in + (size_t)r0 * k) + c + piece);
+        };
+        // four: a lane reads pieces of one row, chunk lane / rows and every 32 / rows after it, a tile ahead
+        constexpr int kPieces = R == 1 ? 1 : S::rows * S::chunks / 32;
+        const int own = lane % S::rows, first_chunk = lane / S::rows;
+        const uint4* xsrc = reinterpret_cast<const uint4*>(in + (size_t)min(r0 + own, rows - 1) * k);
+        uint4 x[kPieces];
+        auto read = [&](int tile) {
+            if (R == 1) return;
 #pragma unroll
-            for (int j = 0; j < S::rows; j += kRowsPerIssue) {
-                if (j + sub_row < S::rows) cp_async16(dst + (uint32_t)(j * S::pitch), xsrc + (size_t)min(r0 + j + sub_row, rows - 1) * chunks + c);
+            for (int i = 0; i < kPieces; ++i) {
+                const int c = tile * S::chunks + first_chunk + i * (32 / S::rows);
+                x[i] = c < chunks ? xsrc[c] : make_uint4(0, 0, 0, 0);
             }
         };
-#pragma unroll
-        for (int t = 0; t < kStages - 1; ++t) {
-            copy_weights(t, t);
-            copy_rows(t, t);
+        auto copy = [&](int tile, int slot) {
+            copy_weights(tile, slot);
+            copy_row(tile, slot);
             asm volatile("cp.async.commit_group;" ::: "memory");
-        }
+        };
+#pragma unroll
+        for (int t = 0; t < kStages - 1; ++t) copy(t, t);
+        read(0);
         int slot = 0, ahead = kStages - 1;   // slots of tile t and of tile t + kStages - 1
         for (int t = 0; t < tiles; ++t) {
+            if constexpr (R > 1) {   // they need nothing but the slot, which was free when its weights were requested
+                float* xf = reinterpret_cast<float*>(project_smem + (size_t)slot * S::stage_bytes + S::x_offset) + own / R * S::x_group + own % R;
+#pragma unroll
+                for (int i = 0; i < kPieces; ++i) {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) xf[(first_chunk + i * (32 / S::rows)) * S::x_pitch + e * R] = bf_half(x[i], e);
+                }
+                read(t + 1);
+            }
             asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");   // tile t; younger copies stay in flight
             __syncwarp();
             stage_barrier<1, kStages, kThreads>(slot, false);
             if (t > 0 && t - 1 + kStages < tiles) stage_barrier<1 + kStages, kStages, kThreads>(ahead, true);   // the consumers have left tile t - 1
-            copy_weights(t + kStages - 1, ahead);
-            copy_rows(t + kStages - 1, ahead);
-            asm volatile("cp.async.commit_group;" ::: "memory");
+            copy(t + kStages - 1, ahead);
             slot = slot + 1 == kStages ? 0 : slot + 1;
             ahead = ahead + 1 == kStages ? 0 : ahead + 1;
         }
         return;
     }
 
-    const int g = (int)threadIdx.x / 32 - 1;
-    float sum[C][R];
+    const int gr = ((int)threadIdx.x / 32 - 1) % V::GR, gc = ((int)threadIdx.x / 32 - 1) / V::GR;
+    using Pair = unsigned long long;
+    constexpr int kPairs = R == 1 ? 1 : R / 2;
+    Pair acc[C][kPairs];
+    float sum = 0.0f;
 #pragma unroll
     for (int c = 0; c < C; ++c) {
 #pragma unroll
-        for (int r = 0; r < R; ++r) sum[c][r] = 0.0f;
+        for (int q = 0; q < kPairs; ++q) acc[c][q] = 0;
     }
     int slot = 0;
     for (int t = 0; t < tiles; ++t) {
         stage_barrier<1, kStages, kThreads>(slot, true);
-        const unsigned char* ws = project_smem + (size_t)slot * S::stage_bytes + lane * S::pitch;
-        const unsigned char* xs = project_smem + (size_t)slot * S::stage_bytes + (S::cols + g * R) * S::pitch;
+        const unsigned char* stage = project_smem + (size_t)slot * S::stage_bytes;
+        const unsigned char* ws = stage + (gc * 32 * C + lane) * S::pitch;
+        const unsigned char* xs = stage + S::x_offset + gr * S::x_group * 4;
         const int count = min(S::chunks, chunks - t * S::chunks);
         auto chunk = [&](int i) {
-            uint4 wv[C], xv[R];
+            uint4 wv[C];
 #pragma unroll
             for (int c = 0; c < C; ++c) wv[c] = *reinterpret_cast<const uint4*>(ws + c * 32 * S::pitch + i * 16);
+            if constexpr (R == 1) {
+                const uint4 xv = *reinterpret_cast<const uint4*>(xs + i * 16);
 #pragma unroll
-            for (int r = 0; r < R; ++r) xv[r] = *reinterpret_cast<const uint4*>(xs + r * S::pitch + i * 16);
+                for (int e = 0; e < 8; ++e) sum = fmaf(bf_half(xv, e), bf_half(wv[0], e), sum);
+            } else {
+                const ulonglong2* x = reinterpret_cast<const ulonglong2*>(xs + i * S::x_pitch * 4);   // the rows of input 0, of input 1, ...
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
+                for (int e = 0; e < 8; ++e) {
 #pragma unroll
-                for (int c = 0; c < C; ++c) {
+                    for (int c = 0; c < C; ++c) {
+                        const float w = bf_half(wv[c], e);
+                        Pair ww;
+                        asm("mov.b64 %0, {%1, %1};" : "=l"(ww) : "f"(w));
 #pragma unroll
-                    for (int r = 0; r < R; ++r) sum[c][r] = fmaf(bf_half(xv[r], e), bf_half(wv[c], e), sum[c][r]);
+                        for (int q = 0; q < kPairs; ++q) {
+                            const ulonglong2 v = x[e * (R / 4) + q / 2];
+                            acc[c][q] = fma_pair(q & 1 ? v.y : v.x, ww, acc[c][q]);
+                        }
+                    }
                 }
             }
         };
         if (count == S::chunks) {
-#pragma unroll(R == 1 ? 8 : 4)
+#pragma unroll(R == 1 ? 8 : 2)
             for (int i = 0; i < S::chunks; ++i) chunk(i);
         } else {
             for (int i = 0; i < count; ++i) chunk(i);
@@ -278,31 +324,38 @@ __global__ void __launch_bounds__(ProjectShape<V>::threads) gm_project_kernel(co
     }
 #pragma unroll
     for (int c = 0; c < C; ++c) {
-        if (lane + 32 * c >= live_cols) break;
-        bf16_t* out = targets.out[which] + col0 + lane + 32 * c;
+        const int col = gc * 32 * C + lane + 32 * c;
+        if (col >= live_cols) break;
+        bf16_t* out = targets.out[which] + col0 + col;
+        const int first = r0 + gr * R;
+        if constexpr (R == 1) {
+            out[(size_t)first * n] = bf_round(sum);
+        } else {
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int row = r0 + g * R + r;
-            if (row < rows) out[(size_t)row * n] = bf_round(sum[c][r]);
+            for (int q = 0; q < kPairs; ++q) {
+                float lo, hi;
+                asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc[c][q]));
+                if (first + 2 * q < rows) out[(size_t)(first + 2 * q) * n] = bf_round(lo);
+                if (first + 2 * q + 1 < rows) out[(size_t)(first + 2 * q + 1) * n] = bf_round(hi);
+            }
         }
     }
 }
 
-// Which variant: the one whose busiest scheduler finishes first.  A warp alone on its scheduler advances one input
-// per 4 cycles (the addition's latency) or per the instructions it issues for an input; warps that share a scheduler
-// add up.  So a narrow projection of a few rows goes to one warp per row and 32 columns (1,152 columns x four rows:
-// 144 warps), and many rows or columns to the variants that issue less per product and read the weights fewer times.
+// Which variant: the one whose busiest scheduler finishes first, by the cycles per input measured above.  A narrow
+// projection of a few rows goes to one warp per row and 32 columns (1,152 columns x four rows: 144 warps), many rows
+// or columns to the variants that spend less per product and read the weights fewer times.
 int project_variant(const int* n, int count, int rows, int sms) {
-    constexpr int kCols[4] = {64, 32, 32, 32}, kRows[4] = {16, 16, 4, 1}, kWarps[4] = {4, 4, 1, 1};
-    constexpr float kIssue[4] = {15.0f, 9.8f, 9.8f, 3.4f};   // per input of a consumer warp, counted from the loop above
+    constexpr int kCols[4] = {64, 32, 128, 32}, kRows[4] = {16, 16, 4, 1};
+    constexpr float kAlone[4] = {19.5f, 14.5f, 14.5f, 5.6f}, kShared[4] = {13.8f, 10.2f, 10.2f, 4.0f};
     int best = 0;
     float best_cost = 0.0f;
     for (int v = 0; v < 4; ++v) {
         int blocks = 0;
         for (int i = 0; i < count; ++i) blocks += (n[i] + kCols[v] - 1) / kCols[v];
         blocks *= (rows + kRows[v] - 1) / kRows[v];
-        const int per_sm = (blocks + sms - 1) / sms, per_scheduler = (per_sm * kWarps[v] + 3) / 4;
-        const float cost = std::max(4.0f, kIssue[v] * (float)per_scheduler);
+        const int per_sm = (blocks + sms - 1) / sms, per_scheduler = v == 3 ? (per_sm + 1) / 2 : per_sm;
+        const float cost = std::max(kAlone[v], kShared[v] * (float)per_scheduler);
         if (v == 0 || cost < best_cost) { best = v; best_cost = cost; }
     }
     return best;
