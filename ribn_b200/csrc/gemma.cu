@@ -74,22 +74,37 @@ __device__ __forceinline__ float block_max(float v, float* scratch) {
     return m;
 }
 
+// values[0 .. n) added in index order by one thread: 4 cycles per addition when the next 128-bit reads are under way
+// while the last ones are added.
+__device__ __forceinline__ float ordered_sum(const float* values, int n) {
+    constexpr int kBatch = 8;
+    const float4* quads = reinterpret_cast<const float4*>(values);
+    const int whole = n / (4 * kBatch) * kBatch;
+    float total = 0.0f;
+    float4 now[kBatch];
+    if (whole > 0) {
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) now[u] = quads[u];
+    }
+    for (int i = 0; i < whole; i += kBatch) {
+        float4 next[kBatch];
+        const float4* ahead = quads + min(i + kBatch, whole - kBatch);
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) next[u] = ahead[u];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) { total += now[u].x; total += now[u].y; total += now[u].z; total += now[u].w; }
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) now[u] = next[u];
+    }
+    for (int i = 4 * whole; i < n; ++i) total += values[i];
+    return total;
+}
+
 // Sum of squares of values[0 .. n) in index order by thread 0, broadcast to the block.  `squares` is a
 // shared staging array of n floats the whole block fills first (each square is exact).
 __device__ __forceinline__ float ordered_energy(const float* squares, int n, float* slot) {
     __syncthreads();
-    if (threadIdx.x == 0) {
-        // 128-bit reads run ahead of the additions; the additions themselves stay in index order
-        const float4* quads = reinterpret_cast<const float4*>(squares);
-        float energy = 0.0f;
-#pragma unroll 8
-        for (int i = 0; i < n / 4; ++i) {
-            const float4 v = quads[i];
-            energy += v.x; energy += v.y; energy += v.z; energy += v.w;
-        }
-        for (int i = n & ~3; i < n; ++i) energy += squares[i];
-        *slot = energy;
-    }
+    if (threadIdx.x == 0) *slot = ordered_sum(squares, n);
     __syncthreads();
     return *slot;
 }
@@ -150,9 +165,7 @@ struct ProjectShape {
     static constexpr int consumers = V::GR * V::GC, threads = 32 * (1 + consumers);
     static constexpr int cols = 32 * V::C * V::GC, rows = V::R * V::GR;
     static constexpr int chunks = V::tile / 8, pitch = V::tile * 2 + 16;        // 16-byte chunks, and bytes between rows of a tile
-    // floats of eight inputs of R expanded rows: padded so that the feeder's stores fall in distinct banks
-    static constexpr int x_group = 9 * V::R, x_pitch = x_group * V::GR;
-    static constexpr int x_offset = cols * pitch, x_bytes = V::R == 1 ? rows * pitch : chunks * x_pitch * 4;
+    static constexpr int x_offset = cols * pitch, x_bytes = rows * pitch;
     static constexpr int stage_bytes = x_offset + x_bytes, smem_bytes = V::stages * stage_bytes;
 };
 
@@ -173,10 +186,14 @@ __device__ __forceinline__ void stage_barrier(int slot, bool wait) {
     else stage_barrier<FIRST + (STAGES > 3 ? 3 : 0), THREADS>(wait);
 }
 
-__device__ __forceinline__ unsigned long long fma_pair(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
+// sum + a.e * b.e for value e of eight BF16 values, one rounding (the product of two BF16 values is exact in FP32):
+// the instruction takes the halves of a register as they are, so nothing is unpacked.
+__device__ __forceinline__ float fma_half(const uint4& a, const uint4& b, float sum, int e) {
+    const uint32_t x = e < 2 ? a.x : e < 4 ? a.y : e < 6 ? a.z : a.w, y = e < 2 ? b.x : e < 4 ? b.y : e < 6 ? b.z : b.w;
+    float out;
+    if (e & 1) asm("{.reg .b16 al, ah, bl, bh; mov.b32 {al, ah}, %1; mov.b32 {bl, bh}, %2; fma.rn.f32.bf16 %0, ah, bh, %3;}" : "=f"(out) : "r"(x), "r"(y), "f"(sum));
+    else asm("{.reg .b16 al, ah, bl, bh; mov.b32 {al, ah}, %1; mov.b32 {bl, bh}, %2; fma.rn.f32.bf16 %0, al, bl, %3;}" : "=f"(out) : "r"(x), "r"(y), "f"(sum));
+    return out;
 }
 
 // Up to three matrices that read the same input rows share one launch (q | k | v, gate | up): their
@@ -221,44 +238,26 @@ __global__ void __launch_bounds__(ProjectShape<V>::threads, 4) gm_project_kernel
                 cp_async16(dst, src);
             }
         };
-        // one row: copied like the weights
-        auto copy_row = [&](int tile, int slot) {
-            const int c = tile * S::chunks;
-            if (R > 1 || tile >= tiles || c + piece >= chunks || sub_row > 0) return;
-            cp_async16(wdst + (uint32_t)(slot * S::stage_bytes + S::x_offset), reinterpret_cast<const uint4*>(in + (size_t)r0 * k) + c + piece);
-        };
-        // four: a lane reads pieces of one row, chunk lane / rows and every 32 / rows after it, a tile ahead
-        constexpr int kPieces = R == 1 ? 1 : S::rows * S::chunks / 32;
-        const int own = lane % S::rows, first_chunk = lane / S::rows;
-        const uint4* xsrc = reinterpret_cast<const uint4*>(in + (size_t)min(r0 + own, rows - 1) * k);
-        uint4 x[kPieces];
-        auto read = [&](int tile) {
-            if (R == 1) return;
+        auto copy_rows = [&](int tile, int slot) {
+            const int c = tile * S::chunks + piece;
+            if (tile >= tiles || c >= chunks) return;
+            const uint32_t dst = wdst + (uint32_t)(slot * S::stage_bytes + S::x_offset);
 #pragma unroll
-            for (int i = 0; i < kPieces; ++i) {
-                const int c = tile * S::chunks + first_chunk + i * (32 / S::rows);
-                x[i] = c < chunks ? xsrc[c] : make_uint4(0, 0, 0, 0);
+            for (int j = 0; j < S::rows; j += kRowsPerIssue) {
+                if (j + sub_row < S::rows) {
+                    cp_async16(dst + (uint32_t)(j * S::pitch), reinterpret_cast<const uint4*>(in) + (size_t)min(r0 + j + sub_row, rows - 1) * chunks + c);
+                }
             }
         };
         auto copy = [&](int tile, int slot) {
             copy_weights(tile, slot);
-            copy_row(tile, slot);
+            copy_rows(tile, slot);
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
 #pragma unroll
         for (int t = 0; t < kStages - 1; ++t) copy(t, t);
-        read(0);
         int slot = 0, ahead = kStages - 1;   // slots of tile t and of tile t + kStages - 1
         for (int t = 0; t < tiles; ++t) {
-            if constexpr (R > 1) {   // they need nothing but the slot, which was free when its weights were requested
-                float* xf = reinterpret_cast<float*>(project_smem + (size_t)slot * S::stage_bytes + S::x_offset) + own / R * S::x_group + own % R;
-#pragma unroll
-                for (int i = 0; i < kPieces; ++i) {
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) xf[(first_chunk + i * (32 / S::rows)) * S::x_pitch + e * R] = bf_half(x[i], e);
-                }
-                read(t + 1);
-            }
             asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");   // tile t; younger copies stay in flight
             __syncwarp();
             stage_barrier<1, kStages, kThreads>(slot, false);
@@ -271,45 +270,31 @@ __global__ void __launch_bounds__(ProjectShape<V>::threads, 4) gm_project_kernel
     }
 
     const int gr = ((int)threadIdx.x / 32 - 1) % V::GR, gc = ((int)threadIdx.x / 32 - 1) / V::GR;
-    using Pair = unsigned long long;
-    constexpr int kPairs = R == 1 ? 1 : R / 2;
-    Pair acc[C][kPairs];
-    float sum = 0.0f;
+    float sum[C][R];
 #pragma unroll
     for (int c = 0; c < C; ++c) {
 #pragma unroll
-        for (int q = 0; q < kPairs; ++q) acc[c][q] = 0;
+        for (int r = 0; r < R; ++r) sum[c][r] = 0.0f;
     }
     int slot = 0;
     for (int t = 0; t < tiles; ++t) {
         stage_barrier<1, kStages, kThreads>(slot, true);
         const unsigned char* stage = project_smem + (size_t)slot * S::stage_bytes;
         const unsigned char* ws = stage + (gc * 32 * C + lane) * S::pitch;
-        const unsigned char* xs = stage + S::x_offset + gr * S::x_group * 4;
+        const unsigned char* xs = stage + S::x_offset + gr * R * S::pitch;
         const int count = min(S::chunks, chunks - t * S::chunks);
         auto chunk = [&](int i) {
-            uint4 wv[C];
+            uint4 w[C], x[R];
 #pragma unroll
-            for (int c = 0; c < C; ++c) wv[c] = *reinterpret_cast<const uint4*>(ws + c * 32 * S::pitch + i * 16);
-            if constexpr (R == 1) {
-                const uint4 xv = *reinterpret_cast<const uint4*>(xs + i * 16);
+            for (int c = 0; c < C; ++c) w[c] = *reinterpret_cast<const uint4*>(ws + c * 32 * S::pitch + i * 16);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) sum = fmaf(bf_half(xv, e), bf_half(wv[0], e), sum);
-            } else {
-                const ulonglong2* x = reinterpret_cast<const ulonglong2*>(xs + i * S::x_pitch * 4);   // the rows of input 0, of input 1, ...
+            for (int r = 0; r < R; ++r) x[r] = *reinterpret_cast<const uint4*>(xs + r * S::pitch + i * 16);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) {
+            for (int e = 0; e < 8; ++e) {
 #pragma unroll
-                    for (int c = 0; c < C; ++c) {
-                        const float w = bf_half(wv[c], e);
-                        Pair ww;
-                        asm("mov.b64 %0, {%1, %1};" : "=l"(ww) : "f"(w));
+                for (int c = 0; c < C; ++c) {
 #pragma unroll
-                        for (int q = 0; q < kPairs; ++q) {
-                            const ulonglong2 v = x[e * (R / 4) + q / 2];
-                            acc[c][q] = fma_pair(q & 1 ? v.y : v.x, ww, acc[c][q]);
-                        }
-                    }
+                    for (int r = 0; r < R; ++r) sum[c][r] = fma_half(x[r], w[c], sum[c][r], e);
                 }
             }
         };
@@ -327,17 +312,10 @@ __global__ void __launch_bounds__(ProjectShape<V>::threads, 4) gm_project_kernel
         const int col = gc * 32 * C + lane + 32 * c;
         if (col >= live_cols) break;
         bf16_t* out = targets.out[which] + col0 + col;
-        const int first = r0 + gr * R;
-        if constexpr (R == 1) {
-            out[(size_t)first * n] = bf_round(sum);
-        } else {
 #pragma unroll
-            for (int q = 0; q < kPairs; ++q) {
-                float lo, hi;
-                asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc[c][q]));
-                if (first + 2 * q < rows) out[(size_t)(first + 2 * q) * n] = bf_round(lo);
-                if (first + 2 * q + 1 < rows) out[(size_t)(first + 2 * q + 1) * n] = bf_round(hi);
-            }
+        for (int r = 0; r < R; ++r) {
+            const int row = r0 + gr * R + r;
+            if (row < rows) out[(size_t)row * n] = bf_round(sum[c][r]);
         }
     }
 }
@@ -347,7 +325,7 @@ __global__ void __launch_bounds__(ProjectShape<V>::threads, 4) gm_project_kernel
 // or columns to the variants that spend less per product and read the weights fewer times.
 int project_variant(const int* n, int count, int rows, int sms) {
     constexpr int kCols[4] = {64, 32, 128, 32}, kRows[4] = {16, 16, 4, 1};
-    constexpr float kAlone[4] = {19.5f, 14.5f, 14.5f, 5.6f}, kShared[4] = {13.8f, 10.2f, 10.2f, 4.0f};
+    constexpr float kAlone[4] = {11.0f, 8.0f, 8.0f, 4.8f}, kShared[4] = {9.5f, 7.5f, 7.5f, 3.1f};
     int best = 0;
     float best_cost = 0.0f;
     for (int v = 0; v < 4; ++v) {
@@ -607,6 +585,119 @@ inline int attention_tile(int visible, int width, int blocks, int sms) {
     return attention_smem_bytes(64, visible, width) <= kAttnSmemLimit ? 64 : 32;
 }
 
+// query . key over 8 * chunks channels, in channel order
+__device__ __forceinline__ float ordered_dot(const uint4* query, const uint4* key, int chunks) {
+    float sum = 0.0f;
+    uint4 kv[2] = {key[0], key[min(1, chunks - 1)]}, qq[2] = {query[0], query[min(1, chunks - 1)]};
+#pragma unroll 2
+    for (int i = 0; i < chunks; i += 2) {   // two chunks read ahead of the two in use
+        uint4 next_k[2], next_q[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int at = min(i + 2 + u, chunks - 1);
+            next_k[u] = key[at];
+            next_q[u] = query[at];
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            if (i + u < chunks) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) sum = fma_half(qq[u], kv[u], sum, e);
+            }
+            kv[u] = next_k[u];
+            qq[u] = next_q[u];
+        }
+    }
+    return sum;
+}
+
+// The same attention with a cluster of four blocks per (row, head), for steps of so few rows that the blocks still fit
+// the GPU once.  Each block scores a quarter of the keys, writes its scores into the shared memory of all four, does
+// the softmax (the same in each) and sums a quarter of the channels, whose values it requested at the start.  Against
+// one block the keys and values arrive over four SMs and the scores take one pass instead of one per 128 keys.
+// Dynamic shared memory: one float per visible key, the block's keys, its quarter of every value row.
+constexpr int kAttnCluster = 4;
+__host__ __device__ inline size_t attention_split_bytes(int visible, int width) {
+    return (((size_t)visible * sizeof(float) + 15) & ~(size_t)15) +
+           (size_t)((visible + kAttnCluster - 1) / kAttnCluster) * ((size_t)width * 2 + 16) + (size_t)visible * (width / kAttnCluster * 2 + 16);
+}
+inline bool attention_splits(int visible, int width, int blocks, int sms) {
+    return blocks * kAttnCluster <= sms && width % (8 * kAttnCluster) == 0 && attention_split_bytes(visible, width) <= kAttnSmemLimit;
+}
+
+__global__ void __launch_bounds__(256, 1) __cluster_dims__(1, 1, kAttnCluster)
+    gm_attention_split_kernel(const bf16_t* q, const int* slot, const int* position, const bf16_t* key_cache, const bf16_t* value_cache,
+                              int heads, int kv_heads, int width, int window, int context, bf16_t* out) {
+    extern __shared__ __align__(16) unsigned char attention_smem[];
+    __shared__ float scratch[8];
+    __shared__ float total_slot;
+    __shared__ uint4 query[64];  // up to 512 BF16 channels
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // this block runs: its scores can be written
+    const int row = blockIdx.x, h = blockIdx.y, rank = blockIdx.z, pos = position[row];
+    const int kv_head = h / (heads / kv_heads);
+    const int last = pos, first = window > 0 ? max(0, pos - (window - 1)) : 0;
+    const int visible = last - first + 1;
+    const int share = (visible + kAttnCluster - 1) / kAttnCluster, key0 = rank * share, keys = max(0, min(share, visible - key0));
+    float* scores = reinterpret_cast<float*>(attention_smem);
+    unsigned char* key_tile = attention_smem + (((size_t)visible * sizeof(float) + 15) & ~(size_t)15);
+    const int key_pitch = width * 2 + 16, part = width / kAttnCluster, value_pitch = part * 2 + 16;
+    unsigned char* value_tile = key_tile + (size_t)share * key_pitch;
+    const size_t stride = (size_t)kv_heads * width;
+    const bf16_t* kbase = key_cache + ((size_t)slot[row] * context + first) * stride + (size_t)kv_head * width;
+    const bf16_t* vbase = value_cache + ((size_t)slot[row] * context + first) * stride + (size_t)kv_head * width + rank * part;
+    const int chunks = width / 8, part_chunks = part / 8;
+    const uint32_t key_dst = (uint32_t)__cvta_generic_to_shared(key_tile), value_dst = (uint32_t)__cvta_generic_to_shared(value_tile);
+#pragma unroll 4
+    for (int key = (int)threadIdx.x / 32; key < keys; key += 8) {
+        for (int c = (int)threadIdx.x % 32; c < chunks; c += 32) {
+            cp_async16(key_dst + (uint32_t)(key * key_pitch + c * 16), reinterpret_cast<const uint4*>(kbase + (size_t)(key0 + key) * stride) + c);
+        }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+#pragma unroll 4
+    for (int i = threadIdx.x; i < visible * part_chunks; i += 256) {
+        const int key = i / part_chunks, c = i - key * part_chunks;
+        cp_async16(value_dst + (uint32_t)(key * value_pitch + c * 16), reinterpret_cast<const uint4*>(vbase + (size_t)key * stride) + c);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    for (int i = threadIdx.x; i < chunks; i += blockDim.x) {
+        query[i] = reinterpret_cast<const uint4*>(q + ((size_t)row * heads + h) * width)[i];
+    }
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    for (int key = threadIdx.x; key < keys; key += blockDim.x) {
+        const float score = bf_load(bf_round(ordered_dot(query, reinterpret_cast<const uint4*>(key_tile + (size_t)key * key_pitch), chunks)));
+        const uint32_t own = (uint32_t)__cvta_generic_to_shared(scores + key0 + key);
+#pragma unroll
+        for (int r = 0; r < kAttnCluster; ++r) {
+            uint32_t there;
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(own), "r"(r));
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(there), "f"(score) : "memory");
+        }
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // the last access to another block's memory is before it
+    float maximum = -INFINITY;
+    for (int t = threadIdx.x; t < visible; t += blockDim.x) maximum = fmaxf(maximum, scores[t]);
+    maximum = block_max(maximum, scratch);
+    for (int t = threadIdx.x; t < visible; t += blockDim.x) scores[t] = (float)exp((double)(scores[t] - maximum));
+    __syncthreads();
+    if (threadIdx.x == 0) total_slot = ordered_sum(scores, visible);
+    __syncthreads();
+    const float total = total_slot;
+    for (int t = threadIdx.x; t < visible; t += blockDim.x) scores[t] = bf_load(bf_round(scores[t] / total));
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    if ((int)threadIdx.x < part) {
+        const bf16_t* column = reinterpret_cast<const bf16_t*>(value_tile) + threadIdx.x;
+        float acc = 0.0f;
+#pragma unroll 16
+        for (int t = 0; t < visible; ++t) acc = fmaf(scores[t], bf_load(column[(size_t)t * (value_pitch / 2)]), acc);
+        out[((size_t)row * heads + h) * width + rank * part + threadIdx.x] = bf_round(acc);
+    }
+}
+
 template <int TILE>
 __global__ void __launch_bounds__(256, 1) gm_attention_kernel(const bf16_t* q, const int* slot, const int* position,
                                                               const bf16_t* key_cache, const bf16_t* value_cache, int heads,
@@ -657,28 +748,7 @@ __global__ void __launch_bounds__(256, 1) gm_attention_kernel(const bf16_t* q, c
         const unsigned char* tile = next_tile(step);
         const int t0 = step * TILE;
         if ((int)threadIdx.x < min(TILE, visible - t0)) {
-            const uint4* key = reinterpret_cast<const uint4*>(tile + (size_t)threadIdx.x * pitch);
-            float sum = 0.0f;
-            uint4 kv[2] = {key[0], key[min(1, chunks - 1)]}, qq[2] = {query[0], query[min(1, chunks - 1)]};
-#pragma unroll 2
-            for (int i = 0; i < chunks; i += 2) {   // two chunks read ahead of the two in use
-                uint4 next_k[2], next_q[2];
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const int at = min(i + 2 + u, chunks - 1);
-                    next_k[u] = key[at];
-                    next_q[u] = query[at];
-                }
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    if (i + u < chunks) {
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) sum = fmaf(bf_half(qq[u], e), bf_half(kv[u], e), sum);
-                    }
-                    kv[u] = next_k[u];
-                    qq[u] = next_q[u];
-                }
-            }
+            const float sum = ordered_dot(query, reinterpret_cast<const uint4*>(tile + (size_t)threadIdx.x * pitch), chunks);
             const float score = bf_load(bf_round(sum));
             scores[t0 + threadIdx.x] = score;
             maximum = fmaxf(maximum, score);
@@ -687,17 +757,7 @@ __global__ void __launch_bounds__(256, 1) gm_attention_kernel(const bf16_t* q, c
     maximum = block_max(maximum, scratch);  // its barriers also order the score writes before the reads below
     for (int t = threadIdx.x; t < visible; t += blockDim.x) scores[t] = (float)exp((double)(scores[t] - maximum));
     __syncthreads();
-    if (threadIdx.x == 0) {
-        const float4* quads = reinterpret_cast<const float4*>(scores);
-        float total = 0.0f;
-#pragma unroll 8
-        for (int t = 0; t < visible / 4; ++t) {
-            const float4 v = quads[t];
-            total += v.x; total += v.y; total += v.z; total += v.w;
-        }
-        for (int t = visible & ~3; t < visible; ++t) total += scores[t];
-        total_slot = total;
-    }
+    if (threadIdx.x == 0) total_slot = ordered_sum(scores, visible);
     __syncthreads();
     const float total = total_slot;
     for (int t = threadIdx.x; t < visible; t += blockDim.x) scores[t] = bf_load(bf_round(scores[t] / total));
@@ -1200,6 +1260,7 @@ RIBN_B200_API int ribn_b200_gemma_finalize(ribn_b200_gemma* m) {
     if (attention_smem_bytes(32, c.context, widest) > kAttnSmemLimit) {
         return fail(m, RIBN_B200_ERROR, "context %d exceeds the attention kernel's score buffer", c.context);
     }
+    GM_CUDA(m, cudaFuncSetAttribute(gm_attention_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAttnSmemLimit));
     GM_CUDA(m, cudaFuncSetAttribute(gm_attention_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAttnSmemLimit));
     GM_CUDA(m, cudaFuncSetAttribute(gm_attention_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAttnSmemLimit));
     GM_CUDA(m, cudaFuncSetAttribute(gm_attention_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAttnSmemLimit));
@@ -1304,11 +1365,17 @@ int enqueue_pass(ribn_b200_gemma* m, int rows, int n_out, int max_position, uint
             m->value_cache[(size_t)cache]);
         const int window = kind ? 0 : c.window;
         const int visible = window > 0 && window < max_position + 1 ? window : max_position + 1;
+        const auto attend = [&](auto kernel, dim3 grid, size_t smem) {
+            p.launch(kernel, grid, 256, smem, m->q2, m->d_slot, m->d_position, m->key_cache[(size_t)cache], m->value_cache[(size_t)cache],
+                     c.heads, c.kv_heads, w, window, c.context, m->attended);
+        };
+        const dim3 grid((unsigned)rows, (unsigned)c.heads);
         const int tile = attention_tile(visible, w, rows * c.heads, m->sms);
-        const auto attention = tile == 128 ? gm_attention_kernel<128> : tile == 64 ? gm_attention_kernel<64> : gm_attention_kernel<32>;
-        p.launch(attention, dim3((unsigned)rows, (unsigned)c.heads), 256, attention_smem_bytes(tile, visible, w),
-            m->q2, m->d_slot, m->d_position, m->key_cache[(size_t)cache], m->value_cache[(size_t)cache], c.heads, c.kv_heads, w,
-            window, c.context, m->attended);
+        const size_t smem = attention_smem_bytes(tile, visible, w);
+        if (attention_splits(visible, w, rows * c.heads, m->sms)) attend(gm_attention_split_kernel, dim3(grid.x, grid.y, kAttnCluster), attention_split_bytes(visible, w));
+        else if (tile == 128) attend(gm_attention_kernel<128>, grid, smem);
+        else if (tile == 64) attend(gm_attention_kernel<64>, grid, smem);
+        else attend(gm_attention_kernel<32>, grid, smem);
         p.project(m->attended, rows, L[L_O].data, H, c.heads * w, m->projected);
         p.rms(m->projected, nullptr, rows, H, L[L_POST_ATTN].data, m->hidden, nullptr, 1, m->mid, L[L_PRE_FFN].data, m->normed);
         // feed-forward (decoder.rs:570-600)

@@ -80,6 +80,31 @@ def test_chunking_and_batching_do_not_change_any_bit():
     model.close()
 
 
+RAGGED = dict(layers=2, hidden=328, heads=4, kv_heads=1, head_dim=256, global_head_dim=256, ffn=9000, vocab=5000, ple=24,
+              ple_vocab=5000, window=100, context=200, kv_shared=0, eps=1.0e-6, softcap=30.0, theta_local=1.0e4,
+              theta_global=1.0e6, layer_types=["sliding", "full"])
+
+
+@pytest.fixture(scope="module")
+def ragged_pair():
+    model, oracle = build_pair(RAGGED, 14, max_sequences=1, max_batch_tokens=128)
+    yield model, oracle
+    model.close(); oracle.close()
+
+
+@pytest.mark.parametrize("rows", [1, 3, 4, 9, 10, 17, 40, 129])
+def test_projection_and_attention_variants_match_the_oracle(ragged_pair, rows):
+    # row counts either side of each variant's tile, widths that leave a remainder in every tile, then a decode row
+    # whose keys are split over a cluster
+    model, oracle = ragged_pair
+    prompt = np.random.default_rng(rows).integers(0, 104, rows).tolist()
+    dev, ref = model.open(), oracle.new_sequence()
+    for tokens in (prompt, [7], [9]):
+        _, same = logits_close(dev.prefill(tokens), ref.prefill(tokens))
+        assert same > 0.9, same
+    dev.close()
+
+
 def test_invalid_rows_are_rejected_without_advancing():
     model, _ = build_pair(SMALL, 13, max_sequences=2, max_batch_tokens=8)
     s = model.open()
