@@ -143,23 +143,23 @@ __global__ void gm_embed_kernel(const uint32_t* tokens, const bf16_t* __restrict
 // ---------------------------------------------------------------------------------------------
 // Projection: out[r][n] = bf16(sum_k in[r][k] * w[n][k]) (linear.rs:23-66), the sum in k order.  A block is a
 // feeder warp and GR x GC consumer warps.  A consumer owns 32 * C output columns for R rows: a thread walks C weight
-// rows and keeps R * C independent accumulation chains, pairs of rows packed (`fma.rn.f32x2` rounds each half as
-// `fmaf` does).  The feeder brings weight tiles by cp.async into a ring of stages (rows pitched 16 bytes apart from a
-// multiple of 128, so the 128-bit reads of a quarter-warp fall in distinct banks) and the input rows beside them: one
-// row as it is, four rows expanded to FP32 and interleaved as the consumers' packed operands.  Named barriers hand
+// rows and keeps R * C independent accumulation chains, fed with BF16 operands as they lie (`fma_half`).  The feeder
+// brings tiles of the weights and of the blocks' input rows by cp.async into a ring of stages (rows pitched 16 bytes
+// apart from a multiple of 128, so the 128-bit reads of a quarter-warp fall in distinct banks).  Named barriers hand
 // the stages over; their ids are constants because an SM has 64 barriers and a block whose ids are computed is given
 // 16 of them.  Four consumer warps per block fall on the four schedulers; two-warp blocks leave two without one.
 //
 // What bounds it: the chain of dependent additions, 4 cycles per input (14.4 us for the 6,912 inputs of a down
 // projection), or, with several chains per scheduler, issue and the shared-memory reads (a 128-bit read occupies a
-// scheduler's return path about 12 cycles, broadcast or not).  Measured per input of a consumer warp, alone and with
-// others on its scheduler: one row 5.6 and 4, 4 rows x 1 column 14.5 and 10.2, 4 x 2 19.5 and 13.8 cycles; 4 x 2 with
-// BF16 input rows 28.
+// scheduler's return path about 12 cycles, broadcast or not).  One warp per 32 columns that copied for itself and
+// unpacked every operand took 24 cycles per input of four rows.  Measured on 1,152-wide models, start -> now: down at
+// 4 rows 97 -> 24.6 us, at 35 rows 150 -> 47.6, at 113 rows 175 -> 66; gate|up 18.6 -> 12.1 (4.9 of HBM time), at 113
+// rows 205 -> 113.
 // ---------------------------------------------------------------------------------------------
 struct ProjectNarrow { static constexpr int R = 1, C = 1, GR = 1, GC = 1, tile = 256, stages = 4; };   // a few rows: chains spread over blocks
 struct ProjectWide { static constexpr int R = 4, C = 1, GR = 1, GC = 4, tile = 128, stages = 3; };     // up to four rows of a wide projection
 struct ProjectRows { static constexpr int R = 4, C = 1, GR = 4, GC = 1, tile = 128, stages = 3; };     // a few tens of rows
-struct ProjectChunk { static constexpr int R = 4, C = 2, GR = 4, GC = 1, tile = 128, stages = 2; };    // prefill
+struct ProjectChunk { static constexpr int R = 4, C = 2, GR = 4, GC = 1, tile = 128, stages = 3; };    // prefill
 template <typename V>
 struct ProjectShape {
     static constexpr int consumers = V::GR * V::GC, threads = 32 * (1 + consumers);
@@ -283,26 +283,35 @@ __global__ void __launch_bounds__(ProjectShape<V>::threads, 4) gm_project_kernel
         const unsigned char* ws = stage + (gc * 32 * C + lane) * S::pitch;
         const unsigned char* xs = stage + S::x_offset + gr * R * S::pitch;
         const int count = min(S::chunks, chunks - t * S::chunks);
-        auto chunk = [&](int i) {
-            uint4 w[C], x[R];
+        struct Group { uint4 w[C], x[R]; };   // eight inputs
+        auto fetch = [&](Group& to, int i) {
 #pragma unroll
-            for (int c = 0; c < C; ++c) w[c] = *reinterpret_cast<const uint4*>(ws + c * 32 * S::pitch + i * 16);
+            for (int c = 0; c < C; ++c) to.w[c] = *reinterpret_cast<const uint4*>(ws + c * 32 * S::pitch + i * 16);
 #pragma unroll
-            for (int r = 0; r < R; ++r) x[r] = *reinterpret_cast<const uint4*>(xs + r * S::pitch + i * 16);
+            for (int r = 0; r < R; ++r) to.x[r] = *reinterpret_cast<const uint4*>(xs + r * S::pitch + i * 16);
+        };
+        auto add = [&](const Group& from) {
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
 #pragma unroll
                 for (int c = 0; c < C; ++c) {
 #pragma unroll
-                    for (int r = 0; r < R; ++r) sum[c][r] = fma_half(x[r], w[c], sum[c][r], e);
+                    for (int r = 0; r < R; ++r) sum[c][r] = fma_half(from.x[r], from.w[c], sum[c][r], e);
                 }
             }
         };
-        if (count == S::chunks) {
-#pragma unroll(R == 1 ? 8 : 2)
-            for (int i = 0; i < S::chunks; ++i) chunk(i);
-        } else {
-            for (int i = 0; i < count; ++i) chunk(i);
+        if (R == 1 && count == S::chunks) {
+#pragma unroll 8
+            for (int i = 0; i < S::chunks; ++i) { Group one; fetch(one, i); add(one); }
+        } else {   // the next group's reads are under way while this one is added
+            Group now, next;
+            fetch(now, 0);
+#pragma unroll 2
+            for (int i = 0; i < count; ++i) {
+                fetch(next, min(i + 1, count - 1));
+                add(now);
+                now = next;
+            }
         }
         if (t + kStages < tiles) stage_barrier<1 + kStages, kStages, kThreads>(slot, false);
         slot = slot + 1 == kStages ? 0 : slot + 1;
@@ -320,7 +329,8 @@ __global__ void __launch_bounds__(ProjectShape<V>::threads, 4) gm_project_kernel
     }
 }
 
-// Which variant: the one whose busiest scheduler finishes first, by the cycles per input measured above.  A narrow
+// Which variant: the one whose busiest scheduler finishes first, by cycles per input of a consumer warp, alone and for
+// each that shares its scheduler (measured for one row, 4.8 and 3.1; for the others near the reads they make).  A narrow
 // projection of a few rows goes to one warp per row and 32 columns (1,152 columns x four rows: 144 warps), many rows
 // or columns to the variants that spend less per product and read the weights fewer times.
 int project_variant(const int* n, int count, int rows, int sms) {
