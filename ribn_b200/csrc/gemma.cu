@@ -152,9 +152,9 @@ __global__ void gm_embed_kernel(const uint32_t* tokens, const bf16_t* __restrict
 // What bounds it: the chain of dependent additions, 4 cycles per input (14.4 us for the 6,912 inputs of a down
 // projection), or, with several chains per scheduler, issue and the shared-memory reads (a 128-bit read occupies a
 // scheduler's return path about 12 cycles, broadcast or not).  One warp per 32 columns that copied for itself and
-// unpacked every operand took 24 cycles per input of four rows.  Measured on 1,152-wide models, start -> now: down at
-// 4 rows 97 -> 24.6 us, at 35 rows 150 -> 47.6, at 113 rows 175 -> 66; gate|up 18.6 -> 12.1 (4.9 of HBM time), at 113
-// rows 205 -> 113.
+// unpacked every operand took 24 cycles per input of four rows.  Measured on a 1,152-wide model, before -> now: a layer's
+// three projections to 1,152 columns (1,024, 6,912 and 256 inputs) 105 -> 35 us at 4 rows, 162 -> 64 at 35, 179 -> 87 at
+// 113; gate|up 18.6 -> 12.1 us at 4 rows (4.9 of HBM time), 205 -> 113 at 113.
 // ---------------------------------------------------------------------------------------------
 struct ProjectNarrow { static constexpr int R = 1, C = 1, GR = 1, GC = 1, tile = 256, stages = 4; };   // a few rows: chains spread over blocks
 struct ProjectWide { static constexpr int R = 4, C = 1, GR = 1, GC = 4, tile = 128, stages = 3; };     // up to four rows of a wide projection
