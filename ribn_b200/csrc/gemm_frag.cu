@@ -3,13 +3,20 @@
 //   y[m][n] = sum_k deq(W[n][k]) x[m][k]
 //
 // The packed tiles already hold, per lane, the bytes of its MMA A fragments, so a weight never passes through
-// shared memory a second time: a lane masks its bytes straight into binary16 SUBNORMALS (the bit pattern of a
-// small integer q is the number q 2^-24, which the tensor core multiplies exactly), one LOP3 per two weights, and
-// `mma.sync.m16n8k16` adds them against the activations' binary16 hi + lo pairs.  One group of inputs that shares a
-// block scale (32 inputs of Q4_K and Q8_0, 16 of Q6_K) is one chain of MMAs; its F32 sum is folded into the tile's
-// sum with the group's exact F32 scale, and the tile's (256 inputs) into the row's sum with the activations' power-
-// of-two scale, both round-to-nearest.  Offsets (Q4_K minima, Q6_K -32, Q8_0 -128) are one more MMA per tile against
-// the activations' group sums.
+// shared memory a second time: a lane masks its bytes straight into binary16 SUBNORMALS (the bit pattern of an
+// integer i below 1024 is the number i 2^-24), about one LOP3 per two weights, and `mma.sync.m16n8k16` adds them against
+// the activations' binary16 hi + lo pairs.  By its errors the tensor core aligns a step's products as if a subnormal
+// were a full-scale 2^-14 and cuts what falls below the sum's F32 resolution there, so an integer has to fill the ten bits to be added as
+// exactly as a normal number: Q8_0's eight bits do (3e-7 of a row's results from the exact ones at K = 4,096), Q4_K's
+// nibbles are taken four bits up (2.6e-7; as they lie 1.8e-6, and 5.6e-6 with the wide-ranging inputs that a gate leaves,
+// against 7e-7 and 8e-7 of the kernel of gemm_tc.cu), and Q6_K's six bits become the signed normal number q - 32, which
+// also spares the cancellation of an offset (1.3e-7; as they lie 5e-7, and 1.5e-6 with those inputs).  The shifts take 0.9 %
+// of a step of 5 rows of the 8B model; without the offset's product a step of 16 rows is 0.6 % faster.
+//
+// One group of inputs that shares a block scale (32 inputs of Q4_K and Q8_0, 16 of Q6_K) is one chain of MMAs; its F32 sum
+// is folded into the tile's sum with the group's exact F32 scale, and the tile's (256 inputs) into the row's sum with the
+// activations' power-of-two scale, both round-to-nearest.  Offsets (Q4_K minima, Q8_0 -128) are one more MMA per tile
+// against the activations' group sums.
 //
 // Why not a tcgen05 pipeline that converts its A operand through shared memory: at these row counts its hand-offs
 // (packed ring -> registers -> shared memory -> MMA -> commit -> tensor memory -> registers) cost several
@@ -39,7 +46,7 @@ constexpr int kTeams = kFragTeams;
 constexpr int kTeamWarps = 4;                    // warps per team, two row tiles each
 constexpr int kWarps = kTeams * kTeamWarps;
 constexpr int kThreads = (kTeams + 1) * kTeamWarps * 32;
-constexpr int kSum16At = 16 * 512, kSum32At = kSum16At + 512, kScaleAt = kSum32At + 256;
+constexpr int kSum32At = 16 * 512, kScaleAt = kSum32At + 256;
 static_assert(kScaleAt + 32 == kFragBlockBytes, "operand block layout");
 constexpr uint32_t kSpinLimit = 1u << 22;
 constexpr size_t kSmemBudget = 220 * 1024;
@@ -133,6 +140,12 @@ __device__ __forceinline__ float half_low(uint32_t w) { return __half2float(__us
 __device__ __forceinline__ float half_high(uint32_t w) { return __half2float(__ushort_as_half((unsigned short)(w >> 16))); }
 
 constexpr float kTwo24 = 16777216.0f, kTwo20 = 1048576.0f;   // an integer masked into binary16 is that integer times 2^-24
+__device__ __forceinline__ __half2 as_half2(uint32_t x) { return *reinterpret_cast<const __half2*>(&x); }
+__device__ __forceinline__ uint32_t as_bits(__half2 x) { return *reinterpret_cast<const uint32_t*>(&x); }
+// bytes i and j of w (selector 0x4j4i) as a pair of normal binary16 integers
+__device__ __forceinline__ uint32_t bytes_half2(uint32_t w, uint32_t selector) {
+    return as_bits(__hsub2(as_half2(__byte_perm(w, 0x64646464u, selector)), __float2half2_rn(1024.0f)));
+}
 
 // c: (row g, columns 2t, 2t + 1), (row g + 8, the same); s0 / s1: factors of rows g / g + 8
 __device__ __forceinline__ void fold(float (&acc)[4], const float (&c)[4], float s0, float s1) {
@@ -172,9 +185,9 @@ __device__ __forceinline__ void group_mma(float (&d)[2][NG][4], const Frag (&a)[
 template <int NG>
 using TileSums = float[2][NG][4];
 
-// A warp's row records: its 32 rows' scales as F32 and its offsets' A operand, written by lane = row (decoding a row's
+// A warp's row records: its 32 rows' scales as F32 and the minima's A operand, written by lane = row (decoding a row's
 // header once instead of in each of the four lanes that need it) and read back in fragment order.
-//   words 0..7 scales, 8..11 offset operand (binary16 pairs), 12 offset factor; a pitch of 20 words is conflict-free
+//   words 0..7 scales, 8..11 Q4_K minima (binary16 pairs), 12 their factor; a pitch of 20 words is conflict-free
 constexpr int kRecWords = 20;
 struct Record {
     uint32_t wr, rd;   // this lane's row / row g of the warp's first row tile
@@ -196,11 +209,11 @@ __device__ __forceinline__ void slot_q4k(uint32_t tile, uint32_t b_at, const Rec
         const float d = half_low(hd.x);
         const uint32_t s_lo = hd.y & 0x3F3F3F3Fu, s_hi = and_or(hd.w, 0x0F0F0F0Fu, (hd.y >> 2) & 0x30303030u);
         const uint32_t m_lo = hd.z & 0x3F3F3F3Fu, m_hi = and_or(hd.w >> 4, 0x0F0F0F0Fu, (hd.z >> 2) & 0x30303030u);
-        const float2 dd = make_float2(d * kTwo24, d * kTwo20);   // odd groups: their nibbles sit 4 bits up
+        const float2 dd = make_float2(d * kTwo20, d * kTwo20);   // the nibbles are taken 4 bits up
         sts128f(rec.wr, bytes_scaled(s_lo, 0, 8388608.0f, dd), bytes_scaled(s_lo, 2, 8388608.0f, dd));
         sts128f(rec.wr + 16, bytes_scaled(s_hi, 0, 8388608.0f, dd), bytes_scaled(s_hi, 2, 8388608.0f, dd));
-        sts128(rec.wr + 32, __byte_perm(m_lo, 0u, 0x4140), __byte_perm(m_lo, 0u, 0x4342), __byte_perm(m_hi, 0u, 0x4140), __byte_perm(m_hi, 0u, 0x4342));
-        sts32f(rec.wr + 48, half_high(hd.x) * -kTwo24);
+        sts128(rec.wr + 32, bytes_half2(m_lo, 0x4140u), bytes_half2(m_lo, 0x4342u), bytes_half2(m_hi, 0x4140u), bytes_half2(m_hi, 0x4342u));
+        sts32f(rec.wr + 48, -half_high(hd.x));
     }
     __syncwarp();
 #pragma unroll kUnroll
@@ -221,15 +234,15 @@ __device__ __forceinline__ void slot_q4k(uint32_t tile, uint32_t b_at, const Rec
 #pragma unroll
                 for (int n = 0; n < NG; ++n) b[part][n] = lds128(b_at + n * kFragBlockBytes + (4 * j + 2 * odd + part) * 512 + lane * 16);
             }
-            const uint32_t mask = odd ? 0x00F000F0u : 0x000F000Fu;
+            constexpr uint32_t mask = 0x00F000F0u;
             Frag a[2][2];
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
 #pragma unroll
                 for (int part = 0; part < 2; ++part) {
                     const uint32_t top = part == 0 ? w[r].x : w[r].y, bottom = part == 0 ? w[r].z : w[r].w;   // rows g, g + 8
-                    a[r][part].r[0] = top & mask; a[r][part].r[2] = (top >> 8) & mask;
-                    a[r][part].r[1] = bottom & mask; a[r][part].r[3] = (bottom >> 8) & mask;
+                    a[r][part].r[0] = (odd ? top : top << 4) & mask; a[r][part].r[2] = (odd ? top >> 8 : top >> 4) & mask;
+                    a[r][part].r[1] = (odd ? bottom : bottom << 4) & mask; a[r][part].r[3] = (odd ? bottom >> 8 : bottom >> 4) & mask;
                 }
             }
             float d[2][NG][4];
@@ -321,20 +334,18 @@ __device__ __forceinline__ void slot_q8_0(uint32_t tile, uint32_t b_at, const Re
 // ---- Q6_K: w = d sc (q - 32), one scale per 16 inputs -----------------------------------------------------------
 template <int NG>
 __device__ __forceinline__ void slot_q6k(uint32_t tile, uint32_t b_at, const Record& rec, int lane, TileSums<NG>& sums) {
-    const int g = lane >> 2, t = lane & 3;
     const uint32_t own = tile + (lane >> 4) * 3360, own_scales = own + 3072 + (lane & 15) * 16;
     const float d = half_low(lds16(own + 3328 + (lane & 15) * 2));
 #pragma unroll 1
     for (int c = 0; c < 2; ++c) {
         if (c == 1) __syncwarp();
         {
-            // the eight 16-input scales of this half: variants 0, 1 (low nibbles), then 2, 3 (their nibbles sit 4 bits up)
+            // the eight 16-input scales of this half
             uint2 sc = lds64(own_scales + c * 8);
             sc.x ^= 0x80808080u; sc.y ^= 0x80808080u;
-            const float2 low = make_float2(d * kTwo24, d * kTwo24), high = make_float2(d * kTwo20, d * kTwo20);
-            sts128f(rec.wr, bytes_scaled(sc.x, 0, 8388736.0f, low), bytes_scaled(sc.x, 2, 8388736.0f, low));
-            sts128f(rec.wr + 16, bytes_scaled(sc.y, 0, 8388736.0f, high), bytes_scaled(sc.y, 2, 8388736.0f, high));
-            if (c == 0) sts32f(rec.wr + 48, -32.0f * d);
+            const float2 dd = make_float2(d, d);
+            sts128f(rec.wr, bytes_scaled(sc.x, 0, 8388736.0f, dd), bytes_scaled(sc.x, 2, 8388736.0f, dd));
+            sts128f(rec.wr + 16, bytes_scaled(sc.y, 0, 8388736.0f, dd), bytes_scaled(sc.y, 2, 8388736.0f, dd));
         }
         __syncwarp();
         uint4 qh[2];
@@ -357,11 +368,12 @@ __device__ __forceinline__ void slot_q6k(uint32_t tile, uint32_t b_at, const Rec
                     for (int h = 0; h < 2; ++h) {
                         const uint32_t low = h == 0 ? ((v & 1) ? w[r].y : w[r].x) : ((v & 1) ? w[r].w : w[r].z);
                         const uint32_t high = h == 0 ? (kh == 0 ? qh[r].x : qh[r].z) : (kh == 0 ? qh[r].y : qh[r].w);
-                        // the variant's two high bits (bits 2v of each byte) go above its nibble
+                        // the variant's two high bits (bits 2v of each byte) go above its nibble: 1024 + q, or 1024 + 16 q
                         const uint32_t up = (v & 1) ? high << 2 : high << 4, down = (v & 1) ? high >> 6 : high >> 4;
                         const uint32_t lm = v < 2 ? 0x000F000Fu : 0x00F000F0u, hm = v < 2 ? 0x00300030u : 0x03000300u;
-                        a[r][0].r[h] = and_or(low, lm, up & hm);
-                        a[r][0].r[h + 2] = and_or(low >> 8, lm, down & hm);
+                        const __half2 mul = __float2half2_rn(v < 2 ? 1.0f : 0.0625f), bias = __float2half2_rn(v < 2 ? -1056.0f : -96.0f);
+                        a[r][0].r[h] = as_bits(__hfma2(as_half2(and_or(low, lm, and_or(up, hm, 0x64006400u))), mul, bias));
+                        a[r][0].r[h + 2] = as_bits(__hfma2(as_half2(and_or(low >> 8, lm, and_or(down, hm, 0x64006400u))), mul, bias));
                     }
                 }
                 float dsum[2][NG][4];
@@ -373,29 +385,6 @@ __device__ __forceinline__ void slot_q6k(uint32_t tile, uint32_t b_at, const Rec
                     for (int n = 0; n < NG; ++n) fold(sums[r][n], dsum[r][n], __uint_as_float(f0), __uint_as_float(f1));
                 }
             }
-        }
-    }
-    // offset: the sixteen subs' scales x their input sums, times 32 d
-    uint32_t sa[2][4];
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {   // fragment register i: row half i & 1, subs 2t + 8 (i >> 1), + 1
-            const uint32_t two = lds16(tile + r * 3360 + 3072 + (g + 8 * (i & 1)) * 16 + 2 * t + 8 * (i >> 1)) ^ 0x8080u;
-            const uint32_t x = __byte_perm(two, 0x64646464u, 0x4140);   // 1024 + (sc + 128)
-            const __half2 hv = __hsub2(*reinterpret_cast<const __half2*>(&x), __float2half2_rn(1152.0f));
-            sa[r][i] = *reinterpret_cast<const uint32_t*>(&hv);
-        }
-    }
-#pragma unroll
-    for (int n = 0; n < NG; ++n) {
-        const uint4 s = lds128(b_at + n * kFragBlockBytes + kSum16At + lane * 16);
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            float dsum[4];
-            mma_first(dsum, sa[r][0], sa[r][1], sa[r][2], sa[r][3], s.z, s.w);
-            mma_next(dsum, sa[r][0], sa[r][1], sa[r][2], sa[r][3], s.x, s.y);
-            fold(sums[r][n], dsum, __uint_as_float(rec_word(rec, r, 0, 12)), __uint_as_float(rec_word(rec, r, 1, 12)));
         }
     }
     __syncwarp();

@@ -235,7 +235,6 @@ int gemm_tc_last_launches();
 // per row and k tile, in one of two block forms:
 //   kFragmentForm (gemm_frag.cu, mma.sync): groups of 8 ng rows (at most 32), ng blocks of eight rows each
 //     [16 steps][lane] 16 bytes   hi pairs (4t, 4t + 2), (4t + 1, 4t + 3) of the step's 16 inputs of row lane / 4, then lo pairs
-//     [lane] 16 bytes             sums of the sixteen 16-input subs as an operand pair (hi, then lo)
 //     [lane] 8 bytes              sums of the eight 32-input groups: hi in the first eight operand rows, lo in the last eight
 //     [8] F32                     the rows' scales
 //   kColumnForm (gemm_ta.cu, tcgen05): groups of mp = 8 ng rows (at most 64), one block
@@ -247,7 +246,7 @@ int gemm_tc_last_launches();
 // Blocks are ordered [group][k tile](ng).  `ss` holds, per row and k tile, the sum of squares of the values before the
 // norm weight, for the RMSNorm factor of the consumer.
 enum StepForm : int { kFragmentForm = 0, kColumnForm = 1, kWideForm = 2 };
-constexpr int kFragBlockBytes = 16 * 512 + 512 + 256 + 32;
+constexpr int kFragBlockBytes = 16 * 512 + 256 + 32;
 
 struct StepOperand {
     unsigned char* blocks = nullptr;

@@ -16,7 +16,7 @@ namespace ribn {
 namespace {
 
 constexpr int kUnitTiles = 8;   // row tiles per tensor copy and per unit: 128 output rows (two units make one of the wide form)
-constexpr int kSum16At = 16 * 512, kSum32At = kSum16At + 512, kScaleAt = kSum32At + 256;   // fragment-form block
+constexpr int kSum32At = 16 * 512, kScaleAt = kSum32At + 256;   // fragment-form block
 
 // RMSNorm factor of one row from the sums of squares of its k tiles (every lane of the warp gets it).
 __device__ __forceinline__ float norm_factor(const float* ss, int tiles, float eps, int lane) {
@@ -152,12 +152,6 @@ __global__ void __launch_bounds__(512, BATCH > 2 ? 1 : 3) step_finish_kernel(con
     *reinterpret_cast<uint4*>(blk + s * 512 + (g * 4 + t) * 16) = make_uint4(pack(hi[0], hi[2]), pack(hi[1], hi[3]), pack(lo[0], lo[2]), pack(lo[1], lo[3]));
     sum += __shfl_xor_sync(0xffffffffu, sum, 1);
     sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-    if (t == 0) {   // sub s: element s & 7 of lanes (g, (s & 7) / 2), register pair half s >> 3
-        const __half h = __float2half_rn(sum), l = __float2half_rn(sum - __half2float(h));
-        __half* at = reinterpret_cast<__half*>(blk + kSum16At + (g * 4 + ((s & 7) >> 1)) * 16 + (s >> 3) * 4) + (s & 1);
-        at[0] = h;
-        at[4] = l;
-    }
     sum += __shfl_xor_sync(0xffffffffu, sum, 4);
     if ((i & 7) == 0) {
         const int q = i >> 3;
