@@ -22,9 +22,15 @@
 // (measured: with the products and the conversion left out, a k tile with three `tcgen05.commit`s still took 1,900 clocks), so
 // a k tile has ONE commit (two for Q6_K, whose A operand fills two stages), which frees its A stage and starts its fold; one
 // arrival per fold warp frees the sums and the activations' slot.
-// Tensor memory: main sums of k tile parity p at columns 64 p, minima sums at 128 + 64 p, A stages at 256 + 128 s (256
-// inputs of Q4_K's one plane, 128 inputs of the others' two).  Slots (unit, row group, k tile) are dealt to the CTAs evenly
-// when another kernel finishes the sums, in whole items otherwise (StepSplit).  Every wait is bounded.
+// Tensor memory: main sums of k tile parity p at columns 64 p, at 128 + 64 p the minima sums of Q4_K or the sums of
+// Q6_K's second half, A stages at 256 + 128 s (256 inputs of Q4_K's one plane, 128 inputs of the others' two).
+// An addition in tensor memory cuts at the sum's last bit, so its error grows with the number of steps that a sum is already
+// large in.  With one sum per tile and p1 before p2, Q6_K was 1.5 times as far from the exact results as the kernel of
+// gemm_tc.cu (6.7e-7 against 4.6e-7 of a row's results at 48 and more columns); with a sum per half and the small parts
+// first it is at 2.0e-7, for 0.7 % of a step of 64 rows.  Q8_0's one sum per tile (5.2e-7, 7.1e-7 at 48 and more columns)
+// replaced one over all inputs there (2.7e-6 to 2.9e-5); a sum per half (2.0e-7) would cost 4 % of a step of 32 rows of
+// the 0.6B model.  Slots (unit, row group, k tile) are dealt to the CTAs evenly when another kernel finishes the sums, in
+// whole items otherwise (StepSplit).  Every wait is bounded.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -139,7 +145,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ta_kernel(const StepGemm a, 
             uint32_t b_parity = 0, fold_parity = 0, a_count = 0, kt = 0, q6_count = 0;
             for (int s = s0; s < s1;) {
                 const int item = s / k_tiles, end = min(s1, (item + 1) * k_tiles);
-                const bool q4k = type_of<TYPE>(a.seg[unit_at(a, item / split.groups, kUnitTiles).seg]) == kQ4_K;
+                const int type = type_of<TYPE>(a.seg[unit_at(a, item / split.groups, kUnitTiles).seg]);
+                const bool q4k = type == kQ4_K, q6k = TYPE == kKQuants ? !q4k : type == kQ6_K;
                 for (; s < end; ++s, ++kt) {
                     const uint32_t p = kt & 1u, d_main = tmem + 64 * p, d_min = tmem + 128 + 64 * p;
                     if (kt >= 2) {   // the fold of k tile kt - 2 has left these sums
@@ -174,18 +181,19 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ta_kernel(const StepGemm a, 
                                 if (alive) alive = mbar_wait(a_full + 8 * hs, (a_count >> 1) & 1u, a.error_flag, 95, spin_limit);
                                 tc_fence_after();
                             }
-                            const uint32_t b_half = b_desc + 8 * half * kStep;
-                            // position i of the stage holds step 4 (i >> 2) + 2 (i & 1) + ((i >> 1) & 1) of the half.
-                            // p2 x lo is below F32's resolution: left out where it costs an MMA.
+                            const uint32_t b_half = b_desc + 8 * half * kStep, d_half = half == 1 && q6k ? d_min : d_main;
+                            // position i of the stage holds step 4 (i >> 2) + 2 (i & 1) + ((i >> 1) & 1) of the half.  The
+                            // small parts first.  p2 x lo is left out where it costs an MMA: at most 2^-22 of a product, and
+                            // only p of more than eleven bits have a p2, so that it is 3e-8 of a row's result
                             if (leader) {
 #pragma unroll
-                                for (int pass = C::kJoined ? 1 : 0; pass < 3; ++pass) {   // (lo x p1 apart,) p1, p2
+                                for (int pass = C::kJoined ? 1 : 0; pass < 3; ++pass) {   // (p1 x lo apart,) p2, p1
 #pragma unroll
                                     for (int i = 0; i < 8; ++i) {
                                         const uint32_t b = b_half + (4 * (i >> 2) + 2 * (i & 1) + ((i >> 1) & 1)) * kStep;
-                                        const uint32_t acc = (i != 0 || pass != (C::kJoined ? 1 : 0)) ? 1u : (uint32_t)half;
-                                        if (pass == 0) umma_ts(d_main, h_at + 8 * i, b + kLo, idesc_one, acc);
-                                        else umma_ts(d_main, h_at + (pass == 2 ? 64 : 0) + 8 * i, b, C::kJoined ? idesc_both : idesc_one, acc);
+                                        const uint32_t acc = i != 0 || pass != (C::kJoined ? 1 : 0) || (half == 1 && !q6k);
+                                        if (pass == 0) umma_ts(d_half, h_at + 8 * i, b + kLo, idesc_one, acc);
+                                        else umma_ts(d_half, h_at + (pass == 1 ? 64 : 0) + 8 * i, b, C::kJoined ? idesc_both : idesc_one, acc);
                                     }
                                 }
                                 umma_commit(half == 0 ? half_done + 8 * (q6_count & 1u) : done + 8 * bs);
@@ -262,7 +270,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ta_kernel(const StepGemm a, 
             const int item = s / k_tiles, unit = item / split.groups, group = item - unit * split.groups;
             const UnitAt at = unit_at(a, unit, kUnitTiles);
             const GemvSegment& seg = a.seg[at.seg];
-            const bool q4k = type_of<TYPE>(seg) == kQ4_K;
+            const int type = type_of<TYPE>(seg);
+            const bool q4k = type == kQ4_K, q6k = TYPE == kKQuants ? !q4k : type == kQ6_K;
             const int end = min(s1, (item + 1) * k_tiles);
             float acc[kChunks][8];
 #pragma unroll
@@ -282,14 +291,15 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ta_kernel(const StepGemm a, 
                 constexpr int kBatch = kChunks < 2 ? 1 : 2;   // eights of columns in flight together
 #pragma unroll
                 for (int j0 = 0; j0 < kChunks; j0 += kBatch) {
-                    float x[kBatch][8], y[kBatch][8], z[kBatch][8];
+                    float x[kBatch][8], y[kBatch][8], z[kBatch][8], w[kBatch][8];
 #pragma unroll
                     for (int b = 0; b < kBatch; ++b) {
                         const int j = j0 + b;
                         if (16 * j + mine < MP) {
                             tmem_ld8(t_main + 16 * j, x[b]);
                             if (C::kJoined) tmem_ld8(t_main + MP + 16 * j, y[b]);
-                            if (q4k) tmem_ld8(t_min + 16 * j, z[b]);
+                            if (q4k || q6k) tmem_ld8(t_min + 16 * j, z[b]);       // minima sums, or the second half's
+                            if (C::kJoined && q6k) tmem_ld8(t_min + MP + 16 * j, w[b]);
                         }
                     }
                     tmem_wait_ld();
@@ -299,7 +309,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ta_kernel(const StepGemm a, 
                         if (j >= kChunks || 16 * j + mine >= MP) continue;
                         tmem_tie(x[b]);
                         if (C::kJoined) tmem_tie(y[b]);
-                        if (q4k) tmem_tie(z[b]);
+                        if (q4k || q6k) tmem_tie(z[b]);
+                        if (C::kJoined && q6k) tmem_tie(w[b]);
 #pragma unroll
                         for (int i = 0; i < 8; i += 4) {
                             float sx[4];
@@ -307,7 +318,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ta_kernel(const StepGemm a, 
                                          : "r"(sx_at + (16 * j + i) * 4));
 #pragma unroll
                             for (int q = 0; q < 4; ++q) {
-                                float v = d * (C::kJoined ? x[b][i + q] + y[b][i + q] : x[b][i + q]);
+                                float v = q6k ? x[b][i + q] + z[b][i + q] : x[b][i + q];
+                                if (C::kJoined) v += q6k ? y[b][i + q] + w[b][i + q] : y[b][i + q];
+                                v *= d;
                                 if (q4k) v = fmaf(-dmin, z[b][i + q], v);
                                 acc[j][i + q] = fmaf(sx[q], v, acc[j][i + q]);
                             }
