@@ -6,10 +6,16 @@
 // L2 delivers to all SMs together.  TWO units per CTA share every activation chunk that arrives (170 KB against 4,096
 // clocks of products per k tile), and the chunk meets the packed weights' conversion once per 128 activation rows.
 //
-// Tensor memory: main sums of unit u at columns 128 u (one accumulator for hi and lo parts, lo first), minima sums at 256
+// Tensor memory: sums of unit u at columns 128 u (one accumulator for hi and lo parts, lo first), minima sums at 256
 // (shared by the units in turn), A stages at 384 + 64 u: 128 inputs of Q4_K's one plane, 64 inputs of the others' two.  The
 // units alternate stage by stage, so a unit's conversion hides under the other unit's products, and so does the fold of
-// its sums once per k tile.  The F32 sums of a work item (2 x 128 x 128) live in the registers of sixteen warps.
+// its sums: once per 128 inputs of the K-quants, once per k tile of Q8_0.  (An addition in tensor memory cuts at the sum's
+// last bit, see gemm_ta.cu.  With one sum per k tile, whose second half's lo parts met a large sum already, the K-quants were
+// 1.5 times as far from the exact results as the kernel of gemm_tc.cu: 1.1e-6 of a row's results against 7.2e-7 for Q4_K,
+// 6.7e-7 against 4.6e-7 for Q6_K; now 3.7e-7 and 3.2e-7.  The additional reads of tensor memory beside the products take
+// 2.2 ms and 2.7 ms of 87 ms of an 8B chunk of 2,048 rows; a third set of sums in turn for Q6_K, or reads of 16 columns at
+// a time, changed nothing.  Q8_0's one sum per tile, 8.4e-7, replaced one over all inputs.)  The F32 sums of a work item
+// (2 x 128 x 128) live in the registers of sixteen warps.
 // Roles of the 28 warps: 0..15 fold and store (one row of each unit and 32 columns per thread), 16..23 convert (two row
 // tiles, half of a stage), 24 / 26 copy weights / activations, 25 issues MMAs.  Every wait is bounded.
 #include <cuda_fp16.h>
@@ -36,22 +42,35 @@ constexpr int kFoldRegs = 88, kConvertRegs = 56, kOtherRegs = 40;
 constexpr uint32_t kSpinLimit = 1u << 22;
 constexpr int kWStages = 4;
 constexpr int kSmemMost = 232448;
+constexpr int kBarBytes = 208;
 
-__device__ __forceinline__ float2 lds64f(uint32_t addr) {
-    float2 v;
-    asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
+__device__ __forceinline__ float4 lds128f(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
     return v;
 }
 
-// acc += sx (f x) over eight columns
-__device__ __forceinline__ void fold8(float* acc, const float (&x)[8], float f, uint32_t sx_at) {
-#pragma unroll
-    for (int i = 0; i < 8; i += 2) {
-        const float2 v = __fmul2_rn(make_float2(x[i], x[i + 1]), make_float2(f, f));
-        const float2 r = __ffma2_rn(lds64f(sx_at + i * 4), v, make_float2(acc[i], acc[i + 1]));
-        acc[i] = r.x; acc[i + 1] = r.y;
-    }
+// acc += sx (f x) over four columns, or sx (f x - g z)
+__device__ __forceinline__ void fold_pair(float* acc, float sx0, float sx1, float2 v) {
+    const float2 r = __ffma2_rn(make_float2(sx0, sx1), v, make_float2(acc[0], acc[1]));
+    acc[0] = r.x; acc[1] = r.y;
 }
+__device__ __forceinline__ void fold4(float* acc, const float* x, float f, uint32_t sx_at) {
+    const float4 s = lds128f(sx_at);
+    const float2 ff = make_float2(f, f);
+    fold_pair(acc, s.x, s.y, __fmul2_rn(make_float2(x[0], x[1]), ff));
+    fold_pair(acc + 2, s.z, s.w, __fmul2_rn(make_float2(x[2], x[3]), ff));
+}
+__device__ __forceinline__ void fold4(float* acc, const float* x, const float* z, float f, float g, uint32_t sx_at) {
+    const float4 s = lds128f(sx_at);
+    const float2 ff = make_float2(f, f), gg = make_float2(-g, -g);
+    fold_pair(acc, s.x, s.y, __ffma2_rn(make_float2(z[0], z[1]), gg, __fmul2_rn(make_float2(x[0], x[1]), ff)));
+    fold_pair(acc + 2, s.z, s.w, __ffma2_rn(make_float2(z[2], z[3]), gg, __fmul2_rn(make_float2(x[2], x[3]), ff)));
+}
+
+// A stages whose products one sum holds: 128 inputs of the K-quants, a whole k tile of Q8_0.
+template <int TYPE>
+__device__ __forceinline__ int stages_per_sum(int type) { return type == kQ4_K ? 1 : TYPE == kKQuants || type == kQ6_K ? 2 : 4; }
 
 template <int TYPE>
 __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, const StepSplit split, const int w_bytes, const int nw) {
@@ -59,9 +78,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const uint32_t spin_limit = a.spin_limit ? a.spin_limit : kSpinLimit;
     const uint32_t b_ring = smem_u32(smem), tails = b_ring + 2 * kChunkBytes, a2_buf = tails + 2 * kTailBytes, scales = a2_buf + 2 * kA2Bytes,
-                   inv_at = scales + 4 * kUnitRows * 4, tmem_slot = inv_at + kCols * 4, bars = tmem_slot + 16, w_ring = (bars + 200 + 127) & ~127u;
+                   inv_at = scales + 4 * kUnitRows * 4, tmem_slot = inv_at + kCols * 4, bars = tmem_slot + 16, w_ring = (bars + kBarBytes + 127) & ~127u;
     const uint32_t w_full = bars, w_empty = bars + 32, b_full = bars + 64, b_empty = bars + 80, a_full = bars + 96, a_free = bars + 112,
-                   d_full = bars + 128, d_free = bars + 144, t_full = bars + 160, t_empty = bars + 176, min_full = bars + 192, min_free = tmem_slot + 8;
+                   d_full = bars + 128, d_free = bars + 152, t_full = bars + 176, t_empty = bars + 192;
     const int k_tiles = split.k_tiles, groups = split.groups, runs = split.runs((int)blockIdx.x);   // item = pair of units * groups + group
 
     if (threadIdx.x == 0) {
@@ -69,11 +88,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
         for (int i = 0; i < 2; ++i) {
             mbar_init(b_full + 8 * i, 1); mbar_init(b_empty + 8 * i, 1);
             mbar_init(a_full + 8 * i, kConvertWarps); mbar_init(a_free + 8 * i, 1);
-            mbar_init(d_full + 8 * i, 1); mbar_init(d_free + 8 * i, kFoldWarps);
             mbar_init(t_full + 8 * i, 1); mbar_init(t_empty + 8 * i, kFoldWarps);
         }
-        mbar_init(min_free, kFoldWarps);
-        mbar_init(min_full, 1);
+        for (int i = 0; i < 3; ++i) { mbar_init(d_full + 8 * i, 1); mbar_init(d_free + 8 * i, kFoldWarps); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kMmaWarp) {
@@ -140,46 +157,48 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
             constexpr uint32_t kBLbo = 2 * kCols * 16, kStep = 2 * kBLbo >> 4, kLo = kCols * 16 >> 4;
             constexpr uint32_t idesc = umma_idesc(kCols);
             const uint32_t b_desc0 = umma_desc(b_ring, kBLbo), sum_desc0 = umma_desc(tails, kCols * 16), a2_desc0 = umma_desc(a2_buf, kA2Lbo);
-            uint32_t n = 0, uses = 0, mins = 0;   // k tiles, A stages per unit, minima products
+            uint32_t n = 0, uses = 0;   // k tiles, A stages per unit
+            uint32_t taken = 0;         // bit i: sums i (a unit's, or 2: the minima's) have been taken an odd number of times
+            auto take = [&](uint32_t i) {
+                if (alive) alive = mbar_wait(d_free + 8 * i, ((taken >> i) & 1u) ^ 1u, a.error_flag, 105, spin_limit);
+                taken ^= 1u << i;
+            };
             for (int r = 0; r < runs; ++r) {
                 const StepRun run = split.run((int)blockIdx.x, r);
                 // broadcast, so that the loop below stays on uniform registers
-                const bool q4k = (TYPE >= 0 ? TYPE : __shfl_sync(0xffffffffu, a.seg[unit_at(a, run.item / groups, 2 * kUnitTiles).seg].type, 0)) == kQ4_K;
-                const int stages = q4k ? 2 : 4, stop = __shfl_sync(0xffffffffu, (int)n + run.end - run.begin, 0);
+                const int type = TYPE >= 0 ? TYPE : __shfl_sync(0xffffffffu, a.seg[unit_at(a, run.item / groups, 2 * kUnitTiles).seg].type, 0);
+                const bool q4k = type == kQ4_K;
+                const int stages = q4k ? 2 : 4, per_sum = stages_per_sum<TYPE>(type), stop = __shfl_sync(0xffffffffu, (int)n + run.end - run.begin, 0);
                 for (; (int)n < stop; ++n) {
 #pragma unroll 1
                     for (int h = 0; h < stages; ++h, ++uses) {
                         const int chunk = q4k ? h : h >> 1;
-                        const bool last = h == stages - 1;
+                        const bool opens = (h & (per_sum - 1)) == 0, closes = (h & (per_sum - 1)) == per_sum - 1;   // a sum
                         if (q4k || !(h & 1)) { if (alive) alive = mbar_wait(b_full + 8 * chunk, n & 1u, a.error_flag, 104, spin_limit); }
                         const uint32_t b_desc = b_desc0 + chunk * (kChunkBytes >> 4) + (q4k ? 0u : (h & 1) * 4 * kStep);
 #pragma unroll
                         for (int u = 0; u < 2; ++u) {
                             const uint32_t d_main = tmem + 128 * u, a_at = tmem + 384 + 64 * u;
-                            if (h == 0 && n >= 1 && alive) alive = mbar_wait(d_free + 8 * u, (n - 1u) & 1u, a.error_flag, 105, spin_limit);
+                            if (opens) take(u);
                             if (alive) alive = mbar_wait(a_full + 8 * u, uses & 1u, a.error_flag, 106, spin_limit);
                             tc_fence_after();
                             if (q4k) {
 #pragma unroll
-                                for (int i = 0; i < 8; ++i) umma_ts_if(leader, d_main, a_at + 8 * i, b_desc + kLo + i * kStep, idesc, (uint32_t)(h | i));
+                                for (int i = 0; i < 8; ++i) umma_ts_if(leader, d_main, a_at + 8 * i, b_desc + kLo + i * kStep, idesc, (uint32_t)(i != 0));
 #pragma unroll
                                 for (int i = 0; i < 8; ++i) umma_ts_if(leader, d_main, a_at + 8 * i, b_desc + i * kStep, idesc, 1u);
                                 if (h == u) {
-                                    // minima x group sums: unit 0's with its first stage, so that they are folded by the time
-                                    // unit 1's, with its last stage, need the columns
+                                    // minima x group sums: unit 0's with its first stage, unit 1's with its last, so that the
+                                    // other unit's have been folded by the time the stage's products are through
                                     if (u == 0 && alive) alive = mbar_wait(t_full + 8 * (n & 1u), (n >> 1) & 1u, a.error_flag, 107, spin_limit);
-                                    if (mins >= 1 && alive) alive = mbar_wait(min_free, (mins - 1u) & 1u, a.error_flag, 108, spin_limit);
+                                    take(2);
                                     tc_fence_after();
-                                    if (leader) {
-                                        umma_ss(tmem + 256, a2_desc0 + u * (kA2Bytes >> 4), sum_desc0 + (n & 1u) * (kTailBytes >> 4), idesc, 0u);
-                                        umma_commit(min_full);
-                                    }
-                                    ++mins;
+                                    if (leader) umma_ss(tmem + 256, a2_desc0 + u * (kA2Bytes >> 4), sum_desc0 + (n & 1u) * (kTailBytes >> 4), idesc, 0u);
                                 }
                             } else {
-                                // position i of the stage holds step 2 (i & 1) + (i >> 1) of its 64 inputs; p2 x lo is below F32's resolution
+                                // position i of the stage holds step 2 (i & 1) + (i >> 1) of its 64 inputs; p2 x lo left out as in gemm_ta.cu
 #pragma unroll
-                                for (int i = 0; i < 4; ++i) umma_ts_if(leader, d_main, a_at + 8 * i, b_desc + kLo + (2 * (i & 1) + (i >> 1)) * kStep, idesc, (uint32_t)(h | i));
+                                for (int i = 0; i < 4; ++i) umma_ts_if(leader, d_main, a_at + 8 * i, b_desc + kLo + (2 * (i & 1) + (i >> 1)) * kStep, idesc, (uint32_t)(!opens || i != 0));
 #pragma unroll
                                 for (int i = 0; i < 4; ++i) umma_ts_if(leader, d_main, a_at + 32 + 8 * i, b_desc + (2 * (i & 1) + (i >> 1)) * kStep, idesc, 1u);
 #pragma unroll
@@ -187,7 +206,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
                             }
                             if (leader) {
                                 umma_commit(a_free + 8 * u);
-                                if (last) umma_commit(d_full + 8 * u);
+                                if (closes) umma_commit(d_full + 8 * u);
                             }
                         }
                         if (leader && (q4k || (h & 1))) umma_commit(b_empty + 8 * chunk);
@@ -246,14 +265,15 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
         const int quadrant = warp & 3, col0 = kMine * (warp >> 2), row = quadrant * 32 + lane;
         bool alive = true;
         int inv_group = -1;
-        uint32_t n = 0, mins = 0;
+        uint32_t n = 0, folds = 0;   // k tiles, sums per unit
         float* inv = reinterpret_cast<float*>(smem + (inv_at - b_ring));
         for (int r = 0; r < runs; ++r) {
             const StepRun run = split.run((int)blockIdx.x, r);
             const int group = run.item % groups;
             const UnitAt at = unit_at(a, run.item / groups, 2 * kUnitTiles);
             const GemvSegment& seg = a.seg[at.seg];
-            const bool q4k = type_of<TYPE>(seg) == kQ4_K;
+            const int type = type_of<TYPE>(seg), sums = (type == kQ4_K ? 2 : 4) / stages_per_sum<TYPE>(type);
+            const bool q4k = type == kQ4_K;
             float acc[2][kMine];
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
@@ -263,38 +283,38 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
             for (int kb = run.begin; kb < run.end; ++kb, ++n) {
                 const uint32_t p = n & 1u, sx_at = tails + p * kTailBytes + kSumBytes + col0 * 4;
                 if (alive) alive = mbar_wait(t_full + 8 * p, (n >> 1) & 1u, a.error_flag, 111, spin_limit);
+#pragma unroll 1
+                for (int i = 0; i < sums; ++i, ++folds) {
 #pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    if (q4k) {
-                        if (alive) alive = mbar_wait(min_full, mins & 1u, a.error_flag, 113, spin_limit);
-                        ++mins;
-                    } else {
-                        if (alive) alive = mbar_wait(d_full + 8 * u, n & 1u, a.error_flag, 112, spin_limit);
-                    }
-                    tc_fence_after();
-                    const float2 d = __half22float2(as_half2(lds32(scales + (2 * p + u) * (kUnitRows * 4) + row * 4)));
-                    const uint32_t t_at = tmem + ((uint32_t)(quadrant * 32) << 16) + col0;
-                    if (q4k) {
-#pragma unroll
-                        for (int c = 0; c < kMine; c += 8) {
-                            float x[8];
-                            tmem_ld8(t_at + 256 + c, x);
-                            tmem_wait_ld();
-                            tmem_tie(x);
-                            if (c == kMine - 8) { tc_fence_before(); __syncwarp(); if (lane == 0) mbar_arrive(min_free); }
-                            fold8(&acc[u][c], x, -d.y, sx_at + c * 4);
-                        }
-                        if (alive) alive = mbar_wait(d_full + 8 * u, n & 1u, a.error_flag, 112, spin_limit);
+                    for (int u = 0; u < 2; ++u) {
+                        if (alive) alive = mbar_wait(d_full + 8 * u, folds & 1u, a.error_flag, 112, spin_limit);
                         tc_fence_after();
-                    }
+                        const float2 d = __half22float2(as_half2(lds32(scales + (2 * p + u) * (kUnitRows * 4) + row * 4)));
+                        const uint32_t t_at = tmem + ((uint32_t)(quadrant * 32) << 16) + col0;
+                        if (q4k && i == u) {   // the minima came with these products
 #pragma unroll
-                    for (int c = 0; c < kMine; c += 8) {
-                        float x[8];
-                        tmem_ld8(t_at + 128 * u + c, x);
-                        tmem_wait_ld();
-                        tmem_tie(x);
-                        if (c == kMine - 8) { tc_fence_before(); __syncwarp(); if (lane == 0) mbar_arrive(d_free + 8 * u); }
-                        fold8(&acc[u][c], x, d.x, sx_at + c * 4);
+                            for (int c = 0; c < kMine; c += 4) {
+                                float x[4], z[4];
+                                tmem_ld4(t_at + 128 * u + c, x);
+                                tmem_ld4(t_at + 256 + c, z);
+                                tmem_wait_ld();
+                                tmem_tie(x);
+                                tmem_tie(z);
+                                if (c == kMine - 4) { tc_fence_before(); __syncwarp(); if (lane == 0) { mbar_arrive(d_free + 8 * u); mbar_arrive(d_free + 16); } }
+                                fold4(&acc[u][c], x, z, d.x, d.y, sx_at + c * 4);
+                            }
+                        } else {
+#pragma unroll
+                            for (int c = 0; c < kMine; c += 8) {
+                                float x[8];
+                                tmem_ld8(t_at + 128 * u + c, x);
+                                tmem_wait_ld();
+                                tmem_tie(x);
+                                if (c == kMine - 8) { tc_fence_before(); __syncwarp(); if (lane == 0) mbar_arrive(d_free + 8 * u); }
+                                fold4(&acc[u][c], x, d.x, sx_at + c * 4);
+                                fold4(&acc[u][c + 4], x + 4, d.x, sx_at + c * 4 + 16);
+                            }
+                        }
                     }
                 }
                 __syncwarp();
@@ -357,7 +377,7 @@ cudaError_t launch_typed(cudaStream_t stream, const StepGemm& a, int w_bytes, bo
         configured[dev] = true;
     }
     w_bytes = (w_bytes + 127) & ~127;
-    const int fixed = 2 * kChunkBytes + 2 * kTailBytes + 2 * kA2Bytes + 4 * kUnitRows * 4 + kCols * 4 + 16 + 200 + 127;
+    const int fixed = 2 * kChunkBytes + 2 * kTailBytes + 2 * kA2Bytes + 4 * kUnitRows * 4 + kCols * 4 + 16 + kBarBytes + 127;
     const int nw = std::min(kWStages, (kSmemMost - fixed) / w_bytes);
     if (nw < 2) return cudaErrorInvalidValue;
     const StepSplit split = step_split(a, a.partial == nullptr);
