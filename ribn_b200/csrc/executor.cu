@@ -1525,22 +1525,18 @@ int ribn_b200_submit(ribn_b200_executor* ex, const ribn_b200_batch_item* items, 
     // launches per step, whose launch gaps a graph closes) once the same shape has come up three times, and while
     // the executor holds fewer than kMaxStepGraphs graphs.
     constexpr size_t kMaxStepGraphs = 192;
-    bool graphable = !(ex->cfg.flags & RIBN_B200_FLAG_NO_GRAPH) && packed_family_applies(ex) &&
-                     plan.n_rows == plan.n_tokens && plan.n_prompt_tokens == 0;
-    if (graphable && !decode_family_applies(ex, plan)) {
-        const int bucket = (plan.max_keys + 511) / 512;
-        const uint64_t key = (uint64_t)plan.n_tokens | ((uint64_t)plan.n_sample << 16) | ((uint64_t)bucket << 32);
-        if (ex->graphs.find(key) == ex->graphs.end()) {
-            graphable = ++ex->graph_seen[key] >= 3 && ex->graphs.size() < kMaxStepGraphs;
-        }
+    const bool decode_only = packed_family_applies(ex) && plan.n_rows == plan.n_tokens && plan.n_prompt_tokens == 0;
+    const int bucket = (plan.max_keys + 511) / 512;
+    const uint64_t key = (uint64_t)plan.n_tokens | ((uint64_t)plan.n_sample << 16) | ((uint64_t)bucket << 32);
+    // The attention cuts its spans by a bound of the longest context, and where they are cut shows in a result's last
+    // bits: a graph serves 512 consecutive positions, and a step that is launched directly takes the same bound.
+    if (decode_only) plan.max_keys = std::min(bucket * 512, ex->cfg.context_tokens);
+    bool graphable = decode_only && !(ex->cfg.flags & RIBN_B200_FLAG_NO_GRAPH);
+    if (graphable && !decode_family_applies(ex, plan) && ex->graphs.find(key) == ex->graphs.end()) {
+        graphable = ++ex->graph_seen[key] >= 3 && ex->graphs.size() < kMaxStepGraphs;
     }
     CU_TRY(ex, cudaEventRecord(ex->ev_start, ex->stream));
     if (graphable) {
-        // Decode-only steps replay a captured graph.  The attention grid is sized by a bucket of the
-        // longest context (results do not depend on it), so a graph serves 512 consecutive positions.
-        const int bucket = (plan.max_keys + 511) / 512;
-        plan.max_keys = std::min(bucket * 512, ex->cfg.context_tokens);
-        const uint64_t key = (uint64_t)plan.n_tokens | ((uint64_t)plan.n_sample << 16) | ((uint64_t)bucket << 32);
         auto found = ex->graphs.find(key);
         if (found == ex->graphs.end()) {
             cudaGraph_t graph = nullptr;

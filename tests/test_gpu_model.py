@@ -404,6 +404,40 @@ def test_batched_decode_graph_replay_changes_no_bit(model):
             assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
 
 
+def test_batched_decode_bits_do_not_depend_on_the_graph_above_512_keys(model):
+    """A batch's spans are cut by the same bound of its longest context (here 520 to 524 keys, where 576 and 1,024 keys
+    would be cut differently) whether the step is launched directly or replayed: the logits of a request are those of
+    its repetition, whose first step finds the captured graph, and those of an executor that never captures."""
+    import ribn_b200
+    from ribn_b200 import BatchItem, StepKind
+    tensors, _ = model
+    lengths = (520, 300, 70)
+    rng = np.random.default_rng(6)
+    prompts = [rng.integers(0, MID["vocab"], size=n, dtype=np.uint32) for n in lengths]
+    runs = []
+    for flags in (0, ribn_b200.FLAG_NO_GRAPH):
+        ex = build(MID, tensors, flags=flags, context_tokens=2048, max_sequences=3, max_batch_tokens=64)
+        for _ in range(2):
+            steps = []
+            for s, prompt in enumerate(prompts):
+                assert ex.admit(s + 1, s + 1, prompt, 8).ready
+                ex.debug_set_context(s + 1, len(prompt), 5 + s, seed=40 + s)
+            for step in range(4):
+                items = [BatchItem(s + 1, StepKind.DECODE, n + step, 1, 1) for s, n in enumerate(lengths)]
+                ex.prepare(items)
+                done = ex.wait(ex.submit(items))
+                steps.append(([d.tokens[0] for d in done], [ex.copy_logits(r).copy() for r in range(3)]))
+            runs.append(steps)
+            for s in range(3):
+                ex.release(s + 1)
+        ex.close()
+    for other in runs[1:]:
+        for (tok_a, log_a), (tok_b, log_b) in zip(runs[0], other):
+            assert tok_a == tok_b
+            for a, b in zip(log_a, log_b):
+                assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+
+
 def test_release_of_prepared_and_in_flight_sequences(model):
     """release() refuses a sequence named by the outstanding preparation ("cannot release prepared Qwen
     state", crates/qwen/src/execution.rs:416-426) and parks one the pending submission still reads until
