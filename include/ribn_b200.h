@@ -463,6 +463,14 @@ RIBN_B200_API int ribn_b200_attention_noalloc(int32_t device, void* stream, cons
 RIBN_B200_API int ribn_b200_debug_repack(int32_t ggml_type, const void* raw, int64_t rows, int64_t cols,
                                          void* out, size_t capacity, size_t* byte_count);
 
+/* How the GEMM of one matrix [rows][cols] is dealt out in a step of `members` rows, without any device work
+ * (`form`: 0 fragment order, 1 column, 2 wide; 148 SMs where there is no device).  A run is eight numbers: worker, item, first
+ * k tile, end, its part of the item's sums, and, as the kernel that adds the parts computes them, the item's parts, its
+ * first worker and the rows of a unit.  Writes up to `capacity` runs, their count, and the floats of scratch that the first
+ * and the further parts take. */
+RIBN_B200_API int ribn_b200_debug_step_deal(int32_t form, int64_t rows, int64_t cols, int32_t members, int32_t* runs, size_t capacity,
+                                            size_t* count, size_t* partial_floats, size_t* further_floats);
+
 /* Library build identification (git-free; the CUDA arch it was built for). */
 RIBN_B200_API const char* ribn_b200_build_info(void);
 

@@ -478,7 +478,8 @@ StepGemm step_base(ribn_b200_executor* ex, int k, int members, bool normed) {
     a.ss = normed ? ex->op_step.ss : nullptr;
     a.eps = ex->cfg.rms_eps;
     a.epilogue = kStore;
-    a.partial = ex->tc_partial;
+    a.partial = ex->gate;   // no projection of a step has its result there
+    a.further = ex->step_further;
     a.error_flag = ex->d_error;
     return a;
 }
@@ -1116,8 +1117,9 @@ int ribn_b200_finalize(ribn_b200_executor* ex) {
     CU_TRY(ex, dev_alloc(ex, &ex->k, T * KD));
     CU_TRY(ex, dev_alloc(ex, &ex->v, T * KD));
     CU_TRY(ex, dev_alloc(ex, &ex->attn, T * QD));
-    CU_TRY(ex, dev_alloc(ex, &ex->gate, T * c.ffn));
-    CU_TRY(ex, dev_alloc(ex, &ex->up, T * c.ffn));
+    // gate and up side by side; the step GEMMs leave their sums there
+    CU_TRY(ex, dev_alloc(ex, &ex->gate, T * std::max({(size_t)2 * c.ffn, QD + 2 * KD, (size_t)c.hidden})));
+    ex->up = ex->gate + T * c.ffn;
     if (ex->tp > 1) CU_TRY(ex, dev_alloc(ex, &ex->proj, T * c.hidden));
     CU_TRY(ex, dev_alloc(ex, &ex->head_in, S * c.hidden));
     CU_TRY(ex, dev_alloc(ex, &ex->logits, S * c.vocab));
@@ -1151,15 +1153,14 @@ int ribn_b200_finalize(ribn_b200_executor* ex) {
                 CU_TRY(ex, dev_alloc(ex, &ex->op_step.blocks, step_bytes));
                 CU_TRY(ex, dev_alloc(ex, &ex->op_step.ss, (size_t)most * (size_t)(kmax / kTileCols)));
                 if (step_gemms(ex)) {
-                    // partial sums of every row count a step can have (their number of parts changes with the row groups)
-                    if (packed_family_applies(ex)) {
-                        for (int m = 1; m <= (int)T; ++m) {
-                            if (m > 64 && m % 8 != 0 && m != (int)T) continue;
-                            for (const StepGemm& g : {step_qkv(ex, 0, m), step_o(ex, 0, m), step_gate_up(ex, 0, m), step_down(ex, 0, m)}) {
-                                ex->tc_partial_floats = std::max(ex->tc_partial_floats, step_partial_floats(g));
-                            }
+                    // of every row count a step can have (how its work is dealt out changes with the row groups)
+                    size_t further = 0;
+                    for (int m = 1; packed_family_applies(ex) && m <= (int)T; ++m) {
+                        for (const StepGemm& g : {step_qkv(ex, 0, m), step_o(ex, 0, m), step_gate_up(ex, 0, m), step_down(ex, 0, m)}) {
+                            further = std::max(further, step_further_floats(g));
                         }
                     }
+                    if (further > 0) CU_TRY(ex, dev_alloc(ex, &ex->step_further, further));
                 } else {
                     // room for every 64-row group of the largest step (one conversion per projection), or one 128-row operand
                     const size_t tc_groups = ((size_t)c.max_batch_tokens + 63) / 64;
@@ -1173,8 +1174,8 @@ int ribn_b200_finalize(ribn_b200_executor* ex) {
                     CU_TRY(ex, dev_alloc(ex, &ex->op_batch.digit_inv, kGemmMaxMembers));
                     // room for four K slices of the widest fused projection at 64 rows
                     ex->tc_partial_floats = (size_t)4 * 64 * (size_t)std::max(std::max(2 * c.ffn, c.hidden), (c.q_heads + 2 * c.kv_heads) * c.head_dim);
+                    CU_TRY(ex, dev_alloc(ex, &ex->tc_partial, ex->tc_partial_floats));
                 }
-                CU_TRY(ex, dev_alloc(ex, &ex->tc_partial, ex->tc_partial_floats));
             }
         }
         CU_TRY(ex, dev_alloc(ex, &ex->d_error, 1));

@@ -122,7 +122,8 @@ struct ribn_b200_executor {
     ribn::BatchOperand op_batch;  // batch form, refilled before every batched projection
     ribn::TcOperand op_tc;        // tensor-memory form (the same, for the tcgen05 kernel)
     ribn::StepOperand op_step;    // operand of the step GEMMs (batches of a few rows; any batch of a Q8_0 model)
-    float* tc_partial = nullptr;  // split-K sums of the batched kernels
+    float* step_further = nullptr;  // the step GEMMs' further partial sums (their first ones lie in `gate`)
+    float* tc_partial = nullptr;  // split-K sums of the batched kernels (tensor parallelism)
     size_t tc_partial_floats = 0;
     // Captured decode steps, keyed by (tokens, sampling rows, attention span bucket).
     struct StepGraph { cudaGraphExec_t exec = nullptr; int launches = 0; };

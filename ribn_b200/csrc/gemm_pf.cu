@@ -334,15 +334,15 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
                 asm volatile("bar.sync 1, 512;" ::: "memory");
             }
             const int live = min(kMine, a.members - group * kCols - col0);
+            const StepSums to = step_sums(a, split, (int)blockIdx.x, run.part, group, col0, at.seg, at.rt0 * kTileRows + row);
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
                 const int n_index = (at.rt0 + kUnitTiles * u) * kTileRows + row;
                 if (n_index >= seg.n) continue;
                 if (a.partial != nullptr) {
-                    float* part = a.partial + ((size_t)run.part * a.members + group * kCols + col0) * a.total_n + a.n_offset[at.seg] + n_index;
 #pragma unroll
                     for (int i = 0; i < kMine; ++i) {
-                        if (i < live) part[(size_t)i * a.total_n] = acc[u][i];
+                        if (i < live) to.at[i * to.stride + kUnitRows * u] = acc[u][i];
                     }
                 } else {
                     float* y = seg.y + (size_t)(group * kCols + col0) * seg.n + n_index;

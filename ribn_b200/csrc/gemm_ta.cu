@@ -347,7 +347,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ta_kernel(const StepGemm a, 
             }
             const int n_index = at.rt0 * kTileRows + row;
             if (n_index < seg.n) {
-                float* part = a.partial + (size_t)((int)blockIdx.x - split.first_worker(item)) * a.members * a.total_n + a.n_offset[at.seg] + n_index;
+                StepSums to{};
+                if (a.partial != nullptr) to = step_sums(a, split, (int)blockIdx.x, split.whole ? 0 : (int)blockIdx.x - split.first_worker(item), group, mine, at.seg, n_index);
 #pragma unroll
                 for (int j = 0; j < kChunks; ++j) {
 #pragma unroll
@@ -355,7 +356,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ta_kernel(const StepGemm a, 
                         const int m = 16 * j + mine + i, member = group * MP + m;
                         if (m >= MP || member >= a.members) continue;
                         if (a.partial != nullptr) {
-                            part[(size_t)member * a.total_n] = acc[j][i];
+                            to.at[(16 * j + i) * to.stride] = acc[j][i];
                         } else {
                             float* y = seg.y + (size_t)member * seg.n + n_index;
                             *y = a.epilogue == kResidual ? *y + acc[j][i] * inv[m] : acc[j][i] * inv[m];

@@ -268,7 +268,8 @@ struct StepGemm {
     const float* ss;               // optional: multiply the results by the RMSNorm factor of these sums of squares
     float eps;
     int epilogue;                  // kStore or kResidual (when partial is null)
-    float* partial;                // not null: leave partial sums [part][member][rows of all segments] for launch_step_finish
+    float* partial;                // not null: leave partial sums for launch_step_finish, items' first parts here (StepSplit)
+    float* further;                // their further parts, step_further_floats
     int* error_flag;
     uint32_t spin_limit;
     int n_offset[3], total_n;      // filled in by the launcher
@@ -310,13 +311,26 @@ struct StepSplit {
         const int lo = b > i * k_tiles ? b - i * k_tiles : 0, hi = e < (i + 1) * k_tiles ? e - i * k_tiles : k_tiles;
         return StepRun{item, lo, hi, whole ? 0 : w - first_worker(item)};
     }
+    // An item's first part lies in the launch's matrix of sums [member][rows of all segments].  A further part begins in the
+    // middle of the item, which only a worker's first run can do: it lies in the slot of its worker, [member of the
+    // group][row of the unit], so an item's further parts are neighbours.
+    __host__ __device__ int slot_floats() const { return group_members << unit_shift; }
 };
+// Where a run's sums of row n of segment `seg` lie, from member `m` of the group on: first value and distance of the members.
+struct StepSums { float* at; size_t stride; };
+__device__ __forceinline__ StepSums step_sums(const StepGemm& a, const StepSplit& s, int worker, int part, int group, int m, int seg, int n) {
+    if (part == 0) return StepSums{a.partial + (size_t)(group * s.group_members + m) * a.total_n + a.n_offset[seg] + n, (size_t)a.total_n};
+    const int unit_rows = 1 << s.unit_shift;
+    return StepSums{a.further + (size_t)worker * s.slot_floats() + m * unit_rows + (n & (unit_rows - 1)), (size_t)unit_rows};
+}
 StepSplit step_split(const StepGemm& a, bool whole_items);
 // A packed matrix as a rank-4 tensor map (128 bytes, to be copied to device memory, 64-byte aligned): one copy then
 // brings a unit's eight row tiles at one k tile; row tiles past the end read zeros.
 constexpr size_t kTileMapBytes = 128;
 cudaError_t make_tile_map(int type, const unsigned char* packed, long long rows, long long cols, void* host_map);
-size_t step_partial_floats(const StepGemm& a);   // scratch a split launch of these arguments needs
+// Scratch that a split launch of these arguments needs.
+size_t step_partial_floats(const StepGemm& a);
+size_t step_further_floats(const StepGemm& a);
 cudaError_t launch_step_gemm(cudaStream_t stream, const StepGemm& args, bool programmatic);
 // The kernels, for launch_step_gemm: `w_bytes` is the largest bytes of eight row tiles at one k tile.
 constexpr int kFragTeams = 2;   // independent workers per CTA of the fragment-order kernel
@@ -338,7 +352,7 @@ struct StepFinish {
     StepOperand out;
     // from the launch's StepGemm, filled in by the launcher
     StepSplit split;
-    const float* partial;
+    const float *partial, *further;
     const float* ss;
     float eps;
     int n_segments, total_n;

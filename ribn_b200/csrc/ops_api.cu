@@ -104,6 +104,34 @@ int ribn_b200_debug_repack(int32_t type, const void* raw, int64_t rows, int64_t 
     return RIBN_B200_OK;
 }
 
+int ribn_b200_debug_step_deal(int32_t form, int64_t rows, int64_t cols, int32_t members, int32_t* runs, size_t capacity, size_t* count,
+                              size_t* partial_floats, size_t* further_floats) {
+    if (form < kFragmentForm || form > kWideForm || rows <= 0 || rows > INT32_MAX / 2 || cols <= 0 || cols % kTileCols != 0 || cols > INT32_MAX ||
+        members <= 0 || count == nullptr || partial_floats == nullptr || further_floats == nullptr || (runs == nullptr && capacity > 0)) {
+        return op_fail("step_deal: invalid argument", cudaSuccess);
+    }
+    StepGemm g{};
+    g.form = form;
+    g.n_segments = 1;
+    g.seg[0] = GemvSegment{nullptr, 8, (int)rows, (int)((rows + kTileRows - 1) / kTileRows), nullptr};
+    g.k = (int)cols;
+    g.members = members;
+    const StepSplit s = step_split(g, false);
+    *partial_floats = step_partial_floats(g);
+    *further_floats = step_further_floats(g);
+    *count = 0;
+    for (int w = 0; w < s.workers; ++w) {
+        for (int r = 0; r < s.runs(w); ++r, ++*count) {
+            if (*count >= capacity) continue;
+            const StepRun run = s.run(w, r);
+            const bool dealt = !s.whole && run.item >= s.rounds * s.workers;
+            const int32_t record[8] = {w, run.item, run.begin, run.end, run.part, s.parts(run.item), dealt ? s.first_worker(run.item) : w, 1 << s.unit_shift};
+            memcpy(runs + 8 * *count, record, sizeof(record));
+        }
+    }
+    return RIBN_B200_OK;
+}
+
 int ribn_b200_debug_unpack(int32_t device, int32_t type, const void* packed, int64_t rows, int64_t cols, float* out) {
     if (!packable(type, rows, cols) || packed == nullptr || out == nullptr) return op_fail("invalid argument, or no usable CUDA device", cudaGetLastError());
     Scope s(device);
@@ -345,7 +373,12 @@ int ribn_b200_op_gemv(int32_t device, int32_t type, const void* weights, int64_t
             g.epilogue = kStore;
             g.error_flag = d_err;
             const bool split = (members <= 64 || variant == 8) && rows % 4 == 0;
-            if (split) { g.partial = s.alloc<float>(step_partial_floats(g)); OP_PTR(g.partial); }
+            if (split) {
+                g.partial = s.alloc<float>(step_partial_floats(g));
+                OP_PTR(g.partial);
+                const size_t further = step_further_floats(g);
+                if (further > 0) { g.further = s.alloc<float>(further); OP_PTR(g.further); }
+            }
             OP_PTR(f.out.blocks); OP_PTR(g.seg[0].map);
             OP_TRY(launch_step_finish(s.stream, kFinishRows, nullptr, f, (int)cols, false));
             OP_TRY(launch_step_gemm(s.stream, g, false));

@@ -29,22 +29,28 @@ __device__ __forceinline__ float norm_factor(const float* ss, int tiles, float e
 
 // ---- consumers of partial sums, producers of operands -----------------------------------------------------------
 
-// The parts of outputs n .. n + 3 (inside segment `seg`) of member m: where the first lies, and how many there are.
-struct Parts { const float* at; int count; };
+// The parts of outputs n .. n + 3 (inside segment `seg`) of member m: where the first lies, how many there are, and the slots
+// of the further ones, counted from the first's worker.
+struct Parts { const float* at; int count; const float* slots; };
 __device__ __forceinline__ Parts parts_of(const StepFinish& a, int seg, int m, int n) {
-    const int unit = a.unit0[seg] + (n >> a.split.unit_shift), item = unit * a.split.groups + m / a.split.group_members;
-    return Parts{a.partial + (size_t)m * a.total_n + a.n_offset[seg] + n, a.split.parts(item)};
+    const int unit = a.unit0[seg] + (n >> a.split.unit_shift), group = m / a.split.group_members, item = unit * a.split.groups + group;
+    Parts p{a.partial + (size_t)m * a.total_n + a.n_offset[seg] + n, a.split.parts(item), nullptr};
+    if (p.count > 1) {
+        p.slots = a.further + (size_t)a.split.first_worker(item) * a.split.slot_floats() +
+                  ((m - group * a.split.group_members) << a.split.unit_shift) + (n & ((1 << a.split.unit_shift) - 1));
+    }
+    return p;
 }
 // Their sum in worker order, `s` holding the first, BATCH at a time in flight.  Prefill-sized launches have one or two parts
 // and want threads (two in flight: 40 registers, SwiGLU of 2,048 x 12,288 in 124 us; eight: 199 us), small ones up to a
 // dozen and want the round trips back (eight in flight: 3.5 us against 5.4).
 template <int BATCH>
 __device__ __forceinline__ float4 add_parts(const StepFinish& a, const Parts& p, float4 s) {
-    const size_t stride = (size_t)a.members * a.total_n;
+    const int slot = a.split.slot_floats();
     for (int i = 1; i < p.count; i += BATCH) {
         float4 v[BATCH];
 #pragma unroll
-        for (int j = 0; j < BATCH; ++j) v[j] = i + j < p.count ? *reinterpret_cast<const float4*>(p.at + (i + j) * stride) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int j = 0; j < BATCH; ++j) v[j] = i + j < p.count ? *reinterpret_cast<const float4*>(p.slots + (i + j) * slot) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
         for (int j = 0; j < BATCH; ++j) {
             if (i + j < p.count) { s.x += v[j].x; s.y += v[j].y; s.z += v[j].z; s.w += v[j].w; }
@@ -273,12 +279,14 @@ StepSplit step_split(const StepGemm& a, bool whole_items) {
 }
 
 size_t step_partial_floats(const StepGemm& a) {
-    const StepSplit s = step_split(a, false);
-    int parts = 1;
-    for (int i = 0; i < s.items; ++i) parts = std::max(parts, s.parts(i));
     size_t total_n = 0;
     for (int i = 0; i < a.n_segments; ++i) total_n += a.seg[i].n;
-    return (size_t)parts * a.members * total_n;
+    return (size_t)a.members * total_n;
+}
+
+size_t step_further_floats(const StepGemm& a) {
+    const StepSplit s = step_split(a, false);
+    return s.whole ? 0 : (size_t)s.spread * s.slot_floats();
 }
 
 cudaError_t launch_step_gemm(cudaStream_t stream, const StepGemm& args, bool programmatic) {
@@ -304,6 +312,7 @@ cudaError_t launch_step_finish(cudaStream_t stream, int mode, const StepGemm* ge
     if (gemm != nullptr) {
         a.split = step_split(*gemm, false);
         a.partial = gemm->partial;
+        a.further = gemm->further;
         a.members = gemm->members;
         a.n_segments = gemm->n_segments;
         a.ss = gemm->ss;

@@ -206,3 +206,14 @@ def repack(ggml_type: int, raw, rows: int, cols: int) -> np.ndarray:
     out = np.empty(need.value, dtype=np.uint8)
     _check(lib().ribn_b200_debug_repack(ggml_type, _p(raw), rows, cols, _p(out), out.size, C.byref(need)), "repack")
     return out
+
+
+def step_deal(form: int, rows: int, cols: int, members: int):
+    """How a step's GEMM is dealt out (ribn_b200_debug_step_deal; no device needed): runs [n][8], and the floats of its
+    first and further partial sums."""
+    count, partial, further = C.c_size_t(0), C.c_size_t(0), C.c_size_t(0)
+    args = (form, rows, cols, members)
+    _check(lib().ribn_b200_debug_step_deal(*args, None, 0, C.byref(count), C.byref(partial), C.byref(further)), "step_deal")
+    runs = np.empty((count.value, 8), dtype=np.int32)
+    _check(lib().ribn_b200_debug_step_deal(*args, _p(runs), runs.shape[0], C.byref(count), C.byref(partial), C.byref(further)), "step_deal")
+    return runs, partial.value, further.value

@@ -635,3 +635,21 @@ def test_host_side_fault_injection_faults_the_executor(model, kind):
     with pytest.raises(ExecutionError, match="faulted"):
         ex.admit(2, 2, [1], 1)
     ex.close()
+
+
+def test_a_larger_batch_limit_takes_memory_for_its_rows_only(built_library):
+    """One layer of the 8B model's shapes, where the partial sums of gate | up were once sized by the parts of its few
+    left-over items: 64 rows more in the limit (17 row groups in place of 16) take what 64 rows take, 0.4 MB each."""
+    import torch
+    import ribn_b200
+    cfg = dict(ribn_b200.QWEN3_8B, layers=1, vocab=1024)
+    used = []
+    for limit in (2048, 2112):
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        ex = ribn_b200.QwenB200(cfg, context_tokens=4096, max_sequences=2, max_batch_tokens=limit)
+        ex.init_synthetic(1, ribn_b200.SCHEME_Q4_K_M)
+        ex.finalize()
+        used.append(before - torch.cuda.mem_get_info()[0])
+        ex.close()
+    assert used[1] - used[0] < 64 << 20, used

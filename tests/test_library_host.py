@@ -218,6 +218,33 @@ def test_repack_feeds_the_mma_fragment_the_raw_integers(built_library, kind, til
                                               blocks[row, kb * 8 + b, 0:2])
 
 
+@pytest.mark.parametrize("form,group,members", [(0, 8, 3), (0, 16, 16), (0, 32, 97), (1, 24, 24), (1, 64, 64), (2, 128, 65), (2, 128, 777), (2, 128, 2112),
+                                                (2, 128, 8192)])
+@pytest.mark.parametrize("rows,cols", [(40, 256), (1024, 3072), (4096, 12288), (6144, 4096), (24576, 4096), (151936, 4096)])
+def test_step_work_is_dealt_out_once_and_further_parts_have_their_own_slots(built_library, form, group, members, rows, cols):
+    """Every (item, k tile) has one worker; an item's parts are consecutive workers, counted as the kernel that adds them
+    counts them; a worker has at most one further part, so that slot `worker` of the scratch is its own; and that scratch
+    is a slot per worker, whatever the rows of the step."""
+    from ribn_b200 import ops
+    runs, partial, further = ops.step_deal(form, rows, cols, members)
+    worker, item, begin, end, part, parts, first, unit_rows = runs.T.astype(np.int64)
+    groups, k_tiles = -(-members // group), cols // 256
+    items = -(-rows // int(unit_rows[0])) * groups
+    covered = np.zeros((items, k_tiles), dtype=np.int32)
+    for i, b, e in zip(item, begin, end):
+        assert b < e
+        covered[i, b:e] += 1
+    assert np.all(covered == 1)
+    assert np.array_equal(part > 0, begin > 0)
+    assert np.array_equal(worker - first, part)
+    assert np.array_equal(np.bincount(item, minlength=items)[item], parts)
+    slots = worker[part > 0]
+    assert np.unique(slots).size == slots.size
+    assert partial == members * rows
+    assert further >= (slots.max(initial=-1) + 1) * group * unit_rows[0]
+    assert further <= 2 * 148 * 128 * 256
+
+
 def test_compute_entry_points_fail_loudly_without_a_gpu(built_library):
     """On a machine without a CUDA device every compute call reports an error
     instead of computing on the CPU."""
