@@ -317,7 +317,7 @@ def test_qwen3_0_6b_q8_0_greedy_agreement_over_256_tokens(built_library):
 
 
 def test_prefill_chunk_of_several_row_groups_matches_oracle(model):
-    """A 150-token chunk runs as three row groups (64 + 64 + 22) over one conversion of all its rows."""
+    """A 150-token chunk runs as two row groups (128 + 22) of the prefill GEMM."""
     from ribn_b200 import BatchItem, StepKind
     tensors, oracle = model
     ex = build(MID, tensors, context_tokens=256, max_sequences=1, max_batch_tokens=192)
@@ -343,9 +343,8 @@ def test_prefill_chunk_of_several_row_groups_matches_oracle(model):
 
 
 def test_operand_cache_changes_no_logit_bit(model):
-    """RIBN_B200_FLAG_OPERAND_CACHE keeps the K-quant matrices as tensor-core operands: a 150-token prefill chunk
-    (a pair of row groups and a partial one) and a ragged decode batch of five rows give the same logits bit for bit
-    and the same tokens as the executor that converts packed tiles on every use."""
+    """RIBN_B200_FLAG_OPERAND_CACHE is accepted on one GPU and changes nothing there (a 150-token prefill chunk, a ragged
+    decode batch of five rows).  test_gpu_tp.py runs the executor that keeps the K-quant matrices as operands."""
     import ribn_b200
     from ribn_b200 import BatchItem, StepKind
     tensors, _ = model
@@ -372,6 +371,40 @@ def test_operand_cache_changes_no_logit_bit(model):
     assert results[0][0] == results[1][0]
     for a, b in zip(results[0][1], results[1][1]):
         assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+
+
+def test_integer_kernels_of_a_batch_match_oracle(model):
+    """FLAG_NO_TCGEN05 on one GPU: a prompt of two row groups (64 + 33), then decode batches of three rows."""
+    import ribn_b200
+    from ribn_b200 import BatchItem, StepKind
+    tensors, oracle = model
+    rng = np.random.default_rng(12)
+    prompts = [rng.integers(0, MID["vocab"], size=n).tolist() for n in (97, 11, 40)]
+    ex = build(MID, tensors, flags=ribn_b200.FLAG_NO_TCGEN05, context_tokens=256, max_sequences=3, max_batch_tokens=128)
+    sequences, feed = [], []
+    for i, prompt in enumerate(prompts):
+        assert ex.admit(i + 1, i + 1, prompt, 8).ready
+        item = BatchItem(i + 1, StepKind.PREFILL, 0, len(prompt), 1)
+        ex.prepare([item])
+        done = ex.wait(ex.submit([item]))
+        seq = oracle.new_sequence()
+        for t in prompt[:-1]:
+            seq.step(t, want_logits=False)
+        assert close(ex.copy_logits(0), seq.step(prompt[-1]))
+        sequences.append(seq)
+        feed.append(done[0].tokens[0])
+    for step in range(4):
+        items = [BatchItem(i + 1, StepKind.DECODE, len(p) + step, 1, 1) for i, p in enumerate(prompts)]
+        ex.prepare(items)
+        done = ex.wait(ex.submit(items))
+        for i, seq in enumerate(sequences):
+            got = ex.copy_logits(i)
+            assert close(got, seq.step(feed[i]))                       # teacher-forced with the device's token
+            feed[i] = done[i].tokens[0]
+            assert feed[i] == orc.argmax(got)
+    for seq in sequences:
+        seq.close()
+    ex.close()
 
 
 def test_batched_decode_graph_replay_changes_no_bit(model):
