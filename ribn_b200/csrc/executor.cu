@@ -583,8 +583,7 @@ cudaError_t batch_project(ribn_b200_executor* ex, int& launches, const float* x,
     const bool tensor_memory = !(ex->cfg.flags & RIBN_B200_FLAG_NO_TCGEN05);
     GemvSegment probe[3];
     for (int i = 0; i < n_mats; ++i) probe[i] = GemvSegment{nullptr, mats[i]->type, 0, 0, nullptr};
-    const bool kquant = tensor_memory && gemm_tc_kquant(probe, n_mats, 1);
-    if (tensor_memory && !kquant) {
+    if (tensor_memory && !gemm_tc_kquant(probe, n_mats, 1)) {
         // matrices with a Q8_0 member: the fragment-order kernel takes every row of the step in one launch
         StepFinish f{};
         f.x = x; f.index = index; f.norm_weight = norm_weight; f.members = tokens; f.out = ex->op_step;
@@ -605,9 +604,9 @@ cudaError_t batch_project(ribn_b200_executor* ex, int& launches, const float* x,
         if (epilogue == kSwiGLU) STEP_TRY(launch_silu_mul(s, ys[0], ys[1], (long long)tokens * mats[0]->rows, ys[0]));
         return cudaSuccess;
     }
-    const int group = !tensor_memory ? kGemmMaxMembers : kquant ? 64 : kGemmTcMaxMembers;
+    const int group = kGemmMaxMembers;
     // K-quant form: one conversion of every row of the step, laid out as one operand per group
-    const bool converted = kquant && tokens > group;
+    const bool converted = tensor_memory && tokens > group;
     if (converted) {
         cudaError_t e = launch_to_tc_operand_groups(s, x, index, norm_weight, tokens, group, k, ex->cfg.rms_eps, ex->op_tc);
         if (e != cudaSuccess) return e;
@@ -631,10 +630,7 @@ cudaError_t batch_project(ribn_b200_executor* ex, int& launches, const float* x,
         if (tensor_memory) {
             // tcgen05 dequant-GEMM; SwiGLU runs as a separate elementwise pass over gate and up
             if (!converted) {
-                cudaError_t e = launch_to_tc_operand(s, index ? x : x + (size_t)base * k, index ? index + base : nullptr,
-                                                     norm_weight, m, k, ex->cfg.rms_eps, kquant, ex->op_tc);
-                if (e != cudaSuccess) return e;
-                launches += kquant ? 1 : 2;
+                STEP_TRY(launch_to_tc_operand(s, x, index, norm_weight, m, k, ex->cfg.rms_eps, true, ex->op_tc));
                 a.chunks = (const signed char*)ex->op_tc.chunks;
                 a.member_scale = ex->op_tc.member_scale;
             } else {
@@ -645,7 +641,7 @@ cudaError_t batch_project(ribn_b200_executor* ex, int& launches, const float* x,
                     a.group_chunk_bytes = tc_operand_bytes(group, k);
                 }
             }
-            a.kquant = kquant ? 1 : 0;
+            a.kquant = 1;
             a.partial = ex->tc_partial;
             a.partial_floats = ex->tc_partial_floats;
             a.epilogue = epilogue == kSwiGLU ? kStore : epilogue;
@@ -1162,13 +1158,11 @@ int ribn_b200_finalize(ribn_b200_executor* ex) {
                     }
                     if (further > 0) CU_TRY(ex, dev_alloc(ex, &ex->step_further, further));
                 } else {
-                    // room for every 64-row group of the largest step (one conversion per projection), or one 128-row operand
-                    const size_t tc_groups = ((size_t)c.max_batch_tokens + 63) / 64;
-                    const size_t tc_rows = std::max<size_t>(tc_groups * 64, kGemmTcMaxMembers);
-                    CU_TRY(ex, dev_alloc(ex, (unsigned char**)&ex->op_tc.chunks,
-                                         std::max(tc_operand_bytes(kGemmTcMaxMembers, kmax), tc_groups * tc_operand_bytes(64, kmax))));
-                    CU_TRY(ex, dev_alloc(ex, &ex->op_tc.scale_in, tc_rows));
-                    CU_TRY(ex, dev_alloc(ex, &ex->op_tc.member_scale, tc_rows));
+                    // room for every 64-row group of the largest step (one conversion per projection)
+                    const size_t tc_groups = (T + 63) / 64;
+                    CU_TRY(ex, dev_alloc(ex, (unsigned char**)&ex->op_tc.chunks, tc_groups * tc_operand_bytes(64, kmax)));
+                    CU_TRY(ex, dev_alloc(ex, &ex->op_tc.scale_in, tc_groups * 64));
+                    CU_TRY(ex, dev_alloc(ex, &ex->op_tc.member_scale, tc_groups * 64));
                     CU_TRY(ex, dev_alloc(ex, &ex->op_batch.chunks, batch_operand_bytes(kGemmMaxMembers, kmax)));
                     CU_TRY(ex, dev_alloc(ex, &ex->op_batch.member_scale, kGemmMaxMembers));
                     CU_TRY(ex, dev_alloc(ex, &ex->op_batch.digit_inv, kGemmMaxMembers));
