@@ -29,7 +29,7 @@
 // gemm_tc.cu (6.7e-7 against 4.6e-7 of a row's results at 48 and more columns); with a sum per half and the small parts
 // first it is at 2.0e-7, for 0.7 % of a step of 64 rows.  Q8_0's one sum per tile (5.2e-7, 7.1e-7 at 48 and more columns)
 // replaced one over all inputs there (2.7e-6 to 2.9e-5); a sum per half (2.0e-7) would cost 4 % of a step of 32 rows of
-// the 0.6B model.  Slots (unit, row group, k tile) are dealt to the CTAs evenly when another kernel finishes the sums, in
+// the 0.6B model.  Slots (unit, k tile) are dealt to the CTAs evenly when another kernel finishes the sums, in
 // whole items otherwise (StepSplit).  Every wait is bounded.
 #include <cuda_fp16.h>
 
@@ -51,11 +51,11 @@ constexpr int kEpilogueRegs = 112, kOtherRegs = 64;
 constexpr uint32_t kSpinLimit = 1u << 22;
 constexpr size_t kSmemBudget = 224 * 1024;
 
-// Columns of a launch's operand: MP rows of activations per group.
+// Columns of a launch's operand: MP rows of activations, in one group.
 template <int MP>
 struct Cols {
     static constexpr bool kJoined = MP <= 32;               // hi and lo parts side by side in one MMA, or one after the other
-    static constexpr int kSumCols = MP < 16 ? 16 : (MP + 15) / 16 * 16;
+    static constexpr int kSumCols = (MP + 15) / 16 * 16;
     static constexpr int kMain = 1024 * MP, kSums = 32 * kSumCols;
     static constexpr int kBlock = kMain + kSums + 4 * MP;
 };
@@ -101,11 +101,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ta_kernel(const StepGemm a, 
             int ws = 0, filled = 0;
             uint32_t parity = 1;
             for (int s = s0; s < s1 && alive;) {
-                const int item = s / k_tiles, end = min(s1, (item + 1) * k_tiles);
-                const UnitAt at = unit_at(a, item / split.groups, kUnitTiles);
+                const int unit = s / k_tiles, end = min(s1, (unit + 1) * k_tiles);
+                const UnitAt at = unit_at(a, unit, kUnitTiles);
                 const GemvSegment& seg = a.seg[at.seg];
                 const uint32_t bytes = kUnitTiles * (uint32_t)packed_tile_bytes(type_of<TYPE>(seg));
-                for (int kb = s - item * k_tiles; s < end; ++s, ++kb) {
+                for (int kb = s - unit * k_tiles; s < end; ++s, ++kb) {
                     if (filled == nw) alive = mbar_wait(w_empty + 8 * ws, parity, a.error_flag, 91, spin_limit);
                     else ++filled;
                     if (!alive) break;
@@ -121,8 +121,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ta_kernel(const StepGemm a, 
             int bs = 0, filled = 0;
             uint32_t parity = 1;
             for (int s = s0; s < s1 && alive;) {
-                const int item = s / k_tiles, end = min(s1, (item + 1) * k_tiles);
-                const unsigned char* from = a.blocks + ((size_t)(item % split.groups) * k_tiles + (s - item * k_tiles)) * C::kBlock;
+                const int unit = s / k_tiles, end = min(s1, (unit + 1) * k_tiles);
+                const unsigned char* from = a.blocks + (size_t)(s - unit * k_tiles) * C::kBlock;
                 for (; s < end; ++s, from += C::kBlock) {
                     if (filled == nb) alive = mbar_wait(folded + 8 * bs, parity, a.error_flag, 92, spin_limit);
                     else ++filled;
@@ -144,8 +144,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ta_kernel(const StepGemm a, 
             int bs = 0, fold_slot = 0;
             uint32_t b_parity = 0, fold_parity = 0, a_count = 0, kt = 0, q6_count = 0;
             for (int s = s0; s < s1;) {
-                const int item = s / k_tiles, end = min(s1, (item + 1) * k_tiles);
-                const int type = type_of<TYPE>(a.seg[unit_at(a, item / split.groups, kUnitTiles).seg]);
+                const int unit = s / k_tiles, end = min(s1, (unit + 1) * k_tiles);
+                const int type = type_of<TYPE>(a.seg[unit_at(a, unit, kUnitTiles).seg]);
                 const bool q4k = type == kQ4_K, q6k = TYPE == kKQuants ? !q4k : type == kQ6_K;
                 for (; s < end; ++s, ++kt) {
                     const uint32_t p = kt & 1u, d_main = tmem + 64 * p, d_min = tmem + 128 + 64 * p;
@@ -224,8 +224,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ta_kernel(const StepGemm a, 
             }
         };
         for (int s = s0; s < s1;) {
-            const int item = s / k_tiles, end = min(s1, (item + 1) * k_tiles);
-            const int type = type_of<TYPE>(a.seg[unit_at(a, item / split.groups, kUnitTiles).seg]);
+            const int unit = s / k_tiles, end = min(s1, (unit + 1) * k_tiles);
+            const int type = type_of<TYPE>(a.seg[unit_at(a, unit, kUnitTiles).seg]);
             for (; s < end; ++s, ++kt) {
                 if (alive) alive = mbar_wait(w_full + 8 * ws, parity, a.error_flag, 96, spin_limit);
                 const uint32_t tile = w_ring + ws * rings.w_bytes + 2 * quadrant * packed_tile_bytes(type);
@@ -263,16 +263,17 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ta_kernel(const StepGemm a, 
         constexpr int kChunks = (MP + 15) / 16;   // eights of columns per thread: 16 j + 8 (warp >> 2)
         const int quadrant = warp & 3, mine = 8 * (warp >> 2), row = quadrant * 32 + lane;
         bool alive = true;
-        int bs = 0, inv_group = -1;
+        int bs = 0;
+        bool factors = a.partial != nullptr;   // the rows' RMSNorm factors are in place, or another kernel applies them
         uint32_t b_parity = 0, kt = 0;
         float* inv = reinterpret_cast<float*>(smem + (inv_at - w_ring));
         for (int s = s0; s < s1;) {
-            const int item = s / k_tiles, unit = item / split.groups, group = item - unit * split.groups;
+            const int unit = s / k_tiles;
             const UnitAt at = unit_at(a, unit, kUnitTiles);
             const GemvSegment& seg = a.seg[at.seg];
             const int type = type_of<TYPE>(seg);
             const bool q4k = type == kQ4_K, q6k = TYPE == kKQuants ? !q4k : type == kQ6_K;
-            const int end = min(s1, (item + 1) * k_tiles);
+            const int end = min(s1, (unit + 1) * k_tiles);
             float acc[kChunks][8];
 #pragma unroll
             for (int j = 0; j < kChunks; ++j) {
@@ -288,7 +289,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ta_kernel(const StepGemm a, 
                 const float2 dd = __half22float2(as_half2(lds32(scales_ring + (kt & 3u) * (kUnitRows * 4) + row * 4)));
                 const float d = dd.x, dmin = dd.y;
                 const uint32_t sx_at = b_ring + bs * kBBytes + C::kMain + C::kSums + mine * 4;
-                constexpr int kBatch = kChunks < 2 ? 1 : 2;   // eights of columns in flight together
+                constexpr int kBatch = 2;   // eights of columns in flight together
 #pragma unroll
                 for (int j0 = 0; j0 < kChunks; j0 += kBatch) {
                     float x[kBatch][8], y[kBatch][8], z[kBatch][8], w[kBatch][8];
@@ -332,13 +333,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ta_kernel(const StepGemm a, 
                 if (lane == 0) mbar_arrive(folded + 8 * bs);
                 if (++bs == nb) { bs = 0; b_parity ^= 1u; }
             }
-            if (a.partial == nullptr && group != inv_group) {
-                inv_group = group;
-                asm volatile("bar.sync 1, 256;" ::: "memory");   // the previous group's factors have been read
+            if (!factors) {
+                factors = true;
                 for (int m = warp; m < MP; m += kEpilogueWarps) {
-                    const int member = group * MP + m;
                     float sum = 0.0f;
-                    if (a.ss != nullptr && member < a.members) for (int i = lane; i < k_tiles; i += 32) sum += a.ss[(size_t)member * k_tiles + i];
+                    if (a.ss != nullptr && m < a.members) for (int i = lane; i < k_tiles; i += 32) sum += a.ss[(size_t)m * k_tiles + i];
 #pragma unroll
                     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
                     if (lane == 0) inv[m] = a.ss != nullptr ? 1.0f / sqrtf(sum / (float)a.k + a.eps) : 1.0f;
@@ -348,17 +347,17 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ta_kernel(const StepGemm a, 
             const int n_index = at.rt0 * kTileRows + row;
             if (n_index < seg.n) {
                 StepSums to{};
-                if (a.partial != nullptr) to = step_sums(a, split, (int)blockIdx.x, split.whole ? 0 : (int)blockIdx.x - split.first_worker(item), group, mine, at.seg, n_index);
+                if (a.partial != nullptr) to = step_sums(a, split, (int)blockIdx.x, split.whole ? 0 : (int)blockIdx.x - split.first_worker(unit), 0, mine, at.seg, n_index);
 #pragma unroll
                 for (int j = 0; j < kChunks; ++j) {
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
-                        const int m = 16 * j + mine + i, member = group * MP + m;
-                        if (m >= MP || member >= a.members) continue;
+                        const int m = 16 * j + mine + i;
+                        if (m >= MP || m >= a.members) continue;
                         if (a.partial != nullptr) {
                             to.at[(16 * j + i) * to.stride] = acc[j][i];
                         } else {
-                            float* y = seg.y + (size_t)member * seg.n + n_index;
+                            float* y = seg.y + (size_t)m * seg.n + n_index;
                             *y = a.epilogue == kResidual ? *y + acc[j][i] * inv[m] : acc[j][i] * inv[m];
                         }
                     }
@@ -389,7 +388,7 @@ cudaError_t launch_variant(cudaStream_t stream, const StepGemm& a, int w_bytes, 
     TaRings rings{};
     rings.w_bytes = (w_bytes + 127) & ~127;
     const size_t b_bytes = (size_t)((Cols<MP>::kBlock + 127) & ~127), fixed = 2 * kA2Bytes + 4 * kUnitRows * 4 + MP * 4 + 16 + 352;
-    rings.b_stages = MP <= 8 ? 5 : MP <= 16 ? 4 : MP <= 32 ? 3 : 2;
+    rings.b_stages = MP <= 32 ? 3 : 2;
     rings.w_stages = (int)std::min<size_t>(8, (kSmemBudget - fixed - rings.b_stages * b_bytes) / rings.w_bytes);
     if (rings.w_stages < 2) return cudaErrorInvalidValue;
     const StepSplit split = step_split(a, a.partial == nullptr);
@@ -409,8 +408,6 @@ cudaError_t launch_variant(cudaStream_t stream, const StepGemm& a, int w_bytes, 
 template <int TYPE>
 cudaError_t launch_typed(cudaStream_t stream, const StepGemm& a, int w_bytes, bool programmatic) {
     switch (step_shape(a.members, kColumnForm).ng) {
-        case 1: return launch_variant<8, TYPE>(stream, a, w_bytes, programmatic);
-        case 2: return launch_variant<16, TYPE>(stream, a, w_bytes, programmatic);
         case 3: return launch_variant<24, TYPE>(stream, a, w_bytes, programmatic);
         case 4: return launch_variant<32, TYPE>(stream, a, w_bytes, programmatic);
         case 6: return launch_variant<48, TYPE>(stream, a, w_bytes, programmatic);
@@ -421,6 +418,7 @@ cudaError_t launch_typed(cudaStream_t stream, const StepGemm& a, int w_bytes, bo
 }  // namespace
 
 cudaError_t launch_gemm_ta(cudaStream_t stream, const StepGemm& a, int w_bytes, bool programmatic) {
+    if (a.members > kColumnMaxMembers) return cudaErrorInvalidValue;
     switch (common_type(a)) {
         case kQ4_K: return launch_typed<kQ4_K>(stream, a, w_bytes, programmatic);
         case kQ6_K: return launch_typed<kQ6_K>(stream, a, w_bytes, programmatic);

@@ -237,15 +237,16 @@ int gemm_tc_last_launches();
 //     [16 steps][lane] 16 bytes   hi pairs (4t, 4t + 2), (4t + 1, 4t + 3) of the step's 16 inputs of row lane / 4, then lo pairs
 //     [lane] 8 bytes              sums of the eight 32-input groups: hi in the first eight operand rows, lo in the last eight
 //     [8] F32                     the rows' scales
-//   kColumnForm (gemm_ta.cu, tcgen05): groups of mp = 8 ng rows (at most 64), one block
+//   kColumnForm (gemm_ta.cu, tcgen05): one group of at most 64 rows in mp = 24, 32, 48 or 64 columns, one block
 //     [32][2 mp] 16 bytes         K-major core matrices: input 16 s + 4 t + i + 2 e is element 2 t + e of 8-input block 2 s + i;
 //                                 columns: hi parts, then lo parts
-//     [2][max(16, mp to 16)] 16 bytes   sums of the eight 32-input groups: hi, then lo
+//     [2][mp to 16] 16 bytes      sums of the eight 32-input groups: hi, then lo
 //     [mp] F32                    the rows' scales
-//   kWideForm (gemm_pf.cu, tcgen05): the column form with mp = 128
+//   kWideForm (gemm_pf.cu, tcgen05): groups of 128 rows, each as the column form with mp = 128
 // Blocks are ordered [group][k tile](ng).  `ss` holds, per row and k tile, the sum of squares of the values before the
 // norm weight, for the RMSNorm factor of the consumer.
 enum StepForm : int { kFragmentForm = 0, kColumnForm = 1, kWideForm = 2 };
+constexpr int kColumnMaxMembers = 64;
 constexpr int kFragBlockBytes = 16 * 512 + 256 + 32;
 
 struct StepOperand {

@@ -353,22 +353,23 @@ int ribn_b200_op_gemv(int32_t device, int32_t type, const void* weights, int64_t
                 OP_TRY(launch_gemm_tc(s.stream, a));
             }
         } else if (variant >= 6 && variant <= 8) {
-            // the kernels of a step of a few rows, in fragment order or with tensor-memory conversion: partial sums finished by a second kernel where a step of a few rows does so
+            // a step's GEMMs in fragment order, with tensor-memory conversion (the column form: up to 64 rows at once) and in
+            // the wide form; partial sums are finished by a second kernel where a step does so
             const int form = variant == 8 ? kWideForm : variant == 7 ? kColumnForm : kFragmentForm;
+            const int per_launch = form == kColumnForm ? std::min(members, kColumnMaxMembers) : members;
             alignas(64) unsigned char map[kTileMapBytes];
             OP_TRY(make_tile_map(type, d_w, rows, cols, map));
             StepFinish f{};
-            f.x = d_x;
-            f.members = members;
-            f.out.blocks = s.alloc<unsigned char>(step_operand_bytes(members, (int)cols, form));
+            f.members = per_launch;
+            f.out.blocks = s.alloc<unsigned char>(step_operand_bytes(per_launch, (int)cols, form));
             f.out.form = form;
             StepGemm g{};
             g.form = form;
             g.n_segments = 1;
-            g.seg[0] = GemvSegment{d_w, type, (int)rows, (int)((rows + kTileRows - 1) / kTileRows), d_y};
+            g.seg[0] = GemvSegment{d_w, type, (int)rows, (int)((rows + kTileRows - 1) / kTileRows), nullptr};
             g.seg[0].map = s.upload(map, sizeof(map));
             g.k = (int)cols;
-            g.members = members;
+            g.members = per_launch;
             g.blocks = f.out.blocks;
             g.epilogue = kStore;
             g.error_flag = d_err;
@@ -380,9 +381,14 @@ int ribn_b200_op_gemv(int32_t device, int32_t type, const void* weights, int64_t
                 if (further > 0) { g.further = s.alloc<float>(further); OP_PTR(g.further); }
             }
             OP_PTR(f.out.blocks); OP_PTR(g.seg[0].map);
-            OP_TRY(launch_step_finish(s.stream, kFinishRows, nullptr, f, (int)cols, false));
-            OP_TRY(launch_step_gemm(s.stream, g, false));
-            if (split) OP_TRY(launch_step_finish(s.stream, kFinishStore, &g, StepFinish{}, 0, false));
+            for (int m0 = 0; m0 < members; m0 += per_launch) {
+                f.x = d_x + (size_t)m0 * cols;
+                g.seg[0].y = d_y + (size_t)m0 * rows;
+                f.members = g.members = std::min(per_launch, members - m0);
+                OP_TRY(launch_step_finish(s.stream, kFinishRows, nullptr, f, (int)cols, false));
+                OP_TRY(launch_step_gemm(s.stream, g, false));
+                if (split) OP_TRY(launch_step_finish(s.stream, kFinishStore, &g, StepFinish{}, 0, false));
+            }
         } else if (variant == 2) {
             // the batched kernel, in groups of up to kGemmMaxMembers members
             BatchOperand bop;

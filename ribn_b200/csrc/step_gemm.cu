@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(512, BATCH > 2 ? 1 : 3) step_finish_kernel(con
     const int s = i >> 2, t = i & 3;
     const float inv_scale = power2(-e);
     if (a.out.form != kFragmentForm) {
-        const int mp = 8 * a.out.ng, sum_cols = max(16, (mp + 15) / 16 * 16), col = ng * 8 + g;
+        const int mp = 8 * a.out.ng, sum_cols = (mp + 15) / 16 * 16, col = ng * 8 + g;
         unsigned char* blk = a.out.blocks + ((size_t)group * k_tiles + kt) * (1028 * mp + 32 * sum_cols);
         // The eight members' 16-byte pieces of an 8-input block lie side by side: through shared memory, so that a warp's
         // stores are whole 128-byte lines.  staged[8-input block][hi, lo][member ^ step % 8]: conflict-free both ways.
@@ -215,16 +215,15 @@ StepShape step_shape(int members, int form) {
     const int eights = (members + 7) / 8;
     if (form == kWideForm) return StepShape{(eights + 15) / 16, 16};
     if (form == kColumnForm) {
-        // one group of up to 64 rows: 8, 16, 24, 32, 48 or 64 columns
-        if (eights <= 4) return StepShape{1, eights};
-        return StepShape{(eights + 7) / 8, eights <= 6 ? 6 : 8};
+        // one group of up to 64 rows: 24, 32, 48 or 64 columns
+        return StepShape{1, eights <= 3 ? 3 : eights <= 4 ? 4 : eights <= 6 ? 6 : 8};
     }
     const int groups = (eights + 3) / 4;
     return StepShape{groups, (eights + groups - 1) / groups};
 }
 
 namespace {
-size_t column_block_bytes(int mp) { return (size_t)1028 * mp + 32 * (size_t)(mp < 16 ? 16 : (mp + 15) / 16 * 16); }
+size_t column_block_bytes(int mp) { return (size_t)1028 * mp + 32 * (size_t)((mp + 15) / 16 * 16); }
 }  // namespace
 
 size_t step_operand_bytes(int members, int k, int form) {
@@ -333,7 +332,7 @@ cudaError_t launch_step_finish(cudaStream_t stream, int mode, const StepGemm* ge
     if (mode == kFinishStore) {
         return launch_pdl(step_store_kernel, dim3((unsigned)((a.total_n / 4 + 255) / 256), (unsigned)a.members), 256, 0, stream, programmatic, a);
     }
-    if (width % kTileCols != 0) return cudaErrorInvalidValue;
+    if (width % kTileCols != 0 || (a.out.form == kColumnForm && a.members > kColumnMaxMembers)) return cudaErrorInvalidValue;
     const StepShape shape = step_shape(a.members, a.out.form);
     a.out.ng = shape.ng;
     const dim3 grid((unsigned)(width / kTileCols), (unsigned)(shape.groups * shape.ng));
