@@ -36,58 +36,19 @@
 
 #include "blocks.cuh"
 #include "gemv.cuh"
+#include "tmem.cuh"
 
 namespace ribn {
 
 namespace {
 
-constexpr int kUnitTiles = 8;                    // row tiles per unit: 128 output rows
 constexpr int kTeams = kFragTeams;
 constexpr int kTeamWarps = 4;                    // warps per team, two row tiles each
 constexpr int kWarps = kTeams * kTeamWarps;
 constexpr int kThreads = (kTeams + 1) * kTeamWarps * 32;
-constexpr int kSum32At = 16 * 512, kScaleAt = kSum32At + 256;
-static_assert(kScaleAt + 32 == kFragBlockBytes, "operand block layout");
 constexpr uint32_t kSpinLimit = 1u << 22;
 constexpr size_t kSmemBudget = 220 * 1024;
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* error_flag, int code, uint32_t limit) {
-    for (uint32_t i = 0; i < limit; ++i) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (ok) return true;
-    }
-    if (error_flag != nullptr) atomicExch(error_flag, code);
-    return false;
-}
-__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-                 "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
-// The box of a packed matrix's tensor map at (k tile, first row tile): eight tiles, kUnitTiles x tile bytes.
-__device__ __forceinline__ void tiles_g2s(uint32_t dst, const void* map, int k_tile, int row_tile, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %2, %3, %4}], [%5];" ::"r"(dst),
-                 "l"(map), "r"(0), "r"(k_tile), "r"(row_tile), "r"(bar) : "memory");
-}
-__device__ __forceinline__ uint4 lds128(uint32_t addr) {
-    uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
-    return v;
-}
 __device__ __forceinline__ uint2 lds64(uint32_t addr) {
     uint2 v;
     asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
@@ -96,16 +57,6 @@ __device__ __forceinline__ uint2 lds64(uint32_t addr) {
 __device__ __forceinline__ float2 lds64f(uint32_t addr) {
     float2 v;
     asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
-    return v;
-}
-__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
-    uint32_t v;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
-    return v;
-}
-__device__ __forceinline__ uint32_t lds16(uint32_t addr) {
-    uint32_t v;
-    asm volatile("{\n\t.reg .u16 t;\n\tld.shared.u16 t, [%1];\n\tcvt.u32.u16 %0, t;\n\t}" : "=r"(v) : "r"(addr));
     return v;
 }
 __device__ __forceinline__ void sts128(uint32_t addr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
@@ -124,12 +75,6 @@ __device__ __forceinline__ void mma_next(float (&c)[4], uint32_t a0, uint32_t a1
     asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// (a & mask) | other in one LOP3
-__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t mask, uint32_t other) {
-    uint32_t r;
-    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(a), "r"(mask), "r"(other));
-    return r;
-}
 // bytes i and i + 1 of w as floats minus `bias` (exact), times f
 __device__ __forceinline__ float2 bytes_scaled(uint32_t w, int i, float bias, float2 f) {
     const float2 raw = make_float2(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540u | (uint32_t)i)),
@@ -140,8 +85,6 @@ __device__ __forceinline__ float half_low(uint32_t w) { return __half2float(__us
 __device__ __forceinline__ float half_high(uint32_t w) { return __half2float(__ushort_as_half((unsigned short)(w >> 16))); }
 
 constexpr float kTwo24 = 16777216.0f, kTwo20 = 1048576.0f;   // an integer masked into binary16 is that integer times 2^-24
-__device__ __forceinline__ __half2 as_half2(uint32_t x) { return *reinterpret_cast<const __half2*>(&x); }
-__device__ __forceinline__ uint32_t as_bits(__half2 x) { return *reinterpret_cast<const uint32_t*>(&x); }
 // bytes i and j of w (selector 0x4j4i) as a pair of normal binary16 integers
 __device__ __forceinline__ uint32_t bytes_half2(uint32_t w, uint32_t selector) {
     return as_bits(__hsub2(as_half2(__byte_perm(w, 0x64646464u, selector)), __float2half2_rn(1024.0f)));
@@ -257,7 +200,7 @@ __device__ __forceinline__ void slot_q4k(uint32_t tile, uint32_t b_at, const Rec
     // minima (groups 2t, 2t + 1) x group sums: hi sums in the operand's first eight rows, lo sums in its last
 #pragma unroll
     for (int n = 0; n < NG; ++n) {
-        const uint2 s = lds64(b_at + n * kFragBlockBytes + kSum32At + lane * 8);
+        const uint2 s = lds64(b_at + n * kFragBlockBytes + kFragSumsAt + lane * 8);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
             const uint32_t m0 = rec_word(rec, r, 0, 8 + t), m1 = rec_word(rec, r, 1, 8 + t);
@@ -318,7 +261,7 @@ __device__ __forceinline__ void slot_q8_0(uint32_t tile, uint32_t b_at, const Re
     // 128 x d of blocks 2t, 2t + 1 (as they lie in the tile) x block sums
 #pragma unroll
     for (int n = 0; n < NG; ++n) {
-        const uint2 s = lds64(b_at + n * kFragBlockBytes + kSum32At + lane * 8);
+        const uint2 s = lds64(b_at + n * kFragBlockBytes + kFragSumsAt + lane * 8);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
             const uint32_t at = tile + r * 4352 + 4096 + g * 16 + 4 * t;
@@ -393,18 +336,6 @@ __device__ __forceinline__ void slot_q6k(uint32_t tile, uint32_t b_at, const Rec
 // A slot: the tiles, then the activations' block; the tensor copy wants 128-byte aligned destinations.
 __host__ __device__ inline int frag_slot_bytes(int w_bytes, int ng) { return (w_bytes + ng * kFragBlockBytes + 127) & ~127; }
 
-struct UnitAt { int seg, rt0; };
-__device__ __forceinline__ UnitAt unit_at(const StepGemm& a, int u) {
-    UnitAt r{0, u * kUnitTiles};
-    while (r.seg + 1 < a.n_segments) {
-        const int tiles = (a.seg[r.seg].row_tiles + kUnitTiles - 1) / kUnitTiles * kUnitTiles;
-        if (r.rt0 < tiles) break;
-        r.rt0 -= tiles;
-        ++r.seg;
-    }
-    return r;
-}
-
 // Register shares: the launch gives each of the 384 threads 168 registers (64,512 in all); the consumers' two warpgroups
 // then take what the producer's warpgroup (one working thread) hands back: 256 x 232 + 128 x 40 = 64,512.
 constexpr int kConsumerRegs = 232, kProducerRegs = 40;
@@ -433,7 +364,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_frag_kernel(const StepGemm a
         if (warp > kWarps || lane != 0) return;
         auto issue = [&](int s, int slot, bool weights, bool activations) {
             const int item = s / k_tiles, kb = s - item * k_tiles;
-            const UnitAt at = unit_at(a, item / split.groups);
+            const UnitAt at = unit_at(a, item / split.groups, kUnitTiles);
             const GemvSegment& seg = a.seg[at.seg];
             const uint32_t bar = full + 8 * slot;
             unsigned char* base = smem + (size_t)slot * slot_bytes;
@@ -500,7 +431,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_frag_kernel(const StepGemm a
     const int s1 = split.begin(worker + 1);
     for (int s = split.begin(worker); s < s1;) {
         const int item = s / k_tiles, unit = item / split.groups, group = item - unit * split.groups;
-        const UnitAt at = unit_at(a, unit);
+        const UnitAt at = unit_at(a, unit, kUnitTiles);
         const GemvSegment& seg = a.seg[at.seg];
         const int type = seg.type;
         const bool present = at.rt0 + 2 * pair < seg.row_tiles;   // a pair's absent second tile reads as zeros and is never stored
@@ -528,7 +459,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_frag_kernel(const StepGemm a
                 else slot_q8_0<NG>(tile, b_at, rec, lane, sums);
 #pragma unroll
                 for (int n = 0; n < NG; ++n) {
-                    const float2 sx = lds64f(b_at + n * kFragBlockBytes + kScaleAt + 8 * t);
+                    const float2 sx = lds64f(b_at + n * kFragBlockBytes + kFragScaleAt + 8 * t);
 #pragma unroll
                     for (int r = 0; r < 2; ++r) {
                         acc[r][n][0] = fmaf(sums[r][n][0], sx.x, acc[r][n][0]);

@@ -247,7 +247,8 @@ int gemm_tc_last_launches();
 // norm weight, for the RMSNorm factor of the consumer.
 enum StepForm : int { kFragmentForm = 0, kColumnForm = 1, kWideForm = 2 };
 constexpr int kColumnMaxMembers = 64;
-constexpr int kFragBlockBytes = 16 * 512 + 256 + 32;
+constexpr int kFragSumsAt = 16 * 512, kFragScaleAt = kFragSumsAt + 256, kFragBlockBytes = kFragScaleAt + 32;
+constexpr int kUnitTiles = 8;   // row tiles per tensor copy and per unit: 128 output rows (two units make one of the wide form)
 
 struct StepOperand {
     unsigned char* blocks = nullptr;

@@ -15,9 +15,6 @@ namespace ribn {
 
 namespace {
 
-constexpr int kUnitTiles = 8;   // row tiles per tensor copy and per unit: 128 output rows (two units make one of the wide form)
-constexpr int kSum32At = 16 * 512, kScaleAt = kSum32At + 256;   // fragment-form block
-
 // RMSNorm factor of one row from the sums of squares of its k tiles (every lane of the warp gets it).
 __device__ __forceinline__ float norm_factor(const float* ss, int tiles, float eps, int lane) {
     float sum = 0.0f;
@@ -162,11 +159,11 @@ __global__ void __launch_bounds__(512, BATCH > 2 ? 1 : 3) step_finish_kernel(con
     if ((i & 7) == 0) {
         const int q = i >> 3;
         const __half h = __float2half_rn(sum), l = __float2half_rn(sum - __half2float(h));
-        __half* at = reinterpret_cast<__half*>(blk + kSum32At + (g * 4 + (q >> 1)) * 8) + (q & 1);
+        __half* at = reinterpret_cast<__half*>(blk + kFragSumsAt + (g * 4 + (q >> 1)) * 8) + (q & 1);
         at[0] = h;
         at[2] = l;
     }
-    if (i == 0) reinterpret_cast<float*>(blk + kScaleAt)[g] = inv_scale;
+    if (i == 0) reinterpret_cast<float*>(blk + kFragScaleAt)[g] = inv_scale;
 }
 
 // Plain outputs of a split launch: y = (sum of the parts) x the RMSNorm factor, four values per thread; blockIdx.y = member.

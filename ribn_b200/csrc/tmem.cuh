@@ -1,5 +1,5 @@
-// What the tcgen05 GEMMs with a tensor-memory A operand share: barriers, copies, tensor-memory accesses, and the
-// conversion of packed Q4_K / Q6_K / Q8_0 tiles to operand columns.
+// What the step GEMMs share: barriers, copies and shared-memory loads, and, of the tcgen05 kernels with a tensor-memory A
+// operand, tensor-memory accesses and the conversion of packed Q4_K / Q6_K / Q8_0 tiles to operand columns.
 #pragma once
 #include <cuda_fp16.h>
 
@@ -8,7 +8,6 @@
 
 namespace ribn {
 
-constexpr int kUnitTiles = 8;
 constexpr int kUnitRows = kUnitTiles * kTileRows;   // 128: tensor-memory lanes
 constexpr int kA2Bytes = kUnitRows * 16 * 2;        // minima operand: 128 rows x (8 minima, twice) halves
 constexpr int kA2Lbo = kUnitRows / 8 * 128;         // bytes between its two 8-input column blocks
