@@ -490,14 +490,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_frag_kernel(const StepGemm a
             }
         }
         const int part = a.partial != nullptr && !split.whole ? worker - split.first_worker(item) : 0;
+        const StepSums to = step_sums(a, split, worker, part, group, 2 * t, at.seg, (at.rt0 + 2 * pair) * kTileRows + g);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int n_index = (at.rt0 + 2 * pair + r) * kTileRows + g + 8 * h;
                 if (n_index >= seg.n) continue;
-                StepSums to{};
-                if (a.partial != nullptr) to = step_sums(a, split, worker, part, group, 2 * t, at.seg, n_index);
 #pragma unroll
                 for (int n = 0; n < NG; ++n) {
 #pragma unroll
@@ -506,7 +505,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_frag_kernel(const StepGemm a
                         if (m >= a.members) continue;
                         const float v = acc[r][n][2 * h + c];
                         if (a.partial != nullptr) {
-                            to.at[(n * 8 + c) * to.stride] = v;
+                            to.at[(n * 8 + c) * to.stride + r * kTileRows + 8 * h] = v;
                         } else {
                             float* y = seg.y + (size_t)m * seg.n + n_index;
                             *y = a.epilogue == kResidual ? *y + v * inv[n][c] : v * inv[n][c];
