@@ -192,7 +192,7 @@ def replica_throughput(dist, world: int, rows: int, steps: int, seconds: float, 
     return world * rows * steps / all_max(dist, seconds, device)
 
 
-EXTRA_FLAGS = 0      # set from --operand-cache: ribn_b200.FLAG_OPERAND_CACHE on every Qwen executor of the run
+EXTRA_FLAGS = 0      # set from --operand-cache with --tp: ribn_b200.FLAG_OPERAND_CACHE on the ranks' executors
 SCHEME = "q4_k_m"   # set from --scheme: "q4_k_m" (Q4_K; Q6_K for attn_v, ffn_down, output) or "q8_0"
 
 
@@ -397,34 +397,6 @@ def run_ours(args):
                           "spread": spreadb,
                           "x_batch1": (world * B * args.steps / devb) / value1}
     ex.close()
-    if B >= 3 and not EXTRA_FLAGS and not args.no_cache_leg and args.scheme == "q4_k_m":
-        # the same batch once more on an executor that keeps the K-quant matrices as tensor-core operands
-        # (RIBN_B200_FLAG_OPERAND_CACHE: 2 or 4 bytes of HBM per weight; same logits bit for bit)
-        # An extra: if the larger executor cannot be built on some rank (memory taken by someone else), every rank
-        # skips the leg together and the line says so.
-        ex, problem = None, ""
-        try:
-            ex = ribn_b200.QwenB200(model, context_tokens=args.context + 2 * total_steps + 20, max_sequences=B,
-                                    max_batch_tokens=max(B, 16), device=local, flags=ribn_b200.FLAG_OPERAND_CACHE)
-            ex.init_synthetic(0x5EED, ribn_b200.SCHEME_Q4_K_M)
-            ex.finalize()
-            seed_sequences(ex, model, B, args.context, 2 * total_steps + 4, seed=1 + rank)
-        except Exception as exc:   # noqa: BLE001
-            problem = str(exc) or type(exc).__name__
-        if all_max(dist, 1.0 if problem else 0.0, local) > 0.0:
-            out["batch64"]["operand_cache"] = {"unavailable": problem or "another rank could not build the executor"}
-        else:
-            positions = {s + 1: args.context for s in range(B)}
-            _, devc, launchesc, _, spreadc = phase(list(range(1, B + 1)), 3)
-            out["batch64"]["operand_cache"] = {"value": world * B * args.steps / devc, "unit": "tok/s",
-                                               "ms_per_step": devc / args.steps * 1e3, "gpu_launches": launchesc,
-                                               "spread": spreadc,
-                                               "note": "K-quant matrices also kept as binary16 operand planes (Q4_K 2 B, Q6_K 4 B per weight)"}
-        if ex is not None:
-            try:
-                ex.close()
-            except Exception:   # noqa: BLE001
-                pass
     if not args.no_serving:
         # p50 time to first token is part of the metric: a bounded serving leg below saturation
         srv = serving_job(args, rank, world, local, dist, n=args.serving_requests, rate=args.arrival_rate_default,
@@ -875,14 +847,14 @@ def main():
     ap.add_argument("--context-max", type=int, default=8192, help="tp: contexts are uniform in [512, this]")
     ap.add_argument("--engine", default="python", choices=["python", "native"],
                     help="serving / mixed: the host engine that drives the executor (ribn_b200/engine.py or the C++ one)")
-    ap.add_argument("--no-cache-leg", action="store_true", help="decode: skip the extra batch leg with the operand cache on")
+    ap.add_argument("--no-cache-leg", action="store_true", help="accepted and without effect: one-GPU executors keep no operand cache to time")
     ap.add_argument("--operand-cache", default="off", choices=["on", "off"],
-                    help="keep the K-quant matrices also as tensor-core operands in HBM (RIBN_B200_FLAG_OPERAND_CACHE)")
+                    help="tp: keep the K-quant matrices also as tensor-core operands in HBM (RIBN_B200_FLAG_OPERAND_CACHE)")
     ap.add_argument("--scheme", default="q4_k_m", choices=["q4_k_m", "q8_0"], help="synthetic checkpoint's block types")
     args = ap.parse_args()
     global SCHEME, EXTRA_FLAGS
     SCHEME = args.scheme
-    if args.operand_cache == "on" and args.impl != "reference":
+    if args.operand_cache == "on" and args.tp > 1 and args.impl != "reference":
         import ribn_b200
         EXTRA_FLAGS = ribn_b200.FLAG_OPERAND_CACHE
     if args.warmup < 3:
