@@ -121,7 +121,7 @@ struct ribn_b200_executor {
     ribn::ActOperand op_hidden, op_attn, op_act, op_head;
     ribn::BatchOperand op_batch;  // batch form, refilled before every batched projection
     ribn::TcOperand op_tc;        // tensor-memory form (the same, for the tcgen05 kernel)
-    ribn::StepOperand op_step;    // operand of the step GEMMs (batches of a few rows; any batch of a Q8_0 model)
+    ribn::StepOperand op_step;    // operand of the step GEMMs
     float* step_further = nullptr;  // the step GEMMs' further partial sums (their first ones lie in `gate`)
     float* tc_partial = nullptr;  // split-K sums of the batched kernels (tensor parallelism)
     size_t tc_partial_floats = 0;
