@@ -13,8 +13,10 @@
 // last bit, see gemm_ta.cu.  With one sum per k tile, whose second half's lo parts met a large sum already, the K-quants were
 // 1.5 times as far from the exact results as the kernel of gemm_tc.cu: 1.1e-6 of a row's results against 7.2e-7 for Q4_K,
 // 6.7e-7 against 4.6e-7 for Q6_K; now 3.7e-7 and 3.2e-7.  The additional reads of tensor memory beside the products take
-// 2.2 ms and 2.7 ms of 87 ms of an 8B chunk of 2,048 rows; a third set of sums in turn for Q6_K, or reads of 16 columns at
-// a time, changed nothing.  Q8_0's one sum per tile, 8.4e-7, replaced one over all inputs.)  The F32 sums of a work item
+// time: gate | up of the 8B model 689 -> 746 us at 2,048 rows, down 450 -> 516 us.  A third set of sums in turn for Q6_K took
+// 490 us for down by itself, and a chunk as long as before; reads of 16 columns at a time, or sums handed back before the
+// reads, changed nothing; both halves' A operand resident, with the minima folded first in the products' columns, took
+// 917 us for gate | up.  Q8_0's one sum per tile, 8.4e-7, replaced one over all inputs.)  The F32 sums of a work item
 // (2 x 128 x 128) live in the registers of sixteen warps.
 // Roles of the 28 warps: 0..15 fold and store (one row of each unit and 32 columns per thread), 16..23 convert (two row
 // tiles, half of a stage), 24 / 26 copy weights / activations, 25 issues MMAs.  Every wait is bounded.
