@@ -63,6 +63,7 @@ struct AttnArgs {
     int run_tokens;            // up to this many consecutive tokens of a sequence share one item (prefill launches); 1: none
     int run_first, run_count;  // host side: tokens [run_first, run_first + run_count) are consecutive tokens of one sequence; -1: unknown
     float* partial;
+    int* error_flag;           // of the tensor-memory kernel's bounded waits
     float* out;                // [T][q_heads][HD]
     ActOperand operand;        // optional operand form of `out`, K = q_heads * HD
 };
@@ -923,6 +924,17 @@ cudaError_t launch_hd(cudaStream_t stream, AttnArgs a, bool fused, int n_tokens,
     const int warp_tokens = std::max(1, 16 / q_per_kv), cta_tokens = kMmaWarps * warp_tokens;
     if (!fused && a.window <= 0 && a.operand.dig == nullptr && a.run_first >= 0 && a.run_count >= 64 &&
         a.run_first + a.run_count <= n_tokens) {
+        if (HD == 128) {
+            const PrefillAttention p{a.q, a.cache_k, a.cache_v, a.page_tables, a.pages_per_sequence, a.token_seq, a.token_pos,
+                                     a.run_first, a.run_count, a.q_heads, a.kv_heads, a.out, a.error_flag};
+            cudaError_t e = launch_attention_tc(stream, p);
+            if (e != cudaSuccess) return e;
+            if (launches) ++*launches;
+            const int behind = a.run_first + a.run_count;
+            if (a.run_first > 0) e = launch_spans_hd<HD>(stream, a, fused, 0, a.run_first, max_keys, partial_bytes, launches, programmatic);
+            if (e == cudaSuccess && behind < n_tokens) e = launch_spans_hd<HD>(stream, a, fused, behind, n_tokens - behind, max_keys, partial_bytes, launches, programmatic);
+            return e;
+        }
         const int aligned = a.run_count / cta_tokens * cta_tokens;
         const bool wide = warp_tokens * q_per_kv > 8;
         const size_t smem = (size_t)(kMmaWarps * 2 * 8 * (wide ? 2 : 1) + 2 * kMmaWarps * 2 * kMmaKeys) * (HD + 8) * sizeof(__half);
@@ -969,7 +981,7 @@ cudaError_t launch_attention(cudaStream_t stream, const float* q, const __half* 
                              const int32_t* page_tables, int pages_per_sequence, const int32_t* token_seq,
                              const int32_t* token_pos, int n_tokens, int q_heads, int kv_heads, int head_dim,
                              int window, int max_keys, float* partial, size_t partial_bytes, float* out,
-                             int* launches, int run_first, int run_count) {
+                             int* launches, int run_first, int run_count, int* error_flag) {
     if (n_tokens <= 0) return cudaSuccess;
     if (q_heads % kv_heads != 0 || q_heads / kv_heads > 16 || max_keys <= 0) return cudaErrorInvalidValue;
     if (head_dim == 32) {
@@ -994,6 +1006,7 @@ cudaError_t launch_attention(cudaStream_t stream, const float* q, const __half* 
     a.partial = partial;
     a.out = out;
     a.run_first = run_first; a.run_count = run_count;
+    a.error_flag = error_flag;
     return dispatch(stream, a, false, head_dim, n_tokens, max_keys, partial_bytes, launches);
 }
 

@@ -1,0 +1,390 @@
+// Attention of a prefill chunk on the tcgen05 tensor cores: consecutive tokens of one sequence against the paged cache.
+//
+// A CTA serves one kv head and two tiles of 128 query rows (row = token x query head of the group), each with its own
+// softmax warps, so that one tile's products run while the other's probabilities are formed.  Per 128 keys and tile:
+//   S = Q K^T   A = Q as binary16 hi + lo in shared memory (converted once), B = the K rows as they lie in the cache: two
+//               products per element, lo first, F32 sums in tensor memory;
+//   P           a thread owns a row: online softmax in base 2, P as binary16 hi + lo written over S in tensor memory;
+//   O += P V    A = P from tensor memory, B = the V rows (the same core matrices, read with the other major order).
+// Q, the probabilities and the sums keep the precision of the span kernels (attention.cu).  A row's reference maximum only
+// moves when a tile's maximum passes it by 2^8 in the exponent, which binary16 pairs and F32 sums hold with the same
+// relative precision; then the row's sums are rescaled where they lie.  Key tiles begin at multiples of 128, and a row's
+// bits depend on its own keys only.
+//
+// What bounds it: the products, 2 x (1,024 + 1,024) clocks per 128 keys and CTA; the shared-memory operand reads of Q K^T
+// (128 bytes per clock) run beside one tile's softmax of about 700 instructions per row.
+// Roles of the 12 warps: 0..3 / 4..7 softmax and output of tile 0 / 1, 8 issues the products, 9..11 copy K / V tiles (keys
+// past the chunk's last one are zero, so that a zero probability meets no NaN).  Every wait is bounded.
+#include <cuda_fp16.h>
+#include <math.h>
+
+#include <algorithm>
+
+#include "kernels.cuh"
+#include "tmem.cuh"
+
+namespace ribn {
+
+namespace {
+
+constexpr int kHd = 128, kRows = 128, kKeys = 128;
+constexpr int kPieceBytes = 128 * 16;                 // one 8-dimension column of 128 rows or keys
+constexpr int kTileBytes = kHd / 8 * kPieceBytes;     // 128 x 128 binary16: 32 KB
+constexpr int kSlots = 3;                             // K / V tiles in shared memory: K0 V0 K1 V1 ..
+constexpr int kSoftmaxWarps = 8, kMmaWarp = 8, kLoadWarp0 = 9, kLoadWarps = 3, kThreads = 12 * 32;
+constexpr size_t kSmem = 4 * kTileBytes + kSlots * kTileBytes + 128;
+constexpr uint32_t kSpinLimit = 1u << 22;
+constexpr float kLog2e = 1.4426950408889634f;
+constexpr float kSlack = 8.0f;                        // the reference maximum may lag by 2^8
+// Register shares: 384 x 168 at launch (64,512); softmax 256 x 208, the others 128 x 88.
+constexpr int kSoftmaxRegs = 208, kOtherRegs = 88;
+
+// B = V: rows are keys (the products' K), 16 bytes of a row are eight of its dimensions (N): N-major core matrices
+constexpr uint32_t kIdescQk = umma_idesc(kKeys), kIdescPv = umma_idesc(kHd) | (1u << 16);
+constexpr uint32_t kDescHighPv = ((uint32_t)kPieceBytes >> 4) | (1u << 14);
+__device__ __forceinline__ void umma_pv(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_desc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "mov.b64 b, {%2, %6};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, {%5, %5, %5, %5}, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "r"(b_desc), "r"(kIdescPv), "r"(accumulate), "r"(0u), "r"(kDescHighPv) : "memory");
+}
+
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,"
+        "%29,%30,%31}, [%32];"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]),
+          "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]), "=f"(v[16]), "=f"(v[17]), "=f"(v[18]), "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]),
+          "=f"(v[23]), "=f"(v[24]), "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31])
+        : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_tie32(float* v) {   // the values of a load, after its wait
+#pragma unroll
+    for (int i = 0; i < 32; i += 8) {
+        asm volatile("" : "+f"(v[i]), "+f"(v[i + 1]), "+f"(v[i + 2]), "+f"(v[i + 3]), "+f"(v[i + 4]), "+f"(v[i + 5]), "+f"(v[i + 6]), "+f"(v[i + 7]) :: "memory");
+    }
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
+                 "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]),
+                 "r"(r[14]), "r"(r[15]) : "memory");
+}
+__device__ __forceinline__ float exp2_approx(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// x0, x1 = hi + lo as binary16 pairs
+__device__ __forceinline__ void split2(float x0, float x1, uint32_t& hi, uint32_t& lo) {
+    const __half2 h = __floats2half2_rn(x0, x1);
+    const float2 back = __half22float2(h), rest = __fadd2_rn(make_float2(x0, x1), make_float2(-back.x, -back.y));
+    hi = as_bits(h);
+    lo = as_bits(__floats2half2_rn(rest.x, rest.y));
+}
+__device__ __forceinline__ void sts128(uint32_t addr, uint4 v) {
+    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+
+__global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const PrefillAttention a, const int tile_tokens) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
+    const uint32_t q_at = smem_u32(smem), ring = q_at + 4 * kTileBytes, bars = ring + kSlots * kTileBytes;
+    const uint32_t q_full = bars, s_full = bars + 16, p_full = bars + 32, o_full = bars + 48, kv_full = bars + 64, kv_empty = bars + 88, tmem_slot = bars + 112;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(q_full + 8 * i, kSoftmaxWarps / 2); mbar_init(s_full + 8 * i, 1); mbar_init(p_full + 8 * i, kSoftmaxWarps / 2); mbar_init(o_full + 8 * i, 1);
+        }
+        for (int i = 0; i < kSlots; ++i) { mbar_init(kv_full + 8 * i, kLoadWarps); mbar_init(kv_empty + 8 * i, 1); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == kMmaWarp) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = lds32(tmem_slot);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
+    // the tile pairs with the most keys first
+    const int q_per_kv = a.q_heads / a.kv_heads, pairs = (int)gridDim.x / a.kv_heads;
+    const int pair = pairs - 1 - (int)blockIdx.x / a.kv_heads, kvh = (int)blockIdx.x % a.kv_heads;
+    const int pos0 = a.token_pos[a.first];
+    int local[2], tokens[2], n[2];   // a tile's first token inside the chunk, its tokens, its key tiles
+    for (int t = 0; t < 2; ++t) {
+        local[t] = (2 * pair + t) * tile_tokens;
+        tokens[t] = max(0, min(tile_tokens, a.count - local[t]));
+        n[t] = tokens[t] > 0 ? (pos0 + local[t] + tokens[t] - 1) / kKeys + 1 : 0;
+    }
+    const int n_tiles = max(n[0], n[1]);
+    bool alive = true;
+
+    if (warp >= kMmaWarp) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
+        if (warp == kMmaWarp) {
+            // ---------------- products (the warp as a whole, one elected lane in it) ----------------
+            const bool leader = elect_one();
+            const uint32_t q_desc = umma_desc(q_at, kPieceBytes), k_desc = umma_desc(ring, kPieceBytes), v_desc = umma_desc(ring, 128);
+            auto slot_wait = [&](int idx) {
+                if (alive) alive = mbar_wait(kv_full + 8 * (idx % kSlots), (uint32_t)(idx / kSlots) & 1u, a.error_flag, 121, kSpinLimit);
+            };
+            auto scores = [&](int t, int j) {
+                slot_wait(2 * j);
+                tc_fence_after();
+                const uint32_t b = k_desc + (2 * j % kSlots) * (kTileBytes >> 4), hi = q_desc + 2 * t * (kTileBytes >> 4), lo = hi + (kTileBytes >> 4);
+                if (leader) {
+#pragma unroll
+                    for (int i = 0; i < kHd / 16; ++i) umma_ss(tmem + 128 * t, lo + i * (2 * kPieceBytes >> 4), b + i * (2 * kPieceBytes >> 4), kIdescQk, (uint32_t)(i != 0));
+#pragma unroll
+                    for (int i = 0; i < kHd / 16; ++i) umma_ss(tmem + 128 * t, hi + i * (2 * kPieceBytes >> 4), b + i * (2 * kPieceBytes >> 4), kIdescQk, 1u);
+                    umma_commit(s_full + 8 * t);
+                }
+            };
+            for (int t = 0; t < 2; ++t) {
+                if (n[t] == 0) continue;
+                if (alive) alive = mbar_wait(q_full + 8 * t, 0, a.error_flag, 122, kSpinLimit);
+                scores(t, 0);
+            }
+            if (leader) umma_commit(kv_empty);
+            for (int j = 0; j < n_tiles; ++j) {
+                const int v_slot = (2 * j + 1) % kSlots, k_next = (2 * j + 2) % kSlots;
+#pragma unroll 1
+                for (int t = 0; t < 2; ++t) {
+                    if (j < n[t]) {
+                        if (alive) alive = mbar_wait(p_full + 8 * t, (uint32_t)j & 1u, a.error_flag, 123, kSpinLimit);
+                        slot_wait(2 * j + 1);
+                        tc_fence_after();
+                        if (leader) {
+                            const uint32_t p_at = tmem + 128 * t, o_at = tmem + 256 + 128 * t, b = v_desc + v_slot * (kTileBytes >> 4);
+#pragma unroll
+                            for (int i = 0; i < kKeys / 16; ++i) umma_pv(o_at, p_at + 64 + 8 * i, b + i * (256 >> 4), (uint32_t)(j != 0 || i != 0));
+#pragma unroll
+                            for (int i = 0; i < kKeys / 16; ++i) umma_pv(o_at, p_at + 8 * i, b + i * (256 >> 4), 1u);
+                            if (j + 1 == n[t]) umma_commit(o_full + 8 * t);
+                        }
+                    }
+                    if (t == 1 && leader) umma_commit(kv_empty + 8 * v_slot);
+                    if (j + 1 < n[t]) scores(t, j + 1);   // over the probabilities that the products above have read
+                    if (t == 1 && j + 1 < n_tiles && leader) umma_commit(kv_empty + 8 * k_next);
+                }
+            }
+            if (!alive) {
+                // let what was issued come to its end before the block can
+                if (leader) umma_commit(q_full);
+                for (uint32_t p = 0; p < 2; ++p) mbar_wait(q_full, p, nullptr, 0, 1u << 16);
+            }
+        } else {
+            // ---------------- K / V tiles: lane = (key of a group of eight, 16-byte piece of four) ----------------
+            const int lw = warp - kLoadWarp0, sub = lane >> 2, last = pos0 + local[0] + tokens[0] + tokens[1] - 1;
+            const int32_t* table = a.page_tables + (long long)(a.token_seq != nullptr ? a.token_seq[a.first] : 0) * a.pages_per_sequence;
+            const long long stride = (long long)a.kv_heads * kHd;
+            constexpr int kGroups = (kKeys / 8 + kLoadWarps - 1) / kLoadWarps;
+            long long rows[kGroups];   // cache rows of this lane's keys of a key tile
+            auto look_up = [&](int j) {
+#pragma unroll
+                for (int i = 0; i < kGroups; ++i) {
+                    const int key = j * kKeys + (lw + i * kLoadWarps) * 8 + sub;
+                    rows[i] = lw + i * kLoadWarps < kKeys / 8 && key <= last ? (long long)table[key / kPageTokens] * kPageTokens + key % kPageTokens : -1;
+                }
+            };
+            auto copy = [&](int idx) {
+                if ((idx & 1) == 0) look_up(idx >> 1);
+                const __half* from = ((idx & 1) ? a.cache_v : a.cache_k) + (long long)kvh * kHd + (lane & 3) * 8;
+                const uint32_t to = ring + (idx % kSlots) * kTileBytes + (lane & 3) * kPieceBytes + (lw * 8 + sub) * 16;
+#pragma unroll
+                for (int i = 0; i < kGroups; ++i) {
+                    if (lw + i * kLoadWarps >= kKeys / 8) break;
+                    const __half* src = from + (rows[i] < 0 ? 0 : rows[i] * stride);
+                    const uint32_t bytes = rows[i] < 0 ? 0u : 16u;   // nothing read, zeros written
+#pragma unroll
+                    for (int p = 0; p < 4; ++p) {
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + i * (kLoadWarps * 128) + p * (4 * kPieceBytes)), "l"(src + p * 32), "r"(bytes) : "memory");
+                    }
+                }
+                asm volatile("cp.async.commit_group;" ::: "memory");
+            };
+            auto landed = [&](int idx) {
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(kv_full + 8 * (idx % kSlots));
+            };
+            const int total = 2 * n_tiles;   // even, at least 2
+            copy(0);
+            copy(1);
+            if (total > 2) copy(2); else asm volatile("cp.async.commit_group;" ::: "memory");
+            asm volatile("cp.async.wait_group 2;" ::: "memory");
+            landed(0);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            landed(1);
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            if (total > 2) landed(2);
+            for (int idx = 3; idx < total; ++idx) {
+                if (alive) alive = mbar_wait(kv_empty + 8 * (idx % kSlots), (uint32_t)(idx / kSlots - 1) & 1u, a.error_flag, 124, kSpinLimit);
+                copy(idx);
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+                landed(idx);
+            }
+        }
+    } else {
+        // ---------------- softmax: one row per thread ----------------
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegs));
+        const int t = warp >> 2, quadrant = warp & 3, row0 = quadrant * 32, row = row0 + lane;
+        const uint32_t q_tile = q_at + 2 * t * kTileBytes;
+        const int live_rows = tokens[t] * q_per_kv;
+        if (n[t] > 0) {
+            {
+                // the warp's 32 query rows as hi + lo: lane = (row of eight, 8-dimension piece of four)
+                const int sub = lane & 7, pc = lane >> 3;
+#pragma unroll 1
+                for (int rg = 0; rg < 4; ++rg) {
+                    const int r = row0 + rg * 8 + sub;
+                    const bool have = r < live_rows;
+                    const float* from = a.q + ((long long)(a.first + local[t] + (have ? r / q_per_kv : 0)) * a.q_heads + kvh * q_per_kv + (have ? r % q_per_kv : 0)) * kHd + pc * 8;
+                    float4 x[4][2];
+#pragma unroll
+                    for (int p = 0; p < 4; ++p) {
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) x[p][h] = have ? *reinterpret_cast<const float4*>(from + p * 32 + 4 * h) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    }
+#pragma unroll
+                    for (int p = 0; p < 4; ++p) {
+                        uint4 hi, lo;
+                        split2(x[p][0].x, x[p][0].y, hi.x, lo.x); split2(x[p][0].z, x[p][0].w, hi.y, lo.y);
+                        split2(x[p][1].x, x[p][1].y, hi.z, lo.z); split2(x[p][1].z, x[p][1].w, hi.w, lo.w);
+                        const uint32_t to = q_tile + (p * 4 + pc) * kPieceBytes + r * 16;
+                        sts128(to, hi);
+                        sts128(to + kTileBytes, lo);
+                    }
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(q_full + 8 * t);
+            }
+            const float c = kLog2e / sqrtf((float)kHd);
+            const int limit = row < live_rows ? pos0 + local[t] + row / q_per_kv : -1;   // the row's last key
+            const int warp_limit = row0 + 31 < live_rows ? pos0 + local[t] + row0 / q_per_kv : -1;   // keys that every row of the warp sees
+            const uint32_t lanes = (uint32_t)row0 << 16, s_at = tmem + lanes + 128 * t, o_at = s_at + 256;
+            float m = -INFINITY;
+            float2 l = make_float2(0.0f, 0.0f);
+            for (int j = 0; j < n[t]; ++j) {
+                if (alive) alive = mbar_wait(s_full + 8 * t, (uint32_t)j & 1u, a.error_flag, 125, kSpinLimit);
+                tc_fence_after();
+                float s[kKeys];
+#pragma unroll
+                for (int i = 0; i < kKeys; i += 32) tmem_ld32(s_at + i, s + i);
+                tmem_wait_ld();
+#pragma unroll
+                for (int i = 0; i < kKeys; i += 32) tmem_tie32(s + i);
+                if (j * kKeys + kKeys - 1 > warp_limit) {
+                    const int see = limit - j * kKeys;
+#pragma unroll
+                    for (int i = 0; i < kKeys; ++i) s[i] = i <= see ? s[i] : -INFINITY;
+                }
+                float top[4] = {s[0], s[1], s[2], s[3]};
+#pragma unroll
+                for (int i = 4; i < kKeys; i += 8) {
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) top[u] = i + 4 + u < kKeys ? fmaxf(top[u], fmaxf(s[i + u], s[i + 4 + u])) : fmaxf(top[u], s[i + u]);
+                }
+                const float mx = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3]));
+                const bool moves = mx > m && (m == -INFINITY || (mx - m) * c > kSlack);
+                if (__any_sync(0xffffffffu, moves)) {
+                    // (the scores' barrier also says that the products into O so far are complete)
+                    const float f = moves ? (m == -INFINITY ? 0.0f : exp2_approx((m - mx) * c)) : 1.0f;
+                    if (moves) m = mx;
+                    l.x *= f; l.y *= f;
+                    if (j > 0) {
+#pragma unroll 1
+                        for (int i = 0; i < kHd; i += 16) {
+                            float o[2][8];
+                            tmem_ld8(o_at + i, o[0]);
+                            tmem_ld8(o_at + i + 8, o[1]);
+                            tmem_wait_ld();
+                            tmem_tie(o[0]);
+                            tmem_tie(o[1]);
+                            uint32_t r[16];
+#pragma unroll
+                            for (int u = 0; u < 16; ++u) r[u] = __float_as_uint(o[u >> 3][u & 7] * f);
+                            tmem_st16(o_at + i, r);
+                        }
+                    }
+                }
+                const float mc = m == -INFINITY ? 0.0f : m * c;
+#pragma unroll
+                for (int i = 0; i < kKeys; i += 32) {
+                    uint32_t hi[16], lo[16];
+#pragma unroll
+                    for (int u = 0; u < 16; ++u) {
+                        const float2 x = __ffma2_rn(make_float2(s[i + 2 * u], s[i + 2 * u + 1]), make_float2(c, c), make_float2(-mc, -mc));
+                        const float2 p = make_float2(exp2_approx(x.x), exp2_approx(x.y));
+                        l = __fadd2_rn(l, p);
+                        split2(p.x, p.y, hi[u], lo[u]);
+                    }
+                    tmem_st16(s_at + i / 2, hi);
+                    tmem_st16(s_at + 64 + i / 2, lo);
+                }
+                tmem_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(p_full + 8 * t);
+            }
+            if (alive) alive = mbar_wait(o_full + 8 * t, 0, a.error_flag, 126, kSpinLimit);
+            tc_fence_after();
+            // rows to memory as whole lines, through the shared memory that the queries have left (a warp's own 16 KB)
+            const float total = l.x + l.y;
+            const uint32_t stage = q_tile + row0 * (kHd * 4);
+#pragma unroll 1
+            for (int i = 0; i < kHd; i += 32) {
+                float o[32];
+                tmem_ld32(o_at + i, o);
+                tmem_wait_ld();
+                tmem_tie32(o);
+#pragma unroll
+                for (int u = 0; u < 32; u += 4) {
+                    const uint4 v = make_uint4(__float_as_uint(o[u] / total), __float_as_uint(o[u + 1] / total), __float_as_uint(o[u + 2] / total), __float_as_uint(o[u + 3] / total));
+                    sts128(stage + lane * (kHd * 4) + ((((i + u) >> 2) ^ (lane & 7)) << 4), v);
+                }
+            }
+            __syncwarp();
+#pragma unroll 4
+            for (int r = 0; r < 32; ++r) {
+                if (row0 + r >= live_rows) break;
+                const uint4 v = lds128(stage + r * (kHd * 4) + ((lane ^ (r & 7)) << 4));
+                const int rr = row0 + r;
+                float* to = a.out + ((long long)(a.first + local[t] + rr / q_per_kv) * a.q_heads + kvh * q_per_kv + rr % q_per_kv) * kHd;
+                *reinterpret_cast<uint4*>(to + lane * 4) = v;
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == kMmaWarp) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    }
+}
+
+}  // namespace
+
+cudaError_t launch_attention_tc(cudaStream_t stream, const PrefillAttention& a) {
+    if (a.count <= 0 || a.q_heads % a.kv_heads != 0 || a.q_heads / a.kv_heads > 16) return cudaErrorInvalidValue;
+    static bool configured[kMaxDevices] = {false};   // function attributes are per device
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
+    if (!configured[dev]) {
+        e = cudaFuncSetAttribute(attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+        if (e != cudaSuccess) return e;
+        configured[dev] = true;
+    }
+    const int tile_tokens = kRows / (a.q_heads / a.kv_heads), pairs = (a.count + 2 * tile_tokens - 1) / (2 * tile_tokens);
+    attention_tc_kernel<<<dim3((unsigned)(pairs * a.kv_heads)), kThreads, kSmem, stream>>>(a, tile_tokens);
+    return cudaGetLastError();
+}
+
+}  // namespace ribn

@@ -248,7 +248,7 @@ cudaError_t run_layers_reference(ribn_b200_executor* ex, const StepPlan& plan, i
             cudaError_t e = launch_attention(s, ex->q, ck, cv, ex->d_page_tables, ex->pages_per_sequence,
                                              ex->meta.token_seq, ex->meta.token_pos, T, c.q_heads, c.kv_heads,
                                              c.head_dim, 0, plan.max_keys, ex->scratch.attn_partial,
-                                             ex->scratch.attn_partial_bytes, ex->attn, &launches, plan.run_first, plan.run_count);
+                                             ex->scratch.attn_partial_bytes, ex->attn, &launches, plan.run_first, plan.run_count, ex->d_error);
             if (e != cudaSuccess) return e;
         }
         if (ex->tp > 1) {
@@ -402,7 +402,7 @@ cudaError_t run_attention(ribn_b200_executor* ex, const StepPlan& plan, int l, b
                                         ex->meta.token_pos, ex->meta.token_slot, T, c.q_heads, c.kv_heads, c.head_dim, c.rms_eps, ck, cv));
     return launch_attention(s, ex->q, ck, cv, ex->d_page_tables, ex->pages_per_sequence, ex->meta.token_seq, ex->meta.token_pos, T, c.q_heads,
                             c.kv_heads, c.head_dim, 0, plan.max_keys, ex->scratch.attn_partial, ex->scratch.attn_partial_bytes, ex->attn,
-                            &launches, plan.run_first, plan.run_count);
+                            &launches, plan.run_first, plan.run_count, ex->d_error);
 }
 
 cudaError_t run_layers_decode(ribn_b200_executor* ex, const StepPlan& plan, int& launches) {

@@ -110,7 +110,23 @@ cudaError_t launch_attention(cudaStream_t stream, const float* q, const __half* 
                              const int32_t* page_tables, int pages_per_sequence, const int32_t* token_seq,
                              const int32_t* token_pos, int n_tokens, int q_heads, int kv_heads, int head_dim,
                              int window, int max_keys, float* partial, size_t partial_bytes, float* out,
-                             int* launches, int run_first = -1, int run_count = 0);
+                             int* launches, int run_first = -1, int run_count = 0, int* error_flag = nullptr);
+
+// Attention of `count` consecutive tokens of one sequence from token `first` on (attention_tc.cu, head width 128): q as for
+// launch_attention, tokens at consecutive positions.
+struct PrefillAttention {
+    const float* q;
+    const __half* cache_k;
+    const __half* cache_v;
+    const int32_t* page_tables;
+    int pages_per_sequence;
+    const int32_t* token_seq;   // may be null: sequence 0
+    const int32_t* token_pos;
+    int first, count, q_heads, kv_heads;
+    float* out;
+    int* error_flag;            // set non-zero when a bounded wait gives up
+};
+cudaError_t launch_attention_tc(cudaStream_t stream, const PrefillAttention& args);
 
 // Decode form of the same attention for rows that add exactly one token: it
 // also applies the per-head Q/K RMSNorm and rotary to the raw projections,

@@ -588,9 +588,14 @@ int ribn_b200_op_attention(int32_t device, const float* q, const uint16_t* keys,
         const size_t per_row = (size_t)q_heads * spans * (head_dim + 2) * sizeof(float);
         const size_t bytes = std::max(per_row, std::min(per_row * (size_t)rows, (size_t)256 << 20));
         float* d_partial = s.alloc<float>(bytes / sizeof(float));
-        OP_PTR(d_partial);
+        int* d_err = s.alloc<int>(1);
+        OP_PTR(d_partial); OP_PTR(d_err);
+        OP_TRY(cudaMemsetAsync(d_err, 0, sizeof(int), s.stream));
         OP_TRY(launch_attention(s.stream, d_q, d_k, d_v, d_table, pages, d_seq, d_pos, rows, q_heads, kv_heads,
-                                head_dim, window, tokens, d_partial, bytes, d_o, nullptr, 0, rows));
+                                head_dim, window, tokens, d_partial, bytes, d_o, nullptr, 0, rows, d_err));
+        int err = 0;
+        if (!s.download(&err, d_err, 1)) return op_fail("attention", cudaGetLastError());
+        if (err != 0) return op_fail("attention: a bounded wait expired", cudaSuccess);
     }
     return s.download(out, d_o, (size_t)rows * q_heads * head_dim) ? RIBN_B200_OK : RIBN_B200_ERROR;
 }

@@ -367,3 +367,29 @@ def test_decode_attention_at_long_contexts(ops, QH, KVH, HD, tokens):
     assert np.array_equal(results[0].view(np.uint32), results[1].view(np.uint32))
     want = orc.attention(q, k.view(np.uint16).reshape(-1), v.view(np.uint16).reshape(-1), tokens, QH, KVH, HD)
     assert np.max(np.abs(results[0] - want)) < 1e-4
+
+
+@pytest.mark.parametrize("QH,KVH,tokens,rows", [(32, 8, 64, 64), (32, 8, 65, 65), (32, 8, 193, 129), (16, 8, 257, 257), (12, 4, 300, 171),
+                                                (8, 8, 400, 400), (16, 1, 130, 100)])
+def test_prefill_chunk_attention_at_the_edges_of_its_tiles(ops, QH, KVH, tokens, rows):
+    """The tensor-memory prefill kernel (head width 128): chunks that end inside a query tile, a key tile and a page, with
+    and without a cached prefix, group sizes 1 to 16 (3: rows of a tile that belong to no token).  Slots of the last page that
+    hold no key carry NaN: nothing may read them.  Scores and probabilities are binary16 hi + lo pairs (22 bits) with F32
+    sums: an error of |q| |k| 2^-22 in a score of a few units, 2e-6 of a result, with room for the sums."""
+    HD = 128
+    rng = np.random.default_rng(tokens * 31 + rows)
+    q = rng.normal(0, 1, size=(rows, QH * HD)).astype(np.float32)
+    k = rng.normal(0, 1, size=(tokens, KVH * HD)).astype(np.float16).view(np.uint16)
+    v = rng.normal(0, 1, size=(tokens, KVH * HD)).astype(np.float16).view(np.uint16)
+    pages = (tokens + 15) // 16
+    results = []
+    for table in (np.arange(pages), rng.permutation(pages)):
+        pk = np.full((pages * 16, KVH * HD), 0x7E00, dtype=np.uint16); pv = pk.copy()
+        order = table[np.arange(tokens) // 16] * 16 + np.arange(tokens) % 16
+        pk[order] = k; pv[order] = v
+        results.append(ops.attention(q, pk, pv, table, tokens, rows, QH, KVH, HD, variant=0))
+    assert np.array_equal(results[0].view(np.uint32), results[1].view(np.uint32))
+    for r in sorted({0, 1, rows // 2, rows - 2, rows - 1} | set(range(0, rows, 37))):
+        seen = tokens - rows + 1 + r
+        want = orc.attention(q[r], k.reshape(-1)[: seen * KVH * HD], v.reshape(-1)[: seen * KVH * HD], seen, QH, KVH, HD)
+        assert np.max(np.abs(results[0][r] - want)) < 1e-5, r
