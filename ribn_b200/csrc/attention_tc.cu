@@ -4,15 +4,19 @@
 // softmax warps, so that one tile's products run while the other's probabilities are formed.  Per 128 keys and tile:
 //   S = Q K^T   A = Q as binary16 hi + lo in shared memory (converted once), B = the K rows as they lie in the cache: two
 //               products per element, lo first, F32 sums in tensor memory;
-//   P           a thread owns a row: online softmax in base 2, P as binary16 hi + lo written over S in tensor memory;
+//   P           a thread owns a row: online softmax in base 2, P as binary16 hi + lo written over S in tensor memory (32 keys
+//               of S become 16 columns of hi and 16 of lo);
 //   O += P V    A = P from tensor memory, B = the V rows (the same core matrices, read with the other major order).
 // Q, the probabilities and the sums keep the precision of the span kernels (attention.cu).  A row's reference maximum only
 // moves when a tile's maximum passes it by 2^8 in the exponent, which binary16 pairs and F32 sums hold with the same
 // relative precision; then the row's sums are rescaled where they lie.  Key tiles begin at multiples of 128, and a row's
 // bits depend on its own keys only.
 //
-// What bounds it: the products, 2 x (1,024 + 1,024) clocks per 128 keys and CTA; the shared-memory operand reads of Q K^T
-// (128 bytes per clock) run beside one tile's softmax of about 700 instructions per row.
+// What bounds it: the products, 2 x (1,024 + 1,024) clocks per 128 keys and CTA, which take about 5,200: those of Q K^T read
+// both operands from shared memory, 128 bytes per clock, beside the copies.  A tile's softmax takes 2,400 clocks beside
+// the other's products.  8B model, 2,048 tokens without prefix: 90 us a layer, against 372 us of the mma.sync kernel that
+// attention.cu keeps for other head widths (0.6B model, 777 tokens: 37 against 64 us, and no spans for the last 9).  All 128
+// scores of a row in registers: 93 us; the next 32 scores requested under the present ones' arithmetic: 91 us.
 // Roles of the 12 warps: 0..3 / 4..7 softmax and output of tile 0 / 1, 8 issues the products, 9..11 copy K / V tiles (keys
 // past the chunk's last one are zero, so that a zero probability meets no NaN).  Every wait is bounded.
 #include <cuda_fp16.h>
@@ -51,7 +55,7 @@ __device__ __forceinline__ void umma_pv(uint32_t d_tmem, uint32_t a_tmem, uint32
         ::"r"(d_tmem), "r"(a_tmem), "r"(b_desc), "r"(kIdescPv), "r"(accumulate), "r"(0u), "r"(kDescHighPv) : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,"
         "%29,%30,%31}, [%32];"
@@ -60,7 +64,7 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
           "=f"(v[23]), "=f"(v[24]), "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31])
         : "r"(taddr));
 }
-__device__ __forceinline__ void tmem_tie32(float* v) {   // the values of a load, after its wait
+__device__ __forceinline__ void tmem_tie32(float (&v)[32]) {   // the values of a load, after its wait
 #pragma unroll
     for (int i = 0; i < 32; i += 8) {
         asm volatile("" : "+f"(v[i]), "+f"(v[i + 1]), "+f"(v[i + 2]), "+f"(v[i + 3]), "+f"(v[i + 4]), "+f"(v[i + 5]), "+f"(v[i + 6]), "+f"(v[i + 7]) :: "memory");
@@ -82,6 +86,11 @@ __device__ __forceinline__ void split2(float x0, float x1, uint32_t& hi, uint32_
     const float2 back = __half22float2(h), rest = __fadd2_rn(make_float2(x0, x1), make_float2(-back.x, -back.y));
     hi = as_bits(h);
     lo = as_bits(__floats2half2_rn(rest.x, rest.y));
+}
+// keys past the row's last one
+__device__ __forceinline__ void mask_keys(float (&s)[32], int see) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) s[i] = i <= see ? s[i] : -INFINITY;
 }
 __device__ __forceinline__ void sts128(uint32_t addr, uint4 v) {
     asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
@@ -161,9 +170,9 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const Prefill
                         if (leader) {
                             const uint32_t p_at = tmem + 128 * t, o_at = tmem + 256 + 128 * t, b = v_desc + v_slot * (kTileBytes >> 4);
 #pragma unroll
-                            for (int i = 0; i < kKeys / 16; ++i) umma_pv(o_at, p_at + 64 + 8 * i, b + i * (256 >> 4), (uint32_t)(j != 0 || i != 0));
+                            for (int i = 0; i < kKeys / 16; ++i) umma_pv(o_at, p_at + 32 * (i >> 1) + 8 * (i & 1) + 16, b + i * (256 >> 4), (uint32_t)(j != 0 || i != 0));
 #pragma unroll
-                            for (int i = 0; i < kKeys / 16; ++i) umma_pv(o_at, p_at + 8 * i, b + i * (256 >> 4), 1u);
+                            for (int i = 0; i < kKeys / 16; ++i) umma_pv(o_at, p_at + 32 * (i >> 1) + 8 * (i & 1), b + i * (256 >> 4), 1u);
                             if (j + 1 == n[t]) umma_commit(o_full + 8 * t);
                         }
                     }
@@ -183,7 +192,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const Prefill
             const int32_t* table = a.page_tables + (long long)(a.token_seq != nullptr ? a.token_seq[a.first] : 0) * a.pages_per_sequence;
             const long long stride = (long long)a.kv_heads * kHd;
             constexpr int kGroups = (kKeys / 8 + kLoadWarps - 1) / kLoadWarps;
-            long long rows[kGroups];   // cache rows of this lane's keys of a key tile
+            long long rows[kGroups];   // cache rows of this lane's keys of the next key tile to copy (K, then V)
             auto look_up = [&](int j) {
 #pragma unroll
                 for (int i = 0; i < kGroups; ++i) {
@@ -192,7 +201,6 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const Prefill
                 }
             };
             auto copy = [&](int idx) {
-                if ((idx & 1) == 0) look_up(idx >> 1);
                 const __half* from = ((idx & 1) ? a.cache_v : a.cache_k) + (long long)kvh * kHd + (lane & 3) * 8;
                 const uint32_t to = ring + (idx % kSlots) * kTileBytes + (lane & 3) * kPieceBytes + (lw * 8 + sub) * 16;
 #pragma unroll
@@ -206,6 +214,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const Prefill
                     }
                 }
                 asm volatile("cp.async.commit_group;" ::: "memory");
+                if (idx & 1) look_up((idx >> 1) + 1);   // under the copies
             };
             auto landed = [&](int idx) {
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -213,6 +222,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const Prefill
                 if (lane == 0) mbar_arrive(kv_full + 8 * (idx % kSlots));
             };
             const int total = 2 * n_tiles;   // even, at least 2
+            look_up(0);
             copy(0);
             copy(1);
             if (total > 2) copy(2); else asm volatile("cp.async.commit_group;" ::: "memory");
@@ -239,23 +249,27 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const Prefill
             {
                 // the warp's 32 query rows as hi + lo: lane = (row of eight, 8-dimension piece of four)
                 const int sub = lane & 7, pc = lane >> 3;
-#pragma unroll 1
+                float4 x[4][4][2];   // everything in flight together
+#pragma unroll
                 for (int rg = 0; rg < 4; ++rg) {
                     const int r = row0 + rg * 8 + sub;
                     const bool have = r < live_rows;
                     const float* from = a.q + ((long long)(a.first + local[t] + (have ? r / q_per_kv : 0)) * a.q_heads + kvh * q_per_kv + (have ? r % q_per_kv : 0)) * kHd + pc * 8;
-                    float4 x[4][2];
 #pragma unroll
                     for (int p = 0; p < 4; ++p) {
 #pragma unroll
-                        for (int h = 0; h < 2; ++h) x[p][h] = have ? *reinterpret_cast<const float4*>(from + p * 32 + 4 * h) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                        for (int h = 0; h < 2; ++h) x[rg][p][h] = have ? *reinterpret_cast<const float4*>(from + p * 32 + 4 * h) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     }
+                }
+#pragma unroll
+                for (int rg = 0; rg < 4; ++rg) {
 #pragma unroll
                     for (int p = 0; p < 4; ++p) {
+                        const float4 x0 = x[rg][p][0], x1 = x[rg][p][1];
                         uint4 hi, lo;
-                        split2(x[p][0].x, x[p][0].y, hi.x, lo.x); split2(x[p][0].z, x[p][0].w, hi.y, lo.y);
-                        split2(x[p][1].x, x[p][1].y, hi.z, lo.z); split2(x[p][1].z, x[p][1].w, hi.w, lo.w);
-                        const uint32_t to = q_tile + (p * 4 + pc) * kPieceBytes + r * 16;
+                        split2(x0.x, x0.y, hi.x, lo.x); split2(x0.z, x0.w, hi.y, lo.y);
+                        split2(x1.x, x1.y, hi.z, lo.z); split2(x1.z, x1.w, hi.w, lo.w);
+                        const uint32_t to = q_tile + (p * 4 + pc) * kPieceBytes + (row0 + rg * 8 + sub) * 16;
                         sts128(to, hi);
                         sts128(to + kTileBytes, lo);
                     }
@@ -273,24 +287,27 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const Prefill
             for (int j = 0; j < n[t]; ++j) {
                 if (alive) alive = mbar_wait(s_full + 8 * t, (uint32_t)j & 1u, a.error_flag, 125, kSpinLimit);
                 tc_fence_after();
-                float s[kKeys];
+                const int see = limit - j * kKeys;
+                const bool masked = j * kKeys + kKeys - 1 > warp_limit;
+                // 32 scores at a time, twice (a read of tensor memory costs less than 128 registers): the maximum, then P
+                float mx = -INFINITY;
+#pragma unroll 1
+                for (int i = 0; i < kKeys; i += 32) {
+                    float s[32];
+                    tmem_ld32(s_at + i, s);
+                    tmem_wait_ld();
+                    tmem_tie32(s);
+                    if (masked) mask_keys(s, see - i);
+                    float top[4] = {s[0], s[1], s[2], s[3]};
 #pragma unroll
-                for (int i = 0; i < kKeys; i += 32) tmem_ld32(s_at + i, s + i);
-                tmem_wait_ld();
+                    for (int u = 4; u < 28; u += 8) {
 #pragma unroll
-                for (int i = 0; i < kKeys; i += 32) tmem_tie32(s + i);
-                if (j * kKeys + kKeys - 1 > warp_limit) {
-                    const int see = limit - j * kKeys;
+                        for (int w = 0; w < 4; ++w) top[w] = fmaxf(top[w], fmaxf(s[u + w], s[u + 4 + w]));
+                    }
 #pragma unroll
-                    for (int i = 0; i < kKeys; ++i) s[i] = i <= see ? s[i] : -INFINITY;
+                    for (int w = 0; w < 4; ++w) top[w] = fmaxf(top[w], s[28 + w]);
+                    mx = fmaxf(mx, fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3])));
                 }
-                float top[4] = {s[0], s[1], s[2], s[3]};
-#pragma unroll
-                for (int i = 4; i < kKeys; i += 8) {
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) top[u] = i + 4 + u < kKeys ? fmaxf(top[u], fmaxf(s[i + u], s[i + 4 + u])) : fmaxf(top[u], s[i + u]);
-                }
-                const float mx = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3]));
                 const bool moves = mx > m && (m == -INFINITY || (mx - m) * c > kSlack);
                 if (__any_sync(0xffffffffu, moves)) {
                     // (the scores' barrier also says that the products into O so far are complete)
@@ -314,18 +331,23 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const Prefill
                     }
                 }
                 const float mc = m == -INFINITY ? 0.0f : m * c;
-#pragma unroll
+#pragma unroll 1
                 for (int i = 0; i < kKeys; i += 32) {
+                    float s[32];
+                    tmem_ld32(s_at + i, s);
+                    tmem_wait_ld();
+                    tmem_tie32(s);
+                    if (masked) mask_keys(s, see - i);
                     uint32_t hi[16], lo[16];
 #pragma unroll
                     for (int u = 0; u < 16; ++u) {
-                        const float2 x = __ffma2_rn(make_float2(s[i + 2 * u], s[i + 2 * u + 1]), make_float2(c, c), make_float2(-mc, -mc));
+                        const float2 x = __ffma2_rn(make_float2(s[2 * u], s[2 * u + 1]), make_float2(c, c), make_float2(-mc, -mc));
                         const float2 p = make_float2(exp2_approx(x.x), exp2_approx(x.y));
                         l = __fadd2_rn(l, p);
                         split2(p.x, p.y, hi[u], lo[u]);
                     }
-                    tmem_st16(s_at + i / 2, hi);
-                    tmem_st16(s_at + 64 + i / 2, lo);
+                    tmem_st16(s_at + i, hi);   // over the 32 scores just read
+                    tmem_st16(s_at + i + 16, lo);
                 }
                 tmem_wait_st();
                 tc_fence_before();
@@ -335,7 +357,11 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const Prefill
             if (alive) alive = mbar_wait(o_full + 8 * t, 0, a.error_flag, 126, kSpinLimit);
             tc_fence_after();
             // rows to memory as whole lines, through the shared memory that the queries have left (a warp's own 16 KB)
-            const float total = l.x + l.y;
+            const float total = l.x + l.y, inv = 1.0f / total;
+            auto over = [&](float o) {   // o / total: the quotient's remainder folded back
+                const float q = o * inv;
+                return fmaf(fmaf(-q, total, o), inv, q);
+            };
             const uint32_t stage = q_tile + row0 * (kHd * 4);
 #pragma unroll 1
             for (int i = 0; i < kHd; i += 32) {
@@ -345,7 +371,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const Prefill
                 tmem_tie32(o);
 #pragma unroll
                 for (int u = 0; u < 32; u += 4) {
-                    const uint4 v = make_uint4(__float_as_uint(o[u] / total), __float_as_uint(o[u + 1] / total), __float_as_uint(o[u + 2] / total), __float_as_uint(o[u + 3] / total));
+                    const uint4 v = make_uint4(__float_as_uint(over(o[u])), __float_as_uint(over(o[u + 1])), __float_as_uint(over(o[u + 2])), __float_as_uint(over(o[u + 3])));
                     sts128(stage + lane * (kHd * 4) + ((((i + u) >> 2) ^ (lane & 7)) << 4), v);
                 }
             }
