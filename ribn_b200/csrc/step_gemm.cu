@@ -10,6 +10,7 @@
 
 #include "blocks.cuh"
 #include "gemv.cuh"
+#include "step_operand.cuh"
 
 namespace ribn {
 
@@ -55,20 +56,27 @@ __device__ __forceinline__ float4 add_parts(const StepFinish& a, const Parts& p,
     }
     return s;
 }
-__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-// 2^k, k in [-126, 127]
-__device__ __forceinline__ float power2(int k) { return __int_as_float((k + 127) << 23); }
 
-// One block: a k tile (256 values of the row) of eight members, 64 threads each, four neighbouring values per thread:
-// lane t of fragment step s holds inputs 16 s + 4 t .. + 3, so a thread writes its member's 16 bytes of the step.
-// MODE: where the values come from (StepFinishMode).
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+
+// One block: a k tile of eight members (write_step_operand).  MODE: where the values come from (StepFinishMode).
 template <int MODE, int BATCH>
 __global__ void __launch_bounds__(512, BATCH > 2 ? 1 : 3) step_finish_kernel(const StepFinish a) {
-    __shared__ float red[16], red_sq[16];
+    __shared__ StepStage stage;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int kt = blockIdx.x, tid = threadIdx.x, g = tid >> 6, i = tid & 63, lane = tid & 31;
     const int m = blockIdx.y * 8 + g, n = kt * kTileCols + 4 * i, k_tiles = gridDim.x, width = k_tiles * kTileCols;
+    // What depends on no earlier kernel comes before the wait: where the parts lie (divisions) and the norm's weights.  A
+    // prefill-sized launch has other blocks to hide them and no registers to hold them.
+    constexpr bool kAhead = MODE == kFinishRows || BATCH > 2;
+    Parts p0{}, p1{};
+    float4 w = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+    if (kAhead && m < a.members) {
+        if (MODE != kFinishRows) p0 = parts_of(a, 0, m, n);
+        if (MODE == kFinishSwiGLU) p1 = parts_of(a, 1, m, n);
+        if (a.norm_weight != nullptr) w = load4(a.norm_weight + n);
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     float square = 0.0f;
     if (m < a.members) {
@@ -76,107 +84,41 @@ __global__ void __launch_bounds__(512, BATCH > 2 ? 1 : 3) step_finish_kernel(con
             v = *reinterpret_cast<const float4*>(a.x + (size_t)(a.index ? a.index[m] : m) * width + n);
         } else if (MODE == kFinishResidual) {
             float4* h = reinterpret_cast<float4*>(a.y[0] + (size_t)m * width + n);
-            const Parts p = parts_of(a, 0, m, n);
-            const float4 before = *h, first = load4(p.at), s = add_parts<BATCH>(a, p, first);
+            if (!kAhead) p0 = parts_of(a, 0, m, n);
+            const float4 before = *h, first = load4(p0.at), s = add_parts<BATCH>(a, p0, first);
             v = make_float4(before.x + s.x, before.y + s.y, before.z + s.z, before.w + s.w);
             *h = v;
         } else {
-            const Parts pg = parts_of(a, 0, m, n), pu = parts_of(a, 1, m, n);
-            const float4 first_g = load4(pg.at), first_u = load4(pu.at);
+            if (!kAhead) { p0 = parts_of(a, 0, m, n); p1 = parts_of(a, 1, m, n); }
+            const float4 first_g = load4(p0.at), first_u = load4(p1.at);
             const float inv = a.ss != nullptr ? norm_factor(a.ss + (size_t)m * a.split.k_tiles, a.split.k_tiles, a.eps, lane) : 1.0f;
-            const float4 gt = add_parts<BATCH>(a, pg, first_g), up = add_parts<BATCH>(a, pu, first_u);
+            const float4 gt = add_parts<BATCH>(a, p0, first_g), up = add_parts<BATCH>(a, p1, first_u);
             auto act = [&](float x, float u) { x *= inv; return x / (1.0f + expf(-x)) * (u * inv); };
             v = make_float4(act(gt.x, up.x), act(gt.y, up.y), act(gt.z, up.z), act(gt.w, up.w));
         }
         square = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w)));
         if (a.norm_weight != nullptr) {
-            const float4 w = *reinterpret_cast<const float4*>(a.norm_weight + n);
+            if (!kAhead) w = load4(a.norm_weight + n);
             v.x *= w.x; v.y *= w.y; v.z *= w.z; v.w *= w.w;
         }
     }
-    // the tile's largest magnitude and sum of squares over the member's 64 threads
-    float top = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-        square += __shfl_xor_sync(0xffffffffu, square, o);
-    }
-    if (lane == 0) { red[tid >> 5] = top; red_sq[tid >> 5] = square; }
-    __syncthreads();
-    top = fmaxf(red[2 * g], red[2 * g + 1]);
-    // a power of two that brings the largest value into [512, 1024): sums of 32 such values still fit binary16
-    const int biased = (int)(__float_as_uint(top) >> 23);   // top is not negative
-    const int e = biased == 255 ? 10 : max(-126, min(126, 136 - biased));
-    const float scale = power2(e);
-    if (i == 0 && m < a.members && a.out.ss != nullptr) a.out.ss[(size_t)m * k_tiles + kt] = red_sq[2 * g] + red_sq[2 * g + 1];
-    const float s4[4] = {v.x * scale, v.y * scale, v.z * scale, v.w * scale};
-    __half hi[4], lo[4];
-    float sum = 0.0f;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        hi[j] = __float2half_rn(s4[j]);
-        lo[j] = __float2half_rn(s4[j] - __half2float(hi[j]));
-        sum += __half2float(hi[j]) + __half2float(lo[j]);   // what the tensor core will see
-    }
-    const int group = blockIdx.y / a.out.ng, ng = blockIdx.y - group * a.out.ng;
-    auto pack = [](__half x, __half y) { const __half2 p = __halves2half2(x, y); return *reinterpret_cast<const uint32_t*>(&p); };
-    const int s = i >> 2, t = i & 3;
-    const float inv_scale = power2(-e);
-    if (a.out.form != kFragmentForm) {
-        const int mp = 8 * a.out.ng, sum_cols = (mp + 15) / 16 * 16, col = ng * 8 + g;
-        unsigned char* blk = a.out.blocks + ((size_t)group * k_tiles + kt) * (1028 * mp + 32 * sum_cols);
-        // The eight members' 16-byte pieces of an 8-input block lie side by side: through shared memory, so that a warp's
-        // stores are whole 128-byte lines.  staged[8-input block][hi, lo][member ^ step % 8]: conflict-free both ways.
-        __shared__ uint4 staged[32][2][8];
-        {
-            uint32_t* at = reinterpret_cast<uint32_t*>(&staged[2 * s][0][g ^ (s & 7)]) + t;
-            at[0] = pack(hi[0], hi[2]);
-            at[32] = pack(lo[0], lo[2]);
-            at[64] = pack(hi[1], hi[3]);          // the next 8-input block
-            at[96] = pack(lo[1], lo[3]);
-        }
-        __syncthreads();
-        {
-            const int kb = tid >> 4, half = (tid >> 3) & 1, member = tid & 7;
-            *reinterpret_cast<uint4*>(blk + ((size_t)kb * 2 * mp + half * mp + ng * 8 + member) * 16) = staged[kb][half][member ^ ((kb >> 1) & 7)];
-        }
-#pragma unroll
-        for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        if ((i & 7) == 0) {
-            const __half h = __float2half_rn(sum), l = __float2half_rn(sum - __half2float(h));
-            __half* to = reinterpret_cast<__half*>(blk + 1024 * mp + col * 16) + (i >> 3);
-            to[0] = h;
-            to[8 * sum_cols] = l;
-        }
-        if (i == 0) reinterpret_cast<float*>(blk + 1024 * mp + 32 * sum_cols)[col] = inv_scale;
-        return;
-    }
-    unsigned char* blk = a.out.blocks + (((size_t)group * k_tiles + kt) * a.out.ng + ng) * kFragBlockBytes;
-    *reinterpret_cast<uint4*>(blk + s * 512 + (g * 4 + t) * 16) = make_uint4(pack(hi[0], hi[2]), pack(hi[1], hi[3]), pack(lo[0], lo[2]), pack(lo[1], lo[3]));
-    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 4);
-    if ((i & 7) == 0) {
-        const int q = i >> 3;
-        const __half h = __float2half_rn(sum), l = __float2half_rn(sum - __half2float(h));
-        __half* at = reinterpret_cast<__half*>(blk + kFragSumsAt + (g * 4 + (q >> 1)) * 8) + (q & 1);
-        at[0] = h;
-        at[2] = l;
-    }
-    if (i == 0) reinterpret_cast<float*>(blk + kFragScaleAt)[g] = inv_scale;
+    write_step_operand(a.out, kt, k_tiles, (int)blockIdx.y, m < a.members, v, square, stage);
 }
 
 // Plain outputs of a split launch: y = (sum of the parts) x the RMSNorm factor, four values per thread; blockIdx.y = member.
+template <int BATCH>
 __global__ void __launch_bounds__(256) step_store_kernel(const StepFinish a) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int m = blockIdx.y, lane = threadIdx.x & 31;
-    const float inv = a.ss != nullptr ? norm_factor(a.ss + (size_t)m * a.split.k_tiles, a.split.k_tiles, a.eps, lane) : 1.0f;
     int n = 4 * (int)(blockIdx.x * blockDim.x + threadIdx.x), seg = 0;
     while (seg < a.n_segments && n >= a.n[seg]) { n -= a.n[seg]; ++seg; }
+    Parts p{};
+    if (seg < a.n_segments) p = parts_of(a, seg, m, n);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const float4 first = seg < a.n_segments ? load4(p.at) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const float inv = a.ss != nullptr ? norm_factor(a.ss + (size_t)m * a.split.k_tiles, a.split.k_tiles, a.eps, lane) : 1.0f;
     if (seg >= a.n_segments) return;
-    const Parts p = parts_of(a, seg, m, n);
-    const float4 s = add_parts<4>(a, p, load4(p.at));
+    const float4 s = add_parts<BATCH>(a, p, first);
     *reinterpret_cast<float4*>(a.y[seg] + (size_t)m * a.n[seg] + n) = make_float4(s.x * inv, s.y * inv, s.z * inv, s.w * inv);
 }
 
@@ -327,14 +269,14 @@ cudaError_t launch_step_finish(cudaStream_t stream, int mode, const StepGemm* ge
     }
     if (a.members < 1) return cudaErrorInvalidValue;
     if (mode == kFinishStore) {
-        return launch_pdl(step_store_kernel, dim3((unsigned)((a.total_n / 4 + 255) / 256), (unsigned)a.members), 256, 0, stream, programmatic, a);
+        return launch_pdl(a.members <= kColumnMaxMembers ? step_store_kernel<7> : step_store_kernel<2>, dim3((unsigned)((a.total_n / 4 + 255) / 256), (unsigned)a.members), 256, 0, stream, programmatic, a);
     }
     if (width % kTileCols != 0 || (a.out.form == kColumnForm && a.members > kColumnMaxMembers)) return cudaErrorInvalidValue;
     const StepShape shape = step_shape(a.members, a.out.form);
     a.out.ng = shape.ng;
     const dim3 grid((unsigned)(width / kTileCols), (unsigned)(shape.groups * shape.ng));
-    // small launches, all of whose items are cut into several parts
-    const bool deep = mode != kFinishRows && !a.split.whole && a.split.rounds == 0 && a.split.workers > 2 * a.split.even();
+    // one block per SM while that is a single wave of blocks (see add_parts)
+    const bool deep = grid.x * grid.y <= (unsigned)device_sms();
     switch (mode) {
         case kFinishRows: return launch_pdl(step_finish_kernel<kFinishRows, 2>, grid, 512, 0, stream, programmatic, a);
         case kFinishResidual:

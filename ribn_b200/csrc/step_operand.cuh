@@ -1,0 +1,94 @@
+// The operand form of a step's GEMMs (StepOperand), written by the kernel that produces the values.
+#pragma once
+#include <cuda_fp16.h>
+
+#include "gemv.cuh"
+
+namespace ribn {
+
+struct StepStage {
+    float tops[16], squares[16];
+    uint4 pieces[32][2][8];   // [8-input block][hi, lo][member ^ step % 8]: conflict-free both ways
+};
+
+// 2^k, k in [-126, 127]
+__device__ __forceinline__ float power2(int k) { return __int_as_float((k + 127) << 23); }
+
+// One block of 512 threads: k tile `kt` (256 values of the row) of the eight members from 8 `eight` on, 64 threads each, four
+// neighbouring values per thread: lane t of fragment step s holds inputs 16 s + 4 t .. + 3, so a thread writes its member's 16
+// bytes of the step.  `v`: the thread's values (zeros where the member does not exist: `have`), `square`: its share of the row's
+// sum of squares.
+__device__ __forceinline__ void write_step_operand(const StepOperand& out, int kt, int k_tiles, int eight, bool have, const float4 v, float square, StepStage& stage) {
+    const int tid = threadIdx.x, g = tid >> 6, i = tid & 63, lane = tid & 31;
+    // the tile's largest magnitude and sum of squares over the member's 64 threads
+    float top = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+        square += __shfl_xor_sync(0xffffffffu, square, o);
+    }
+    if (lane == 0) { stage.tops[tid >> 5] = top; stage.squares[tid >> 5] = square; }
+    __syncthreads();
+    top = fmaxf(stage.tops[2 * g], stage.tops[2 * g + 1]);
+    // a power of two that brings the largest value into [512, 1024): sums of 32 such values still fit binary16
+    const int biased = (int)(__float_as_uint(top) >> 23);   // top is not negative
+    const int e = biased == 255 ? 10 : max(-126, min(126, 136 - biased));
+    const float scale = power2(e);
+    if (i == 0 && have && out.ss != nullptr) out.ss[(size_t)(eight * 8 + g) * k_tiles + kt] = stage.squares[2 * g] + stage.squares[2 * g + 1];
+    const float s4[4] = {v.x * scale, v.y * scale, v.z * scale, v.w * scale};
+    __half hi[4], lo[4];
+    float sum = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        hi[j] = __float2half_rn(s4[j]);
+        lo[j] = __float2half_rn(s4[j] - __half2float(hi[j]));
+        sum += __half2float(hi[j]) + __half2float(lo[j]);   // what the tensor core will see
+    }
+    const int group = eight / out.ng, ng = eight - group * out.ng;
+    auto pack = [](__half x, __half y) { const __half2 p = __halves2half2(x, y); return *reinterpret_cast<const uint32_t*>(&p); };
+    const int s = i >> 2, t = i & 3;
+    const float inv_scale = power2(-e);
+    if (out.form != kFragmentForm) {
+        const int mp = 8 * out.ng, sum_cols = (mp + 15) / 16 * 16, col = ng * 8 + g;
+        unsigned char* blk = out.blocks + ((size_t)group * k_tiles + kt) * (1028 * mp + 32 * sum_cols);
+        // The eight members' 16-byte pieces of an 8-input block lie side by side: through shared memory, so that a warp's
+        // stores are whole 128-byte lines.  stage.pieces[8-input block][hi, lo][member ^ step % 8]: conflict-free both ways.
+        {
+            uint32_t* at = reinterpret_cast<uint32_t*>(&stage.pieces[2 * s][0][g ^ (s & 7)]) + t;
+            at[0] = pack(hi[0], hi[2]);
+            at[32] = pack(lo[0], lo[2]);
+            at[64] = pack(hi[1], hi[3]);          // the next 8-input block
+            at[96] = pack(lo[1], lo[3]);
+        }
+        __syncthreads();
+        {
+            const int kb = tid >> 4, half = (tid >> 3) & 1, member = tid & 7;
+            *reinterpret_cast<uint4*>(blk + ((size_t)kb * 2 * mp + half * mp + ng * 8 + member) * 16) = stage.pieces[kb][half][member ^ ((kb >> 1) & 7)];
+        }
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if ((i & 7) == 0) {
+            const __half h = __float2half_rn(sum), l = __float2half_rn(sum - __half2float(h));
+            __half* to = reinterpret_cast<__half*>(blk + 1024 * mp + col * 16) + (i >> 3);
+            to[0] = h;
+            to[8 * sum_cols] = l;
+        }
+        if (i == 0) reinterpret_cast<float*>(blk + 1024 * mp + 32 * sum_cols)[col] = inv_scale;
+        return;
+    }
+    unsigned char* blk = out.blocks + (((size_t)group * k_tiles + kt) * out.ng + ng) * kFragBlockBytes;
+    *reinterpret_cast<uint4*>(blk + s * 512 + (g * 4 + t) * 16) = make_uint4(pack(hi[0], hi[2]), pack(hi[1], hi[3]), pack(lo[0], lo[2]), pack(lo[1], lo[3]));
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+    if ((i & 7) == 0) {
+        const int q = i >> 3;
+        const __half h = __float2half_rn(sum), l = __float2half_rn(sum - __half2float(h));
+        __half* at = reinterpret_cast<__half*>(blk + kFragSumsAt + (g * 4 + (q >> 1)) * 8) + (q & 1);
+        at[0] = h;
+        at[2] = l;
+    }
+    if (i == 0) reinterpret_cast<float*>(blk + kFragScaleAt)[g] = inv_scale;
+}
+
+}  // namespace ribn
