@@ -26,6 +26,7 @@
 #include "gemv.cuh"
 #include "kernels.cuh"
 #include "operand.cuh"
+#include "step_operand.cuh"
 
 namespace ribn {
 
@@ -66,6 +67,7 @@ struct AttnArgs {
     int* error_flag;           // of the tensor-memory kernel's bounded waits
     float* out;                // [T][q_heads][HD]
     ActOperand operand;        // optional operand form of `out`, K = q_heads * HD
+    StepOperand step_operand;  // the same for a step's GEMMs (null blocks: not asked for)
 };
 
 // RMSNorm + NeoX rotary of one head vector held lane-strided: element i of a
@@ -767,12 +769,60 @@ __global__ void __launch_bounds__(kMmaWarps * 32) attention_prefill_mma_kernel(c
 template <int HD>
 __global__ void __launch_bounds__(kMmaWarps * 32) attention_merge_kernel(const AttnArgs a) {
     __shared__ float sums[kMmaWarps][HD + 1];
+    const int t = a.token_base + (int)blockIdx.x / a.q_heads, qh = (int)blockIdx.x % a.q_heads;
+    const int spans = token_spans(a, a.token_pos[t]);   // positions are older than the kernel before this one
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const int t = a.token_base + (int)blockIdx.x / a.q_heads, qh = (int)blockIdx.x % a.q_heads;
-    const int spans = token_spans(a, a.token_pos[t]);
     if (spans <= 1) return;  // written directly by the span kernel
     merge_head<HD>(a, t, qh, spans, threadIdx.x >> 5, threadIdx.x & 31, sums);
+}
+
+// The merge of a step that feeds a step GEMM, in one pass with the operand form: a block takes a k tile (256 / HD heads) of eight
+// tokens, a thread four dimensions of one; spans in order, eight in flight.  A token with one span has its result in `out`.
+template <int HD>
+__global__ void __launch_bounds__(512) attention_merge_operand_kernel(const AttnArgs a, const int n_tokens) {
+    __shared__ StepStage stage;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    constexpr int REC = HD + 2, kBatch = 8;
+    const int g = threadIdx.x >> 6, i = threadIdx.x & 63, local = (int)blockIdx.y * 8 + g, t = a.token_base + local;
+    const int head = (int)blockIdx.x * (kTileCols / HD) + 4 * i / HD, d = 4 * i % HD;
+    const bool have = local < n_tokens;
+    const int spans = have ? token_spans(a, a.token_pos[t]) : 0;   // positions are older than the kernel before this one
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (spans == 1) {
+        v = *reinterpret_cast<const float4*>(a.out + ((long long)t * a.q_heads + head) * HD + d);
+    } else if (spans > 1) {
+        const float* pp = a.partial + ((long long)local * a.q_heads + head) * a.max_spans * REC;
+        float top = -INFINITY, denom = 0.0f;
+        for (int s0 = 0; s0 < spans; s0 += kBatch) {
+            float2 x[kBatch], y[kBatch], ml[kBatch];   // four dimensions; maximum and sum
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) {
+                const bool in = s0 + u < spans;
+                const float* rec = pp + (long long)(s0 + u) * REC;
+                x[u] = in ? *reinterpret_cast<const float2*>(rec + d) : make_float2(0.0f, 0.0f);
+                y[u] = in ? *reinterpret_cast<const float2*>(rec + d + 2) : make_float2(0.0f, 0.0f);
+                ml[u] = in ? *reinterpret_cast<const float2*>(rec + HD) : make_float2(-INFINITY, 0.0f);
+            }
+            float m = top;
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) m = fmaxf(m, ml[u].x);
+            const float f = __expf(top - m);   // 0 the first time
+            top = m;
+            denom *= f; v.x *= f; v.y *= f; v.z *= f; v.w *= f;
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) {
+                const float w = __expf(ml[u].x - m);   // 0 past the last span
+                denom = fmaf(ml[u].y, w, denom);
+                v.x = fmaf(x[u].x, w, v.x); v.y = fmaf(x[u].y, w, v.y); v.z = fmaf(y[u].x, w, v.z); v.w = fmaf(y[u].y, w, v.w);
+            }
+        }
+        v.x /= denom; v.y /= denom; v.z /= denom; v.w /= denom;
+    }
+    StepOperand out = a.step_operand;
+    out.ss = nullptr;
+    write_step_operand(out, (int)blockIdx.x, (int)gridDim.x, (int)blockIdx.y, have, v, 0.0f, stage);
 }
 
 int attn_sm_count() {
@@ -836,7 +886,7 @@ cudaError_t launch_pdl(cudaStream_t stream, Kernel kernel, dim3 grid, int thread
 // The span kernel and its merge over tokens [first_token, first_token + n_tokens) of the launch.
 template <int HD>
 cudaError_t launch_spans_hd(cudaStream_t stream, AttnArgs a, bool fused, int first_token, int n_tokens, int max_keys,
-                            size_t partial_bytes, int* launches, bool programmatic) {
+                            size_t partial_bytes, int* launches, bool programmatic, bool* operand_written = nullptr) {
     const int q_per_kv = a.q_heads / a.kv_heads;
     const int max_tiles = (max_keys + kAttnSpanKeys - 1) / kAttnSpanKeys;
     if (max_tiles > kAttnMaxSpans) return cudaErrorInvalidValue;
@@ -905,7 +955,14 @@ cudaError_t launch_spans_hd(cudaStream_t stream, AttnArgs a, bool fused, int fir
         }
         if (e != cudaSuccess) return e;
         if (launches) ++*launches;
-        if (a.max_spans > 1) {
+        if (a.max_spans > 1 && n == n_tokens && a.step_operand.blocks != nullptr && operand_written != nullptr) {
+            const StepShape shape = step_shape(n, a.step_operand.form);
+            a.step_operand.ng = shape.ng;
+            e = launch_pdl(stream, attention_merge_operand_kernel<HD>, dim3((unsigned)(a.q_heads * HD / kTileCols), (unsigned)(shape.groups * shape.ng)), 512, 0, a, programmatic, n);
+            if (e != cudaSuccess) return e;
+            if (launches) ++*launches;
+            *operand_written = true;
+        } else if (a.max_spans > 1) {
             e = launch_pdl(stream, attention_merge_kernel<HD>, dim3(n * a.q_heads), kMmaWarps * 32, 0, a, programmatic);
             if (e != cudaSuccess) return e;
             if (launches) ++*launches;
@@ -916,7 +973,7 @@ cudaError_t launch_spans_hd(cudaStream_t stream, AttnArgs a, bool fused, int fir
 
 template <int HD>
 cudaError_t launch_hd(cudaStream_t stream, AttnArgs a, bool fused, int n_tokens, int max_keys, size_t partial_bytes,
-                      int* launches, bool programmatic = false) {
+                      int* launches, bool programmatic = false, bool* operand_written = nullptr) {
     const int q_per_kv = a.q_heads / a.kv_heads;
     if (q_per_kv > 16) return cudaErrorInvalidValue;  // the group is the 16 columns of two MMA tiles
     // A long run of consecutive tokens of one sequence (a prefill chunk; the caller says where it lies) takes the
@@ -962,15 +1019,15 @@ cudaError_t launch_hd(cudaStream_t stream, AttnArgs a, bool fused, int n_tokens,
         if (behind < n_tokens) e = launch_spans_hd<HD>(stream, a, fused, behind, n_tokens - behind, max_keys, partial_bytes, launches, programmatic);
         return e;
     }
-    return launch_spans_hd<HD>(stream, a, fused, 0, n_tokens, max_keys, partial_bytes, launches, programmatic);
+    return launch_spans_hd<HD>(stream, a, fused, 0, n_tokens, max_keys, partial_bytes, launches, programmatic, operand_written);
 }
 
 cudaError_t dispatch(cudaStream_t stream, const AttnArgs& a, bool fused, int head_dim, int n_tokens, int max_keys,
-                     size_t partial_bytes, int* launches, bool programmatic = false) {
+                     size_t partial_bytes, int* launches, bool programmatic = false, bool* operand_written = nullptr) {
     switch (head_dim) {
-        case 64: return launch_hd<64>(stream, a, fused, n_tokens, max_keys, partial_bytes, launches, programmatic);
-        case 128: return launch_hd<128>(stream, a, fused, n_tokens, max_keys, partial_bytes, launches, programmatic);
-        case 256: return launch_hd<256>(stream, a, fused, n_tokens, max_keys, partial_bytes, launches, programmatic);
+        case 64: return launch_hd<64>(stream, a, fused, n_tokens, max_keys, partial_bytes, launches, programmatic, operand_written);
+        case 128: return launch_hd<128>(stream, a, fused, n_tokens, max_keys, partial_bytes, launches, programmatic, operand_written);
+        case 256: return launch_hd<256>(stream, a, fused, n_tokens, max_keys, partial_bytes, launches, programmatic, operand_written);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -1010,7 +1067,8 @@ cudaError_t launch_attention(cudaStream_t stream, const float* q, const __half* 
     return dispatch(stream, a, false, head_dim, n_tokens, max_keys, partial_bytes, launches);
 }
 
-cudaError_t launch_attention_decode(cudaStream_t stream, const DecodeAttention& d, int* launches) {
+cudaError_t launch_attention_decode(cudaStream_t stream, const DecodeAttention& d, int* launches, bool* operand_written) {
+    if (operand_written) *operand_written = false;
     if (d.n_tokens <= 0) return cudaSuccess;
     if (d.q_heads % d.kv_heads != 0 || d.q_heads / d.kv_heads > 16 || d.max_keys <= 0) return cudaErrorInvalidValue;
     AttnArgs a{};
@@ -1022,8 +1080,9 @@ cudaError_t launch_attention_decode(cudaStream_t stream, const DecodeAttention& 
     a.q_heads = d.q_heads; a.kv_heads = d.kv_heads; a.window = d.window;
     a.partial = d.partial; a.out = d.out; a.operand = d.operand;
     a.run_first = -1; a.run_count = 0;
+    if (d.step_operand.blocks != nullptr && d.q_heads * d.head_dim % kTileCols == 0) a.step_operand = d.step_operand;
     const int max_keys = d.window > 0 ? std::min(d.max_keys, d.window) : d.max_keys;
-    return dispatch(stream, a, true, d.head_dim, d.n_tokens, max_keys, d.partial_bytes, launches, d.programmatic);
+    return dispatch(stream, a, true, d.head_dim, d.n_tokens, max_keys, d.partial_bytes, launches, d.programmatic, operand_written);
 }
 
 }  // namespace ribn

@@ -376,7 +376,9 @@ GemvArgs head_args(ribn_b200_executor* ex, int rows, const ActOperand& in) {
 // one token (fused_attention) it is one pass, which can also leave the result in `operand`.
 bool fused_attention(const ribn_b200_executor* ex, const StepPlan& plan) { return plan.n_rows == plan.n_tokens && ex->cfg.head_dim >= 64; }
 
-cudaError_t run_attention(ribn_b200_executor* ex, const StepPlan& plan, int l, bool programmatic, const ActOperand& operand, int& launches) {
+// `step_operand`, `operand_written`: see DecodeAttention (one pass only).
+cudaError_t run_attention(ribn_b200_executor* ex, const StepPlan& plan, int l, bool programmatic, const ActOperand& operand, int& launches,
+                          StepOperand step_operand = StepOperand{}, bool* operand_written = nullptr) {
     const ribn_b200_config& c = ex->cfg;
     cudaStream_t s = ex->stream;
     const int T = plan.n_tokens;
@@ -396,7 +398,8 @@ cudaError_t run_attention(ribn_b200_executor* ex, const StepPlan& plan, int l, b
         d.partial = ex->scratch.attn_partial; d.partial_bytes = ex->scratch.attn_partial_bytes;
         d.out = ex->attn; d.operand = operand;
         d.programmatic = programmatic;
-        return launch_attention_decode(s, d, &launches);
+        d.step_operand = step_operand;
+        return launch_attention_decode(s, d, &launches, operand_written);
     }
     STEP_TRY(launch_qk_norm_rope_append(s, ex->q, ex->k, ex->v, (const float*)t[kAttnQNorm].raw, (const float*)t[kAttnKNorm].raw, ex->inv_freq,
                                         ex->meta.token_pos, ex->meta.token_slot, T, c.q_heads, c.kv_heads, c.head_dim, c.rms_eps, ck, cv));
@@ -530,16 +533,17 @@ cudaError_t run_layers_step(ribn_b200_executor* ex, const StepPlan& plan, int& l
     STEP_TRY(rows(ex->hidden, nullptr, (const float*)ex->lt(0, kAttnNorm).raw, T, c.hidden));
     for (int l = 0; l < c.layers; ++l) {
         Tensor* t = &ex->lt(l, 0);
+        bool operand_written = false;
         {
             const StepGemm g = step_qkv(ex, l, T);
             STEP_TRY(launch_step_gemm(s, g, pdl));
             STEP_TRY(launch_step_finish(s, kFinishStore, &g, StepFinish{}, 0, pdl));
         }
         {
-            cudaError_t e = run_attention(ex, plan, l, pdl, ActOperand{}, launches);
+            cudaError_t e = run_attention(ex, plan, l, pdl, ActOperand{}, launches, plain, &operand_written);
             if (e != cudaSuccess) return e;
         }
-        STEP_TRY(rows(ex->attn, nullptr, nullptr, T, QD));
+        if (!operand_written) STEP_TRY(rows(ex->attn, nullptr, nullptr, T, QD));
         StepFinish f{};
         {
             const StepGemm g = step_o(ex, l, T);

@@ -152,9 +152,11 @@ struct DecodeAttention {
     size_t partial_bytes;
     float* out;
     ActOperand operand;
+    StepOperand step_operand;  // steps of three rows and more, optional (null blocks): the operand form of their output projection
     bool programmatic;  // launch as programmatic dependents of the previous kernel in the stream
 };
-cudaError_t launch_attention_decode(cudaStream_t stream, const DecodeAttention& d, int* launches);
+// `operand_written`: whether the result lies in d.step_operand (else in d.out: one span per row, or several launches).
+cudaError_t launch_attention_decode(cudaStream_t stream, const DecodeAttention& d, int* launches, bool* operand_written = nullptr);
 
 // Decode steps of a Gated-DeltaNet recurrent layer behind its projections, for `members` sequences with their own
 // states, `tokens` consecutive tokens each (1: a decode step; more: a prefill chunk, token by token inside the

@@ -686,3 +686,31 @@ def test_a_larger_batch_limit_takes_memory_for_its_rows_only(built_library):
         used.append(before - torch.cuda.mem_get_info()[0])
         ex.close()
     assert used[1] - used[0] < 64 << 20, used
+
+
+@pytest.mark.parametrize("head_dim", [64, 128])
+@pytest.mark.parametrize("rows", [3, 9, 17, 40])
+def test_decode_rows_of_one_and_of_many_spans_share_a_step(built_library, rows, head_dim):
+    """A ragged decode step whose attention merge also writes the output projection's operand: rows whose keys are one span
+    (their result is not a partial one), a few and many spans side by side, in row counts that leave operand blocks of eight
+    rows part empty, in the fragment and the column form; against the plain reference-style kernels on the same cache."""
+    import ribn_b200
+    from ribn_b200 import BatchItem, StepKind
+    cfg = dict(layers=2, hidden=512, q_heads=8, kv_heads=2, head_dim=head_dim, ffn=1024, vocab=1024, rope_base=1.0e6, rms_eps=1.0e-6)
+    cycle = (16, 63, 64, 65, 600, 129, 1500)
+    lengths = [cycle[i % len(cycle)] for i in range(rows)]
+    logits = []
+    for flags in (0, ribn_b200.FLAG_REFERENCE_KERNELS):
+        ex = ribn_b200.QwenB200(cfg, flags=flags | ribn_b200.FLAG_KEEP_LOGITS, context_tokens=2048, max_sequences=rows, max_batch_tokens=64)
+        ex.init_synthetic(23, ribn_b200.SCHEME_Q4_K_M)
+        ex.finalize()
+        for s, n in enumerate(lengths):
+            assert ex.admit(s + 1, s + 1, [1] * n, 4).ready
+            ex.debug_set_context(s + 1, n, 5 + s, seed=70 + s)
+        items = [BatchItem(s + 1, StepKind.DECODE, n, 1, 1) for s, n in enumerate(lengths)]
+        ex.prepare(items)
+        ex.wait(ex.submit(items))
+        logits.append(np.stack([ex.copy_logits(r) for r in range(rows)]))
+        ex.close()
+    assert np.all(np.isfinite(logits[0]))
+    assert close(logits[0], logits[1])
