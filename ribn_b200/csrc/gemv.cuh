@@ -242,7 +242,10 @@ int gemm_tc_last_launches();
 //                                 columns: hi parts, then lo parts
 //     [2][mp to 16] 16 bytes      sums of the eight 32-input groups: hi, then lo
 //     [mp] F32                    the rows' scales
-//   kWideForm (gemm_pf.cu, tcgen05): groups of 128 rows, each as the column form with mp = 128
+//   kWideForm (gemm_pf.cu, tcgen05): groups of 128 rows, a pair of CTAs taking 64 of them each
+//     [2 x 64 rows][2 x 128 inputs][hi, lo][16][64] 16 bytes   K-major core matrices as above
+//     [2 x 64 rows][2][64] 16 bytes                            sums, as above
+//     [128] F32                                                the rows' scales
 // Blocks are ordered [group][k tile](ng).  `ss` holds, per row and k tile, the sum of squares of the values before the
 // norm weight, for the RMSNorm factor of the consumer.
 enum StepForm : int { kFragmentForm = 0, kColumnForm = 1, kWideForm = 2 };
@@ -276,16 +279,19 @@ struct StepGemm {
     uint32_t spin_limit;
     int n_offset[3], total_n;      // filled in by the launcher
 };
-// An item is one group of rows of a unit of weight rows (128; 256 in the wide form).  How a launch's (item, k tile) slots are
-// dealt to its workers (CTAs, or a CTA's teams of warps): in whole items, or evenly, an item's slots then lying with
-// consecutive workers.  The wide form takes whole items in rounds, neighbouring workers the same activations side by side,
-// and deals out only the last, incomplete round evenly.  It depends on the matrices and the row groups only.
+// An item is one group of rows of a unit of weight rows (128; 256 in the wide form), in the wide form up to two neighbouring
+// groups (`joint`).  How a launch's (item, k tile) slots are dealt to its workers (CTAs, a CTA's teams of warps, or in the wide
+// form pairs of CTAs): in whole items, or evenly, an item's slots then lying with consecutive workers.  The wide form takes
+// whole items in rounds, neighbouring workers the same activations side by side, and deals out only the last, incomplete
+// round evenly.  It depends on the matrices and the row groups only.
 struct StepRun { int item, begin, end, part; };   // k tiles [begin, end) of an item, whose sums are its part `part`
 struct StepSplit {
-    int k_tiles, groups, group_members, items, workers, whole, unit_shift;   // unit_shift: log2 of a unit's weight rows
-    int rounds;                                                              // wide form: rounds of whole items
+    int k_tiles, groups, group_members, joint, items, workers, whole, unit_shift;   // unit_shift: log2 of a unit's weight rows
+    int rounds;                                                                     // wide form: rounds of whole items
     int spread;   // workers that share the even slots: never more than there are slots, so that an item's parts have no gaps
     __host__ __device__ int even() const { return items - rounds * workers; }   // items dealt out evenly
+    __host__ __device__ int item_groups() const { return (groups + joint - 1) / joint; }   // items per unit
+    __host__ __device__ int item_of(int unit, int group) const { return unit * item_groups() + group / joint; }
     // (32-bit arithmetic: step_split deals out whole items where slots x workers would not fit)
     __host__ __device__ int begin(int w) const {   // first even slot of worker w; workers past the last one have nothing
         const uint32_t v = (uint32_t)(w < spread ? w : spread) * (uint32_t)even(), n = (uint32_t)spread;
@@ -314,16 +320,18 @@ struct StepSplit {
         return StepRun{item, lo, hi, whole ? 0 : w - first_worker(item)};
     }
     // An item's first part lies in the launch's matrix of sums [member][rows of all segments].  A further part begins in the
-    // middle of the item, which only a worker's first run can do: it lies in the slot of its worker, [member of the
-    // group][row of the unit], so an item's further parts are neighbours.
+    // middle of the item, which only a worker's first run can do: each of its groups lies in a slot of its worker, [member of
+    // the group][row of the unit]; the slots of first groups, then those of second ones, so an item's further parts are
+    // neighbours.
     __host__ __device__ int slot_floats() const { return group_members << unit_shift; }
+    __host__ __device__ size_t slot_of(int group, int worker) const { return (size_t)(group % joint * workers + worker) * (size_t)slot_floats(); }
 };
 // Where a run's sums of row n of segment `seg` lie, from member `m` of the group on: first value and distance of the members.
 struct StepSums { float* at; size_t stride; };
 __device__ __forceinline__ StepSums step_sums(const StepGemm& a, const StepSplit& s, int worker, int part, int group, int m, int seg, int n) {
     if (part == 0) return StepSums{a.partial + (size_t)(group * s.group_members + m) * a.total_n + a.n_offset[seg] + n, (size_t)a.total_n};
     const int unit_rows = 1 << s.unit_shift;
-    return StepSums{a.further + (size_t)worker * s.slot_floats() + m * unit_rows + (n & (unit_rows - 1)), (size_t)unit_rows};
+    return StepSums{a.further + s.slot_of(group, worker) + m * unit_rows + (n & (unit_rows - 1)), (size_t)unit_rows};
 }
 StepSplit step_split(const StepGemm& a, bool whole_items);
 // A packed matrix as a rank-4 tensor map (128 bytes, to be copied to device memory, 64-byte aligned): one copy then

@@ -121,12 +121,18 @@ int ribn_b200_debug_step_deal(int32_t form, int64_t rows, int64_t cols, int32_t 
     *further_floats = step_further_floats(g);
     *count = 0;
     for (int w = 0; w < s.workers; ++w) {
-        for (int r = 0; r < s.runs(w); ++r, ++*count) {
-            if (*count >= capacity) continue;
+        for (int r = 0; r < s.runs(w); ++r) {
             const StepRun run = s.run(w, r);
-            const bool dealt = !s.whole && run.item >= s.rounds * s.workers;
-            const int32_t record[8] = {w, run.item, run.begin, run.end, run.part, s.parts(run.item), dealt ? s.first_worker(run.item) : w, 1 << s.unit_shift};
-            memcpy(runs + 8 * *count, record, sizeof(record));
+            const int unit = run.item / s.item_groups(), group0 = run.item % s.item_groups() * s.joint;
+            // a worker of two groups at a time counts as two, each with its own slots of sums
+            for (int u = 0; u < s.joint && group0 + u < s.groups; ++u, ++*count) {
+                if (*count >= capacity) continue;
+                const bool dealt = !s.whole && run.item >= s.rounds * s.workers;
+                const int own = u * s.workers;
+                const int32_t record[8] = {own + w, unit * s.groups + group0 + u, run.begin, run.end, run.part, s.parts(run.item),
+                                           own + (dealt ? s.first_worker(run.item) : w), 1 << s.unit_shift};
+                memcpy(runs + 8 * *count, record, sizeof(record));
+            }
         }
     }
     return RIBN_B200_OK;

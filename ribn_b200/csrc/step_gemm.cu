@@ -31,10 +31,10 @@ __device__ __forceinline__ float norm_factor(const float* ss, int tiles, float e
 // of the further ones, counted from the first's worker.
 struct Parts { const float* at; int count; const float* slots; };
 __device__ __forceinline__ Parts parts_of(const StepFinish& a, int seg, int m, int n) {
-    const int unit = a.unit0[seg] + (n >> a.split.unit_shift), group = m / a.split.group_members, item = unit * a.split.groups + group;
+    const int unit = a.unit0[seg] + (n >> a.split.unit_shift), group = m / a.split.group_members, item = a.split.item_of(unit, group);
     Parts p{a.partial + (size_t)m * a.total_n + a.n_offset[seg] + n, a.split.parts(item), nullptr};
     if (p.count > 1) {
-        p.slots = a.further + (size_t)a.split.first_worker(item) * a.split.slot_floats() +
+        p.slots = a.further + a.split.slot_of(group, a.split.first_worker(item)) +
                   ((m - group * a.split.group_members) << a.split.unit_shift) + (n & ((1 << a.split.unit_shift) - 1));
     }
     return p;
@@ -206,10 +206,12 @@ StepSplit step_split(const StepGemm& a, bool whole_items) {
     s.k_tiles = a.k / kTileCols;
     s.groups = shape.groups;
     s.group_members = shape.ng * 8;
-    for (int i = 0; i < a.n_segments; ++i) s.items += (a.seg[i].row_tiles + tiles - 1) / tiles * shape.groups;
+    s.joint = a.form == kWideForm ? 2 : 1;
+    for (int i = 0; i < a.n_segments; ++i) s.items += (a.seg[i].row_tiles + tiles - 1) / tiles * s.item_groups();
     if ((unsigned long long)s.items * s.k_tiles * (device_sms() * kFragTeams) >> 32) whole_items = true;
     s.whole = whole_items ? 1 : 0;
-    s.workers = std::min(device_sms() * (a.form == kFragmentForm ? kFragTeams : 1), whole_items ? s.items : s.items * s.k_tiles);
+    const int workers = a.form == kWideForm ? device_sms() / 2 : device_sms() * (a.form == kFragmentForm ? kFragTeams : 1);
+    s.workers = std::min(std::max(1, workers), whole_items ? s.items : s.items * s.k_tiles);
     s.rounds = a.form == kWideForm ? s.items / s.workers : 0;
     if (s.rounds * s.workers == s.items && s.rounds > 0) s.whole = 1;   // nothing is left to deal out evenly
     s.spread = std::max(1, s.whole ? std::min(s.workers, s.even()) : std::min(s.workers, s.even() * s.k_tiles));
@@ -224,7 +226,7 @@ size_t step_partial_floats(const StepGemm& a) {
 
 size_t step_further_floats(const StepGemm& a) {
     const StepSplit s = step_split(a, false);
-    return s.whole ? 0 : (size_t)s.spread * s.slot_floats();
+    return s.whole ? 0 : s.slot_of(s.joint - 1, s.spread);
 }
 
 cudaError_t launch_step_gemm(cudaStream_t stream, const StepGemm& args, bool programmatic) {

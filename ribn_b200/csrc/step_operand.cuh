@@ -50,6 +50,7 @@ __device__ __forceinline__ void write_step_operand(const StepOperand& out, int k
     const float inv_scale = power2(-e);
     if (out.form != kFragmentForm) {
         const int mp = 8 * out.ng, sum_cols = (mp + 15) / 16 * 16, col = ng * 8 + g;
+        const bool wide = out.form == kWideForm;   // 64 rows of a block at a time, and 128 inputs of them
         unsigned char* blk = out.blocks + ((size_t)group * k_tiles + kt) * (1028 * mp + 32 * sum_cols);
         // The eight members' 16-byte pieces of an 8-input block lie side by side: through shared memory, so that a warp's
         // stores are whole 128-byte lines.  stage.pieces[8-input block][hi, lo][member ^ step % 8]: conflict-free both ways.
@@ -63,15 +64,18 @@ __device__ __forceinline__ void write_step_operand(const StepOperand& out, int k
         __syncthreads();
         {
             const int kb = tid >> 4, half = (tid >> 3) & 1, member = tid & 7;
-            *reinterpret_cast<uint4*>(blk + ((size_t)kb * 2 * mp + half * mp + ng * 8 + member) * 16) = stage.pieces[kb][half][member ^ ((kb >> 1) & 7)];
+            const int c = ng * 8 + member;
+            const int at = wide ? (((c >> 6) * 2 + (kb >> 4)) * 2 + half) * 1024 + (kb & 15) * 64 + (c & 63) : (kb * 2 + half) * mp + c;
+            *reinterpret_cast<uint4*>(blk + (size_t)at * 16) = stage.pieces[kb][half][member ^ ((kb >> 1) & 7)];
         }
 #pragma unroll
         for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
         if ((i & 7) == 0) {
             const __half h = __float2half_rn(sum), l = __float2half_rn(sum - __half2float(h));
-            __half* to = reinterpret_cast<__half*>(blk + 1024 * mp + col * 16) + (i >> 3);
+            const int cols = wide ? 64 : sum_cols, at = wide ? (col >> 6) * 128 + (col & 63) : col;
+            __half* to = reinterpret_cast<__half*>(blk + 1024 * mp + at * 16) + (i >> 3);
             to[0] = h;
-            to[8 * sum_cols] = l;
+            to[8 * cols] = l;
         }
         if (i == 0) reinterpret_cast<float*>(blk + 1024 * mp + 32 * sum_cols)[col] = inv_scale;
         return;
