@@ -409,8 +409,17 @@ cudaError_t launch_attention_tc(cudaStream_t stream, const PrefillAttention& a) 
         configured[dev] = true;
     }
     const int tile_tokens = kRows / (a.q_heads / a.kv_heads), pairs = (a.count + 2 * tile_tokens - 1) / (2 * tile_tokens);
-    attention_tc_kernel<<<dim3((unsigned)(pairs * a.kv_heads)), kThreads, kSmem, stream>>>(a, tile_tokens);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(pairs * a.kv_heads));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = kSmem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];   // barriers and tensor memory are set up under the kernel before
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, attention_tc_kernel, a, tile_tokens);
 }
 
 }  // namespace ribn

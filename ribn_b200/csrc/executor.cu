@@ -376,9 +376,9 @@ GemvArgs head_args(ribn_b200_executor* ex, int rows, const ActOperand& in) {
 // one token (fused_attention) it is one pass, which can also leave the result in `operand`.
 bool fused_attention(const ribn_b200_executor* ex, const StepPlan& plan) { return plan.n_rows == plan.n_tokens && ex->cfg.head_dim >= 64; }
 
-// `step_operand`, `operand_written`: see DecodeAttention (one pass only).
+// `step_operand`, `operand_written`: see DecodeAttention (one pass only); `appended`: launch_step_qkv has done all before attention.
 cudaError_t run_attention(ribn_b200_executor* ex, const StepPlan& plan, int l, bool programmatic, const ActOperand& operand, int& launches,
-                          StepOperand step_operand = StepOperand{}, bool* operand_written = nullptr) {
+                          StepOperand step_operand = StepOperand{}, bool* operand_written = nullptr, bool appended = false) {
     const ribn_b200_config& c = ex->cfg;
     cudaStream_t s = ex->stream;
     const int T = plan.n_tokens;
@@ -401,8 +401,10 @@ cudaError_t run_attention(ribn_b200_executor* ex, const StepPlan& plan, int l, b
         d.step_operand = step_operand;
         return launch_attention_decode(s, d, &launches, operand_written);
     }
-    STEP_TRY(launch_qk_norm_rope_append(s, ex->q, ex->k, ex->v, (const float*)t[kAttnQNorm].raw, (const float*)t[kAttnKNorm].raw, ex->inv_freq,
-                                        ex->meta.token_pos, ex->meta.token_slot, T, c.q_heads, c.kv_heads, c.head_dim, c.rms_eps, ck, cv));
+    if (!appended) {
+        STEP_TRY(launch_qk_norm_rope_append(s, ex->q, ex->k, ex->v, (const float*)t[kAttnQNorm].raw, (const float*)t[kAttnKNorm].raw, ex->inv_freq,
+                                            ex->meta.token_pos, ex->meta.token_slot, T, c.q_heads, c.kv_heads, c.head_dim, c.rms_eps, ck, cv));
+    }
     return launch_attention(s, ex->q, ck, cv, ex->d_page_tables, ex->pages_per_sequence, ex->meta.token_seq, ex->meta.token_pos, T, c.q_heads,
                             c.kv_heads, c.head_dim, 0, plan.max_keys, ex->scratch.attn_partial, ex->scratch.attn_partial_bytes, ex->attn,
                             &launches, plan.run_first, plan.run_count, ex->d_error);
@@ -523,6 +525,7 @@ cudaError_t run_layers_step(ribn_b200_executor* ex, const StepPlan& plan, int& l
     StepOperand normed = ex->op_step, plain = ex->op_step;   // operands a norm's consumer reads / no norm follows
     normed.form = plain.form = step_form(T);
     plain.ss = nullptr;
+    const bool whole_heads = !fused_attention(ex, plan) && c.head_dim == 128;   // the kernel of other widths takes q, k, v as stored
     auto rows = [&](const float* x, const int32_t* index, const float* norm, int members, int k) -> cudaError_t {
         StepFinish f{};
         f.x = x; f.index = index; f.norm_weight = norm; f.members = members;
@@ -537,10 +540,16 @@ cudaError_t run_layers_step(ribn_b200_executor* ex, const StepPlan& plan, int& l
         {
             const StepGemm g = step_qkv(ex, l, T);
             STEP_TRY(launch_step_gemm(s, g, pdl));
-            STEP_TRY(launch_step_finish(s, kFinishStore, &g, StepFinish{}, 0, pdl));
+            if (whole_heads) {
+                const StepQkv qkv{(const float*)t[kAttnQNorm].raw, (const float*)t[kAttnKNorm].raw, ex->inv_freq, ex->meta.token_pos, ex->meta.token_slot,
+                                  c.q_heads, c.kv_heads, c.rms_eps, ex->q, ex->cache_k + (long long)l * ex->layer_stride, ex->cache_v + (long long)l * ex->layer_stride};
+                STEP_TRY(launch_step_qkv(s, g, qkv, pdl));
+            } else {
+                STEP_TRY(launch_step_finish(s, kFinishStore, &g, StepFinish{}, 0, pdl));
+            }
         }
         {
-            cudaError_t e = run_attention(ex, plan, l, pdl, ActOperand{}, launches, plain, &operand_written);
+            cudaError_t e = run_attention(ex, plan, l, pdl, ActOperand{}, launches, plain, &operand_written, whole_heads);
             if (e != cudaSuccess) return e;
         }
         if (!operand_written) STEP_TRY(rows(ex->attn, nullptr, nullptr, T, QD));

@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
     // a: A stages, d: sums, m: the minima's sums; a_full, d_free and m_free are rank 0's
     const uint32_t w_full = bars, w_empty = bars + 32, b_full = bars + 64, b_peer = bars + 96, b_empty = bars + 128, t_full = bars + 160, t_peer = bars + 192,
                    t_empty = bars + 224, a_full = bars + 256, a_free = bars + 272, d_full = bars + 288, d_free = bars + 304, m_free = bars + 320;
-    const int k_tiles = split.k_tiles, groups = split.groups, item_groups = split.item_groups(), runs = split.runs(worker);
+    const int k_tiles = split.k_tiles, groups = split.groups, item_groups = split.unit_items, runs = split.runs(worker);
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < nw; ++i) { mbar_init(w_full + 8 * i, 1); mbar_init(w_empty + 8 * i, kConvertWarps); }

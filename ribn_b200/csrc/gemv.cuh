@@ -280,31 +280,34 @@ struct StepGemm {
     int n_offset[3], total_n;      // filled in by the launcher
 };
 // An item is one group of rows of a unit of weight rows (128; 256 in the wide form), in the wide form up to two neighbouring
-// groups (`joint`).  How a launch's (item, k tile) slots are dealt to its workers (CTAs, a CTA's teams of warps, or in the wide
+// groups.  How a launch's (item, k tile) slots are dealt to its workers (CTAs, a CTA's teams of warps, or in the wide
 // form pairs of CTAs): in whole items, or evenly, an item's slots then lying with consecutive workers.  The wide form takes
 // whole items in rounds, neighbouring workers the same activations side by side, and deals out only the last, incomplete
 // round evenly.  It depends on the matrices and the row groups only.
 struct StepRun { int item, begin, end, part; };   // k tiles [begin, end) of an item, whose sums are its part `part`
 struct StepSplit {
-    int k_tiles, groups, group_members, joint, items, workers, whole, unit_shift;   // unit_shift: log2 of a unit's weight rows
-    int rounds;                                                                     // wide form: rounds of whole items
+    int k_tiles, groups, group_members, joint_shift, items, workers, whole, unit_shift;   // log2 of an item's groups, of a unit's weight rows
+    int unit_items;   // items per unit
+    int rounds;       // wide form: rounds of whole items
     int spread;   // workers that share the even slots: never more than there are slots, so that an item's parts have no gaps
+    uint32_t even_magic;   // 2^32 / even slots, rounded down
     __host__ __device__ int even() const { return items - rounds * workers; }   // items dealt out evenly
-    __host__ __device__ int item_groups() const { return (groups + joint - 1) / joint; }   // items per unit
-    __host__ __device__ int item_of(int unit, int group) const { return unit * item_groups() + group / joint; }
+    __host__ __device__ int item_of(int unit, int group) const { return unit * unit_items + (group >> joint_shift); }
+    __host__ __device__ int first_group(int item) const { return item % unit_items << joint_shift; }
     // (32-bit arithmetic: step_split deals out whole items where slots x workers would not fit)
     __host__ __device__ int begin(int w) const {   // first even slot of worker w; workers past the last one have nothing
         const uint32_t v = (uint32_t)(w < spread ? w : spread) * (uint32_t)even(), n = (uint32_t)spread;
         return (int)(whole ? v / n * (uint32_t)k_tiles : v * (uint32_t)k_tiles / n);
     }
-    __host__ __device__ int first_worker(int item) const {
-        const uint32_t slot = (uint32_t)(item - rounds * workers) * (uint32_t)k_tiles;
-        return (int)(((slot + 1) * (uint32_t)spread - 1) / (uint32_t)(even() * k_tiles));
+    // The worker of an even slot: (slot + 1) x spread - 1 over all even slots.  The finish kernels ask for every thread's, so the
+    // division is a multiplication whose result is at most one too small.
+    __host__ __device__ int worker_of(uint32_t slot) const {
+        const uint32_t v = (slot + 1) * (uint32_t)spread - 1, n = (uint32_t)(even() * k_tiles);
+        const uint32_t q = (uint32_t)((unsigned long long)v * even_magic >> 32);
+        return (int)(v - q * n >= n ? q + 1 : q);
     }
-    __host__ __device__ int last_worker(int item) const {
-        const uint32_t slot = (uint32_t)(item + 1 - rounds * workers) * (uint32_t)k_tiles;
-        return (int)((slot * (uint32_t)spread - 1) / (uint32_t)(even() * k_tiles));
-    }
+    __host__ __device__ int first_worker(int item) const { return worker_of((uint32_t)(item - rounds * workers) * (uint32_t)k_tiles); }
+    __host__ __device__ int last_worker(int item) const { return worker_of((uint32_t)(item + 1 - rounds * workers) * (uint32_t)k_tiles - 1); }
     __host__ __device__ int parts(int item) const {
         return whole || item < rounds * workers ? 1 : last_worker(item) - first_worker(item) + 1;
     }
@@ -324,7 +327,7 @@ struct StepSplit {
     // the group][row of the unit]; the slots of first groups, then those of second ones, so an item's further parts are
     // neighbours.
     __host__ __device__ int slot_floats() const { return group_members << unit_shift; }
-    __host__ __device__ size_t slot_of(int group, int worker) const { return (size_t)(group % joint * workers + worker) * (size_t)slot_floats(); }
+    __host__ __device__ size_t slot_of(int group, int worker) const { return (size_t)((group & ((1 << joint_shift) - 1)) * workers + worker) * (size_t)slot_floats(); }
 };
 // Where a run's sums of row n of segment `seg` lie, from member `m` of the group on: first value and distance of the members.
 struct StepSums { float* at; size_t stride; };
@@ -369,6 +372,17 @@ struct StepFinish {
     float* y[3];
     int n[3], unit0[3], n_offset[3];
 };
+// What follows the q | k | v projection of a step with prompts (head width 128): q, k and v as sums * RMSNorm factor, q and k
+// normalised per head and rotated; q [T][q_heads][128], k and v appended to the paged cache.
+struct StepQkv {
+    const float *q_norm, *k_norm, *inv_freq;
+    const int32_t *token_pos, *token_slot;
+    int q_heads, kv_heads;
+    float eps;
+    float* q;
+    __half *cache_k, *cache_v;
+};
+cudaError_t launch_step_qkv(cudaStream_t stream, const StepGemm& gemm, const StepQkv& args, bool programmatic);
 // `gemm`: the split launch whose sums are finished (null for kFinishRows); `width`: values per row of the operand.
 cudaError_t launch_step_finish(cudaStream_t stream, int mode, const StepGemm* gemm, StepFinish args, int width, bool programmatic);
 

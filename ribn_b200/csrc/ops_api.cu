@@ -123,9 +123,9 @@ int ribn_b200_debug_step_deal(int32_t form, int64_t rows, int64_t cols, int32_t 
     for (int w = 0; w < s.workers; ++w) {
         for (int r = 0; r < s.runs(w); ++r) {
             const StepRun run = s.run(w, r);
-            const int unit = run.item / s.item_groups(), group0 = run.item % s.item_groups() * s.joint;
+            const int unit = run.item / s.unit_items, group0 = s.first_group(run.item);
             // a worker of two groups at a time counts as two, each with its own slots of sums
-            for (int u = 0; u < s.joint && group0 + u < s.groups; ++u, ++*count) {
+            for (int u = 0; u < 1 << s.joint_shift && group0 + u < s.groups; ++u, ++*count) {
                 if (*count >= capacity) continue;
                 const bool dealt = !s.whole && run.item >= s.rounds * s.workers;
                 const int own = u * s.workers;

@@ -122,6 +122,64 @@ __global__ void __launch_bounds__(256) step_store_kernel(const StepFinish a) {
     *reinterpret_cast<float4*>(a.y[seg] + (size_t)m * a.n[seg] + n) = make_float4(s.x * inv, s.y * inv, s.z * inv, s.w * inv);
 }
 
+// One block per token: the rotation's factors once for all its heads, then a warp per head, four neighbouring dimensions per
+// thread; the next head's first sums are requested under the present one.  (A store of q, k and v and a warp per token and
+// head behind it took 15.5 + 16.5 us at 777 tokens of the 0.6B model, 35 + 41 us at 2,048 of the 8B model; this 17 and 34 us,
+// with eight or sixteen warps 18 to 19 and 36 to 41 us.)
+constexpr int kQkvHead = 128, kQkvWarps = 4;
+__global__ void __launch_bounds__(kQkvWarps * 32) step_qkv_kernel(const StepFinish a, const StepQkv c) {
+    __shared__ float2 turn[kQkvHead / 2];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, heads = c.q_heads + 2 * c.kv_heads;
+    if (threadIdx.x < kQkvHead / 2) {   // positions are older than the projection
+        const float theta = (float)c.token_pos[t] * c.inv_freq[threadIdx.x];
+        turn[threadIdx.x] = make_float2(cosf(theta), sinf(theta));
+    }
+    const long long slot = c.token_slot[t];
+    const float4 wq = load4(c.q_norm + 4 * lane), wk = load4(c.k_norm + 4 * lane);
+    auto place = [&](int h) {
+        const int seg = h < c.q_heads ? 0 : h < c.q_heads + c.kv_heads ? 1 : 2;
+        return parts_of(a, seg, t, (h - (seg == 0 ? 0 : seg == 1 ? c.q_heads : c.q_heads + c.kv_heads)) * kQkvHead + 4 * lane);
+    };
+    Parts p{};
+    if (warp < heads) p = place(warp);
+    __syncthreads();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    float4 first = warp < heads ? load4(p.at) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const float inv = a.ss != nullptr ? norm_factor(a.ss + (size_t)t * a.split.k_tiles, a.split.k_tiles, a.eps, lane) : 1.0f;
+    for (int h = warp; h < heads; h += kQkvWarps) {
+        Parts next{};
+        float4 next_first = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (h + kQkvWarps < heads) { next = place(h + kQkvWarps); next_first = load4(next.at); }
+        float4 x = add_parts<2>(a, p, first);
+        x.x *= inv; x.y *= inv; x.z *= inv; x.w *= inv;
+        auto append = [&](__half* cache, int head) {
+            const __half2 lo = __floats2half2_rn(x.x, x.y), hi = __floats2half2_rn(x.z, x.w);
+            *reinterpret_cast<uint2*>(cache + (slot * c.kv_heads + head) * kQkvHead + 4 * lane) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+        };
+        if (h >= c.q_heads + c.kv_heads) {
+            append(c.cache_v, h - c.q_heads - c.kv_heads);
+        } else {
+            float sum = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, x.w * x.w)));
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            const float r = 1.0f / sqrtf(sum / (float)kQkvHead + c.eps);
+            const float4 w = h < c.q_heads ? wq : wk;
+            x.x = x.x * r * w.x; x.y = x.y * r * w.y; x.z = x.z * r * w.z; x.w = x.w * r * w.w;
+            // dimension d turns with d + 64, sixteen lanes further
+            const float4 o = make_float4(__shfl_xor_sync(0xffffffffu, x.x, 16), __shfl_xor_sync(0xffffffffu, x.y, 16),
+                                         __shfl_xor_sync(0xffffffffu, x.z, 16), __shfl_xor_sync(0xffffffffu, x.w, 16));
+            const float4 t0 = *reinterpret_cast<const float4*>(&turn[4 * (lane & 15)]), t1 = *reinterpret_cast<const float4*>(&turn[4 * (lane & 15) + 2]);
+            auto rotate = [&](float mine, float other, float cosine, float sine) { return lane < 16 ? mine * cosine - other * sine : other * sine + mine * cosine; };
+            x = make_float4(rotate(x.x, o.x, t0.x, t0.y), rotate(x.y, o.y, t0.z, t0.w), rotate(x.z, o.z, t1.x, t1.y), rotate(x.w, o.w, t1.z, t1.w));
+            if (h < c.q_heads) *reinterpret_cast<float4*>(c.q + ((size_t)t * c.q_heads + h) * kQkvHead + 4 * lane) = x;
+            else append(c.cache_k, h - c.q_heads);
+        }
+        p = next;
+        first = next_first;
+    }
+}
+
 int device_sms() {
     static int counts[kMaxDevices] = {0};
     int dev = 0;
@@ -206,8 +264,9 @@ StepSplit step_split(const StepGemm& a, bool whole_items) {
     s.k_tiles = a.k / kTileCols;
     s.groups = shape.groups;
     s.group_members = shape.ng * 8;
-    s.joint = a.form == kWideForm ? 2 : 1;
-    for (int i = 0; i < a.n_segments; ++i) s.items += (a.seg[i].row_tiles + tiles - 1) / tiles * s.item_groups();
+    s.joint_shift = a.form == kWideForm ? 1 : 0;
+    s.unit_items = (s.groups + s.joint_shift) >> s.joint_shift;
+    for (int i = 0; i < a.n_segments; ++i) s.items += (a.seg[i].row_tiles + tiles - 1) / tiles * s.unit_items;
     if ((unsigned long long)s.items * s.k_tiles * (device_sms() * kFragTeams) >> 32) whole_items = true;
     s.whole = whole_items ? 1 : 0;
     const int workers = a.form == kWideForm ? device_sms() / 2 : device_sms() * (a.form == kFragmentForm ? kFragTeams : 1);
@@ -218,6 +277,7 @@ StepSplit step_split(const StepGemm& a, bool whole_items) {
     s.rounds = a.form == kWideForm && s.groups != 3 ? s.items / s.workers : 0;
     if (s.rounds * s.workers == s.items && s.rounds > 0) s.whole = 1;   // nothing is left to deal out evenly
     s.spread = std::max(1, s.whole ? std::min(s.workers, s.even()) : std::min(s.workers, s.even() * s.k_tiles));
+    s.even_magic = (uint32_t)std::min<unsigned long long>(0xFFFFFFFFull, (1ull << 32) / (unsigned long long)std::max(1, s.even() * s.k_tiles));
     return s;
 }
 
@@ -229,7 +289,7 @@ size_t step_partial_floats(const StepGemm& a) {
 
 size_t step_further_floats(const StepGemm& a) {
     const StepSplit s = step_split(a, false);
-    return s.whole ? 0 : s.slot_of(s.joint - 1, s.spread);
+    return s.whole ? 0 : s.slot_of((1 << s.joint_shift) - 1, s.spread);
 }
 
 cudaError_t launch_step_gemm(cudaStream_t stream, const StepGemm& args, bool programmatic) {
@@ -250,28 +310,43 @@ cudaError_t launch_step_gemm(cudaStream_t stream, const StepGemm& args, bool pro
     return a.form == kColumnForm ? launch_gemm_ta(stream, a, w_bytes, programmatic) : launch_gemm_frag(stream, a, w_bytes, programmatic);
 }
 
+namespace {
+// The fields that come from a split launch; false where its outputs are not multiples of four.
+bool fill_parts(const StepGemm& gemm, StepFinish& a) {
+    a.split = step_split(gemm, false);
+    a.partial = gemm.partial;
+    a.further = gemm.further;
+    a.members = gemm.members;
+    a.n_segments = gemm.n_segments;
+    a.ss = gemm.ss;
+    a.eps = gemm.eps;
+    int units = 0;
+    a.total_n = 0;
+    for (int i = 0; i < gemm.n_segments; ++i) {
+        a.y[i] = gemm.seg[i].y;
+        a.n[i] = gemm.seg[i].n;
+        a.unit0[i] = units;
+        a.n_offset[i] = a.total_n;
+        units += (gemm.seg[i].n + (1 << a.split.unit_shift) - 1) >> a.split.unit_shift;
+        a.total_n += gemm.seg[i].n;
+        if (gemm.seg[i].n % 4 != 0) return false;
+    }
+    return true;
+}
+}  // namespace
+
+cudaError_t launch_step_qkv(cudaStream_t stream, const StepGemm& gemm, const StepQkv& args, bool programmatic) {
+    StepFinish a{};
+    if (gemm.members < 1 || gemm.n_segments != 3 || gemm.seg[0].n != args.q_heads * kQkvHead || gemm.seg[1].n != args.kv_heads * kQkvHead ||
+        gemm.seg[2].n != gemm.seg[1].n || !fill_parts(gemm, a)) {
+        return cudaErrorInvalidValue;
+    }
+    return launch_pdl(step_qkv_kernel, dim3((unsigned)gemm.members), kQkvWarps * 32, 0, stream, programmatic, a, args);
+}
+
 cudaError_t launch_step_finish(cudaStream_t stream, int mode, const StepGemm* gemm, StepFinish a, int width, bool programmatic) {
     a.n_segments = 0;
-    if (gemm != nullptr) {
-        a.split = step_split(*gemm, false);
-        a.partial = gemm->partial;
-        a.further = gemm->further;
-        a.members = gemm->members;
-        a.n_segments = gemm->n_segments;
-        a.ss = gemm->ss;
-        a.eps = gemm->eps;
-        int units = 0;
-        a.total_n = 0;
-        for (int i = 0; i < gemm->n_segments; ++i) {
-            a.y[i] = gemm->seg[i].y;
-            a.n[i] = gemm->seg[i].n;
-            a.unit0[i] = units;
-            a.n_offset[i] = a.total_n;
-            units += (gemm->seg[i].n + (1 << a.split.unit_shift) - 1) >> a.split.unit_shift;
-            a.total_n += gemm->seg[i].n;
-            if (gemm->seg[i].n % 4 != 0) return cudaErrorInvalidValue;
-        }
-    }
+    if (gemm != nullptr && !fill_parts(*gemm, a)) return cudaErrorInvalidValue;
     if (a.members < 1) return cudaErrorInvalidValue;
     if (mode == kFinishStore) {
         return launch_pdl(a.members <= kColumnMaxMembers ? step_store_kernel<7> : step_store_kernel<2>, dim3((unsigned)((a.total_n / 4 + 255) / 256), (unsigned)a.members), 256, 0, stream, programmatic, a);

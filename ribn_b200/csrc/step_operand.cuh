@@ -20,12 +20,13 @@ __device__ __forceinline__ float power2(int k) { return __int_as_float((k + 127)
 // sum of squares.
 __device__ __forceinline__ void write_step_operand(const StepOperand& out, int kt, int k_tiles, int eight, bool have, const float4 v, float square, StepStage& stage) {
     const int tid = threadIdx.x, g = tid >> 6, i = tid & 63, lane = tid & 31;
-    // the tile's largest magnitude and sum of squares over the member's 64 threads
+    // the tile's largest magnitude and, for a norm's consumer, its sum of squares, over the member's 64 threads
     float top = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-        square += __shfl_xor_sync(0xffffffffu, square, o);
+    for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+    if (out.ss != nullptr) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) square += __shfl_xor_sync(0xffffffffu, square, o);
     }
     if (lane == 0) { stage.tops[tid >> 5] = top; stage.squares[tid >> 5] = square; }
     __syncthreads();
@@ -35,17 +36,14 @@ __device__ __forceinline__ void write_step_operand(const StepOperand& out, int k
     const int e = biased == 255 ? 10 : max(-126, min(126, 136 - biased));
     const float scale = power2(e);
     if (i == 0 && have && out.ss != nullptr) out.ss[(size_t)(eight * 8 + g) * k_tiles + kt] = stage.squares[2 * g] + stage.squares[2 * g + 1];
-    const float s4[4] = {v.x * scale, v.y * scale, v.z * scale, v.w * scale};
-    __half hi[4], lo[4];
-    float sum = 0.0f;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        hi[j] = __float2half_rn(s4[j]);
-        lo[j] = __float2half_rn(s4[j] - __half2float(hi[j]));
-        sum += __half2float(hi[j]) + __half2float(lo[j]);   // what the tensor core will see
-    }
+    // hi and lo of inputs 0, 2 and 1, 3; the sum of what the tensor core will see
+    const __half2 h02 = __floats2half2_rn(v.x * scale, v.z * scale), h13 = __floats2half2_rn(v.y * scale, v.w * scale);
+    const float2 b02 = __half22float2(h02), b13 = __half22float2(h13);
+    const __half2 l02 = __floats2half2_rn(v.x * scale - b02.x, v.z * scale - b02.y), l13 = __floats2half2_rn(v.y * scale - b13.x, v.w * scale - b13.y);
+    const float2 r02 = __half22float2(l02), r13 = __half22float2(l13);
+    float sum = (((b02.x + r02.x) + (b13.x + r13.x)) + (b02.y + r02.y)) + (b13.y + r13.y);
+    auto bits = [](const __half2& x) { return *reinterpret_cast<const uint32_t*>(&x); };
     const int group = eight / out.ng, ng = eight - group * out.ng;
-    auto pack = [](__half x, __half y) { const __half2 p = __halves2half2(x, y); return *reinterpret_cast<const uint32_t*>(&p); };
     const int s = i >> 2, t = i & 3;
     const float inv_scale = power2(-e);
     if (out.form != kFragmentForm) {
@@ -56,10 +54,10 @@ __device__ __forceinline__ void write_step_operand(const StepOperand& out, int k
         // stores are whole 128-byte lines.  stage.pieces[8-input block][hi, lo][member ^ step % 8]: conflict-free both ways.
         {
             uint32_t* at = reinterpret_cast<uint32_t*>(&stage.pieces[2 * s][0][g ^ (s & 7)]) + t;
-            at[0] = pack(hi[0], hi[2]);
-            at[32] = pack(lo[0], lo[2]);
-            at[64] = pack(hi[1], hi[3]);          // the next 8-input block
-            at[96] = pack(lo[1], lo[3]);
+            at[0] = bits(h02);
+            at[32] = bits(l02);
+            at[64] = bits(h13);          // the next 8-input block
+            at[96] = bits(l13);
         }
         __syncthreads();
         {
@@ -81,7 +79,7 @@ __device__ __forceinline__ void write_step_operand(const StepOperand& out, int k
         return;
     }
     unsigned char* blk = out.blocks + (((size_t)group * k_tiles + kt) * out.ng + ng) * kFragBlockBytes;
-    *reinterpret_cast<uint4*>(blk + s * 512 + (g * 4 + t) * 16) = make_uint4(pack(hi[0], hi[2]), pack(hi[1], hi[3]), pack(lo[0], lo[2]), pack(lo[1], lo[3]));
+    *reinterpret_cast<uint4*>(blk + s * 512 + (g * 4 + t) * 16) = make_uint4(bits(h02), bits(h13), bits(l02), bits(l13));
     sum += __shfl_xor_sync(0xffffffffu, sum, 1);
     sum += __shfl_xor_sync(0xffffffffu, sum, 2);
     sum += __shfl_xor_sync(0xffffffffu, sum, 4);

@@ -714,3 +714,30 @@ def test_decode_rows_of_one_and_of_many_spans_share_a_step(built_library, rows, 
         ex.close()
     assert np.all(np.isfinite(logits[0]))
     assert close(logits[0], logits[1])
+
+
+@pytest.mark.parametrize("q_heads,kv_heads", [(8, 2), (4, 4), (2, 1)])
+@pytest.mark.parametrize("tokens", [3, 17, 65, 130, 300])
+def test_prompt_rows_are_normalised_rotated_and_appended_in_one_pass(built_library, tokens, q_heads, kv_heads):
+    """The kernel behind a prompt's q | k | v projection (head width 128) in each operand form and row-group count, group sizes 1
+    to 4: cached keys and values against the plain reference-style kernels' to the last binary16 place or two (F32 sums in
+    another order can move a rounding), and the logits that follow."""
+    import ribn_b200
+    from ribn_b200 import BatchItem, StepKind
+    cfg = dict(layers=2, hidden=512, q_heads=q_heads, kv_heads=kv_heads, head_dim=128, ffn=1024, vocab=1024, rope_base=1.0e6, rms_eps=1.0e-6)
+    prompt = np.random.default_rng(tokens).integers(0, cfg["vocab"], tokens).tolist()
+    results = []
+    for flags in (0, ribn_b200.FLAG_REFERENCE_KERNELS):
+        ex = ribn_b200.QwenB200(cfg, flags=flags | ribn_b200.FLAG_KEEP_LOGITS, context_tokens=512, max_sequences=1, max_batch_tokens=512)
+        ex.init_synthetic(29, ribn_b200.SCHEME_Q4_K_M)
+        ex.finalize()
+        assert ex.admit(1, 1, prompt, 4).ready
+        item = BatchItem(1, StepKind.PREFILL, 0, tokens, 1)
+        ex.prepare([item])
+        ex.wait(ex.submit([item]))
+        results.append([ex.copy_logits(0).copy()] + [np.asarray(ex.copy_kv(1, layer, which, tokens)).view(np.float16).astype(np.float32).copy()
+                                                     for layer in range(2) for which in range(2)])
+        ex.close()
+    assert close(results[0][0], results[1][0])
+    for got, want in zip(results[0][1:], results[1][1:]):
+        assert np.all(np.abs(got - want) <= 2.0 ** -9 * np.abs(want) + 2.0 ** -11 * np.abs(want).max())
