@@ -506,7 +506,9 @@ struct Cursor {
 // SHARED = false: each team of eight warps owns whole units (many units per CTA: the output head).
 // SHARED = true: all 24 warps cooperate on every unit, the teams taking alternate stages (the layer
 // projections, which give a CTA only one to three units).
-template <int MEMBERS, bool SHARED>
+// TYPE: the block type of all the launch's matrices, or kAnyType.
+constexpr int kAnyType = -1;
+template <int MEMBERS, bool SHARED, int TYPE>
 __global__ void __launch_bounds__(kThreads, 1) gemv_mma_kernel(const GemvArgs a, const int slots_per_team,
                                                                const int slot_bytes) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -734,50 +736,46 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_mma_kernel(const GemvArgs a,
     int turn = 0;
     int buf = 0, done = 0;
     for (int u = u0 + set; u < u1; u += unit_step, buf ^= 1, ++done) {
-        Accum acc[kMaxRuns];
-#pragma unroll
-        for (int r = 0; r < kMaxRuns; ++r) {
-            acc[r].c[0] = acc[r].c[1] = acc[r].c[2] = acc[r].c[3] = 0.0f;
-            acc[r].s[0] = acc[r].s[1] = 0.0f;
-        }
-#pragma unroll
-        for (int r = 0; r < kMaxRuns; ++r) {
-            if (r >= runs) break;
-            const GemvSegment* seg = nullptr;
-            int rt = 0;
-            if (!locate(u, r, seg, rt)) continue;
-            const int type = seg->type;
-            const int tile_bytes = packed_tile_bytes(type);
-            for (int st = 0; st < stages_per_run; ++st) {
-                if (!SHARED || turn == team) {  // SHARED: the teams take the stages in turn
-                    const uint32_t slot = SHARED ? ring_pos : ring_pos * kTeams + team;
-                    if (alive) alive = mbar_wait(sh.full + slot * 8, ring_parity, a.error_flag, 3, spin_limit);
-                    const int kb = st * kStageTiles + member_warp;
-                    if (kb < k_tiles) {
-                        const uint32_t tile = ring + slot * (uint32_t)slot_bytes + (uint32_t)(member_warp * tile_bytes);
-                        if (type == kQ4_K) tile_q4k<MEMBERS>(tile, ln, kb, lane, acc[r]);
-                        else if (type == kQ6_K) tile_q6k<MEMBERS>(tile, ln, kb, lane, acc[r]);
-                        else tile_q8_0<MEMBERS>(tile, ln, kb, lane, acc[r]);
-                    }
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(sh.empty + slot * 8);  // this warp has left the stage
-                }
-                if (++ring_pos == ring_len) { ring_pos = 0; ring_parity ^= 1u; }
-                if (++turn == kTeams) turn = 0;
-            }
-        }
-        // Per-warp partial of (row, member): digits 1 and 2 are this lane's two columns, digit 3 is the
-        // first column of the next lane; lanes with even t own member t / 2.
         if (done >= 2) bar_sync(kBarFree + set * 4 + buf, bar_threads);  // the epilogue warp has read this buffer
         float* red = sh.red + ((size_t)(set * 2 + buf) * kSetWarps + set_warp) * kMaxRuns * MEMBERS * 16;
-#pragma unroll
-        for (int r = 0; r < kMaxRuns; ++r) {
-            if (r >= runs) break;
-            const float d3a = __shfl_down_sync(0xffffffffu, acc[r].c[0], 1);
-            const float d3b = __shfl_down_sync(0xffffffffu, acc[r].c[2], 1);
+        // One copy of the tile code for all runs: a launch is a few tiles per warp, and with a copy per run and block type
+        // most of its time went into fetching instructions (see the file's head).
+#pragma unroll 1
+        for (int r = 0; r < runs; ++r) {
+            Accum acc;
+            acc.c[0] = acc.c[1] = acc.c[2] = acc.c[3] = 0.0f;
+            acc.s[0] = acc.s[1] = 0.0f;
+            const GemvSegment* seg = nullptr;
+            int rt = 0;
+            if (locate(u, r, seg, rt)) {
+                const int type = TYPE == kAnyType ? seg->type : TYPE;
+                const int tile_bytes = packed_tile_bytes(type);
+#pragma unroll 1
+                for (int st = 0; st < stages_per_run; ++st) {
+                    if (!SHARED || turn == team) {  // SHARED: the teams take the stages in turn
+                        const uint32_t slot = SHARED ? ring_pos : ring_pos * kTeams + team;
+                        if (alive) alive = mbar_wait(sh.full + slot * 8, ring_parity, a.error_flag, 3, spin_limit);
+                        const int kb = st * kStageTiles + member_warp;
+                        if (kb < k_tiles) {
+                            const uint32_t tile = ring + slot * (uint32_t)slot_bytes + (uint32_t)(member_warp * tile_bytes);
+                            if (type == kQ4_K) tile_q4k<MEMBERS>(tile, ln, kb, lane, acc);
+                            else if (type == kQ6_K) tile_q6k<MEMBERS>(tile, ln, kb, lane, acc);
+                            else tile_q8_0<MEMBERS>(tile, ln, kb, lane, acc);
+                        }
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(sh.empty + slot * 8);  // this warp has left the stage
+                    }
+                    if (++ring_pos == ring_len) { ring_pos = 0; ring_parity ^= 1u; }
+                    if (++turn == kTeams) turn = 0;
+                }
+            }
+            // Per-warp partial of (row, member): digits 1 and 2 are this lane's two columns, digit 3 is the
+            // first column of the next lane; lanes with even t own member t / 2.
+            const float d3a = __shfl_down_sync(0xffffffffu, acc.c[0], 1);
+            const float d3b = __shfl_down_sync(0xffffffffu, acc.c[2], 1);
             if ((t & 1) == 0 && (t >> 1) < MEMBERS) {
-                const float va = acc[r].c[0] + acc[r].c[1] * (1.0f / 128.0f) + d3a * (1.0f / 16384.0f) + acc[r].s[0];
-                const float vb = acc[r].c[2] + acc[r].c[3] * (1.0f / 128.0f) + d3b * (1.0f / 16384.0f) + acc[r].s[1];
+                const float va = acc.c[0] + acc.c[1] * (1.0f / 128.0f) + d3a * (1.0f / 16384.0f) + acc.s[0];
+                const float vb = acc.c[2] + acc.c[3] * (1.0f / 128.0f) + d3b * (1.0f / 16384.0f) + acc.s[1];
                 float* dst = red + ((size_t)r * MEMBERS + (t >> 1)) * 16;
                 dst[g] = va;
                 dst[g + 8] = vb;
@@ -831,17 +829,37 @@ int sm_count() {
 // Leaves a few KB of the SM's shared memory to small kernels that overlap this one's tail or head.
 constexpr size_t kSmemBudget = 208 * 1024;
 
+namespace {
+using GemvKernel = void (*)(GemvArgs, int, int);
+template <int MEMBERS, bool SHARED>
+GemvKernel gemv_kernel_of(int type) {
+    switch (type) {
+        case kQ4_K: return gemv_mma_kernel<MEMBERS, SHARED, kQ4_K>;
+        case kQ6_K: return gemv_mma_kernel<MEMBERS, SHARED, kQ6_K>;
+        case kQ8_0: return gemv_mma_kernel<MEMBERS, SHARED, kQ8_0>;
+        default: return gemv_mma_kernel<MEMBERS, SHARED, kAnyType>;
+    }
+}
+GemvKernel gemv_kernel(int members, bool shared, int type) {
+    if (members == 1) return shared ? gemv_kernel_of<1, true>(type) : gemv_kernel_of<1, false>(type);
+    return shared ? gemv_kernel_of<2, true>(type) : gemv_kernel_of<2, false>(type);
+}
+}  // namespace
+
 cudaError_t gemv_prepare() {
     static bool configured_on[kMaxDevices] = {false};  // function attributes are per device
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
     bool& configured = configured_on[dev];
     if (!configured) {
-        const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
-        cudaError_t e = cudaFuncSetAttribute(gemv_mma_kernel<1, false>, at, (int)kSmemBudget);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemv_mma_kernel<1, true>, at, (int)kSmemBudget);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemv_mma_kernel<2, false>, at, (int)kSmemBudget);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemv_mma_kernel<2, true>, at, (int)kSmemBudget);
+        cudaError_t e = cudaSuccess;
+        for (int members = 1; members <= kGemvMaxMembers; ++members) {
+            for (int shared = 0; shared < 2; ++shared) {
+                for (const int type : {(int)kQ4_K, (int)kQ6_K, (int)kQ8_0, kAnyType}) {
+                    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemv_kernel(members, shared != 0, type), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget);
+                }
+            }
+        }
         if (e != cudaSuccess) return e;
         sm_count();
         configured = true;
@@ -935,12 +953,9 @@ cudaError_t launch_gemv_mma(cudaStream_t stream, const GemvArgs& args, bool prog
     cfg.numAttrs = programmatic ? 1 : 0;
     // Few units per CTA: let all the warps cooperate on each unit.
     const bool shared = units < 2 * kTeams * grid;
-    if (args.members == 1) {
-        return shared ? cudaLaunchKernelEx(&cfg, gemv_mma_kernel<1, true>, args, slots_per_team, slot_bytes)
-                      : cudaLaunchKernelEx(&cfg, gemv_mma_kernel<1, false>, args, slots_per_team, slot_bytes);
-    }
-    return shared ? cudaLaunchKernelEx(&cfg, gemv_mma_kernel<2, true>, args, slots_per_team, slot_bytes)
-                  : cudaLaunchKernelEx(&cfg, gemv_mma_kernel<2, false>, args, slots_per_team, slot_bytes);
+    int type = args.seg[0].type;
+    for (int i = 1; i < args.n_segments; ++i) if (args.seg[i].type != type) type = kAnyType;
+    return cudaLaunchKernelEx(&cfg, gemv_kernel(args.members, shared, type), args, slots_per_team, slot_bytes);
 }
 
 }  // namespace ribn
