@@ -983,7 +983,7 @@ cudaError_t launch_hd(cudaStream_t stream, AttnArgs a, bool fused, int n_tokens,
         a.run_first + a.run_count <= n_tokens) {
         if (HD == 128) {
             const PrefillAttention p{a.q, a.cache_k, a.cache_v, a.page_tables, a.pages_per_sequence, a.token_seq, a.token_pos,
-                                     a.run_first, a.run_count, a.q_heads, a.kv_heads, a.out, a.error_flag};
+                                     a.run_first, a.run_count, a.q_heads, a.kv_heads, max_keys, a.out, a.error_flag};
             cudaError_t e = launch_attention_tc(stream, p);
             if (e != cudaSuccess) return e;
             if (launches) ++*launches;

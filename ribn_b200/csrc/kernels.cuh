@@ -123,6 +123,7 @@ struct PrefillAttention {
     const int32_t* token_seq;   // may be null: sequence 0
     const int32_t* token_pos;
     int first, count, q_heads, kv_heads;
+    int max_keys;               // at least the keys of the last token
     float* out;
     int* error_flag;            // set non-zero when a bounded wait gives up
 };

@@ -370,10 +370,11 @@ def test_decode_attention_at_long_contexts(ops, QH, KVH, HD, tokens):
 
 
 @pytest.mark.parametrize("QH,KVH,tokens,rows", [(32, 8, 64, 64), (32, 8, 65, 65), (32, 8, 193, 129), (16, 8, 257, 257), (12, 4, 300, 171),
-                                                (8, 8, 400, 400), (16, 1, 130, 100)])
+                                                (8, 8, 400, 400), (16, 1, 130, 100), (32, 8, 737, 641), (32, 8, 1300, 70)])
 def test_prefill_chunk_attention_at_the_edges_of_its_tiles(ops, QH, KVH, tokens, rows):
     """The tensor-memory prefill kernel (head width 128): chunks that end inside a query tile, a key tile and a page, with
-    and without a cached prefix, group sizes 1 to 16 (3: rows of a tile that belong to no token).  Slots of the last page that
+    and without a cached prefix, group sizes 1 to 16 (3: rows of a tile that belong to no token); one, two and many key tiles
+    shared by the softmax groups of a CTA, and the launch of pairs of query tiles (641 rows).  Slots of the last page that
     hold no key carry NaN: nothing may read them.  Scores and probabilities are binary16 hi + lo pairs (22 bits) with F32
     sums: an error of |q| |k| 2^-22 in a score of a few units, 2e-6 of a result, with room for the sums."""
     HD = 128
