@@ -63,6 +63,7 @@ __device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_ca
 template <int MODE, int BATCH>
 __global__ void __launch_bounds__(512, BATCH > 2 ? 1 : 3) step_finish_kernel(const StepFinish a) {
     __shared__ StepStage stage;
+    __shared__ float factors[8];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int kt = blockIdx.x, tid = threadIdx.x, g = tid >> 6, i = tid & 63, lane = tid & 31;
     const int m = blockIdx.y * 8 + g, n = kt * kTileCols + 4 * i, k_tiles = gridDim.x, width = k_tiles * kTileCols;
@@ -77,7 +78,7 @@ __global__ void __launch_bounds__(512, BATCH > 2 ? 1 : 3) step_finish_kernel(con
         if (a.norm_weight != nullptr) w = load4(a.norm_weight + n);
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f), gt = v, up = v;
     float square = 0.0f;
     if (m < a.members) {
         if (MODE == kFinishRows) {
@@ -91,11 +92,34 @@ __global__ void __launch_bounds__(512, BATCH > 2 ? 1 : 3) step_finish_kernel(con
         } else {
             if (!kAhead) { p0 = parts_of(a, 0, m, n); p1 = parts_of(a, 1, m, n); }
             const float4 first_g = load4(p0.at), first_u = load4(p1.at);
-            const float inv = a.ss != nullptr ? norm_factor(a.ss + (size_t)m * a.split.k_tiles, a.split.k_tiles, a.eps, lane) : 1.0f;
-            const float4 gt = add_parts<BATCH>(a, p0, first_g), up = add_parts<BATCH>(a, p1, first_u);
-            auto act = [&](float x, float u) { x *= inv; return x / (1.0f + expf(-x)) * (u * inv); };
-            v = make_float4(act(gt.x, up.x), act(gt.y, up.y), act(gt.z, up.z), act(gt.w, up.w));
+            if (tid < 32) {
+                // the eight members' RMSNorm factors, four lanes each, once for the block: in every warp they were a third of its instructions
+                const int row = blockIdx.y * 8 + (lane >> 2);
+                float sum = 0.0f;
+                if (a.ss != nullptr && row < a.members) for (int j = lane & 3; j < a.split.k_tiles; j += 4) sum += a.ss[(size_t)row * a.split.k_tiles + j];
+                sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+                sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+                if ((lane & 3) == 0) factors[lane >> 2] = a.ss != nullptr ? 1.0f / sqrtf(sum / (float)(a.split.k_tiles * kTileCols) + a.eps) : 1.0f;
+            }
+            gt = add_parts<BATCH>(a, p0, first_g);
+            up = add_parts<BATCH>(a, p1, first_u);
         }
+    }
+    if (MODE == kFinishSwiGLU) {
+        __syncthreads();
+        const float inv = factors[g];
+        // silu(x) u: the quotient by 1 + e^-x from the reciprocal, its remainder folded back (e^87: the quotient is below 1e-35)
+        auto act = [&](float x, float u) {
+            x *= inv;
+            const float den = 1.0f + expf(fminf(-x, 87.0f));
+            float r;
+            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(den));
+            const float q = x * r, exact = fmaf(fmaf(-q, den, x), r, q);
+            return (fabsf(q) < INFINITY ? exact : q) * (u * inv);
+        };
+        v = make_float4(act(gt.x, up.x), act(gt.y, up.y), act(gt.z, up.z), act(gt.w, up.w));
+    }
+    if (m < a.members) {
         square = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w)));
         if (a.norm_weight != nullptr) {
             if (!kAhead) w = load4(a.norm_weight + n);
