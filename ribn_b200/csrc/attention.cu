@@ -895,15 +895,17 @@ cudaError_t launch_spans_hd(cudaStream_t stream, AttnArgs a, bool fused, int fir
     a.run_tokens = (!fused && a.window <= 0 && a.operand.dig == nullptr && n_tokens >= 16) ? std::max(1, 16 / q_per_kv) : 1;
     const long long item_tokens = (n_tokens + a.run_tokens - 1) / a.run_tokens;
     // Tiles per span: the fewest tile-times on the busiest of the resident CTAs (three per SM), an item's set-up and fold
-    // counted as one tile and a span's share of the merge as a quarter.  (One tile per span while that did not fill the
-    // GPU sixteen times over left two rows at 6,144 keys with 104 spans: 24 us of spans and 18 us of merge per layer.)
+    // counted as one and a half and every eight spans, which the merge requests together, as a half.  (One tile per span while
+    // that did not fill the GPU sixteen times over left two rows at 6,144 keys with 104 spans: 24 us of spans and 18 us of
+    // merge per layer.  A quarter per span, as if the merge took them one by one, gave one row at 1,024 keys two tiles a span:
+    // its step took 0.79 ms against 0.755 of the 0.6B model.)
     const long long ctas = 3ll * attn_sm_count();
     float best = 0.0f;
     a.tiles = 1;
     for (int tiles = 1; tiles <= std::min(16, max_tiles); ++tiles) {
         const int spans = (max_tiles + tiles - 1) / tiles;
         const long long waves = (item_tokens * a.kv_heads * spans + ctas - 1) / ctas;
-        const float cost = (float)waves * (float)(tiles + 1) + 0.25f * (float)spans;
+        const float cost = (float)waves * ((float)tiles + 1.5f) + 0.45f * (float)((spans + 7) / 8);
         if (tiles == 1 || cost < best) { best = cost; a.tiles = tiles; }
     }
     a.max_spans = (max_tiles + a.tiles - 1) / a.tiles;
