@@ -61,7 +61,7 @@ __device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_ca
 
 // One block: a k tile of eight members (write_step_operand).  MODE: where the values come from (StepFinishMode).
 template <int MODE, int BATCH>
-__global__ void __launch_bounds__(512, BATCH > 2 ? 1 : 3) step_finish_kernel(const StepFinish a) {
+__global__ void __launch_bounds__(512, BATCH > 4 ? 1 : BATCH > 2 ? 2 : 3) step_finish_kernel(const StepFinish a) {
     __shared__ StepStage stage;
     __shared__ float factors[8];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -382,14 +382,18 @@ cudaError_t launch_step_finish(cudaStream_t stream, int mode, const StepGemm* ge
     const StepShape shape = step_shape(a.members, a.out.form);
     a.out.ng = shape.ng;
     const dim3 grid((unsigned)(width / kTileCols), (unsigned)(shape.groups * shape.ng));
-    // one block per SM while that is a single wave of blocks (see add_parts)
-    const bool deep = grid.x * grid.y <= (unsigned)device_sms();
+    // one block per SM while that is a single wave of blocks, two less deep ones, then three (see add_parts; the middle form: 300
+    // tokens of the 0.6B model 3.57 -> 3.46 ms; for all larger launches 1 % slower at 2,048 tokens of the 8B model)
+    const unsigned blocks = grid.x * grid.y, sms = (unsigned)device_sms();
+    const int deep = blocks <= sms ? 7 : blocks <= 3 * sms ? 4 : 2;
     switch (mode) {
         case kFinishRows: return launch_pdl(step_finish_kernel<kFinishRows, 2>, grid, 512, 0, stream, programmatic, a);
         case kFinishResidual:
-            return launch_pdl(deep ? step_finish_kernel<kFinishResidual, 7> : step_finish_kernel<kFinishResidual, 2>, grid, 512, 0, stream, programmatic, a);
+            return launch_pdl(deep == 7 ? step_finish_kernel<kFinishResidual, 7> : deep == 4 ? step_finish_kernel<kFinishResidual, 4> : step_finish_kernel<kFinishResidual, 2>,
+                              grid, 512, 0, stream, programmatic, a);
         case kFinishSwiGLU:
-            return launch_pdl(deep ? step_finish_kernel<kFinishSwiGLU, 7> : step_finish_kernel<kFinishSwiGLU, 2>, grid, 512, 0, stream, programmatic, a);
+            return launch_pdl(deep == 7 ? step_finish_kernel<kFinishSwiGLU, 7> : deep == 4 ? step_finish_kernel<kFinishSwiGLU, 4> : step_finish_kernel<kFinishSwiGLU, 2>,
+                              grid, 512, 0, stream, programmatic, a);
         default: return cudaErrorInvalidValue;
     }
 }
