@@ -741,3 +741,30 @@ def test_prompt_rows_are_normalised_rotated_and_appended_in_one_pass(built_libra
     assert close(results[0][0], results[1][0])
     for got, want in zip(results[0][1:], results[1][1:]):
         assert np.all(np.abs(got - want) <= 2.0 ** -9 * np.abs(want) + 2.0 ** -11 * np.abs(want).max())
+
+
+@pytest.mark.parametrize("kinds", [(H.Q4_K, H.Q6_K, H.Q8_0), (H.Q6_K, H.Q4_K, H.Q6_K), (H.Q8_0, H.Q8_0, H.Q8_0)], ids=["all", "k-quants", "one"])
+@pytest.mark.parametrize("tokens", [3, 12, 16, 24, 70])
+def test_launches_of_one_and_of_several_block_types(built_library, tokens, kinds):
+    """q, k and v of the given types in one launch, gate of the first and up of the second: the kernels that are compiled for a
+    launch's common type, for both K-quants and for any type, in each operand form, against the plain reference-style kernels."""
+    import ribn_b200
+    from ribn_b200 import BatchItem, StepKind
+    cfg = dict(MID, layers=1)
+    tensors = dict(H.make_model(cfg, seed=31, scheme="q8_0"))
+    rng = np.random.default_rng(37)
+    for part, kind in (("attn_q", kinds[0]), ("attn_k", kinds[1]), ("attn_v", kinds[2]), ("ffn_gate", kinds[0]), ("ffn_up", kinds[1])):
+        name = f"blk.0.{part}.weight"
+        _, rows, cols, _ = tensors[name]
+        tensors[name] = (kind, rows, cols, H.quantize(kind, rng.normal(0.0, 0.02, size=(rows, cols)).astype(np.float32)))
+    prompt = rng.integers(0, cfg["vocab"], tokens).tolist()
+    logits = []
+    for flags in (0, ribn_b200.FLAG_REFERENCE_KERNELS):
+        ex = build(cfg, tensors, flags, context_tokens=256, max_sequences=1, max_batch_tokens=128)
+        assert ex.admit(1, 1, prompt, 4).ready
+        item = BatchItem(1, StepKind.PREFILL, 0, tokens, 1)
+        ex.prepare([item])
+        ex.wait(ex.submit([item]))
+        logits.append(ex.copy_logits(0).copy())
+        ex.close()
+    assert close(logits[0], logits[1])
