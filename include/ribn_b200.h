@@ -464,7 +464,8 @@ RIBN_B200_API int ribn_b200_debug_repack(int32_t ggml_type, const void* raw, int
                                          void* out, size_t capacity, size_t* byte_count);
 
 /* How the GEMM of one matrix [rows][cols] is dealt out in a step of `members` rows, without any device work
- * (`form`: 0 fragment order, 1 column, 2 wide; 148 SMs where there is no device).  A run is eight numbers: worker, item, first
+ * (`form`: 0 fragment order, 1 column, 2 wide; 148 SMs where there is no device).  A worker that takes two row groups at a time
+ * (a CTA pair of the wide form) counts as two, one per group.  A run is eight numbers: worker, item, first
  * k tile, end, its part of the item's sums, and, as the kernel that adds the parts computes them, the item's parts, its
  * first worker and the rows of a unit.  Writes up to `capacity` runs, their count, and the floats of scratch that the first
  * and the further parts take. */

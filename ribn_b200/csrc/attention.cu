@@ -4,9 +4,10 @@
 //
 // Launches run the tensor-core span kernel below (the GQA group's query heads
 // against 16-key slices as m16n8k16 MMAs, K / V staged in shared memory by
-// asynchronous copies), then the merge kernel; the whole sixteen-token groups
-// of a prefill chunk run the prefill kernel instead (a key tile staged once per
-// group, every warp walks all the keys of its own tokens, no merge).  A token's
+// asynchronous copies), then the merge kernel; a prefill chunk of 64 tokens or
+// more runs a prefill kernel instead: heads of 128 that of attention_tc.cu,
+// others the one below for the chunk's whole groups of tokens (a key tile staged
+// once per group, every warp walks all the keys of its own tokens, no merge).  A token's
 // result depends only on its own keys and on the launch's size class (tiles
 // per span; chunk or not), never on where its pages live.
 //
@@ -625,7 +626,7 @@ __global__ void __launch_bounds__(kMmaWarps * 32, HD <= 128 && NT == 1 ? 3 : 1) 
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-// ---- prefill kernel: a run of consecutive tokens of one sequence ---------------------------------------
+// ---- prefill kernel: a run of consecutive tokens of one sequence, head widths 64 and 256 -----------------
 //
 // A CTA serves (4 x warp_tokens consecutive tokens, kv head); warp w owns warp_tokens of them (their query heads
 // are its MMA columns) and walks ALL their keys, so there are no spans to merge and the result is final.  The
@@ -978,12 +979,13 @@ cudaError_t launch_hd(cudaStream_t stream, AttnArgs a, bool fused, int n_tokens,
                       int* launches, bool programmatic = false, bool* operand_written = nullptr) {
     const int q_per_kv = a.q_heads / a.kv_heads;
     if (q_per_kv > 16) return cudaErrorInvalidValue;  // the group is the 16 columns of two MMA tiles
-    // A long run of consecutive tokens of one sequence (a prefill chunk; the caller says where it lies) takes the
-    // prefill kernel for as many whole CTA groups as it holds; what lies before, behind and beyond takes the spans.
+    // A long run of consecutive tokens of one sequence (a prefill chunk; the caller says where it lies) takes a prefill
+    // kernel: with heads of 128 the whole run the tcgen05 kernel's, else as many whole CTA groups as it holds the kernel's
+    // above; what lies before, behind and beyond takes the spans.
     const int warp_tokens = std::max(1, 16 / q_per_kv), cta_tokens = kMmaWarps * warp_tokens;
     if (!fused && a.window <= 0 && a.operand.dig == nullptr && a.run_first >= 0 && a.run_count >= 64 &&
         a.run_first + a.run_count <= n_tokens) {
-        if (HD == 128) {
+        if constexpr (HD == 128) {
             const PrefillAttention p{a.q, a.cache_k, a.cache_v, a.page_tables, a.pages_per_sequence, a.token_seq, a.token_pos,
                                      a.run_first, a.run_count, a.q_heads, a.kv_heads, max_keys, a.out, a.error_flag};
             cudaError_t e = launch_attention_tc(stream, p);
@@ -993,33 +995,34 @@ cudaError_t launch_hd(cudaStream_t stream, AttnArgs a, bool fused, int n_tokens,
             if (a.run_first > 0) e = launch_spans_hd<HD>(stream, a, fused, 0, a.run_first, max_keys, partial_bytes, launches, programmatic);
             if (e == cudaSuccess && behind < n_tokens) e = launch_spans_hd<HD>(stream, a, fused, behind, n_tokens - behind, max_keys, partial_bytes, launches, programmatic);
             return e;
-        }
-        const int aligned = a.run_count / cta_tokens * cta_tokens;
-        const bool wide = warp_tokens * q_per_kv > 8;
-        const size_t smem = (size_t)(kMmaWarps * 2 * 8 * (wide ? 2 : 1) + 2 * kMmaWarps * 2 * kMmaKeys) * (HD + 8) * sizeof(__half);
-        static bool configured_on[kMaxDevices] = {false};  // function attributes are per device
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
-        if (!configured_on[dev]) {
-            cudaError_t e = cudaFuncSetAttribute(attention_prefill_mma_kernel<HD, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_prefill_mma_kernel<HD, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        } else {
+            const int aligned = a.run_count / cta_tokens * cta_tokens;
+            const bool wide = warp_tokens * q_per_kv > 8;
+            const size_t smem = (size_t)(kMmaWarps * 2 * 8 * (wide ? 2 : 1) + 2 * kMmaWarps * 2 * kMmaKeys) * (HD + 8) * sizeof(__half);
+            static bool configured_on[kMaxDevices] = {false};  // function attributes are per device
+            int dev = 0;
+            if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
+            if (!configured_on[dev]) {
+                cudaError_t e = cudaFuncSetAttribute(attention_prefill_mma_kernel<HD, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+                if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_prefill_mma_kernel<HD, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+                if (e != cudaSuccess) return e;
+                configured_on[dev] = true;
+            }
+            AttnArgs p = a;
+            p.token_base = a.run_first;
+            const dim3 grid((unsigned)(aligned / cta_tokens * a.kv_heads));
+            cudaError_t e = wide ? launch_pdl(stream, attention_prefill_mma_kernel<HD, 2>, grid, kMmaWarps * 32, smem, p, programmatic, aligned, warp_tokens)
+                                 : launch_pdl(stream, attention_prefill_mma_kernel<HD, 1>, grid, kMmaWarps * 32, smem, p, programmatic, aligned, warp_tokens);
             if (e != cudaSuccess) return e;
-            configured_on[dev] = true;
+            if (launches) ++*launches;
+            if (a.run_first > 0) {
+                e = launch_spans_hd<HD>(stream, a, fused, 0, a.run_first, max_keys, partial_bytes, launches, programmatic);
+                if (e != cudaSuccess) return e;
+            }
+            const int behind = a.run_first + aligned;
+            if (behind < n_tokens) e = launch_spans_hd<HD>(stream, a, fused, behind, n_tokens - behind, max_keys, partial_bytes, launches, programmatic);
+            return e;
         }
-        AttnArgs p = a;
-        p.token_base = a.run_first;
-        const dim3 grid((unsigned)(aligned / cta_tokens * a.kv_heads));
-        cudaError_t e = wide ? launch_pdl(stream, attention_prefill_mma_kernel<HD, 2>, grid, kMmaWarps * 32, smem, p, programmatic, aligned, warp_tokens)
-                             : launch_pdl(stream, attention_prefill_mma_kernel<HD, 1>, grid, kMmaWarps * 32, smem, p, programmatic, aligned, warp_tokens);
-        if (e != cudaSuccess) return e;
-        if (launches) ++*launches;
-        if (a.run_first > 0) {
-            e = launch_spans_hd<HD>(stream, a, fused, 0, a.run_first, max_keys, partial_bytes, launches, programmatic);
-            if (e != cudaSuccess) return e;
-        }
-        const int behind = a.run_first + aligned;
-        if (behind < n_tokens) e = launch_spans_hd<HD>(stream, a, fused, behind, n_tokens - behind, max_keys, partial_bytes, launches, programmatic);
-        return e;
     }
     return launch_spans_hd<HD>(stream, a, fused, 0, n_tokens, max_keys, partial_bytes, launches, programmatic, operand_written);
 }

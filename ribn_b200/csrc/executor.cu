@@ -457,11 +457,11 @@ cudaError_t run_layers_decode(ribn_b200_executor* ex, const StepPlan& plan, int&
 // ---- three rows and more: one GEMM launch per projection over the whole step, its partial sums finished by the kernel
 // that makes the next projection's operand -----------------------------------------------------------------------------
 // The block form of a step's activations, which selects its GEMM kernel.  A projection of the 8B model (gate | up, 57 MB,
-// from HBM, serialised) takes 23 / 33 / 43 / 63 us in fragment order at 8 / 16 / 24 / 32 rows, 30 / 31 / 34 / 36 us with
-// tensor-memory conversion at 24 / 32 / 48 / 64 (30 us at 16) and 58 / 61 us in the wide form at 65 / 128: the lines lie at
-// 16, where the smaller projections decide, and at 64 rows.  Q8_0 (a layer's four projections of the 0.6B model): 33 / 60 us
-// in fragment order at 16 / 32 rows against 36 / 37 us; the wide form takes 57 us at 128 rows and 122 us at 777, against 82
-// and 161 us of the column form in groups of 64.
+// from HBM, serialised) takes 23 / 29 / 40 / 54 us in fragment order at 8 / 16 / 24 / 32 rows, 29 / 31 / 34 / 35 us with
+// tensor-memory conversion at 24 / 32 / 48 / 64 (30 us at 16) and 60 / 64 us in the wide form at 65 / 128: the lines lie at
+// 16, where the smaller projections decide, and at 64 rows, the column form's most.  Q8_0 (a layer's four projections of the
+// 0.6B model): 29 / 46 us in fragment order at 16 / 32 rows against 35 / 36 us; the wide form takes 54 us at 64 rows against
+// 40 us of the column form, and at 128 rows 56 us against 79 us of two launches of it.
 int step_form(int members) {
     return members <= 16 ? kFragmentForm : members <= 64 ? kColumnForm : kWideForm;
 }

@@ -101,9 +101,10 @@ cudaError_t launch_attention_ref(cudaStream_t stream, const float* q, const __ha
 // incremented per kernel launch.  `token_seq` may be null: every token then
 // belongs to sequence 0 (one page-table row).  A GQA group has at most
 // 16 query heads.  `run_first`, `run_count` (optional) tell where a run of
-// consecutive tokens of ONE sequence lies in the launch (a prefill chunk):
-// its whole groups of 4 x (16 / group size) tokens take a kernel that stages
-// each key tile once for such a group and walks all its keys, no merge.
+// consecutive tokens of ONE sequence lies in the launch (a prefill chunk): from
+// 64 tokens on it takes a prefill kernel that stages each key tile once for many
+// tokens and walks all their keys, no merge (heads of 128: attention_tc.cu for the
+// whole run; else whole groups of 4 x (16 / group size) tokens).
 constexpr int kAttnSpanKeys = 64;
 constexpr int kAttnMaxSpans = 1024;  // tiles per token: 65536 keys
 cudaError_t launch_attention(cudaStream_t stream, const float* q, const __half* cache_k, const __half* cache_v,
