@@ -407,7 +407,7 @@ cudaError_t run_attention(ribn_b200_executor* ex, const StepPlan& plan, int l, b
     }
     return launch_attention(s, ex->q, ck, cv, ex->d_page_tables, ex->pages_per_sequence, ex->meta.token_seq, ex->meta.token_pos, T, c.q_heads,
                             c.kv_heads, c.head_dim, 0, plan.max_keys, ex->scratch.attn_partial, ex->scratch.attn_partial_bytes, ex->attn,
-                            &launches, plan.run_first, plan.run_count, ex->d_error);
+                            &launches, plan.run_first, plan.run_count, ex->d_error, step_operand, operand_written);
 }
 
 cudaError_t run_layers_decode(ribn_b200_executor* ex, const StepPlan& plan, int& launches) {

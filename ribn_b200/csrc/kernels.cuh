@@ -104,14 +104,16 @@ cudaError_t launch_attention_ref(cudaStream_t stream, const float* q, const __ha
 // consecutive tokens of ONE sequence lies in the launch (a prefill chunk): from
 // 64 tokens on it takes a prefill kernel that stages each key tile once for many
 // tokens and walks all their keys, no merge (heads of 128: attention_tc.cu for the
-// whole run; else whole groups of 4 x (16 / group size) tokens).
+// whole run; else whole groups of 4 x (16 / group size) tokens).  `step_operand`,
+// `operand_written`: as in DecodeAttention.
 constexpr int kAttnSpanKeys = 64;
 constexpr int kAttnMaxSpans = 1024;  // tiles per token: 65536 keys
 cudaError_t launch_attention(cudaStream_t stream, const float* q, const __half* cache_k, const __half* cache_v,
                              const int32_t* page_tables, int pages_per_sequence, const int32_t* token_seq,
                              const int32_t* token_pos, int n_tokens, int q_heads, int kv_heads, int head_dim,
                              int window, int max_keys, float* partial, size_t partial_bytes, float* out,
-                             int* launches, int run_first = -1, int run_count = 0, int* error_flag = nullptr);
+                             int* launches, int run_first = -1, int run_count = 0, int* error_flag = nullptr,
+                             StepOperand step_operand = StepOperand{}, bool* operand_written = nullptr);
 
 // Attention of `count` consecutive tokens of one sequence from token `first` on (attention_tc.cu, head width 128): q as for
 // launch_attention, tokens at consecutive positions.
@@ -127,6 +129,8 @@ struct PrefillAttention {
     int max_keys;               // at least the keys of the last token
     float* out;
     int* error_flag;            // set non-zero when a bounded wait gives up
+    // optional: the result in this form in place of `out` (wide form, the tokens of the launch from 0 on, groups of 2 or 4 heads)
+    StepOperand operand;
 };
 cudaError_t launch_attention_tc(cudaStream_t stream, const PrefillAttention& args);
 

@@ -768,3 +768,28 @@ def test_launches_of_one_and_of_several_block_types(built_library, tokens, kinds
         logits.append(ex.copy_logits(0).copy())
         ex.close()
     assert close(logits[0], logits[1])
+
+
+@pytest.mark.parametrize("q_heads,kv_heads", [(8, 2), (4, 2), (16, 2)])
+@pytest.mark.parametrize("tokens", [639, 640, 647, 705, 897])
+def test_prompt_attention_leaves_the_operand_of_its_consumer(built_library, tokens, q_heads, kv_heads):
+    """A long prompt alone in a step: prefill attention that writes the output projection's operand (from 640 tokens on, groups of 2
+    and 4 heads; 8 take the launch that converts F32 results), for last blocks of one to eight tokens, part of a query tile and of
+    a row group, without and behind a cached prefix; against the reference-style kernels."""
+    import ribn_b200
+    from ribn_b200 import BatchItem, StepKind
+    cfg = dict(layers=2, hidden=512, q_heads=q_heads, kv_heads=kv_heads, head_dim=128, ffn=1024, vocab=1024, rope_base=1.0e6, rms_eps=1.0e-6)
+    prompt = np.random.default_rng(tokens).integers(0, cfg["vocab"], 2 * tokens).tolist()
+    logits = []
+    for flags in (0, ribn_b200.FLAG_REFERENCE_KERNELS):
+        ex = ribn_b200.QwenB200(cfg, flags=flags | ribn_b200.FLAG_KEEP_LOGITS, context_tokens=2048, max_sequences=1, max_batch_tokens=960)
+        ex.init_synthetic(41, ribn_b200.SCHEME_Q4_K_M)
+        ex.finalize()
+        assert ex.admit(1, 1, prompt, 4).ready
+        for first in (0, tokens):
+            item = BatchItem(1, StepKind.PREFILL, first, tokens, 1 if first else 0)
+            ex.prepare([item])
+            ex.wait(ex.submit([item]))
+        logits.append(ex.copy_logits(0).copy())
+        ex.close()
+    assert close(logits[0], logits[1])
