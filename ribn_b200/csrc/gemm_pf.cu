@@ -221,6 +221,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
                     }
                 }
             }
+            // the leader's tensor core still arrives here for the last slots: not after this block has ended
+            for (uint32_t i = pos > kBSlots ? pos - kBSlots : 0u; i < pos && alive; ++i) alive = mbar_wait(b_empty + 8 * (i % kBSlots), (i / kBSlots) & 1u, a.error_flag, 115, spin_limit);
             if (!alive) {
                 for (int i = 0; i < 8; ++i) { mbar_wait(b_full + 8 * (i & 3), (uint32_t)(i >> 2), nullptr, 0, spin_limit); mbar_wait(t_full + 8 * (i & 3), (uint32_t)(i >> 2), nullptr, 0, spin_limit); }
             }
@@ -355,6 +357,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
                 if (++ws == (uint32_t)nw) { ws = 0; parity ^= 1u; }
             }
         }
+        // likewise the arrivals that give the last stages back
+        for (uint32_t i = uses > 2u ? uses - 2u : 0u; i < uses && alive; ++i) alive = mbar_wait(a_free + 8 * (i & 1u), (i >> 1) & 1u, a.error_flag, 116, spin_limit);
     } else {
         // ---------------- fold and store: one row and 32 columns of each group ----------------
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kFoldRegs));

@@ -290,3 +290,19 @@ def test_step_gemm_is_no_further_from_exact_sums_than_the_chunk_kernels(ops, kin
         want = xs.astype(np.float64) @ weights.T
         off = {v: float(np.linalg.norm(ops.gemv(kind, enc, rows, cols, xs, variant=v) - want) / np.linalg.norm(want)) for v in (3, variant)}
         assert off[variant] <= 1.1 * off[3], off
+
+
+@pytest.mark.parametrize("kind", [H.Q4_K, H.Q6_K, H.Q8_0])
+@pytest.mark.parametrize("cols,members", [(256, 70), (256, 129), (512, 70), (768, 129), (1280, 257), (1536, 300)])
+def test_wide_gemm_ends_with_its_rings_at_any_fill(ops, kind, cols, members):
+    # 2 to 24 activation chunks through a ring of four, 2 to 24 operand stages through two: a block waits for the last of
+    # them before it ends (a wait for one that never comes would expire and be reported), launches follow one another at once
+    rng = np.random.default_rng(cols + members + kind)
+    rows = 300
+    enc = H.quantize(kind, rng.normal(0, 0.02, size=(rows, cols)).astype(np.float32))
+    xs = rng.normal(0, 1, (members, cols)).astype(np.float32)
+    want = xs @ H.np_dequant(kind, enc).reshape(rows, cols).T
+    first = ops.gemv(kind, enc, rows, cols, xs, variant=8)
+    assert np.max(np.abs(first - want)) / np.max(np.abs(want)) < 3e-6
+    for _ in range(3):
+        assert np.array_equal(ops.gemv(kind, enc, rows, cols, xs, variant=8).view(np.uint32), first.view(np.uint32))
