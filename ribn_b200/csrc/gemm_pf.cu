@@ -57,25 +57,16 @@ __device__ __forceinline__ uint32_t cluster_rank() {
     return r;
 }
 __device__ __forceinline__ void cluster_sync() { asm volatile("barrier.cluster.arrive;\n\tbarrier.cluster.wait;" ::: "memory"); }
+// An arrival at rank 0's barrier, in the default form, which like mbar_wait synchronises threads of one CTA only; the pair's
+// barriers rely on no more.  No thread reads what a thread of the other CTA wrote: what passes between them is tensor memory
+// (behind tcgen05.wait and tcgen05.fence on both sides of the barrier) and shared memory that the tensor core reads through the
+// asynchronous proxy (bulk copies that have landed, and the minima operand behind fence.proxy.async).  A fold thread reads its
+// rows' scales, which threads of its own CTA stored before they arrived here.
 __device__ __forceinline__ void arrive_leader(uint32_t bar) {
     asm volatile(
         "{\n\t.reg .b32 r;\n\t"
         "mapa.shared::cluster.u32 r, %0, 0;\n\t"
         "mbarrier.arrive.shared::cluster.b64 _, [r];\n\t}" ::"r"(bar) : "memory");
-}
-// mbar_wait for a barrier that the other CTA's threads arrive on
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, int* error_flag, int code, uint32_t limit) {
-    for (uint32_t i = 0; i < limit; ++i) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (ok) return true;
-    }
-    if (error_flag != nullptr) atomicExch(error_flag, code);
-    return false;
 }
 // to the barrier at this place in both CTAs
 __device__ __forceinline__ void commit_both(uint32_t bar) {
@@ -255,7 +246,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
             uint32_t n = 0, pos = 0, uses = 0, sums = 0;   // k tiles, ring slots, A stages and sums so far
             uint32_t taken = 0, t_used = 0;                // bit i: sums i (2: the minima's), tail i, used an odd number of times
             auto take = [&](uint32_t i) {
-                if (alive) alive = mbar_wait_cluster(i == 2 ? m_free : d_free + 8 * i, ((taken >> i) & 1u) ^ 1u, a.error_flag, 105, spin_limit);
+                if (alive) alive = mbar_wait(i == 2 ? m_free : d_free + 8 * i, ((taken >> i) & 1u) ^ 1u, a.error_flag, 105, spin_limit);
                 taken ^= 1u << i;
             };
             for (int r = 0; r < runs; ++r) {
@@ -271,14 +262,14 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
                         const bool opens = (h & (per_sum - 1)) == 0, closes = (h & (per_sum - 1)) == per_sum - 1;   // a sum
                         const bool first = q4k || (h & 1) == 0, last = q4k || (h & 1) == 1;                        // stage of a chunk
                         const uint32_t st = uses & 1u, a_at = tmem + 384 + 64 * st;
-                        if (alive) alive = mbar_wait_cluster(a_full + 8 * st, (uses >> 1) & 1u, a.error_flag, 106, spin_limit);
+                        if (alive) alive = mbar_wait(a_full + 8 * st, (uses >> 1) & 1u, a.error_flag, 106, spin_limit);
 #pragma unroll 1
                         for (int u = 0; u < both; ++u) {
                             const uint32_t db = (sums + u) & 1u, d_main = tmem + 128 * db, slot = (pos + u) % kBSlots;
                             if (opens) take(db);
                             if (first) {
                                 if (alive) alive = mbar_wait(b_full + 8 * slot, ((pos + u) / kBSlots) & 1u, a.error_flag, 104, spin_limit);
-                                if (alive) alive = mbar_wait_cluster(b_peer + 8 * slot, ((pos + u) / kBSlots) & 1u, a.error_flag, 104, spin_limit);
+                                if (alive) alive = mbar_wait(b_peer + 8 * slot, ((pos + u) / kBSlots) & 1u, a.error_flag, 104, spin_limit);
                             }
                             tc_fence_after();
                             const uint32_t b_desc = b_desc0 + slot * (kChunkBytes >> 4) + (q4k ? 0u : (h & 1) * 4 * kStep);
@@ -292,7 +283,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
                                     // the other's have been folded by the time the stage's products are through
                                     const uint32_t i = 2 * (n & 1u) + u;
                                     if (alive) alive = mbar_wait(t_full + 8 * i, (t_used >> i) & 1u, a.error_flag, 107, spin_limit);
-                                    if (alive) alive = mbar_wait_cluster(t_peer + 8 * i, (t_used >> i) & 1u, a.error_flag, 107, spin_limit);
+                                    if (alive) alive = mbar_wait(t_peer + 8 * i, (t_used >> i) & 1u, a.error_flag, 107, spin_limit);
                                     take(2);
                                     tc_fence_after();
                                     if (leader) pair_mma_ss(tmem + 256, a2_desc0 + (n & 1u) * (kA2Bytes >> 4), sum_desc0 + i * (kTailBytes >> 4));
