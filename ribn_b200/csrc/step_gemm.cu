@@ -153,12 +153,12 @@ __global__ void __launch_bounds__(256) step_store_kernel(const StepFinish a) {
 constexpr int kQkvHead = 128;
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) step_qkv_kernel(const StepFinish a, const StepQkv c) {
-    __shared__ float2 turn[kQkvHead / 2];
+    __shared__ float4 turn[kQkvHead / 4];   // (cosine, sine) of two neighbouring dimensions
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, heads = c.q_heads + 2 * c.kv_heads;
     if (threadIdx.x < kQkvHead / 2) {   // positions are older than the projection
         const float theta = (float)c.token_pos[t] * c.inv_freq[threadIdx.x];
-        turn[threadIdx.x] = make_float2(cosf(theta), sinf(theta));
+        reinterpret_cast<float2*>(turn)[threadIdx.x] = make_float2(cosf(theta), sinf(theta));
     }
     const long long slot = c.token_slot[t];
     const float4 wq = load4(c.q_norm + 4 * lane), wk = load4(c.k_norm + 4 * lane);
@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(WARPS * 32) step_qkv_kernel(const StepFinish a
             // dimension d turns with d + 64, sixteen lanes further
             const float4 o = make_float4(__shfl_xor_sync(0xffffffffu, x.x, 16), __shfl_xor_sync(0xffffffffu, x.y, 16),
                                          __shfl_xor_sync(0xffffffffu, x.z, 16), __shfl_xor_sync(0xffffffffu, x.w, 16));
-            const float4 t0 = *reinterpret_cast<const float4*>(&turn[4 * (lane & 15)]), t1 = *reinterpret_cast<const float4*>(&turn[4 * (lane & 15) + 2]);
+            const float4 t0 = turn[2 * (lane & 15)], t1 = turn[2 * (lane & 15) + 1];
             auto rotate = [&](float mine, float other, float cosine, float sine) { return lane < 16 ? mine * cosine - other * sine : other * sine + mine * cosine; };
             x = make_float4(rotate(x.x, o.x, t0.x, t0.y), rotate(x.y, o.y, t0.z, t0.w), rotate(x.z, o.z, t1.x, t1.y), rotate(x.w, o.w, t1.z, t1.w));
             if (h < c.q_heads) *reinterpret_cast<float4*>(c.q + ((size_t)t * c.q_heads + h) * kQkvHead + 4 * lane) = x;
