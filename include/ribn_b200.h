@@ -472,6 +472,13 @@ RIBN_B200_API int ribn_b200_debug_repack(int32_t ggml_type, const void* raw, int
 RIBN_B200_API int ribn_b200_debug_step_deal(int32_t form, int64_t rows, int64_t cols, int32_t members, int32_t* runs, size_t capacity,
                                             size_t* count, size_t* partial_floats, size_t* further_floats);
 
+/* The operand form of a step's GEMMs (`form` as above) as the step's kernels write it: of the rows x [members][width], or,
+ * with `up`, of silu(gate) * up from the sums gate = x and up that a gate | up projection of 1,024 inputs left; `ss` (may be
+ * NULL: no RMSNorm) is that projection's input as [members][4] sums of squares.  `bytes` may be NULL to query the size; what
+ * the kernels leave untouched reads zero. */
+RIBN_B200_API int ribn_b200_debug_step_operand(int32_t device, int32_t form, const float* x, const float* up, const float* ss, int32_t members,
+                                               int32_t width, void* bytes, size_t capacity, size_t* byte_count);
+
 /* Library build identification (git-free; the CUDA arch it was built for). */
 RIBN_B200_API const char* ribn_b200_build_info(void);
 

@@ -606,6 +606,53 @@ int ribn_b200_op_attention(int32_t device, const float* q, const uint16_t* keys,
     return s.download(out, d_o, (size_t)rows * q_heads * head_dim) ? RIBN_B200_OK : RIBN_B200_ERROR;
 }
 
+int ribn_b200_debug_step_operand(int32_t device, int32_t form, const float* x, const float* up, const float* ss, int32_t members, int32_t width,
+                                 void* bytes, size_t capacity, size_t* byte_count) {
+    if (form < kFragmentForm || form > kWideForm || members <= 0 || (form == kColumnForm && members > kColumnMaxMembers) || width <= 0 ||
+        width % kTileCols != 0 || byte_count == nullptr) {
+        return op_fail("step_operand: invalid argument", cudaSuccess);
+    }
+    *byte_count = step_operand_bytes(members, width, form);
+    if (bytes == nullptr) return RIBN_B200_OK;
+    if (x == nullptr || capacity < *byte_count) return op_fail("step_operand: invalid argument", cudaSuccess);
+    Scope s(device);
+    if (!s.ok) return op_fail("invalid argument, or no usable CUDA device", cudaGetLastError());
+    constexpr int kInputs = 4;   // k tiles of the projection whose sums gate | up stand for
+    const size_t values = (size_t)members * width;
+    StepFinish f{};
+    f.members = members;
+    f.out.form = form;
+    f.out.blocks = s.alloc<unsigned char>(*byte_count);
+    OP_PTR(f.out.blocks);
+    OP_TRY(cudaMemsetAsync(f.out.blocks, 0, *byte_count, s.stream));
+    if (up == nullptr) {
+        f.x = s.upload(x, values);
+        OP_PTR(f.x);
+        OP_TRY(launch_step_finish(s.stream, kFinishRows, nullptr, f, width, false));
+    } else {
+        StepGemm g{};
+        g.form = form;
+        g.n_segments = 2;
+        for (int i = 0; i < 2; ++i) g.seg[i] = GemvSegment{nullptr, kQ8_0, width, width / kTileRows, nullptr};
+        g.k = kInputs * kTileCols;
+        g.members = members;
+        g.eps = 1e-6f;
+        std::vector<float> sums(2 * values);
+        for (int m = 0; m < members; ++m) {
+            memcpy(&sums[(size_t)m * 2 * width], x + (size_t)m * width, (size_t)width * sizeof(float));
+            memcpy(&sums[((size_t)m * 2 + 1) * width], up + (size_t)m * width, (size_t)width * sizeof(float));
+        }
+        g.partial = s.upload(sums.data(), sums.size());
+        const size_t further = step_further_floats(g);
+        g.further = s.alloc<float>(further);
+        OP_PTR(g.partial); OP_PTR(g.further);
+        OP_TRY(cudaMemsetAsync(g.further, 0, further * sizeof(float), s.stream));
+        if (ss != nullptr) { g.ss = s.upload(ss, (size_t)members * kInputs); OP_PTR(g.ss); }
+        OP_TRY(launch_step_finish(s.stream, kFinishSwiGLU, &g, f, width, false));
+    }
+    return s.download((unsigned char*)bytes, f.out.blocks, *byte_count) ? RIBN_B200_OK : op_fail("step_operand", cudaGetLastError());
+}
+
 int ribn_b200_op_batch_metadata(int32_t device, const int32_t* row_slot, const int32_t* row_prefix,
                                 const int32_t* row_tokens, int32_t rows, const int32_t* page_tables,
                                 int32_t pages_per_sequence, int32_t page_tokens, int32_t* cu_seqlens,

@@ -117,7 +117,8 @@ __global__ void __launch_bounds__(512, BATCH > 4 ? 1 : BATCH > 2 ? 2 : 3) step_f
             const float q = x * r, exact = fmaf(fmaf(-q, den, x), r, q);
             return (fabsf(q) < INFINITY ? exact : q) * (u * inv);
         };
-        v = make_float4(act(gt.x, up.x), act(gt.y, up.y), act(gt.z, up.z), act(gt.w, up.w));
+        // rows past the last one stay zero; a block without any row has no factors either
+        if (m < a.members) v = make_float4(act(gt.x, up.x), act(gt.y, up.y), act(gt.z, up.z), act(gt.w, up.w));
     }
     if (m < a.members) {
         square = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w)));

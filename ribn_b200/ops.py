@@ -217,3 +217,15 @@ def step_deal(form: int, rows: int, cols: int, members: int):
     runs = np.empty((count.value, 8), dtype=np.int32)
     _check(lib().ribn_b200_debug_step_deal(*args, _p(runs), runs.shape[0], C.byref(count), C.byref(partial), C.byref(further)), "step_deal")
     return runs, partial.value, further.value
+
+
+def step_operand(form: int, x, up=None, ss=None, device: int = 0) -> np.ndarray:
+    """The operand form of a step's GEMMs, as bytes (ribn_b200_debug_step_operand): of rows, or of silu(x) * up."""
+    x = np.ascontiguousarray(x, dtype=np.float32)
+    rest = [None if a is None else np.ascontiguousarray(a, dtype=np.float32) for a in (up, ss)]
+    need = C.c_size_t(0)
+    head = (device, form, _p(x), *(None if a is None else _p(a) for a in rest), x.shape[0], x.shape[1])
+    _check(lib().ribn_b200_debug_step_operand(*head, None, 0, C.byref(need)), "step_operand size")
+    out = np.empty(need.value, dtype=np.uint8)
+    _check(lib().ribn_b200_debug_step_operand(*head, _p(out), out.size, C.byref(need)), "step_operand")
+    return out

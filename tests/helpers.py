@@ -226,3 +226,53 @@ def oracle_config(cfg: dict, context: int) -> dict:
     return dict(layers=cfg["layers"], hidden=cfg["hidden"], q_heads=cfg["q_heads"], kv_heads=cfg["kv_heads"],
                 head_dim=cfg["head_dim"], ffn=cfg["ffn"], vocab=cfg["vocab"], context=context,
                 rope_base=cfg["rope_base"], eps=cfg["rms_eps"])
+
+
+# --- the operand form of a step's GEMMs (ribn_b200/csrc/gemv.cuh: StepForm) ------------------------------------------
+FRAGMENT, COLUMN, WIDE = 0, 1, 2
+
+
+def step_operand_fields(form: int, blocks: np.ndarray, members: int, width: int):
+    """The fields of an operand, over all rows that the blocks have room for (rows past `members` included): binary16 bits
+    hi [rows][width] and lo [rows][width] in input order, the 32-input group sums [rows][k tiles][8 groups][hi, lo] and the
+    scales [rows][k tiles]."""
+    k_tiles, eights = width // 256, (members + 7) // 8
+    if form == WIDE:
+        groups, ng = (eights + 15) // 16, 16
+    elif form == COLUMN:
+        groups, ng = 1, next(n for n in (3, 4, 6, 8) if n >= eights)
+    else:
+        groups = (eights + 3) // 4
+        ng = (eights + groups - 1) // groups
+    mp, rows = 8 * ng, groups * 8 * ng
+    blocks = np.ascontiguousarray(blocks)
+    parts = np.empty((2, rows, k_tiles, 16, 4, 4), dtype=np.uint16)   # hi / lo, row, k tile, step, lane's quarter, input
+    if form == FRAGMENT:
+        b = blocks.reshape(groups, k_tiles, ng, 16 * 512 + 256 + 32)
+        pairs = b[..., :16 * 512].copy().view(np.uint16).reshape(groups, k_tiles, ng, 16, 8, 4, 2, 4)   # .. step, row, t, hi / lo, inputs 0 2 1 3
+        parts[...] = pairs[..., [0, 2, 1, 3]].transpose(6, 0, 2, 4, 1, 3, 5, 7).reshape(parts.shape)
+        sums = b[..., 16 * 512:16 * 512 + 256].copy().view(np.uint16).reshape(groups, k_tiles, ng, 8, 4, 2, 2)   # .. row, pair of groups, hi / lo, group
+        sums = sums.transpose(0, 2, 3, 1, 4, 6, 5).reshape(rows, k_tiles, 8, 2)
+        scales = b[..., 16 * 512 + 256:].copy().view(np.float32).transpose(0, 2, 3, 1).reshape(rows, k_tiles)
+    else:
+        sum_cols = (mp + 15) // 16 * 16
+        b = blocks.reshape(groups, k_tiles, 1028 * mp + 32 * sum_cols)
+        main, tail = b[..., :1024 * mp].copy().view(np.uint16), b[..., 1024 * mp:1024 * mp + 32 * sum_cols].copy().view(np.uint16)
+        if form == COLUMN:   # [8-input block][hi, lo][column]
+            main = main.reshape(groups, k_tiles, 32, 2, mp, 8).transpose(3, 0, 4, 1, 2, 5)
+            tail = tail.reshape(groups, k_tiles, 2, sum_cols, 8)[:, :, :, :mp].transpose(0, 3, 1, 4, 2)
+        else:                # [64 rows][128 inputs][hi, lo][8-input block][row]
+            main = main.reshape(groups, k_tiles, 2, 2, 2, 16, 64, 8).transpose(4, 0, 2, 6, 1, 3, 5, 7)
+            tail = tail.reshape(groups, k_tiles, 2, 2, 64, 8).transpose(0, 2, 4, 1, 5, 3)
+        # 8-input block 2 s + i, element 2 t + e: input 16 s + 4 t + i + 2 e
+        main = main.reshape(2, rows, k_tiles, 16, 2, 4, 2)
+        parts[...] = main.transpose(0, 1, 2, 3, 5, 6, 4).reshape(parts.shape)
+        sums = tail.reshape(rows, k_tiles, 8, 2)
+        scales = b[..., 1024 * mp + 32 * sum_cols:].copy().view(np.float32).transpose(0, 2, 1).reshape(rows, k_tiles)
+    return dict(hi=parts[0].reshape(rows, width), lo=parts[1].reshape(rows, width), sums=np.ascontiguousarray(sums), scale=np.ascontiguousarray(scales))
+
+
+def step_operand_values(fields) -> np.ndarray:
+    """What the tensor core is given: (hi + lo) x scale in 64 bits."""
+    hi, lo = (fields[f].view(np.float16).astype(np.float64) for f in ("hi", "lo"))
+    return (hi + lo) * np.repeat(fields["scale"].astype(np.float64), 256, axis=1)

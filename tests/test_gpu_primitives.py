@@ -394,3 +394,28 @@ def test_prefill_chunk_attention_at_the_edges_of_its_tiles(ops, QH, KVH, tokens,
         seen = tokens - rows + 1 + r
         want = orc.attention(q[r], k.reshape(-1)[: seen * KVH * HD], v.reshape(-1)[: seen * KVH * HD], seen, QH, KVH, HD)
         assert np.max(np.abs(results[0][r] - want)) < 1e-5, r
+
+
+# ---- the operand form of a step's GEMMs -------------------------------------------------------------------
+@pytest.mark.parametrize("form,members", [(H.FRAGMENT, 5), (H.FRAGMENT, 65), (H.COLUMN, 3), (H.COLUMN, 33), (H.COLUMN, 64), (H.WIDE, 65), (H.WIDE, 100), (H.WIDE, 129)])
+def test_swiglu_operand_rows_past_the_last_one_are_zero(ops, form, members):
+    """Blocks of eight rows that are part empty and, in the column and wide forms, wholly so (33 rows: one of six blocks; 65: seven of
+    sixteen): their rows read zero with the scale of a zero row.  The launch before leaves NaN factors where the kernel keeps
+    its own in shared memory.  The other rows: silu(gate) up in 64 bits, to the units in the last place of the exponential (2),
+    three roundings and the operand's 22 bits."""
+    width, eps = 512, 1e-6
+    rng = np.random.default_rng(members + 7 * form)
+    rows = H.step_operand_fields(form, ops.step_operand(form, np.zeros((members, width), np.float32)), members, width)["hi"].shape[0]
+    gate, up = (rng.normal(0, 2, (rows, width)).astype(np.float32) for _ in range(2))
+    ss = rng.uniform(200, 300, (rows, 4)).astype(np.float32)
+    ops.step_operand(form, gate, up, ss=np.full((rows, 4), np.nan, np.float32))
+    got = H.step_operand_fields(form, ops.step_operand(form, gate[:members], up[:members], ss=ss[:members]), members, width)
+    for field in ("hi", "lo", "sums"):
+        assert not np.any(got[field][members:]), field
+    assert np.all(got["scale"][members:] == np.float32(2.0 ** -126))
+    factor = 1.0 / np.sqrt(ss.astype(np.float64).sum(axis=1) / 1024 + eps)
+    x = gate * factor[:, None]
+    want = (x / (1.0 + np.exp(-x)) * (up * factor[:, None]))[:members]
+    off = np.abs(H.step_operand_values(got)[:members] - want)
+    # 8 units of 2^-24 of the value (the factor: 2, twice; e^-x: 2; sums and products), 2^-23 of the tile's largest for the operand
+    assert np.all(off <= 10 * 2.0 ** -24 * np.abs(want) + 2.0 ** -23 * np.abs(want).max(axis=1, keepdims=True))
