@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const Prefill
         n[t] = tokens[t] > 0 ? (pos0 + local[t] + tokens[t] - 1) / kKeys + 1 : 0;
         if (SPLIT) n[t] = (n[t] + 1 - t) / 2;
     }
-    const int n_tiles = max(n[0], n[1]);
+    const int n_tiles = max(n[0], n[1]), all_tiles = SPLIT ? n[0] + n[1] : n_tiles, total_copies = 2 * all_tiles;
     bool alive = true;
 
     if (warp >= kMmaWarp) {
@@ -252,7 +252,8 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const Prefill
                     if (j + 1 == n[t]) umma_commit(o_full + 8 * t);
                 }
             };
-            auto release = [&](int idx) { if (leader) umma_commit(kv_empty + 8 * (idx % kSlots)); };
+            // (the last copies' slots are not asked for again: an arrival there could come after the block's end)
+            auto release = [&](int idx) { if (leader && idx + kSlots < total_copies) umma_commit(kv_empty + 8 * (idx % kSlots)); };
             if (SPLIT) {
                 int idx = 0;   // copies in the order of their use, each used once
                 if (alive) alive = mbar_wait(q_full, 0, a.error_flag, 122, kSpinLimit);
@@ -293,7 +294,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const Prefill
             const long long stride = (long long)a.kv_heads * kHd;
             constexpr int kGroups = (kKeys / 8 + kLoadWarps - 1) / kLoadWarps;
             // Copy `idx`: K0 V0 K1 V1 .., or (SPLIT) K0 K1, then V j, K j + 2 in turn: 2 (j + 1) and 2 (j + 1) + 1, what does not exist left out
-            const int all_tiles = SPLIT ? n[0] + n[1] : n_tiles, total = 2 * all_tiles;
+            const int total = total_copies;
             auto what = [&](int idx, bool& v) -> int {   // its key tile
                 if (!SPLIT) { v = idx & 1; return idx >> 1; }
                 if (idx < 2 || all_tiles == 1) { v = all_tiles == 1 ? idx == 1 : false; return all_tiles == 1 ? 0 : idx; }
