@@ -183,12 +183,13 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const Prefill
     extern __shared__ __align__(128) unsigned char smem[];
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const uint32_t q_at = smem_u32(smem), ring = q_at + 4 * kTileBytes, bars = ring + kSlots * kTileBytes;
-    const uint32_t q_full = bars, s_full = bars + 16, p_full = bars + 32, o_full = bars + 48, kv_full = bars + 64, kv_empty = bars + 88, tmem_slot = bars + 112;
+    const uint32_t q_full = bars, s_full = bars + 16, p_full = bars + 32, o_full = bars + 48, kv_full = bars + 64, kv_empty = bars + 88, tmem_slot = bars + 112, drained = bars + 120;
     if (threadIdx.x == 0) {
         for (int i = 0; i < 2; ++i) {
             mbar_init(q_full + 8 * i, kSoftmaxWarps / 2); mbar_init(s_full + 8 * i, 1); mbar_init(p_full + 8 * i, kSoftmaxWarps / 2); mbar_init(o_full + 8 * i, 1);
         }
         for (int i = 0; i < kSlots; ++i) { mbar_init(kv_full + 8 * i, kLoadWarps); mbar_init(kv_empty + 8 * i, 1); }
+        mbar_init(drained, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kMmaWarp) {
@@ -230,27 +231,27 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const Prefill
                 slot_wait(idx);
                 tc_fence_after();
                 const uint32_t b = k_desc + (idx % kSlots) * (kTileBytes >> 4), hi = q_desc + (SPLIT ? 0 : 2 * t) * (kTileBytes >> 4), lo = hi + (kTileBytes >> 4);
-                if (leader) {
+                if (leader && alive) {
 #pragma unroll
                     for (int i = 0; i < kHd / 16; ++i) umma_ss(tmem + 128 * t, lo + i * (2 * kPieceBytes >> 4), b + i * (2 * kPieceBytes >> 4), kIdescQk, (uint32_t)(i != 0));
 #pragma unroll
                     for (int i = 0; i < kHd / 16; ++i) umma_ss(tmem + 128 * t, hi + i * (2 * kPieceBytes >> 4), b + i * (2 * kPieceBytes >> 4), kIdescQk, 1u);
-                    umma_commit(s_full + 8 * t);
                 }
+                if (leader) umma_commit(s_full + 8 * t);
             };
             // O of tile t += P of its j-th key tile times the V tile that is copy `idx`
             auto values = [&](int t, int j, int idx) {
                 if (alive) alive = mbar_wait(p_full + 8 * t, (uint32_t)j & 1u, a.error_flag, 123, kSpinLimit);
                 slot_wait(idx);
                 tc_fence_after();
-                if (leader) {
+                if (leader && alive) {
                     const uint32_t p_at = tmem + 128 * t, o_at = tmem + 256 + 128 * t, b = v_desc + (idx % kSlots) * (kTileBytes >> 4);
 #pragma unroll
                     for (int i = 0; i < kKeys / 16; ++i) umma_pv(o_at, p_at + 32 * (i >> 1) + 8 * (i & 1) + 16, b + i * (256 >> 4), (uint32_t)(j != 0 || i != 0));
 #pragma unroll
                     for (int i = 0; i < kKeys / 16; ++i) umma_pv(o_at, p_at + 32 * (i >> 1) + 8 * (i & 1), b + i * (256 >> 4), 1u);
-                    if (j + 1 == n[t]) umma_commit(o_full + 8 * t);
                 }
+                if (leader && j + 1 == n[t]) umma_commit(o_full + 8 * t);
             };
             // (the last copies' slots are not asked for again: an arrival there could come after the block's end)
             auto release = [&](int idx) { if (leader && idx + kSlots < total_copies) umma_commit(kv_empty + 8 * (idx % kSlots)); };
@@ -283,9 +284,9 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const Prefill
                 }
             }
             if (!alive) {
-                // let what was issued come to its end before the block can
-                if (leader) umma_commit(q_full);
-                for (uint32_t p = 0; p < 2; ++p) mbar_wait(q_full, p, nullptr, 0, 1u << 16);
+                // let what was issued come to its end before the block, and its tensor memory, can: a commit follows all products before it
+                if (leader) umma_commit(drained);
+                mbar_wait(drained, 0, nullptr, 0, kSpinLimit);
             }
         } else {
             // ---------------- K / V tiles: lane = (key of a group of eight, 16-byte piece of four) ----------------
