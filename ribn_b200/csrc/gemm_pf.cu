@@ -72,6 +72,9 @@ __device__ __forceinline__ void arrive_leader(uint32_t bar) {
 __device__ __forceinline__ void commit_both(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
 }
+__device__ __forceinline__ void commit_own(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
 // M = 256: 128 rows from each CTA, N / 2 columns from each
 constexpr uint32_t kIdescPair = (1u << 4) | ((uint32_t)(kCols >> 3) << 17) | ((uint32_t)(2 * kUnitRows >> 4) << 24);
 __device__ __forceinline__ void pair_mma_ts(bool leader, uint32_t d_tmem, uint32_t a_tmem, uint32_t b_desc, uint32_t accumulate) {
@@ -133,7 +136,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
     // b / t: a ring slot of activations, the tail of (k tile parity, group); _peer (of rank 0): the other CTA's has landed.
     // a: A stages, d: sums, m: the minima's sums; a_full, d_free and m_free are rank 0's
     const uint32_t w_full = bars, w_empty = bars + 32, b_full = bars + 64, b_peer = bars + 96, b_empty = bars + 128, t_full = bars + 160, t_peer = bars + 192,
-                   t_empty = bars + 224, a_full = bars + 256, a_free = bars + 272, d_full = bars + 288, d_free = bars + 304, m_free = bars + 320;
+                   t_empty = bars + 224, a_full = bars + 256, a_free = bars + 272, d_full = bars + 288, d_free = bars + 304, m_free = bars + 320, drained = bars + 328;
     const int k_tiles = split.k_tiles, groups = split.groups, item_groups = split.unit_items, runs = split.runs(worker);
 
     if (threadIdx.x == 0) {
@@ -147,6 +150,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
             mbar_init(d_full + 8 * i, 1); mbar_init(d_free + 8 * i, 2 * kFoldWarps);
         }
         mbar_init(m_free, 2 * kFoldWarps);
+        mbar_init(drained, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kMmaWarp) {
@@ -272,12 +276,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
                                 if (alive) alive = mbar_wait(b_peer + 8 * slot, ((pos + u) / kBSlots) & 1u, a.error_flag, 104, spin_limit);
                             }
                             tc_fence_after();
+                            const bool issue = leader && alive;   // after an expired wait no product is added to those in flight
                             const uint32_t b_desc = b_desc0 + slot * (kChunkBytes >> 4) + (q4k ? 0u : (h & 1) * 4 * kStep);
                             if (q4k) {
 #pragma unroll
-                                for (int i = 0; i < 8; ++i) pair_mma_ts(leader, d_main, a_at + 8 * i, b_desc + kLo + i * kStep, (uint32_t)(i != 0));
+                                for (int i = 0; i < 8; ++i) pair_mma_ts(issue, d_main, a_at + 8 * i, b_desc + kLo + i * kStep, (uint32_t)(i != 0));
 #pragma unroll
-                                for (int i = 0; i < 8; ++i) pair_mma_ts(leader, d_main, a_at + 8 * i, b_desc + i * kStep, 1u);
+                                for (int i = 0; i < 8; ++i) pair_mma_ts(issue, d_main, a_at + 8 * i, b_desc + i * kStep, 1u);
                                 if (h == u) {
                                     // minima x group sums: the first group's with its first sum, the second's with its last, so that
                                     // the other's have been folded by the time the stage's products are through
@@ -286,16 +291,16 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
                                     if (alive) alive = mbar_wait(t_peer + 8 * i, (t_used >> i) & 1u, a.error_flag, 107, spin_limit);
                                     take(2);
                                     tc_fence_after();
-                                    if (leader) pair_mma_ss(tmem + 256, a2_desc0 + (n & 1u) * (kA2Bytes >> 4), sum_desc0 + i * (kTailBytes >> 4));
+                                    if (leader && alive) pair_mma_ss(tmem + 256, a2_desc0 + (n & 1u) * (kA2Bytes >> 4), sum_desc0 + i * (kTailBytes >> 4));
                                 }
                             } else {
                                 // position i of the stage holds step 2 (i & 1) + (i >> 1) of its 64 inputs; p2 x lo left out as in gemm_ta.cu
 #pragma unroll
-                                for (int i = 0; i < 4; ++i) pair_mma_ts(leader, d_main, a_at + 8 * i, b_desc + kLo + (2 * (i & 1) + (i >> 1)) * kStep, (uint32_t)(!opens || i != 0));
+                                for (int i = 0; i < 4; ++i) pair_mma_ts(issue, d_main, a_at + 8 * i, b_desc + kLo + (2 * (i & 1) + (i >> 1)) * kStep, (uint32_t)(!opens || i != 0));
 #pragma unroll
-                                for (int i = 0; i < 4; ++i) pair_mma_ts(leader, d_main, a_at + 32 + 8 * i, b_desc + (2 * (i & 1) + (i >> 1)) * kStep, 1u);
+                                for (int i = 0; i < 4; ++i) pair_mma_ts(issue, d_main, a_at + 32 + 8 * i, b_desc + (2 * (i & 1) + (i >> 1)) * kStep, 1u);
 #pragma unroll
-                                for (int i = 0; i < 4; ++i) pair_mma_ts(leader, d_main, a_at + 8 * i, b_desc + (2 * (i & 1) + (i >> 1)) * kStep, 1u);
+                                for (int i = 0; i < 4; ++i) pair_mma_ts(issue, d_main, a_at + 8 * i, b_desc + (2 * (i & 1) + (i >> 1)) * kStep, 1u);
                             }
                             if (leader) {
                                 if (last) commit_both(b_empty + 8 * slot);
@@ -308,6 +313,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_pf_kernel(const StepGemm a, 
                     }
                     t_used ^= (both == 2 ? 3u : 1u) << (2 * (n & 1u));   // waited for or not
                 }
+            }
+            if (!alive) {
+                // products in flight read both CTAs' memory, which the other gives up behind the barrier below: a commit follows them all
+                if (leader) commit_own(drained);
+                mbar_wait(drained, 0, nullptr, 0, kSpinLimit);
             }
         }
     } else if (warp >= kConvertWarp0) {
