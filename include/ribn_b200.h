@@ -88,7 +88,8 @@ enum {
     RIBN_B200_FLAG_REFERENCE_KERNELS = 2, /* run the plain one-warp-per-row CUDA kernels
                                              (slow; used to cross-check the fast path) */
     RIBN_B200_FLAG_NO_GRAPH = 4,      /* launch kernels directly instead of replaying graphs */
-    RIBN_B200_FLAG_NO_TCGEN05 = 8,    /* batches of 3+ rows on the integer mma.sync kernel instead of tcgen05 */
+    RIBN_B200_FLAG_NO_TCGEN05 = 8,    /* no tcgen05 kernel: batches of 3+ rows on the integer mma.sync GEMM, prompts of 64
+                                         tokens and more on the mma.sync attention */
     RIBN_B200_FLAG_KV_ON_DEMAND = 16, /* admit reserves the prompt's KV pages only; prepare takes the pages a row's
                                          range needs and defers the rows the arena cannot serve */
     RIBN_B200_FLAG_OPERAND_CACHE = 32 /* tensor-parallel executors: finalize also keeps every Q4_K / Q6_K matrix as tcgen05

@@ -5,8 +5,8 @@
 // Launches run the tensor-core span kernel below (the GQA group's query heads
 // against 16-key slices as m16n8k16 MMAs, K / V staged in shared memory by
 // asynchronous copies), then the merge kernel; a prefill chunk of 64 tokens or
-// more runs a prefill kernel instead: heads of 128 that of attention_tc.cu,
-// others the one below for the chunk's whole groups of tokens (a key tile staged
+// more runs a prefill kernel instead: heads of 128 that of attention_tc.cu, where
+// the tcgen05 kernels are asked for, others the one below for the chunk's whole groups of tokens (a key tile staged
 // once per group, every warp walks all the keys of its own tokens, no merge).  A token's
 // result depends only on its own keys and on the launch's size class (tiles
 // per span; chunk or not), never on where its pages live.
@@ -66,6 +66,7 @@ struct AttnArgs {
     int run_first, run_count;  // host side: tokens [run_first, run_first + run_count) are consecutive tokens of one sequence; -1: unknown
     float* partial;
     int* error_flag;           // of the tensor-memory kernel's bounded waits
+    bool tensor_memory;        // host side: prefill chunks may take the tcgen05 kernel
     float* out;                // [T][q_heads][HD]
     ActOperand operand;        // optional operand form of `out`, K = q_heads * HD
     StepOperand step_operand;  // the same for a step's GEMMs (null blocks: not asked for)
@@ -626,7 +627,7 @@ __global__ void __launch_bounds__(kMmaWarps * 32, HD <= 128 && NT == 1 ? 3 : 1) 
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-// ---- prefill kernel: a run of consecutive tokens of one sequence, head widths 64 and 256 -----------------
+// ---- prefill kernel: a run of consecutive tokens of one sequence; head width 128 without the tcgen05 kernels only ----
 //
 // A CTA serves (4 x warp_tokens consecutive tokens, kv head); warp w owns warp_tokens of them (their query heads
 // are its MMA columns) and walks ALL their keys, so there are no spans to merge and the result is final.  The
@@ -980,12 +981,12 @@ cudaError_t launch_hd(cudaStream_t stream, AttnArgs a, bool fused, int n_tokens,
     const int q_per_kv = a.q_heads / a.kv_heads;
     if (q_per_kv > 16) return cudaErrorInvalidValue;  // the group is the 16 columns of two MMA tiles
     // A long run of consecutive tokens of one sequence (a prefill chunk; the caller says where it lies) takes a prefill
-    // kernel: with heads of 128 the whole run the tcgen05 kernel's, else as many whole CTA groups as it holds the kernel's
-    // above; what lies before, behind and beyond takes the spans.
+    // kernel: with heads of 128 the whole run the tcgen05 kernel's (unless the caller wants none of those), else as many whole
+    // CTA groups as it holds the kernel's above; what lies before, behind and beyond takes the spans.
     const int warp_tokens = std::max(1, 16 / q_per_kv), cta_tokens = kMmaWarps * warp_tokens;
     if (!fused && a.window <= 0 && a.operand.dig == nullptr && a.run_first >= 0 && a.run_count >= 64 &&
         a.run_first + a.run_count <= n_tokens) {
-        if constexpr (HD == 128) {
+        if (HD == 128 && a.tensor_memory) {
             PrefillAttention p{a.q, a.cache_k, a.cache_v, a.page_tables, a.pages_per_sequence, a.token_seq, a.token_pos,
                                      a.run_first, a.run_count, a.q_heads, a.kv_heads, max_keys, a.out, a.error_flag, StepOperand{}};
             // A long step that is this run alone leaves the next projection's operand itself, where a warp holds eight tokens at a
@@ -1051,7 +1052,8 @@ cudaError_t launch_attention(cudaStream_t stream, const float* q, const __half* 
                              const int32_t* page_tables, int pages_per_sequence, const int32_t* token_seq,
                              const int32_t* token_pos, int n_tokens, int q_heads, int kv_heads, int head_dim,
                              int window, int max_keys, float* partial, size_t partial_bytes, float* out,
-                             int* launches, int run_first, int run_count, int* error_flag, StepOperand step_operand, bool* operand_written) {
+                             int* launches, int run_first, int run_count, int* error_flag, StepOperand step_operand, bool* operand_written,
+                             bool tensor_memory) {
     if (operand_written) *operand_written = false;
     if (n_tokens <= 0) return cudaSuccess;
     if (q_heads % kv_heads != 0 || q_heads / kv_heads > 16 || max_keys <= 0) return cudaErrorInvalidValue;
@@ -1078,6 +1080,7 @@ cudaError_t launch_attention(cudaStream_t stream, const float* q, const __half* 
     a.out = out;
     a.run_first = run_first; a.run_count = run_count;
     a.error_flag = error_flag;
+    a.tensor_memory = tensor_memory;
     if (step_operand.blocks != nullptr && q_heads * head_dim % kTileCols == 0) a.step_operand = step_operand;
     return dispatch(stream, a, false, head_dim, n_tokens, max_keys, partial_bytes, launches, false, operand_written);
 }

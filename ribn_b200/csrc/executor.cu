@@ -248,7 +248,8 @@ cudaError_t run_layers_reference(ribn_b200_executor* ex, const StepPlan& plan, i
             cudaError_t e = launch_attention(s, ex->q, ck, cv, ex->d_page_tables, ex->pages_per_sequence,
                                              ex->meta.token_seq, ex->meta.token_pos, T, c.q_heads, c.kv_heads,
                                              c.head_dim, 0, plan.max_keys, ex->scratch.attn_partial,
-                                             ex->scratch.attn_partial_bytes, ex->attn, &launches, plan.run_first, plan.run_count, ex->d_error);
+                                             ex->scratch.attn_partial_bytes, ex->attn, &launches, plan.run_first, plan.run_count, ex->d_error,
+                                             StepOperand{}, nullptr, !(c.flags & RIBN_B200_FLAG_NO_TCGEN05));
             if (e != cudaSuccess) return e;
         }
         if (ex->tp > 1) {
@@ -407,7 +408,8 @@ cudaError_t run_attention(ribn_b200_executor* ex, const StepPlan& plan, int l, b
     }
     return launch_attention(s, ex->q, ck, cv, ex->d_page_tables, ex->pages_per_sequence, ex->meta.token_seq, ex->meta.token_pos, T, c.q_heads,
                             c.kv_heads, c.head_dim, 0, plan.max_keys, ex->scratch.attn_partial, ex->scratch.attn_partial_bytes, ex->attn,
-                            &launches, plan.run_first, plan.run_count, ex->d_error, step_operand, operand_written);
+                            &launches, plan.run_first, plan.run_count, ex->d_error, step_operand, operand_written,
+                            !(c.flags & RIBN_B200_FLAG_NO_TCGEN05));
 }
 
 cudaError_t run_layers_decode(ribn_b200_executor* ex, const StepPlan& plan, int& launches) {

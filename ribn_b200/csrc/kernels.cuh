@@ -104,8 +104,8 @@ cudaError_t launch_attention_ref(cudaStream_t stream, const float* q, const __ha
 // consecutive tokens of ONE sequence lies in the launch (a prefill chunk): from
 // 64 tokens on it takes a prefill kernel that stages each key tile once for many
 // tokens and walks all their keys, no merge (heads of 128: attention_tc.cu for the
-// whole run; else whole groups of 4 x (16 / group size) tokens).  `step_operand`,
-// `operand_written`: as in DecodeAttention.
+// whole run, unless `tensor_memory` is false; else whole groups of 4 x (16 / group
+// size) tokens).  `step_operand`, `operand_written`: as in DecodeAttention.
 constexpr int kAttnSpanKeys = 64;
 constexpr int kAttnMaxSpans = 1024;  // tiles per token: 65536 keys
 cudaError_t launch_attention(cudaStream_t stream, const float* q, const __half* cache_k, const __half* cache_v,
@@ -113,7 +113,7 @@ cudaError_t launch_attention(cudaStream_t stream, const float* q, const __half* 
                              const int32_t* token_pos, int n_tokens, int q_heads, int kv_heads, int head_dim,
                              int window, int max_keys, float* partial, size_t partial_bytes, float* out,
                              int* launches, int run_first = -1, int run_count = 0, int* error_flag = nullptr,
-                             StepOperand step_operand = StepOperand{}, bool* operand_written = nullptr);
+                             StepOperand step_operand = StepOperand{}, bool* operand_written = nullptr, bool tensor_memory = true);
 
 // Attention of `count` consecutive tokens of one sequence from token `first` on (attention_tc.cu, head width 128): q as for
 // launch_attention, tokens at consecutive positions.

@@ -407,6 +407,29 @@ def test_integer_kernels_of_a_batch_match_oracle(model):
     ex.close()
 
 
+def test_prompts_without_tcgen05_take_the_mma_sync_attention(model):
+    """FLAG_NO_TCGEN05, head width 128: the mma.sync prefill kernel takes whole groups of tokens and leaves the rest to the span
+    kernels, so that one token more than a whole group is more launches; the tcgen05 kernel takes any number in one."""
+    import ribn_b200
+    from ribn_b200 import BatchItem, StepKind
+    tensors, _ = model
+    prompt = np.random.default_rng(14).integers(0, MID["vocab"], 97).tolist()
+    assert MID["head_dim"] == 128 and 96 % (4 * 16 // (MID["q_heads"] // MID["kv_heads"])) == 0
+    more = {}
+    for flags in (0, ribn_b200.FLAG_NO_TCGEN05):
+        ex = build(MID, tensors, flags=flags, context_tokens=256, max_sequences=2, max_batch_tokens=128)
+        launches = []
+        for sequence, tokens in ((1, 96), (2, 97)):
+            assert ex.admit(sequence, sequence, prompt[:tokens], 4).ready
+            item = BatchItem(sequence, StepKind.PREFILL, 0, tokens, 1)
+            ex.prepare([item])
+            ex.wait(ex.submit([item]))
+            launches.append(ex.last_step_stats()[1])
+        more[flags] = launches[1] - launches[0]
+        ex.close()
+    assert more[0] == 0 and more[ribn_b200.FLAG_NO_TCGEN05] >= MID["layers"], more
+
+
 def test_batched_decode_graph_replay_changes_no_bit(model):
     """Batched decode steps of a recurring shape replay a captured graph from their third occurrence on; the
     logits must equal those of an executor that never captures (RIBN_B200_FLAG_NO_GRAPH), bit for bit."""
