@@ -480,6 +480,10 @@ RIBN_B200_API int ribn_b200_debug_step_deal(int32_t form, int64_t rows, int64_t 
 RIBN_B200_API int ribn_b200_debug_step_operand(int32_t device, int32_t form, const float* x, const float* up, const float* ss, int32_t members,
                                                int32_t width, void* bytes, size_t capacity, size_t* byte_count);
 
+/* The quotient of the kernels' x / den that are not divisions, from an approximate reciprocal of den (`approximate`: SwiGLU)
+ * and from 1 / den (`divided`: the attention's rows). */
+RIBN_B200_API int ribn_b200_debug_quotient(int32_t device, const float* x, const float* den, int64_t length, float* approximate, float* divided);
+
 /* Library build identification (git-free; the CUDA arch it was built for). */
 RIBN_B200_API const char* ribn_b200_build_info(void);
 

@@ -504,10 +504,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const Prefill
             }
             if (SPLIT && t == 1) live = 0;
             const float inv = 1.0f / total;
-            auto over = [&](float o) {   // o / total: the quotient's remainder folded back
-                const float q = o * inv;
-                return fmaf(fmaf(-q, total, o), inv, q);
-            };
+            auto over = [&](float o) { return quotient(o, total, inv); };
             if (!SPLIT || t == 0) {
 #pragma unroll 1
                 for (int i = 0; i < kHd; i += 32) {

@@ -17,6 +17,7 @@
 #include "blocks.cuh"
 #include "gemv.cuh"
 #include "kernels.cuh"
+#include "step_operand.cuh"
 
 using namespace ribn;
 
@@ -78,6 +79,13 @@ size_t encoded_bytes(int type, long long rows, long long cols) {
     const int e = block_elems(type);
     if (e == 0 || cols % e != 0) return 0;
     return (size_t)rows * (size_t)(cols / e) * (size_t)block_bytes(type);
+}
+
+__global__ void quotient_kernel(const float* x, const float* den, size_t n, float* approximate, float* divided) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    approximate[i] = quotient(x[i], den[i], reciprocal(den[i]));
+    divided[i] = quotient(x[i], den[i], 1.0f / den[i]);
 }
 
 }  // namespace
@@ -604,6 +612,17 @@ int ribn_b200_op_attention(int32_t device, const float* q, const uint16_t* keys,
         if (err != 0) return op_fail("attention: a bounded wait expired", cudaSuccess);
     }
     return s.download(out, d_o, (size_t)rows * q_heads * head_dim) ? RIBN_B200_OK : RIBN_B200_ERROR;
+}
+
+int ribn_b200_debug_quotient(int32_t device, const float* x, const float* den, int64_t length, float* approximate, float* divided) {
+    Scope s(device);
+    if (!s.ok || length <= 0) return op_fail("invalid argument, or no usable CUDA device", cudaGetLastError());
+    const size_t n = (size_t)length;
+    float *d_x = s.upload(x, n), *d_den = s.upload(den, n), *d_a = s.alloc<float>(n), *d_b = s.alloc<float>(n);
+    OP_PTR(d_x); OP_PTR(d_den); OP_PTR(d_a); OP_PTR(d_b);
+    quotient_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s.stream>>>(d_x, d_den, n, d_a, d_b);
+    OP_TRY(cudaGetLastError());
+    return s.download(approximate, d_a, n) && s.download(divided, d_b, n) ? RIBN_B200_OK : op_fail("quotient", cudaGetLastError());
 }
 
 int ribn_b200_debug_step_operand(int32_t device, int32_t form, const float* x, const float* up, const float* ss, int32_t members, int32_t width,

@@ -108,14 +108,11 @@ __global__ void __launch_bounds__(512, BATCH > 4 ? 1 : BATCH > 2 ? 2 : 3) step_f
     if (MODE == kFinishSwiGLU) {
         __syncthreads();
         const float inv = factors[g];
-        // silu(x) u: the quotient by 1 + e^-x from the reciprocal, its remainder folded back (e^87: the quotient is below 1e-35)
+        // silu(x) u, a quarter of x by a quarter of 1 + e^-x: the reciprocal of any finite denominator is a normal number
         auto act = [&](float x, float u) {
             x *= inv;
-            const float den = 1.0f + expf(fminf(-x, 87.0f));
-            float r;
-            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(den));
-            const float q = x * r, exact = fmaf(fmaf(-q, den, x), r, q);
-            return (fabsf(q) < INFINITY ? exact : q) * (u * inv);
+            const float den = fmaf(expf(-x), 0.25f, 0.25f);
+            return quotient(0.25f * x, den, reciprocal(den)) * (u * inv);
         };
         // rows past the last one stay zero; a block without any row has no factors either
         if (m < a.members) v = make_float4(act(gt.x, up.x), act(gt.y, up.y), act(gt.z, up.z), act(gt.w, up.w));

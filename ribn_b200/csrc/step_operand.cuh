@@ -1,6 +1,7 @@
 // The operand form of a step's GEMMs (StepOperand), written by the kernel that produces the values.
 #pragma once
 #include <cuda_fp16.h>
+#include <math.h>
 
 #include "gemv.cuh"
 
@@ -10,6 +11,20 @@ struct StepStage {
     float tops[16], squares[16];
     uint4 pieces[32][2][8];   // [8-input block][hi, lo][member ^ step % 8]: conflict-free both ways
 };
+
+// x / den from a reciprocal r of den: the remainder of x r, which a fused multiply-add gives exactly, times r is folded back
+// (P. Markstein, Computation of elementary functions on the IBM RISC System/6000 processor, IBM J. Res. Dev. 34, 1990).  With r
+// good to a unit in the last place the result is x / den but for near ties.  An infinite x or den leaves no remainder: x r.
+__device__ __forceinline__ float quotient(float x, float den, float r) {
+    const float q = x * r, rest = fmaf(-q, den, x);
+    return fabsf(rest) < INFINITY ? fmaf(rest, r, q) : q;
+}
+// 1 / x to a unit in the last place; a result below 2^-126 is zero
+__device__ __forceinline__ float reciprocal(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
 
 // 2^k, k in [-126, 127]
 __device__ __forceinline__ float power2(int k) { return __int_as_float((k + 127) << 23); }

@@ -229,3 +229,11 @@ def step_operand(form: int, x, up=None, ss=None, device: int = 0) -> np.ndarray:
     out = np.empty(need.value, dtype=np.uint8)
     _check(lib().ribn_b200_debug_step_operand(*head, _p(out), out.size, C.byref(need)), "step_operand")
     return out
+
+
+def quotient(x, den, device: int = 0):
+    """x / den as the kernels form it from an approximate and from a divided reciprocal (ribn_b200_debug_quotient)."""
+    x, den = (np.ascontiguousarray(a, dtype=np.float32) for a in (x, den))
+    out = np.empty_like(x), np.empty_like(x)
+    _check(lib().ribn_b200_debug_quotient(device, _p(x), _p(den), x.size, _p(out[0]), _p(out[1])), "quotient")
+    return out

@@ -419,3 +419,36 @@ def test_swiglu_operand_rows_past_the_last_one_are_zero(ops, form, members):
     off = np.abs(H.step_operand_values(got)[:members] - want)
     # 8 units of 2^-24 of the value (the factor: 2, twice; e^-x: 2; sums and products), 2^-23 of the tile's largest for the operand
     assert np.all(off <= 10 * 2.0 ** -24 * np.abs(want) + 2.0 ** -23 * np.abs(want).max(axis=1, keepdims=True))
+
+
+def test_quotients_from_a_reciprocal_are_divisions(ops):
+    """x / den from a reciprocal with its remainder folded back: an error of q of two units in the last place leaves, through a
+    reciprocal good to one, 2^-21 of a unit before the last rounding, so that only near ties round the other way (2^-20 of random
+    quotients), and then by one unit; infinities as division has them."""
+    rng = np.random.default_rng(5)
+    n = 1 << 20
+    x = (rng.choice([-1.0, 1.0], n) * np.exp2(rng.uniform(-60, 60, n))).astype(np.float32)
+    den = np.exp2(rng.uniform(0, 60, n)).astype(np.float32)
+    den[:4096] = 0.25 * (1 + np.exp(rng.uniform(-20, 20, 4096)))
+    want = x / den
+    for got in ops.quotient(x, den):
+        units = np.abs(got.view(np.int32).astype(np.int64) - want.view(np.int32).astype(np.int64))
+        assert units.max() <= 1 and np.count_nonzero(units) <= 16, (units.max(), np.count_nonzero(units))
+    x, den = np.array([np.inf, -np.inf, 3, -3, np.inf, 0], np.float32), np.array([2, 2, np.inf, np.inf, np.inf, 5], np.float32)
+    with np.errstate(invalid="ignore"):
+        want = x / den
+    for got in ops.quotient(x, den):
+        assert np.array_equal(got, want, equal_nan=True), got
+
+
+def test_swiglu_of_large_gates_follows_the_division(ops):
+    """silu(x) u = x u / (1 + e^-x) up to where e^-x is no longer finite, and zero beyond, however large the gate."""
+    gates = np.array([-1e30, -1e6, -700, -100, -89, -88.5, -88, -87.4, -87.2, -80, -20, 20, 80, 100, 1e6], np.float32)
+    x = np.repeat(gates, 256)[None, :]
+    up = np.full(x.shape, 1e30, np.float32)
+    got = H.step_operand_values(H.step_operand_fields(H.FRAGMENT, ops.step_operand(H.FRAGMENT, x, up), 1, x.shape[1]))[0]
+    x64 = x[0].astype(np.float64)
+    with np.errstate(over="ignore"):
+        want = np.where(x64 > -88.72, x64 / (1 + np.exp(-x64)), 0) * np.float64(up[0, 0])
+    # the exponential (2 units of 2^-24 for each unit in the last place), four roundings; the operand's 22 bits
+    assert np.all(np.abs(got - want) <= (10 * 2.0 ** -24 + 2.0 ** -22) * np.abs(want)), np.stack([gates, got[::256], want[::256]])
