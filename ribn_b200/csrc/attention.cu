@@ -64,6 +64,7 @@ struct AttnArgs {
     int tiles;                 // 64-key tiles per span (tensor-core span kernel and its merge); 1 elsewhere
     int run_tokens;            // up to this many consecutive tokens of a sequence share one item (prefill launches); 1: none
     int run_first, run_count;  // host side: tokens [run_first, run_first + run_count) are consecutive tokens of one sequence; -1: unknown
+    int run_keys;              // host side: the keys of the run's last token
     float* partial;
     int* error_flag;           // of the tensor-memory kernel's bounded waits
     bool tensor_memory;        // host side: prefill chunks may take the tcgen05 kernel
@@ -988,7 +989,7 @@ cudaError_t launch_hd(cudaStream_t stream, AttnArgs a, bool fused, int n_tokens,
         a.run_first + a.run_count <= n_tokens) {
         if (HD == 128 && a.tensor_memory) {
             PrefillAttention p{a.q, a.cache_k, a.cache_v, a.page_tables, a.pages_per_sequence, a.token_seq, a.token_pos,
-                                     a.run_first, a.run_count, a.q_heads, a.kv_heads, max_keys, a.out, a.error_flag, StepOperand{}};
+                                     a.run_first, a.run_count, a.q_heads, a.kv_heads, a.run_keys, a.out, a.error_flag, StepOperand{}};
             // A long step that is this run alone leaves the next projection's operand itself, where a warp holds eight tokens at a
             // time, so that its stores are whole lines (groups of 2 and 4 heads).  The launch that is saved grows with the tokens,
             // the kernel's longer tail does not: against F32 results, 8B model 512 tokens 0.5 % of a step slower, 640 0.7 %, 800 0.9 % and
@@ -1052,7 +1053,7 @@ cudaError_t launch_attention(cudaStream_t stream, const float* q, const __half* 
                              const int32_t* page_tables, int pages_per_sequence, const int32_t* token_seq,
                              const int32_t* token_pos, int n_tokens, int q_heads, int kv_heads, int head_dim,
                              int window, int max_keys, float* partial, size_t partial_bytes, float* out,
-                             int* launches, int run_first, int run_count, int* error_flag, StepOperand step_operand, bool* operand_written,
+                             int* launches, int run_first, int run_count, int run_keys, int* error_flag, StepOperand step_operand, bool* operand_written,
                              bool tensor_memory) {
     if (operand_written) *operand_written = false;
     if (n_tokens <= 0) return cudaSuccess;
@@ -1078,7 +1079,7 @@ cudaError_t launch_attention(cudaStream_t stream, const float* q, const __half* 
     a.window = window;
     a.partial = partial;
     a.out = out;
-    a.run_first = run_first; a.run_count = run_count;
+    a.run_first = run_first; a.run_count = run_count; a.run_keys = run_keys;
     a.error_flag = error_flag;
     a.tensor_memory = tensor_memory;
     if (step_operand.blocks != nullptr && q_heads * head_dim % kTileCols == 0) a.step_operand = step_operand;

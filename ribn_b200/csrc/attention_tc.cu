@@ -10,7 +10,8 @@
 // Q, the probabilities and the sums keep the precision of the span kernels (attention.cu).  A row's reference maximum only
 // moves when a tile's maximum passes it by 2^8 in the exponent, which binary16 pairs and F32 sums hold with the same
 // relative precision; then the row's sums are rescaled where they lie.  Key tiles begin at multiples of 128, and a row's
-// bits depend on its own keys only.
+// bits depend on its own keys and on its chunk's tokens and prefix (which choose between the two forms of the kernel), never
+// on the other rows of a step.
 //
 // What bounds it: the products, 2 x (1,024 + 1,024) clocks per 128 keys and CTA, which take about 5,200: those of Q K^T read
 // both operands from shared memory, 128 bytes per clock, beside the copies.  A tile's softmax takes 2,400 clocks beside
@@ -571,7 +572,7 @@ cudaError_t launch_attention_tc(cudaStream_t stream, const PrefillAttention& a) 
     // While every query tile can have an SM of its own, half of its key tiles per softmax group take half as long: 777 tokens of
     // the 0.6B model (7 key tiles) 37 -> 33 us a layer; with one or two key tiles there is nothing to share (65 tokens: 2 % of
     // the step slower).
-    const bool split = tiles * a.kv_heads <= sms[dev] && a.max_keys > 2 * kKeys;
+    const bool split = tiles * a.kv_heads <= sms[dev] && a.keys > 2 * kKeys;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)((split ? tiles : (tiles + 1) / 2) * a.kv_heads));
     cfg.blockDim = dim3(kThreads);

@@ -198,7 +198,7 @@ int pages_for(uint32_t tokens) { return (int)((tokens + kPageTokens - 1) / kPage
 struct StepPlan {
     int n_rows = 0, n_tokens = 0, n_sample = 0, n_prompt_tokens = 0;
     int max_keys = 0;  // longest prefix + tokens of any row
-    int run_first = -1, run_count = 0;  // the longest row's tokens: consecutive positions of one sequence (a prefill chunk)
+    int run_first = -1, run_count = 0, run_keys = 0;  // the longest row's tokens (consecutive positions of one sequence: a prefill chunk), the last one's keys
 };
 
 #define STEP_TRY(expr)                          \
@@ -248,7 +248,7 @@ cudaError_t run_layers_reference(ribn_b200_executor* ex, const StepPlan& plan, i
             cudaError_t e = launch_attention(s, ex->q, ck, cv, ex->d_page_tables, ex->pages_per_sequence,
                                              ex->meta.token_seq, ex->meta.token_pos, T, c.q_heads, c.kv_heads,
                                              c.head_dim, 0, plan.max_keys, ex->scratch.attn_partial,
-                                             ex->scratch.attn_partial_bytes, ex->attn, &launches, plan.run_first, plan.run_count, ex->d_error,
+                                             ex->scratch.attn_partial_bytes, ex->attn, &launches, plan.run_first, plan.run_count, plan.run_keys, ex->d_error,
                                              StepOperand{}, nullptr, !(c.flags & RIBN_B200_FLAG_NO_TCGEN05));
             if (e != cudaSuccess) return e;
         }
@@ -408,7 +408,7 @@ cudaError_t run_attention(ribn_b200_executor* ex, const StepPlan& plan, int l, b
     }
     return launch_attention(s, ex->q, ck, cv, ex->d_page_tables, ex->pages_per_sequence, ex->meta.token_seq, ex->meta.token_pos, T, c.q_heads,
                             c.kv_heads, c.head_dim, 0, plan.max_keys, ex->scratch.attn_partial, ex->scratch.attn_partial_bytes, ex->attn,
-                            &launches, plan.run_first, plan.run_count, ex->d_error, step_operand, operand_written,
+                            &launches, plan.run_first, plan.run_count, plan.run_keys, ex->d_error, step_operand, operand_written,
                             !(c.flags & RIBN_B200_FLAG_NO_TCGEN05));
 }
 
@@ -1477,7 +1477,7 @@ int ribn_b200_submit(ribn_b200_executor* ex, const ribn_b200_batch_item* items, 
         r.sample_row = it.output_budget > 0 ? plan.n_sample++ : -1;
         p.sample_row[i] = r.sample_row;
         r.pad[0] = r.pad[1] = r.pad[2] = 0;
-        if ((int)it.token_budget > plan.run_count) { plan.run_first = plan.n_tokens; plan.run_count = (int)it.token_budget; }
+        if ((int)it.token_budget > plan.run_count) { plan.run_first = plan.n_tokens; plan.run_count = (int)it.token_budget; plan.run_keys = (int)(it.prefix + it.token_budget); }
         plan.n_tokens += (int)it.token_budget;
         plan.max_keys = std::max(plan.max_keys, (int)(it.prefix + it.token_budget));
     }

@@ -104,7 +104,8 @@ cudaError_t launch_attention_ref(cudaStream_t stream, const float* q, const __ha
 // consecutive tokens of ONE sequence lies in the launch (a prefill chunk): from
 // 64 tokens on it takes a prefill kernel that stages each key tile once for many
 // tokens and walks all their keys, no merge (heads of 128: attention_tc.cu for the
-// whole run, unless `tensor_memory` is false; else whole groups of 4 x (16 / group
+// whole run, unless `tensor_memory` is false, in a form chosen by `run_keys`, the
+// keys of the run's last token; else whole groups of 4 x (16 / group
 // size) tokens).  `step_operand`, `operand_written`: as in DecodeAttention.
 constexpr int kAttnSpanKeys = 64;
 constexpr int kAttnMaxSpans = 1024;  // tiles per token: 65536 keys
@@ -112,7 +113,7 @@ cudaError_t launch_attention(cudaStream_t stream, const float* q, const __half* 
                              const int32_t* page_tables, int pages_per_sequence, const int32_t* token_seq,
                              const int32_t* token_pos, int n_tokens, int q_heads, int kv_heads, int head_dim,
                              int window, int max_keys, float* partial, size_t partial_bytes, float* out,
-                             int* launches, int run_first = -1, int run_count = 0, int* error_flag = nullptr,
+                             int* launches, int run_first = -1, int run_count = 0, int run_keys = 0, int* error_flag = nullptr,
                              StepOperand step_operand = StepOperand{}, bool* operand_written = nullptr, bool tensor_memory = true);
 
 // Attention of `count` consecutive tokens of one sequence from token `first` on (attention_tc.cu, head width 128): q as for
@@ -126,7 +127,7 @@ struct PrefillAttention {
     const int32_t* token_seq;   // may be null: sequence 0
     const int32_t* token_pos;
     int first, count, q_heads, kv_heads;
-    int max_keys;               // at least the keys of the last token
+    int keys;                   // of the last token
     float* out;
     int* error_flag;            // set non-zero when a bounded wait gives up
     // optional: the result in this form in place of `out` (wide form, the tokens of the launch from 0 on, groups of 2 or 4 heads)

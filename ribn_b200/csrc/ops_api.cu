@@ -606,7 +606,7 @@ int ribn_b200_op_attention(int32_t device, const float* q, const uint16_t* keys,
         OP_PTR(d_partial); OP_PTR(d_err);
         OP_TRY(cudaMemsetAsync(d_err, 0, sizeof(int), s.stream));
         OP_TRY(launch_attention(s.stream, d_q, d_k, d_v, d_table, pages, d_seq, d_pos, rows, q_heads, kv_heads,
-                                head_dim, window, tokens, d_partial, bytes, d_o, nullptr, 0, rows, d_err));
+                                head_dim, window, tokens, d_partial, bytes, d_o, nullptr, 0, rows, tokens, d_err));
         int err = 0;
         if (!s.download(&err, d_err, 1)) return op_fail("attention", cudaGetLastError());
         if (err != 0) return op_fail("attention: a bounded wait expired", cudaSuccess);

@@ -816,3 +816,28 @@ def test_prompt_attention_leaves_the_operand_of_its_consumer(built_library, toke
         logits.append(ex.copy_logits(0).copy())
         ex.close()
     assert close(logits[0], logits[1])
+
+
+def test_a_prompt_beside_decode_rows_has_the_same_bits_whatever_their_contexts(built_library):
+    """Decode rows and a prompt of 100 tokens in one step (head width 128): the prompt's cached keys and values, those behind its own
+    attention included, are the same to the bit beside short and beside long contexts."""
+    import ribn_b200
+    from ribn_b200 import BatchItem, StepKind
+    cfg = dict(layers=2, hidden=512, q_heads=8, kv_heads=2, head_dim=128, ffn=1024, vocab=1024, rope_base=1.0e6, rms_eps=1.0e-6)
+    prompt = np.random.default_rng(3).integers(0, cfg["vocab"], 100).tolist()
+    caches = []
+    for context in (16, 900):
+        ex = ribn_b200.QwenB200(cfg, flags=ribn_b200.FLAG_KEEP_LOGITS, context_tokens=1024, max_sequences=4, max_batch_tokens=128)
+        ex.init_synthetic(17, ribn_b200.SCHEME_Q4_K_M)
+        ex.finalize()
+        for s in (1, 2):
+            assert ex.admit(s, s, [1] * context, 4).ready
+            ex.debug_set_context(s, context, 5 + s, seed=70 + s)
+        assert ex.admit(3, 3, prompt, 4).ready
+        items = [BatchItem(1, StepKind.DECODE, context, 1, 1), BatchItem(3, StepKind.PREFILL, 0, len(prompt), 1), BatchItem(2, StepKind.DECODE, context, 1, 1)]
+        ex.prepare(items)
+        ex.wait(ex.submit(items))
+        caches.append([np.asarray(ex.copy_kv(3, layer, which, len(prompt))).copy() for layer in range(2) for which in range(2)])
+        ex.close()
+    for a, b in zip(*caches):
+        assert np.array_equal(a, b)
