@@ -480,6 +480,13 @@ RIBN_B200_API int ribn_b200_debug_step_deal(int32_t form, int64_t rows, int64_t 
 RIBN_B200_API int ribn_b200_debug_step_operand(int32_t device, int32_t form, const float* x, const float* up, const float* ss, int32_t members,
                                                int32_t width, void* bytes, size_t capacity, size_t* byte_count);
 
+/* ribn_b200_op_attention (head width 128, no window) of a chunk that leaves the output projection's operand in place of F32 results
+ * (640 rows and more, 2 or 4 query heads per kv head; refused otherwise): its bytes in the wide form, those of rows past the
+ * last one zero.  `bytes` may be NULL to query the size. */
+RIBN_B200_API int ribn_b200_debug_attention_operand(int32_t device, const float* q, const uint16_t* keys, const uint16_t* values,
+                                                    const int32_t* page_table, int32_t physical_tokens, int32_t tokens, int32_t rows,
+                                                    int32_t q_heads, int32_t kv_heads, void* bytes, size_t capacity, size_t* byte_count);
+
 /* The quotient of the kernels' x / den that are not divisions, from an approximate reciprocal of den (`approximate`: SwiGLU)
  * and from 1 / den (`divided`: the attention's rows). */
 RIBN_B200_API int ribn_b200_debug_quotient(int32_t device, const float* x, const float* den, int64_t length, float* approximate, float* divided);

@@ -118,6 +118,8 @@ SIGNATURES = {
     "ribn_b200_debug_step_deal": (C.c_int, [C.c_int32, C.c_int64, C.c_int64, C.c_int32, _P, C.c_size_t, C.POINTER(C.c_size_t),
                                             C.POINTER(C.c_size_t), C.POINTER(C.c_size_t)]),
     "ribn_b200_debug_step_operand": (C.c_int, [C.c_int32, C.c_int32, _P, _P, _P, C.c_int32, C.c_int32, _P, C.c_size_t, C.POINTER(C.c_size_t)]),
+    "ribn_b200_debug_attention_operand": (C.c_int, [C.c_int32, _P, _P, _P, _P, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32, _P,
+                                                    C.c_size_t, C.POINTER(C.c_size_t)]),
     "ribn_b200_debug_quotient": (C.c_int, [C.c_int32, _P, _P, C.c_int64, _P, _P]),
     "ribn_b200_debug_repack": (C.c_int, [C.c_int32, _P, C.c_int64, C.c_int64, _P, C.c_size_t,
                                          C.POINTER(C.c_size_t)]),

@@ -573,10 +573,11 @@ int ribn_b200_op_f32_to_f16(int32_t device, const float* in, int64_t length, uin
     return s.download(out, d_o, (size_t)length) ? RIBN_B200_OK : RIBN_B200_ERROR;
 }
 
-int ribn_b200_op_attention(int32_t device, const float* q, const uint16_t* keys, const uint16_t* values,
-                           const int32_t* page_table, int32_t page_tokens, int32_t physical_tokens, int32_t tokens,
-                           int32_t rows, int32_t q_heads, int32_t kv_heads, int32_t head_dim, int32_t window,
-                           float* out, int32_t variant) {
+namespace {
+// `operand` (optional): the wide operand form in place of `out`, which the kernel of long chunks writes.
+int attention_op(int32_t device, const float* q, const uint16_t* keys, const uint16_t* values, const int32_t* page_table, int32_t page_tokens,
+                 int32_t physical_tokens, int32_t tokens, int32_t rows, int32_t q_heads, int32_t kv_heads, int32_t head_dim, int32_t window,
+                 float* out, int32_t variant, unsigned char* operand) {
     Scope s(device);
     if (!s.ok || rows <= 0 || tokens < rows || page_tokens != kPageTokens || q_heads % kv_heads != 0) {
         return op_fail("invalid argument, or no usable CUDA device", cudaGetLastError());
@@ -592,6 +593,7 @@ int ribn_b200_op_attention(int32_t device, const float* q, const uint16_t* keys,
     int32_t* d_seq = s.upload(seq.data(), seq.size());
     int32_t* d_pos = s.upload(pos.data(), pos.size());
     float* d_o = s.alloc<float>((size_t)rows * q_heads * head_dim);
+    const size_t operand_bytes = operand != nullptr ? step_operand_bytes(rows, q_heads * head_dim, kWideForm) : 0;
     OP_PTR(d_q); OP_PTR(d_k); OP_PTR(d_v); OP_PTR(d_table); OP_PTR(d_seq); OP_PTR(d_pos); OP_PTR(d_o);
     if (variant == 1) {
         OP_TRY(launch_attention_ref(s.stream, d_q, d_k, d_v, d_table, pages, d_seq, d_pos, rows, q_heads, kv_heads,
@@ -603,15 +605,47 @@ int ribn_b200_op_attention(int32_t device, const float* q, const uint16_t* keys,
         const size_t bytes = std::max(per_row, std::min(per_row * (size_t)rows, (size_t)256 << 20));
         float* d_partial = s.alloc<float>(bytes / sizeof(float));
         int* d_err = s.alloc<int>(1);
+        StepOperand step{};
+        bool operand_written = false;
+        if (operand != nullptr) {
+            step.form = kWideForm;
+            step.blocks = s.alloc<unsigned char>(operand_bytes);
+            OP_PTR(step.blocks);
+            OP_TRY(cudaMemsetAsync(step.blocks, 0, operand_bytes, s.stream));
+        }
         OP_PTR(d_partial); OP_PTR(d_err);
         OP_TRY(cudaMemsetAsync(d_err, 0, sizeof(int), s.stream));
         OP_TRY(launch_attention(s.stream, d_q, d_k, d_v, d_table, pages, d_seq, d_pos, rows, q_heads, kv_heads,
-                                head_dim, window, tokens, d_partial, bytes, d_o, nullptr, 0, rows, tokens, d_err));
+                                head_dim, window, tokens, d_partial, bytes, d_o, nullptr, 0, rows, tokens, d_err, step, &operand_written));
         int err = 0;
         if (!s.download(&err, d_err, 1)) return op_fail("attention", cudaGetLastError());
         if (err != 0) return op_fail("attention: a bounded wait expired", cudaSuccess);
+        if (operand != nullptr) {
+            if (!operand_written) return op_fail("attention: chunks of this size and group leave no operand", cudaSuccess);
+            return s.download(operand, step.blocks, operand_bytes) ? RIBN_B200_OK : RIBN_B200_ERROR;
+        }
     }
     return s.download(out, d_o, (size_t)rows * q_heads * head_dim) ? RIBN_B200_OK : RIBN_B200_ERROR;
+}
+}  // namespace
+
+int ribn_b200_op_attention(int32_t device, const float* q, const uint16_t* keys, const uint16_t* values,
+                           const int32_t* page_table, int32_t page_tokens, int32_t physical_tokens, int32_t tokens,
+                           int32_t rows, int32_t q_heads, int32_t kv_heads, int32_t head_dim, int32_t window,
+                           float* out, int32_t variant) {
+    return attention_op(device, q, keys, values, page_table, page_tokens, physical_tokens, tokens, rows, q_heads, kv_heads, head_dim, window, out,
+                        variant, nullptr);
+}
+
+int ribn_b200_debug_attention_operand(int32_t device, const float* q, const uint16_t* keys, const uint16_t* values, const int32_t* page_table,
+                                      int32_t physical_tokens, int32_t tokens, int32_t rows, int32_t q_heads, int32_t kv_heads, void* bytes,
+                                      size_t capacity, size_t* byte_count) {
+    if (rows <= 0 || q_heads <= 0 || q_heads * 128 % kTileCols != 0 || byte_count == nullptr) return op_fail("attention_operand: invalid argument", cudaSuccess);
+    *byte_count = step_operand_bytes(rows, q_heads * 128, kWideForm);
+    if (bytes == nullptr) return RIBN_B200_OK;
+    if (capacity < *byte_count) return op_fail("attention_operand: invalid argument", cudaSuccess);
+    return attention_op(device, q, keys, values, page_table, kPageTokens, physical_tokens, tokens, rows, q_heads, kv_heads, 128, 0, nullptr, 0,
+                        (unsigned char*)bytes);
 }
 
 int ribn_b200_debug_quotient(int32_t device, const float* x, const float* den, int64_t length, float* approximate, float* divided) {

@@ -231,6 +231,19 @@ def step_operand(form: int, x, up=None, ss=None, device: int = 0) -> np.ndarray:
     return out
 
 
+def attention_operand(q, keys_f16, values_f16, page_table, tokens: int, rows: int, q_heads: int, kv_heads: int, device: int = 0) -> np.ndarray:
+    """The operand that the attention of a long chunk leaves, as bytes (ribn_b200_debug_attention_operand)."""
+    q = np.ascontiguousarray(q, dtype=np.float32)
+    k, v = (np.ascontiguousarray(a, dtype=np.uint16) for a in (keys_f16, values_f16))
+    table = np.ascontiguousarray(page_table, dtype=np.int32)
+    need = C.c_size_t(0)
+    head = (device, _p(q), _p(k), _p(v), _p(table), k.size // (kv_heads * 128), tokens, rows, q_heads, kv_heads)
+    _check(lib().ribn_b200_debug_attention_operand(*head, None, 0, C.byref(need)), "attention_operand size")
+    out = np.empty(need.value, dtype=np.uint8)
+    _check(lib().ribn_b200_debug_attention_operand(*head, _p(out), out.size, C.byref(need)), "attention_operand")
+    return out
+
+
 def quotient(x, den, device: int = 0):
     """x / den as the kernels form it from an approximate and from a divided reciprocal (ribn_b200_debug_quotient)."""
     x, den = (np.ascontiguousarray(a, dtype=np.float32) for a in (x, den))

@@ -793,19 +793,20 @@ def test_launches_of_one_and_of_several_block_types(built_library, tokens, kinds
     assert close(logits[0], logits[1])
 
 
-@pytest.mark.parametrize("q_heads,kv_heads", [(8, 2), (4, 2), (16, 2)])
-@pytest.mark.parametrize("tokens", [639, 640, 647, 705, 897])
+@pytest.mark.parametrize("q_heads,kv_heads,tokens", [(q, 2, n) for q in (8, 4, 16) for n in (639, 640, 647, 705, 897)] + [(32, 8, 705), (32, 8, 768), (16, 8, 1281)])
 def test_prompt_attention_leaves_the_operand_of_its_consumer(built_library, tokens, q_heads, kv_heads):
     """A long prompt alone in a step: prefill attention that writes the output projection's operand (from 640 tokens on, groups of 2
     and 4 heads; 8 take the launch that converts F32 results), for last blocks of one to eight tokens, part of a query tile and of
-    a row group, without and behind a cached prefix; against the reference-style kernels."""
+    a row group, without and behind a cached prefix, in both forms of the kernel (eight kv heads: more than 148 query tiles);
+    against the reference-style kernels, in the second layer's keys and values of every token (as in the test of q | k | v
+    above) and the logits of the last."""
     import ribn_b200
     from ribn_b200 import BatchItem, StepKind
     cfg = dict(layers=2, hidden=512, q_heads=q_heads, kv_heads=kv_heads, head_dim=128, ffn=1024, vocab=1024, rope_base=1.0e6, rms_eps=1.0e-6)
     prompt = np.random.default_rng(tokens).integers(0, cfg["vocab"], 2 * tokens).tolist()
-    logits = []
+    results = []
     for flags in (0, ribn_b200.FLAG_REFERENCE_KERNELS):
-        ex = ribn_b200.QwenB200(cfg, flags=flags | ribn_b200.FLAG_KEEP_LOGITS, context_tokens=2048, max_sequences=1, max_batch_tokens=960)
+        ex = ribn_b200.QwenB200(cfg, flags=flags | ribn_b200.FLAG_KEEP_LOGITS, context_tokens=2624, max_sequences=1, max_batch_tokens=1344)
         ex.init_synthetic(41, ribn_b200.SCHEME_Q4_K_M)
         ex.finalize()
         assert ex.admit(1, 1, prompt, 4).ready
@@ -813,9 +814,48 @@ def test_prompt_attention_leaves_the_operand_of_its_consumer(built_library, toke
             item = BatchItem(1, StepKind.PREFILL, first, tokens, 1 if first else 0)
             ex.prepare([item])
             ex.wait(ex.submit([item]))
-        logits.append(ex.copy_logits(0).copy())
+        results.append([ex.copy_logits(0).copy()] + [np.asarray(ex.copy_kv(1, 1, which, 2 * tokens)).view(np.float16).astype(np.float32).copy() for which in range(2)])
         ex.close()
-    assert close(logits[0], logits[1])
+    assert close(results[0][0], results[1][0])
+    for got, want in zip(results[0][1:], results[1][1:]):
+        assert np.all(np.abs(got - want) <= 2.0 ** -9 * np.abs(want) + 2.0 ** -11 * np.abs(want).max())
+
+
+@pytest.mark.parametrize("q_heads,kv_heads", [(8, 2), (4, 4)])
+@pytest.mark.parametrize("tokens", [64, 100, 333])
+def test_decode_rows_and_a_long_prompt_share_a_step(built_library, tokens, q_heads, kv_heads):
+    """Continuous batching at head width 128: two decode rows before a prompt's second chunk and one behind it, so that the prefill
+    attention begins in the middle of the step and the span kernels take what lies before and behind; against the reference-style
+    kernels, in the second layer's keys and values of every token of the step and the logits of every row."""
+    import ribn_b200
+    from ribn_b200 import BatchItem, StepKind
+    cfg = dict(layers=2, hidden=512, q_heads=q_heads, kv_heads=kv_heads, head_dim=128, ffn=1024, vocab=1024, rope_base=1.0e6, rms_eps=1.0e-6)
+    contexts, before = (40, 700, 129), 70
+    prompt = np.random.default_rng(tokens).integers(0, cfg["vocab"], before + tokens).tolist()
+    results = []
+    for flags in (0, ribn_b200.FLAG_REFERENCE_KERNELS):
+        ex = ribn_b200.QwenB200(cfg, flags=flags | ribn_b200.FLAG_KEEP_LOGITS, context_tokens=1024, max_sequences=4, max_batch_tokens=384)
+        ex.init_synthetic(43, ribn_b200.SCHEME_Q4_K_M)
+        ex.finalize()
+        for s, n in enumerate(contexts):
+            assert ex.admit(s + 1, s + 1, [1] * n, 4).ready
+            ex.debug_set_context(s + 1, n, 5 + s, seed=70 + s)
+        assert ex.admit(9, 9, prompt, 4).ready
+        item = BatchItem(9, StepKind.PREFILL, 0, before, 0)
+        ex.prepare([item])
+        ex.wait(ex.submit([item]))
+        rows = [BatchItem(s + 1, StepKind.DECODE, n, 1, 1) for s, n in enumerate(contexts)]
+        items = rows[:2] + [BatchItem(9, StepKind.PREFILL, before, tokens, 1)] + rows[2:]
+        ex.prepare(items)
+        ex.wait(ex.submit(items))
+        caches = [np.asarray(ex.copy_kv(s, 1, which, n)).view(np.float16).astype(np.float32).copy()
+                  for s, n in [(9, before + tokens)] + [(i + 1, n + 1) for i, n in enumerate(contexts)] for which in range(2)]
+        results.append(([ex.copy_logits(r).copy() for r in range(len(items))], caches))
+        ex.close()
+    for got, want in zip(results[0][0], results[1][0]):
+        assert close(got, want)
+    for got, want in zip(results[0][1], results[1][1]):
+        assert np.all(np.abs(got - want) <= 2.0 ** -9 * np.abs(want) + 2.0 ** -11 * np.abs(want).max())
 
 
 def test_a_prompt_beside_decode_rows_has_the_same_bits_whatever_their_contexts(built_library):

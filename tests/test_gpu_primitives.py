@@ -452,3 +452,19 @@ def test_swiglu_of_large_gates_follows_the_division(ops):
         want = np.where(x64 > -88.72, x64 / (1 + np.exp(-x64)), 0) * np.float64(up[0, 0])
     # the exponential (2 units of 2^-24 for each unit in the last place), four roundings; the operand's 22 bits
     assert np.all(np.abs(got - want) <= (10 * 2.0 ** -24 + 2.0 ** -22) * np.abs(want)), np.stack([gates, got[::256], want[::256]])
+
+
+@pytest.mark.parametrize("QH,KVH,tokens,rows", [(8, 2, 640, 640), (8, 2, 900, 647), (4, 2, 900, 705), (32, 8, 705, 705), (32, 8, 1500, 768), (16, 8, 1281, 1281)])
+def test_prompt_attention_operand_is_that_of_its_results(ops, QH, KVH, tokens, rows):
+    """The operand that the attention of a long chunk writes, bit for bit that of its F32 results as the step's kernels write it: both
+    forms of the kernel (up to 148 query tiles and more), last pairs of one and two tiles, ragged tiles, blocks of eight and groups of rows."""
+    rng = np.random.default_rng(tokens + rows)
+    q = rng.normal(0, 1, size=(rows, QH * 128)).astype(np.float32)
+    k, v = (rng.normal(0, 1, size=((tokens + 15) // 16 * 16, KVH * 128)).astype(np.float16).view(np.uint16) for _ in range(2))
+    table = np.arange((tokens + 15) // 16)
+    want = ops.step_operand(H.WIDE, ops.attention(q, k, v, table, tokens, rows, QH, KVH, 128))
+    got = ops.attention_operand(q, k, v, table, tokens, rows, QH, KVH)
+    fields = [H.step_operand_fields(H.WIDE, a, rows, QH * 128) for a in (got, want)]
+    for name in fields[0]:
+        a, b = (np.ascontiguousarray(f[name][:rows]) for f in fields)
+        assert np.array_equal(a.view(np.uint8), b.view(np.uint8)), name
