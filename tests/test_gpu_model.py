@@ -859,15 +859,15 @@ def test_decode_rows_and_a_long_prompt_share_a_step(built_library, tokens, q_hea
 
 
 def test_a_prompt_beside_decode_rows_has_the_same_bits_whatever_their_contexts(built_library):
-    """Decode rows and a prompt of 100 tokens in one step (head width 128): the prompt's cached keys and values, those behind its own
+    """Decode rows and a prompt of 200 tokens (two key tiles) in one step (head width 128): the prompt's cached keys and values, those behind its own
     attention included, are the same to the bit beside short and beside long contexts."""
     import ribn_b200
     from ribn_b200 import BatchItem, StepKind
     cfg = dict(layers=2, hidden=512, q_heads=8, kv_heads=2, head_dim=128, ffn=1024, vocab=1024, rope_base=1.0e6, rms_eps=1.0e-6)
-    prompt = np.random.default_rng(3).integers(0, cfg["vocab"], 100).tolist()
+    prompt = np.random.default_rng(3).integers(0, cfg["vocab"], 200).tolist()
     caches = []
     for context in (16, 900):
-        ex = ribn_b200.QwenB200(cfg, flags=ribn_b200.FLAG_KEEP_LOGITS, context_tokens=1024, max_sequences=4, max_batch_tokens=128)
+        ex = ribn_b200.QwenB200(cfg, flags=ribn_b200.FLAG_KEEP_LOGITS, context_tokens=1024, max_sequences=4, max_batch_tokens=256)
         ex.init_synthetic(17, ribn_b200.SCHEME_Q4_K_M)
         ex.finalize()
         for s in (1, 2):
