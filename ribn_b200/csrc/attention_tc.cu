@@ -10,7 +10,7 @@
 // Q, the probabilities and the sums keep the precision of the span kernels (attention.cu).  A row's reference maximum only
 // moves when a tile's maximum passes it by 2^8 in the exponent, which binary16 pairs and F32 sums hold with the same
 // relative precision; then the row's sums are rescaled where they lie.  Key tiles begin at multiples of 128, and a row's
-// bits depend on its own keys and on its chunk's tokens and prefix (which choose between the two forms of the kernel), never
+// bits depend on its own keys and on its chunk's tokens and prefix (which choose among the kernel's forms), never
 // on the other rows of a step.
 //
 // What bounds it: the products, 2 x (1,024 + 1,024) clocks per 128 keys and CTA, which take about 5,200: those of Q K^T read
@@ -42,6 +42,7 @@ constexpr size_t kSmem = 4 * kTileBytes + kSlots * kTileBytes + 128 + kRows * 8;
 constexpr uint32_t kSpinLimit = 1u << 22;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr size_t kWideBlock = 1028 * 128 + 32 * 128;  // one k tile of 128 rows in the wide operand form
+constexpr int kWindow = 4;                            // key tiles whose products one sum in tensor memory holds
 constexpr float kSlack = 8.0f;                        // the reference maximum may lag by 2^8
 // Register shares: 384 x 168 at launch (64,512); softmax 256 x 208, the others 128 x 88.
 constexpr int kSoftmaxRegs = 208, kOtherRegs = 88;
@@ -177,10 +178,18 @@ __device__ __forceinline__ void write_wide_operand(const StepOperand& out, uint3
     }
 }
 
-// SPLIT: one query tile per CTA, whose even key tiles are the first four softmax warps' and odd ones the others'; their two
-// results meet at the end.  For launches that would leave half of the SMs without a pair of tiles.
-template <bool SPLIT>
+// kPairs: two query tiles per CTA.  kWindows: the same for more keys than a window, whose sum in tensor memory is added to the
+// rows' sums in the softmax warps' registers at each window's end.  An addition in tensor memory cuts at the sum's last bit:
+// with one sum over all keys a result was 3.4e-5 from the exact one at 8,838 keys and 6.4e-5 at 16,384 (the mma.sync kernel:
+// 2.6e-5 and 5.0e-5), with windows of 512 keys 1.8e-6 at either.  2,048 tokens of the 8B model behind 14,336 (4 layers): 11.6 ms
+// before, 11.7 with windows; compiled for short chunks too, its longer code cost them 2 % of a step.
+// kShared (SPLIT): one query tile per CTA, whose even key tiles are the first four softmax warps' and odd ones the others'; their
+// two results meet at the end.  For launches that would leave half of the SMs without a pair of tiles.  (1.6e-5 at 8,262 keys:
+// half as many additions per sum.)
+enum Form : int { kPairs, kWindows, kShared };
+template <int FORM>
 __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const PrefillAttention a, const int tile_tokens) {
+    constexpr bool SPLIT = FORM == kShared, WINDOWS = FORM == kWindows;
     extern __shared__ __align__(128) unsigned char smem[];
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const uint32_t q_at = smem_u32(smem), ring = q_at + 4 * kTileBytes, bars = ring + kSlots * kTileBytes;
@@ -246,9 +255,9 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const Prefill
                 slot_wait(idx);
                 tc_fence_after();
                 if (leader && alive) {
-                    const uint32_t p_at = tmem + 128 * t, o_at = tmem + 256 + 128 * t, b = v_desc + (idx % kSlots) * (kTileBytes >> 4);
+                    const uint32_t goes_on = WINDOWS ? j % kWindow != 0 : j != 0, p_at = tmem + 128 * t, o_at = tmem + 256 + 128 * t, b = v_desc + (idx % kSlots) * (kTileBytes >> 4);
 #pragma unroll
-                    for (int i = 0; i < kKeys / 16; ++i) umma_pv(o_at, p_at + 32 * (i >> 1) + 8 * (i & 1) + 16, b + i * (256 >> 4), (uint32_t)(j != 0 || i != 0));
+                    for (int i = 0; i < kKeys / 16; ++i) umma_pv(o_at, p_at + 32 * (i >> 1) + 8 * (i & 1) + 16, b + i * (256 >> 4), goes_on | (uint32_t)(i != 0));
 #pragma unroll
                     for (int i = 0; i < kKeys / 16; ++i) umma_pv(o_at, p_at + 32 * (i >> 1) + 8 * (i & 1), b + i * (256 >> 4), 1u);
                 }
@@ -401,11 +410,27 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const Prefill
             const uint32_t lanes = (uint32_t)row0 << 16, s_at = tmem + lanes + 128 * t, o_at = s_at + 256;
             float m = -INFINITY;
             float2 l = make_float2(0.0f, 0.0f);
+            float sum[WINDOWS ? kHd : 1], since = 1.0f;   // earlier windows' results; the factor that has come to them since the last one's end
+#pragma unroll
+            for (int i = 0; i < (WINDOWS ? kHd : 1); ++i) sum[i] = 0.0f;
             for (int j = 0; j < n[t]; ++j) {
                 if (alive) alive = mbar_wait(s_full + 8 * t, (uint32_t)j & 1u, a.error_flag, 125, kSpinLimit);
                 tc_fence_after();
                 const int key0 = (SPLIT ? 2 * j + t : j) * kKeys, see = limit - key0;
                 const bool masked = key0 + kKeys - 1 > warp_limit;
+                const bool fresh = WINDOWS ? j % kWindow == 0 : j == 0;
+                if (WINDOWS && fresh && j > 0) {   // (the scores' barrier also says that the products into O so far are complete)
+#pragma unroll
+                    for (int i = 0; i < kHd; i += 32) {
+                        float o[32];
+                        tmem_ld32(o_at + i, o);
+                        tmem_wait_ld();
+                        tmem_tie32(o);
+#pragma unroll
+                        for (int u = 0; u < 32; ++u) sum[WINDOWS ? i + u : 0] = fmaf(sum[WINDOWS ? i + u : 0], since, o[u]);
+                    }
+                    since = 1.0f;
+                }
                 // 32 scores at a time, twice (a read of tensor memory costs less than 128 registers): the maximum, then P
                 float mx = -INFINITY;
 #pragma unroll 1
@@ -427,11 +452,11 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const Prefill
                 }
                 const bool moves = mx > m && (m == -INFINITY || (mx - m) * c > kSlack);
                 if (__any_sync(0xffffffffu, moves)) {
-                    // (the scores' barrier also says that the products into O so far are complete)
                     const float f = moves ? (m == -INFINITY ? 0.0f : exp2_approx((m - mx) * c)) : 1.0f;
                     if (moves) m = mx;
                     l.x *= f; l.y *= f;
-                    if (j > 0) {
+                    if (WINDOWS) since *= f;
+                    if (!fresh) {
 #pragma unroll 1
                         for (int i = 0; i < kHd; i += 16) {
                             float o[2][8];
@@ -507,12 +532,16 @@ __global__ void __launch_bounds__(kThreads, 1) attention_tc_kernel(const Prefill
             const float inv = 1.0f / total;
             auto over = [&](float o) { return quotient(o, total, inv); };
             if (!SPLIT || t == 0) {
-#pragma unroll 1
+#pragma unroll (WINDOWS ? kHd / 32 : 1)
                 for (int i = 0; i < kHd; i += 32) {
                     float o[32];
                     tmem_ld32(o_at + i, o);
                     tmem_wait_ld();
                     tmem_tie32(o);
+                    if (WINDOWS) {
+#pragma unroll
+                        for (int u = 0; u < 32; ++u) o[u] = fmaf(sum[WINDOWS ? i + u : 0], since, o[u]);
+                    }
                     if (SPLIT && n[1] > 0) {
 #pragma unroll
                         for (int u = 0; u < 32; u += 4) {
@@ -562,8 +591,9 @@ cudaError_t launch_attention_tc(cudaStream_t stream, const PrefillAttention& a) 
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
     if (!configured[dev]) {
-        e = cudaFuncSetAttribute(attention_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+        e = cudaFuncSetAttribute(attention_tc_kernel<kPairs>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_tc_kernel<kWindows>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_tc_kernel<kShared>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) return e;
         configured[dev] = true;
@@ -583,7 +613,8 @@ cudaError_t launch_attention_tc(cudaStream_t stream, const PrefillAttention& a) 
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return split ? cudaLaunchKernelEx(&cfg, attention_tc_kernel<true>, a, tile_tokens) : cudaLaunchKernelEx(&cfg, attention_tc_kernel<false>, a, tile_tokens);
+    return cudaLaunchKernelEx(&cfg, split ? attention_tc_kernel<kShared> : a.keys > kWindow * kKeys ? attention_tc_kernel<kWindows> : attention_tc_kernel<kPairs>,
+                              a, tile_tokens);
 }
 
 }  // namespace ribn

@@ -468,3 +468,32 @@ def test_prompt_attention_operand_is_that_of_its_results(ops, QH, KVH, tokens, r
     for name in fields[0]:
         a, b = (np.ascontiguousarray(f[name][:rows]) for f in fields)
         assert np.array_equal(a.view(np.uint8), b.view(np.uint8)), name
+
+
+@pytest.mark.parametrize("QH,KVH,tokens,rows", [(32, 8, 8262, 70), (32, 8, 8838, 646), (32, 8, 4500, 705), (16, 8, 2600, 1281), (40, 8, 1100, 700)])
+def test_prompt_attention_behind_a_long_prefix(ops, QH, KVH, tokens, rows):
+    """Chunks behind thousands of cached keys, few query tiles (key tiles shared by the softmax groups) and many (windows of 512
+    keys, added up outside the tensor core; ragged last windows; a group of five heads).  Against 64 bits, in units of sum p |v|: an addition in tensor memory
+    cuts less than a unit in the last place, 2^-23; two per 16 keys of a sum, which holds half of the keys or a window.  Scores,
+    exponentials, probabilities and F32 sums are 2^-19 together."""
+    HD, group = 128, QH // KVH
+    rng = np.random.default_rng(tokens + rows)
+    q = rng.normal(0, 1, size=(rows, QH * HD)).astype(np.float32)
+    k = rng.normal(0, 1, size=(tokens, KVH * HD)).astype(np.float16)
+    v = (rng.normal(0, 1, size=(tokens, KVH * HD)) + 0.5).astype(np.float16)   # sums that grow
+    pages = (tokens + 15) // 16
+    table = rng.permutation(pages)
+    order = table[np.arange(tokens) // 16] * 16 + np.arange(tokens) % 16
+    pk, pv = (np.full((pages * 16, KVH * HD), 0x7E00, dtype=np.uint16) for _ in range(2))
+    pk[order], pv[order] = k.view(np.uint16), v.view(np.uint16)
+    got = ops.attention(q, pk, pv, table, tokens, rows, QH, KVH, HD, variant=0)
+    shared = -(-rows // (128 // group)) * KVH <= 148
+    bound = (tokens / 2 if shared else 512) / 16 * 2 * 2.0 ** -23 + 2.0 ** -19
+    for r in (0, 1, rows // 2, rows - 1):
+        seen = tokens - rows + 1 + r
+        keys, values = (a[:seen].astype(np.float64).reshape(seen, KVH, HD).transpose(1, 0, 2) for a in (k, v))
+        s = q[r].astype(np.float64).reshape(KVH, group, HD) @ keys.transpose(0, 2, 1) / np.sqrt(HD)
+        p = np.exp(s - s.max(-1, keepdims=True))
+        p /= p.sum(-1, keepdims=True)
+        off = np.abs(got[r].reshape(KVH, group, HD) - p @ values) / (p @ np.abs(values))
+        assert off.max() <= bound, (r, off.max(), bound)
