@@ -15,9 +15,10 @@
 //
 // What bounds it: the products, 2 x (1,024 + 1,024) clocks per 128 keys and CTA, which take about 5,200: those of Q K^T read
 // both operands from shared memory, 128 bytes per clock, beside the copies.  A tile's softmax takes 2,400 clocks beside
-// the other's products.  8B model, 2,048 tokens without prefix: 90 us a layer, against 372 us of the mma.sync kernel that
-// attention.cu keeps for other head widths (0.6B model, 777 tokens: 33 against 64 us, and no spans for the last 9).  All 128
-// scores of a row in registers: 93 us; the next 32 scores requested under the present ones' arithmetic: 91 us.
+// the other's products.  8B model, 2,048 tokens without prefix: 90 us a layer as first built (108 with the windows below, cold),
+// against 372 us of the mma.sync kernel that attention.cu keeps for other head widths (0.6B model, 777 tokens: 33 against 64 us,
+// and no spans for the last 9); behind 14,336 tokens 943 against 5,338 us.  All 128 scores of a row in registers: 93 us against
+// 90; the next 32 scores requested under the present ones' arithmetic: 91 us.
 // Roles of the 12 warps: 0..3 / 4..7 softmax and output of tile 0 / 1, 8 issues the products, 9..11 copy K / V tiles (keys
 // past the chunk's last one are zero, so that a zero probability meets no NaN).  Every wait is bounded.
 #include <cuda_fp16.h>
@@ -181,8 +182,9 @@ __device__ __forceinline__ void write_wide_operand(const StepOperand& out, uint3
 // kPairs: two query tiles per CTA.  kWindows: the same for more keys than a window, whose sum in tensor memory is added to the
 // rows' sums in the softmax warps' registers at each window's end.  An addition in tensor memory cuts at the sum's last bit:
 // with one sum over all keys a result was 3.4e-5 from the exact one at 8,838 keys and 6.4e-5 at 16,384 (the mma.sync kernel:
-// 2.6e-5 and 5.0e-5), with windows of 512 keys 1.8e-6 at either.  2,048 tokens of the 8B model behind 14,336 (4 layers): 11.6 ms
-// before, 11.7 with windows; compiled for short chunks too, its longer code cost them 2 % of a step.
+// 2.6e-5 and 5.0e-5), with windows of 512 keys 1.8e-6 at either.  2,048 tokens of the 8B model (4 layers): 102 to 107 us a layer
+// without, 108 with windows (of 1,024 keys: 108), a step of 6.94 and 6.97 ms; behind 14,336 tokens 11.6 and 11.6 ms.  In short
+// chunks its longer code cost 2 % of a step: they take kPairs.
 // kShared (SPLIT): one query tile per CTA, whose even key tiles are the first four softmax warps' and odd ones the others'; their
 // two results meet at the end.  For launches that would leave half of the SMs without a pair of tiles.  (1.6e-5 at 8,262 keys:
 // half as many additions per sum.)

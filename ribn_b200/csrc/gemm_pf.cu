@@ -19,7 +19,10 @@
 // What bounds it now: the folds, 5,300 of 6,500 clocks per k tile when they read eight columns at a time (694 and 434 us); they
 // read sixteen, as many as the registers hold (32: 712 us).  A thread's arrival at the other CTA's barrier must not be
 // `.release.cluster`: its wait for all earlier accesses doubled the fold (1,060 us).  Fewer product columns for a group of
-// few rows gained nothing at 777 and 1,047 rows: its conversion and folds remain.
+// few rows gained nothing at 777 and 1,047 rows: its conversion and folds remain.  An item of one row group (65 to 128 rows) pays
+// for the pair's barriers without sharing a conversion: gate | up 59.5 and 63.6 us at 65 and 128 rows against 57.9 and 61.4 of
+// one CTA per item.  Whole steps gained all the same (8 layers of the 8B model, 65 / 80 / 100 / 128 tokens: 1.70 / 1.64 / 1.79 / 1.76
+// -> 1.59 / 1.60 / 1.64 / 1.69 ms), so the pair serves every size.
 // Roles of the 28 warps: 0..15 fold and store (one row and 32 columns of each group per thread), 16..23 convert (two row
 // tiles, half of a stage), 24 / 26 copy weights / activations, 25 issues MMAs in the leading CTA and tells it in the other
 // what has landed there.  Every wait is bounded.
