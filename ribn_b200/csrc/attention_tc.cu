@@ -103,7 +103,8 @@ __device__ __forceinline__ void sts128(uint32_t addr, uint4 v) {
 
 // The wide operand form of a warp's 32 result rows (32 / heads tokens from `token0` on), which lie in `stage` as 512 bytes each,
 // 16-byte pieces in the order of their number ^ (row % 8): the values and bits of write_step_operand (step_operand.cuh), eight
-// tokens of a pair of heads (one k tile) at a time.  A lane holds eight neighbouring inputs of each; its halves go back to where the
+// tokens of a pair of heads (one k tile) at a time.  Rows past the last token keep what they held: only their own columns of the
+// products see them, and nothing stores those.  A lane holds eight neighbouring inputs of each; its halves go back to where the
 // 16 rows lay, so that the stores are the eight tokens' 16-byte pieces side by side.
 // In place of F32 results and a launch that reads them: 2,048 tokens of the 8B model (4 layers) 7.15 -> 7.10 ms, 777 of the 0.6B
 // model 4.96 -> 4.87 ms.
